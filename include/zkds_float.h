@@ -219,7 +219,8 @@ typedef struct {
 } zkfp_gated_norm_args;
 int zkfp_gated_norm(const zkfp_gated_norm_args* a, void* stream);
 
-/* which kernel a call takes: 0 plain CUDA cores, 1 tensor cores, 2 weight streaming; for tests and reports */
+/* which kernel a call takes: 0 plain CUDA cores, 1 tensor cores, 2 weight streaming, 3 weight streaming through
+ * warp-level tensor-core products; for tests and reports */
 int zkfp_linear_path(const zkfp_linear_args* a);
 int zkfp_attention_path(const zkfp_attention_args* a);
 int zkfp_scan_path(const zkfp_scan_args* a);

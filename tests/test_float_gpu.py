@@ -102,6 +102,16 @@ def test_linear_and_its_epilogues(K, dtype, M, N, Kd):
     K.device_status(sync=True)
 
 
+@pytest.mark.parametrize("M,N,Kd", [(3, 16, 136), (8, 1000, 520), (9, 2120, 264), (16, 40, 7168), (17, 72, 1032), (32, 2120, 1544),
+                                    (32, 9000, 136)])
+def test_linear_of_few_bfloat16_rows(K, M, N, Kd):
+    """the streamed tensor-core products: edges of the tiles of eight rows and sixteen columns, ragged blocks of K, shares"""
+    a = K.LinearArgs()
+    a.M, a.N, a.K, a.dtype = M, N, Kd, K.BF16
+    assert K.linear_path(ctypes.byref(a)) == 3
+    test_linear_and_its_epilogues(K, "bfloat16", M, N, Kd)
+
+
 def test_linear_takes_the_kernel_meant_for_the_shape(K):
     def path(M, dtype):
         a = K.LinearArgs()

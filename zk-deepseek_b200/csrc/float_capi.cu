@@ -97,6 +97,7 @@ extern "C" {
 int zkfp_linear_path(const zkfp_linear_args* a)
 {
     if (a->M <= (a->dtype == ZKFP_BF16 ? kStreamRowsBf16 : kStreamRowsF32)) return 2;
+    if (a->dtype == ZKFP_BF16 && linear_skinny_takes(*a)) return 3;
     return a->dtype == ZKFP_BF16 ? 1 : 0;
 }
 
@@ -113,6 +114,7 @@ int zkfp_linear(const zkfp_linear_args* a, void* stream)
     e.bias = a->bias; e.out2 = a->out2; e.ldo2 = a->ldo2; e.split = a->out2 ? a->split : a->N;
     cudaStream_t st = (cudaStream_t)stream;
     switch (zkfp_linear_path(a)) {
+    case 3: return launch_linear_skinny(*a, e, st);
     case 2: return launch_linear_stream(*a, e, st);
     case 1: return launch_linear_tc(*a, e, st);
     default: return launch_linear_plain(*a, e, st);

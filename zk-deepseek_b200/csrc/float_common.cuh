@@ -167,6 +167,8 @@ __device__ __forceinline__ void epilogue8(const LinEpi& e, int pos, long long m,
 // ---- launchers (float_ops.cu, float_gemm.cu, float_attention.cu) -------------------------------------------
 int launch_linear_plain(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
 int launch_linear_stream(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
+bool linear_skinny_takes(const zkfp_linear_args& a);
+int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
 int launch_linear_tc(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
 int launch_attention_plain(const zkfp_attention_args& a, cudaStream_t st);
 bool attention_prefill_tc_takes(const zkfp_attention_args& a);

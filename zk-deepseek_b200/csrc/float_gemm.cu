@@ -1,5 +1,6 @@
 // Linear layers of the floating-point decoders: out = epilogue(A W^T) with 32-bit accumulation.
 //   few rows (decode)   linear_stream_kernel: every weight is read once, sixteen bytes a lane
+//   up to 32, bfloat16  linear_skinny_kernel: the same with warp-level tensor-core products
 //   many rows, bfloat16 linear_tc_kernel (float_gemm_tc.cu): tcgen05 tiles fed by TMA
 //   many rows, float32  linear_plain_kernel: true 32-bit products on the CUDA cores
 #include "float_common.cuh"
@@ -138,6 +139,107 @@ linear_stream_kernel(const T* __restrict__ A, long long lda, const T* __restrict
     }
 }
 
+// ---- few rows, bfloat16: weights streamed through warp-level tensor-core products -----------------------------------
+// out^T = W A^T in 16 x 8 x 16 products: a warp owns sixteen weight rows, the rows of A are the eight columns of a
+// product.  The order of K inside a product is free as long as both operands agree, so a lane takes eight consecutive k
+// of its row (one 16-byte load) as the fragments of two products: no shared memory and no shuffles on the way in.
+// Bound by the bytes of the weights; a warp keeps two blocks of 128 k (4 KB each) in flight.  4 rows, against the tcgen05
+// tiles that these sizes took before (split sums, a start of 18 us): 4096 x 4096 9.8 us against 23.1, 10304 x 2048 13.1
+// against 18.8, 28672 x 4096 46 (5.1 TB/s) against 68, 36864 x 7168 86 (6.1 TB/s) against 119.
+__device__ __forceinline__ uint4 stream16(const bf16* p)
+{
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                          uint32_t b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+constexpr int kSkinnyRows = 32;
+constexpr int kSkinnyK = 128;            // k of a block: four 16-byte loads a lane and weight row
+
+template <int NT>                        // tiles of eight rows of A
+__global__ void __launch_bounds__(256, NT <= 2 ? 2 : 1)
+linear_skinny_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ W, long long ldw, int M, int N, int K,
+                     int ksplit, const LinEpi e)
+{
+    __shared__ float part[8][16][NT * 8 + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int groups = 8 / ksplit, ks = warp % ksplit;
+    const int n0 = (blockIdx.x * groups + warp / ksplit) * 16;
+    float acc[NT][4] = {}, sum[NT][4] = {};
+    if (n0 < N) {
+        // rows beyond the last are read as the last one; what they give is not stored
+        const bf16 *w0 = W + (long long)min(n0 + g, N - 1) * ldw + t * 8, *w1 = W + (long long)min(n0 + g + 8, N - 1) * ldw + t * 8;
+        const bf16* a[NT];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) a[j] = A + (long long)min(j * 8 + g, M - 1) * lda + t * 8;
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        uint4 cur[2][4], nxt[2][4];
+        auto fetch = [&](uint4 (&v)[2][4], int k) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool in = k + u * 32 + t * 8 < K;
+                v[0][u] = in ? stream16(w0 + k + u * 32) : zero;
+                v[1][u] = in ? stream16(w1 + k + u * 32) : zero;
+            }
+        };
+        const int step = ksplit * kSkinnyK;
+        int k = ks * kSkinnyK;
+        if (k < K) fetch(cur, k);
+        for (int it = 0; k < K; k += step, ++it) {
+            if (k + step < K) fetch(nxt, k + step);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool in = k + u * 32 + t * 8 < K;
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const uint4 x = in ? *reinterpret_cast<const uint4*>(a[j] + k + u * 32) : zero;
+                    mma_16816(acc[j], cur[0][u].x, cur[1][u].x, cur[0][u].y, cur[1][u].y, x.x, x.y);
+                    mma_16816(acc[j], cur[0][u].z, cur[1][u].z, cur[0][u].w, cur[1][u].w, x.z, x.w);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { cur[0][u] = nxt[0][u]; cur[1][u] = nxt[1][u]; }
+            // fresh accumulators every 512 k: a product's own additions are cut off rather than rounded
+            if ((it & 3) == 3) {
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        sum[j][i] += acc[j][i];
+                        acc[j][i] = 0.f;
+                    }
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[warp][g + (i >> 1) * 8][j * 8 + t * 2 + (i & 1)] = sum[j][i] + acc[j][i];
+    __syncthreads();
+    // eight columns of one row an item, the shares of K added in a fixed order
+    for (int it = threadIdx.x; it < groups * 2 * M; it += 256) {
+        const int m = it % M, o = it / M, grp = o >> 1, n = (blockIdx.x * groups + grp) * 16 + (o & 1) * 8;
+        if (n >= N) continue;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            v[i] = 0.f;
+            for (int s = 0; s < ksplit; ++s) v[i] += part[grp * ksplit + s][(o & 1) * 8 + i][m];
+        }
+        epilogue8(e, e.kind == ZKFP_EPI_ROTATE ? epi_position(e, m) : 0, m, n, v);
+    }
+}
+
 template <typename T>
 int linear_stream(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
 {
@@ -165,6 +267,34 @@ int linear_plain(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
 }
 
 }  // namespace
+
+bool linear_skinny_takes(const zkfp_linear_args& a)
+{
+    // Up to eight rows always.  Beyond, every eight rows cost a product and a load of A per sixteen bytes of weights, and
+    // the tcgen05 tiles win once the weights are large enough to hide their start and split sums (16 rows: 7168 x 18432
+    // 60 against 65 us, 36864 x 7168 104 against 96; 32 rows: 2048 x 8192 20 against 30, 10304 x 2048 26 against 19).
+    const long long weights = a.N * a.K;
+    return a.M <= 8 || (a.M <= 16 && weights <= 140000000) || (a.M <= kSkinnyRows && weights <= 20000000);
+}
+
+int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
+{
+    // warps on the same rows until every SM has a block.  More of them leave a last wave that is nearly empty and cost
+    // more reductions (16384 x 2048, 4 rows: 2 shares 15.5 us, 4: 17.5, 8: 20.5), fewer leave SMs idle (4096 x 4096:
+    // 8 shares 10.3 us, 4: 12.8, 2: 18.4)
+    const long long tiles = (a.N + 15) / 16;
+    int ksplit = 1;
+    while (ksplit < 8 && tiles * ksplit < 8LL * fp_sm_count() && (long long)ksplit * kSkinnyK < a.K) ksplit *= 2;
+    const int groups = 8 / ksplit;
+    const unsigned grid = (unsigned)((tiles + groups - 1) / groups);
+    const bf16 *A = (const bf16*)a.A, *W = (const bf16*)a.W;
+    const int M = (int)a.M, N = (int)a.N, K = (int)a.K;
+    if (M <= 8) linear_skinny_kernel<1><<<grid, 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
+    else if (M <= 16) linear_skinny_kernel<2><<<grid, 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
+    else if (M <= kSkinnyRows) linear_skinny_kernel<4><<<grid, 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
+    else return ZKDS_ERR_UNSUPPORTED;
+    return fp_launched();
+}
 
 int launch_linear_plain(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
 {
