@@ -112,6 +112,12 @@ def test_linear_of_few_bfloat16_rows(K, M, N, Kd):
     test_linear_and_its_epilogues(K, "bfloat16", M, N, Kd)
 
 
+@pytest.mark.parametrize("M,N,Kd", [(17, 24, 8), (32, 136, 24), (33, 128, 2056), (64, 264, 8192), (65, 2120, 40), (97, 16, 4104)])
+def test_linear_of_float32_tiles(K, M, N, Kd):
+    """edges of the tiles of 32 and 64 rows and 128 columns, blocks of K, and shares of K of which some are empty"""
+    test_linear_and_its_epilogues(K, "float32", M, N, Kd)
+
+
 def test_linear_takes_the_kernel_meant_for_the_shape(K):
     def path(M, dtype):
         a = K.LinearArgs()

@@ -117,7 +117,7 @@ int zkfp_linear(const zkfp_linear_args* a, void* stream)
     case 3: return launch_linear_skinny(*a, e, st);
     case 2: return launch_linear_stream(*a, e, st);
     case 1: return launch_linear_tc(*a, e, st);
-    default: return launch_linear_plain(*a, e, st);
+    default: return launch_linear_f32(*a, e, st);
     }
 }
 

@@ -165,7 +165,7 @@ __device__ __forceinline__ void epilogue8(const LinEpi& e, int pos, long long m,
 }
 
 // ---- launchers (float_ops.cu, float_gemm.cu, float_attention.cu) -------------------------------------------
-int launch_linear_plain(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
+int launch_linear_f32(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
 int launch_linear_stream(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
 bool linear_skinny_takes(const zkfp_linear_args& a);
 int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
