@@ -659,3 +659,38 @@ def test_fused_gate_selection(M, mo, kmod, dev, E, groups, keep, topk, with_bias
     same(idx2, oi2, "tied scores: the lower index first, as the oracle's stable sort")
     check_selection(masked2, idx2.cpu().numpy())
     kmod.device_status()
+
+
+@pytest.mark.parametrize("T,k,first,E,bound", [(0, 8, 0, 16, None), (1, 8, 0, 32, None), (33, 8, 8, 16, None), (64, 8, 16, 16, 300),
+                                               (1001, 8, 0, 64, None), (4099, 2, 3, 7, None), (300, 8, 0, 512, None)])
+def test_route_kernel(M, kmod, dev, T, k, first, E, bound):
+    """rows of the routed experts: counted here pair by pair; experts outside the range, shares of a warp that end inside a
+    step of 32 pairs, tiles that stay unused"""
+    rng = np.random.default_rng(T + E)
+    total = first + E + 5
+    idx = np.stack([rng.permutation(total)[:k] for _ in range(T)]) if T else np.zeros((0, k))
+    n_tiles = ((T * k if bound is None else bound) + E * 127) // 128
+    row_src, pos, group, counts = [v.cpu().numpy() for v in kmod.moe_route(t(idx.astype(np.int64), dev), first, E, n_tiles)]
+    want_src, want_pos = np.full(n_tiles * 128, -1), np.full((T, k), -1)
+    want_group, row = np.full(n_tiles, -1), 0
+    for e in range(E):
+        where = np.argwhere(idx == first + e)
+        assert counts[e] == len(where)
+        for i, (token, slot) in enumerate(where):
+            want_src[row + i], want_pos[token, slot] = token, row + i
+        tiles = (len(where) + 127) // 128
+        want_group[row // 128:row // 128 + tiles] = e
+        row += tiles * 128
+    assert (row_src == want_src).all() and (pos == want_pos).all() and (group == want_group).all()
+
+
+@pytest.mark.parametrize("slots,cols", [(1, 2), (3, 514), (8, 7168), (9, 1030)])
+def test_combine_over_column_parts(kmod, dev, slots, cols):
+    rng = np.random.default_rng(slots)
+    out, w = rng.integers(-2**40, 2**40, (20, cols)), rng.integers(0, 2**22, (5, slots))
+    pos, base = rng.integers(-1, 20, (5, slots)).astype(np.int32), rng.integers(-2**40, 2**40, (5, cols))
+    got = kmod.moe_combine(t(out, dev), torch.from_numpy(pos).to(dev), t(w, dev), t(base, dev))
+    want = base.copy()
+    for s in range(slots):
+        want += np.where(pos[:, s:s + 1] >= 0, (out[pos[:, s]] * w[:, s:s + 1]) >> 23, 0)
+    assert (got.cpu().numpy() == want).all()

@@ -849,6 +849,17 @@ int zkds_gate_select(const int64_t* sigma, const int32_t* bias, int64_t tokens, 
     return finish(rc, "zkds_gate_select");
 }
 
+int zkds_moe_route(const int64_t* indices, int64_t tokens, int slots, int64_t first_expert, int experts, int64_t n_tiles,
+                   int* row_src, int* pos, int* tile_group, int64_t* counts, void* stream)
+{
+    int rc = (tokens < 0 || n_tiles < 0 || !counts || (tokens && (!indices || !pos)) || (n_tiles && (!row_src || !tile_group)))
+                 ? ZKDS_ERR_ARG
+                 : launch_moe_route(indices, tokens, slots, first_expert, experts, n_tiles, row_src, pos, tile_group, counts,
+                                    ST(stream));
+    if (rc == ZKDS_ERR_UNSUPPORTED) { t_status = rc; return rc; }       // silent: the caller falls back
+    return finish(rc, "zkds_moe_route");
+}
+
 int zkds_lut(int64_t* host_lut, int kind) { return finish(make_lut(host_lut, kind), "zkds_lut"); }
 
 // ---- the reference's 21 symbols ---------------------------------------------------

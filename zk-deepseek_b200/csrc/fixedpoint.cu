@@ -1249,21 +1249,30 @@ int launch_gather_rows(const int64_t* src, const int* index, int64_t* dst, int64
 
 // y[t][:] = base[t][:] + sum_slot floor(out[pos[t][slot]][:] * w[t][slot] / 2^23)   (model.py:1379-1383:
 // wrapping int64 product, floor division by 2^23, order-free integer sum); pos < 0 skips a slot
+// One block per token and 256 column pairs, four slots' rows in flight: bound by the bytes of the rows.  One token x 8 slots
+// x 7168 columns 55 -> 5 us (it was one block walking the columns, a chain of two loads per slot), 1001 tokens 99 -> 94 us.
 __global__ void __launch_bounds__(kThreads)
 moe_combine_kernel(const longlong2* __restrict__ out, const int* __restrict__ pos,
                    const int64_t* __restrict__ w, const longlong2* __restrict__ base,
                    longlong2* __restrict__ y, int slots, int64_t cols2)
 {
     const int64_t t = blockIdx.x;
-    for (int64_t c = threadIdx.x; c < cols2; c += kThreads) {
+    for (int64_t c = (int64_t)blockIdx.y * kThreads + threadIdx.x; c < cols2; c += (int64_t)gridDim.y * kThreads) {
         longlong2 acc = base ? base[t * cols2 + c] : make_longlong2(0, 0);
-        for (int s = 0; s < slots; ++s) {
-            const int r = pos[t * slots + s];
-            if (r < 0) continue;
-            const int64_t ws = w[t * slots + s];
-            const longlong2 v = out[(int64_t)r * cols2 + c];
-            acc.x = (int64_t)((uint64_t)acc.x + (uint64_t)((int64_t)((uint64_t)v.x * (uint64_t)ws) >> 23));
-            acc.y = (int64_t)((uint64_t)acc.y + (uint64_t)((int64_t)((uint64_t)v.y * (uint64_t)ws) >> 23));
+        for (int s0 = 0; s0 < slots; s0 += 4) {
+            longlong2 v[4];
+            int64_t ws[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = s0 + i < slots ? pos[t * slots + s0 + i] : -1;
+                ws[i] = r < 0 ? 0 : w[t * slots + s0 + i];
+                v[i] = r < 0 ? make_longlong2(0, 0) : out[(int64_t)r * cols2 + c];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc.x = (int64_t)((uint64_t)acc.x + (uint64_t)((int64_t)((uint64_t)v[i].x * (uint64_t)ws[i]) >> 23));
+                acc.y = (int64_t)((uint64_t)acc.y + (uint64_t)((int64_t)((uint64_t)v[i].y * (uint64_t)ws[i]) >> 23));
+            }
         }
         y[t * cols2 + c] = acc;
     }
@@ -1276,7 +1285,8 @@ int launch_moe_combine(const int64_t* out, const int* pos, const int64_t* w, con
     if ((cols & 1) || tokens > 0x7fffffffll ||
         ((((uintptr_t)out | (uintptr_t)base | (uintptr_t)y) & 15) != 0))
         return ZKDS_ERR_ARG;
-    moe_combine_kernel<<<(unsigned)tokens, kThreads, 0, st>>>(
+    const int64_t parts = (cols / 2 + kThreads - 1) / kThreads;
+    moe_combine_kernel<<<dim3((unsigned)tokens, (unsigned)(parts < 65535 ? parts : 65535)), kThreads, 0, st>>>(
         reinterpret_cast<const longlong2*>(out), pos, w, reinterpret_cast<const longlong2*>(base),
         reinterpret_cast<longlong2*>(y), slots, cols / 2);
     return check_launch();
@@ -1550,6 +1560,97 @@ int launch_gate_select(const int64_t* sig, const int32_t* bias, int64_t T, int E
     if (blocks > 0x7fffffffll) return ZKDS_ERR_RANGE;
     gate_select_kernel<<<(unsigned)blocks, 32 * kGateWarps, (size_t)kGateWarps * E * sizeof(int64_t), st>>>(
         sig, bias, T, E, n_groups, topk_groups, topk, indices, raw, w);
+    return check_launch();
+}
+
+// Places of the (token, slot) pairs in the experts' row order: rows sorted by expert, pairs of an expert in their own
+// order, every expert padded to tiles of 128 rows.  One CTA: a warp owns a consecutive share of the pairs, counts its
+// experts, and after a scan over experts and warps places its pairs 32 at a time (pairs of one expert in a warp step find
+// their order from a vote).  Bound by the latency of its few passes: 8008 pairs of 32 experts 12.5 us, 512 pairs of 64 4.9 us; a
+// sort, scans and sixty launches in all took 165 us of kernels for the 8008 pairs and 600 us of a host thread.
+namespace {
+
+constexpr int kRouteThreads = 1024, kRouteWarps = 32;
+constexpr int kRouteMaxE = 512;
+constexpr int64_t kRouteMaxPairs = 1 << 17;      // beyond, one CTA takes longer than a sort over the whole GPU
+
+__global__ void __launch_bounds__(kRouteThreads)
+moe_route_kernel(const int64_t* __restrict__ indices, int pairs, int slots, int64_t first, int E, int n_tiles,
+                 int* __restrict__ row_src, int* __restrict__ pos, int* __restrict__ tile_group, int64_t* __restrict__ counts)
+{
+    extern __shared__ int route_smem[];
+    int* place = route_smem;                             // [warp][E]: counts, then the next row of the warp's pairs
+    int* total = route_smem + kRouteWarps * E;           // [E]
+    int* begin = total + E;                              // [E + 1]: first row of the expert
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rows = n_tiles * 128;
+    for (int i = threadIdx.x; i < kRouteWarps * E; i += kRouteThreads) place[i] = 0;
+    for (int i = threadIdx.x; i < rows; i += kRouteThreads) row_src[i] = -1;
+    for (int i = threadIdx.x; i < n_tiles; i += kRouteThreads) tile_group[i] = -1;
+    __syncthreads();
+    const int share = ((pairs + kRouteWarps - 1) / kRouteWarps + 31) & ~31;
+    const int p0 = warp * share, p1 = min(pairs, p0 + share);
+    for (int p = p0 + lane; p < p1; p += 32) {
+        const int64_t e = indices[p] - first;
+        if (e >= 0 && e < E) atomicAdd(&place[warp * E + (int)e], 1);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += kRouteThreads) {
+        int n = 0;
+        for (int w = 0; w < kRouteWarps; ++w) {
+            const int c = place[w * E + e];
+            place[w * E + e] = n;
+            n += c;
+        }
+        total[e] = n;
+        counts[e] = n;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int at = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane, v = e < E ? (total[e] + 127) & ~127 : 0;
+            int sum = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += u;
+            }
+            if (e < E) begin[e] = at + sum - v;
+            at += __shfl_sync(0xffffffffu, sum, 31);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < E; i += kRouteThreads)
+        for (int t = begin[i] / 128; t < (begin[i] + total[i] + 127) / 128 && t < n_tiles; ++t) tile_group[t] = i;
+    for (int p = p0; p < p1; p += 32) {
+        const bool in = p + lane < p1;
+        const int64_t key = in ? indices[p + lane] - first : -1;
+        const int e = key >= 0 && key < E ? (int)key : E;
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        int row = -1;
+        if (e < E) row = begin[e] + place[warp * E + e] + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (e < E && lane == __ffs(same) - 1) place[warp * E + e] += __popc(same);
+        __syncwarp();
+        if (row >= rows) row = -1;                       // more pairs than the caller said there can be
+        if (row >= 0) row_src[row] = (p + lane) / slots;
+        if (in) pos[p + lane] = row;
+    }
+}
+
+}  // namespace
+
+int launch_moe_route(const int64_t* indices, int64_t tokens, int slots, int64_t first_expert, int experts, int64_t n_tiles,
+                     int* row_src, int* pos, int* tile_group, int64_t* counts, cudaStream_t st)
+{
+    if (slots < 1 || experts < 1 || experts > kRouteMaxE || tokens > kRouteMaxPairs / slots || n_tiles > (1 << 23))
+        return ZKDS_ERR_UNSUPPORTED;
+    const size_t smem = ((size_t)(kRouteWarps + 2) * experts + 1) * sizeof(int);
+    ZKDS_CUDA(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(((kRouteWarps + 2) * kRouteMaxE + 1) * sizeof(int))));
+    moe_route_kernel<<<1, kRouteThreads, smem, st>>>(indices, (int)(tokens * slots), slots, first_expert, experts, (int)n_tiles,
+                                                     row_src, pos, tile_group, counts);
     return check_launch();
 }
 

@@ -63,6 +63,8 @@ int launch_gather_rows(const int64_t* src, const int* index, int64_t* dst, int64
 // normalised weights; one warp per token.  ZKDS_ERR_UNSUPPORTED for shapes it does not take.
 int launch_gate_select(const int64_t* sig, const int32_t* bias, int64_t T, int E, int n_groups, int topk_groups,
                        int topk, int64_t* indices, int64_t* raw, int64_t* w, cudaStream_t st);
+int launch_moe_route(const int64_t* indices, int64_t tokens, int slots, int64_t first_expert, int experts, int64_t n_tiles,
+                     int* row_src, int* pos, int* tile_group, int64_t* counts, cudaStream_t st);
 int launch_moe_combine(const int64_t* out, const int* pos, const int64_t* w, const int64_t* base,
                        int64_t* y, int64_t tokens, int slots, int64_t cols, cudaStream_t st);
 // expert parallelism over peer memory (see include/zkds_int64.h)

@@ -107,6 +107,7 @@ _sig("zkds_grouped_gather_prepared", [_vp, _vp, _vp, _vp, _ll, _vp, _ll, _ll, _l
 _sig("zkds_glu_q23", [_vp, _vp, _ll, _vp, _vp, _vp, _ll, _ll, _vp])
 _sig("zkds_gather_rows", [_vp, _vp, _vp, _ll, _ll, _vp])
 _sig("zkds_moe_combine", [_vp, _vp, _vp, _vp, _vp, _ll, _i, _ll, _vp])
+_sig("zkds_moe_route", [_vp, _ll, _i, _ll, _i, _ll, _vp, _vp, _vp, _vp, _vp])
 _sig("zkds_gate_select", [_vp, _vp, _ll, _i, _i, _i, _i, _vp, _vp, _vp, _vp])
 _sig("zkds_cache_planes_append", [_vp, _vp, _vp, _vp, _ll, _ll, _ll, _ll, _ll, _ll, _i, _vp])
 _sig("zkds_mla_scores_cached", [_vp, _vp, _vp, _ll, _vp, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _i, _ll,
@@ -590,6 +591,25 @@ class CachePlanes:
             return None
         _check(rc, "softmax_pv_cached")
         return out
+
+
+def moe_route(indices, first_expert, experts, n_tiles):
+    """Rows of the routed experts in one kernel: indices int64 [T, k] -> (row_src int32 [n_tiles * 128], pos int32 [T, k],
+    tile_group int32 [n_tiles], counts int64 [experts]), as MoE.route describes them.  Returns None for shapes the
+    kernel does not take."""
+    T, k = indices.shape
+    if not indices.is_cuda or indices.dtype != torch.int64 or not indices.is_contiguous():
+        return None
+    i32 = dict(dtype=torch.int32, device=indices.device)
+    row_src, pos, group = torch.empty(n_tiles * 128, **i32), torch.empty((T, k), **i32), torch.empty(n_tiles, **i32)
+    counts = torch.empty(experts, dtype=torch.int64, device=indices.device)
+    with _on(indices.device):
+        rc = lib.zkds_moe_route(indices.data_ptr(), T, k, int(first_expert), int(experts), n_tiles, row_src.data_ptr(),
+                                pos.data_ptr(), group.data_ptr(), counts.data_ptr(), _stream())
+    if rc == 6:
+        return None
+    _check(rc, "moe_route")
+    return row_src, pos, group, counts
 
 
 def gate_select(sigma, bias, n_groups, topk_groups, topk):

@@ -815,6 +815,10 @@ class MoE(nn.Module):
         T, k = indices.shape
         E = self.n_local_experts
         dev = indices.device
+        n_tiles = ((T * k if max_pairs is None else min(T * k, max_pairs)) + E * 127) // 128
+        routed = K.moe_route(indices, self.experts_start_idx, E, n_tiles)
+        if routed is not None:
+            return routed
         flat = indices.flatten() - self.experts_start_idx
         local = (flat >= 0) & (flat < E)
         key = torch.where(local, flat, torch.full_like(flat, E))
@@ -826,7 +830,6 @@ class MoE(nn.Module):
         pad_end = torch.cumsum(padded, 0)
         pad_start = pad_end - padded
         start = torch.cumsum(counts, 0) - counts
-        n_tiles = ((T * k if max_pairs is None else min(T * k, max_pairs)) + E * 127) // 128
         R = n_tiles * 128
         ar = torch.arange(T * k, device=dev)
         valid = skey < E
