@@ -758,3 +758,11 @@ def test_converters_against_the_reference_kernels(libpath, reflib, dev):
             outs.append(o.cpu().numpy())
         ok = exf + rescale > -32
         assert np.array_equal(outs[0][ok], outs[1][ok]), "float32_to_int64_2d rescale %d" % rescale
+
+
+@pytest.mark.parametrize("M,K,N,abits,bbits,s", [(1, 1100, 8, 20, 15, 16), (16, 2064, 136, 22, 15, 16), (17, 7168, 129, 22, 30, 29),
+                                                 (33, 1500, 40, 30, 31, 30), (64, 4096, 300, 21, 15, 16), (5, 18432, 64, 16, 8, 70)])
+def test_few_rows_against_many_weights(kmod, orc, dev, M, K, N, abits, bbits, s):
+    """the weights as the MMA's rows: edges of the boxes of 16, 32 and 64 rows and of 128 columns, ragged and empty shares of
+    K, sums of one and of two words.  (Not 23 bits: three signed limbs end at 8355711, below 2^23.)"""
+    test_small_m_gemm_split_over_k(kmod, orc, dev, M, K, N, abits, bbits, s)

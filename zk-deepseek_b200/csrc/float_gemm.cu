@@ -42,7 +42,7 @@ __device__ __forceinline__ float4 peer_float4(uint32_t own, unsigned rank)
 
 __device__ __forceinline__ void cluster_barrier()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 template <int TM>                        // rows a thread: 8 (64-row tiles) or 4 (32-row tiles)

@@ -1097,6 +1097,225 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------
+// few rows against many weights (decode): the weights are the MMA's 128 rows
+// ------------------------------------------------------------------------------------
+// limb_gemm_kernel gives the MMA's M to the activations: with at most 64 rows of them it multiplies 128 all the same,
+// 12 MMAs of 128 x 256 (three limbs on two) per 32 KB of weights, which caps an SM at 40 GB/s.  Here 128 weight rows are
+// M and the R = 16, 32 or 64 activation rows of all limbs are stacked along N: 8 MMAs of 128 x 3 R for the same 32 KB, so
+// that the weight bytes are the bound.  Limb j of the weights against the stack lands on diagonals j .. j + La - 1, which
+// again are adjacent column ranges.  An accumulator lane is an output column: a warp stores 256 consecutive bytes of a row.
+// K is shared by the CTAs of a cluster: each leaves its sums in its own shared memory, then all of them add up and finish a
+// slice through distributed shared memory, so a split needs neither a workspace nor atomics.  A CTA gives its tensor memory
+// back before it waits for its cluster: what holds tensor memory never waits for another CTA, so CTAs of several launches
+// on one SM cannot block one another.
+// 64 sequences through a dense and a routed block (decoding): all its contractions of this kind 2400 -> 1949 us, the whole
+// step 4239 -> 3823 us; one sequence 1116 -> 671 us with its per-head products left out, the step 1982 -> 1835 us.
+constexpr int kRowsEpiWarps = 4, kRowsThreads = 64 + 32 * kRowsEpiWarps;
+
+__device__ __forceinline__ uint64_t peer_u64(uint32_t own, uint32_t rank)
+{
+    uint64_t v;
+    asm volatile("{\n\t.reg .b32 p;\n\tmapa.shared::cluster.u32 p, %1, %2;\n\tld.shared::cluster.u64 %0, [p];\n\t}"
+                 : "=l"(v) : "r"(own), "r"(rank) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// quotient and remainder of one element whose sum (addend included) is complete
+__device__ __forceinline__ void rows_store(const LimbParams& p, i128w sum, int shift, int64_t z, int64_t m, int64_t n)
+{
+    const int64_t at = z * p.c_sz + m * p.c_sm + n;
+    if (p.fits64) {
+        const int64_t v = (int64_t)sum.lo;
+        p.C[at] = shift >= 63 ? (v >> 63) : (v >> shift);
+        if (p.R) p.R[at] = gemm_remainder(make_i128(v), shift, p.r_legacy);
+    } else {
+        p.C[at] = sar128_lo(sum, shift);
+        if (p.R) p.R[at] = gemm_remainder(sum, shift, p.r_legacy);
+    }
+}
+
+// p.NT = R rows of activations (tmA's box); tmW's box holds 128 weight rows.  grid (n_tiles * ksplit, row tiles, batches)
+__global__ void __launch_bounds__(kRowsThreads)
+limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const LimbParams p,
+                 const uint32_t pipe_bytes)
+{
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * 8 + 2];
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int share = blockIdx.x % p.ksplit, R = p.NT;
+    const int64_t n0 = (int64_t)(blockIdx.x / p.ksplit) * kTileM, z = blockIdx.z, m0 = (int64_t)blockIdx.y * kTileM;
+    const int group = p.tile_group ? p.tile_group[blockIdx.y] : 0;
+    if (group < 0) {              // unused row tile, the same for the whole cluster: zeros, as limb_gemm_kernel leaves them
+        for (int i = share * kRowsThreads + threadIdx.x; i < kTileM * kTileM; i += p.ksplit * kRowsThreads) {
+            const int64_t r = m0 + (i >> 7), c = n0 + (i & 127);
+            if (r < p.M && c < p.N) p.C[r * p.c_sm + c] = 0;
+        }
+        return;
+    }
+    int La = p.La;
+    if (p.a_absmax) {
+        const int need = limbs_needed_dev(*p.a_absmax);
+        if (need > La) {
+            if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) *p.overflow_flag = 1u;
+        } else La = need;
+    }
+    const int D = La + p.Lb - 1;
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t w_bytes = (uint32_t)p.Lb * kTileM * kBlockK, a_limb = (uint32_t)R * kBlockK;
+    const uint32_t stage_bytes = w_bytes + (uint32_t)La * a_limb;
+    const int stages = min(8, (int)(pipe_bytes / stage_bytes));
+    const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = smem_u32(&bars[8]);
+    const uint32_t bar_zeroed = smem_u32(&bars[16]), bar_accum = smem_u32(&bars[17]);
+    const int kb_begin = share * p.kb_per_split;
+    const int kb_end = min(p.kblocks, kb_begin + p.kb_per_split);       // may be empty: such a share adds zeros
+    const bool some = kb_begin < kb_end;
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        mbar_init(bar_zeroed, kRowsEpiWarps);
+        mbar_init(bar_accum, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&s_tmem_base), p.tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem_base;
+    volatile int* abort_flag = &s_abort;
+    // the sums of a split tile: [row][128 columns], one word or (a second plane behind it) two
+    uint64_t* red = reinterpret_cast<uint64_t*>(smem_raw + (smem_base - smem_u32(smem_raw)));
+    const int rows = p.tile_group ? R : (int)p.M;
+
+    if (warp == 0) {
+        if (lane == 0 && some) {
+            const int64_t zb = p.tile_group ? group : (p.b_batched ? z : 0);
+            const int a_row = (int)(z * p.M + m0), w_row = (int)(zb * p.b_batch_rows + n0);
+            int armed = 0;
+            for (int kb = kb_begin; kb < kb_end; ++kb) {
+                const int it = kb - kb_begin, s = it % stages;
+                if (!mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag)) break;
+                const uint32_t full = bar_full + 8 * s, sw = smem_base + s * stage_bytes;
+                mbar_expect_tx(full, stage_bytes);
+                for (int j = 0; j < p.Lb; ++j)
+                    tma_load_2d(sw + j * (kTileM * kBlockK), &tmW, kb * kBlockK, (int)(j * p.b_rows_per_limb) + w_row, full);
+                for (int i = 0; i < La; ++i)
+                    tma_load_2d(sw + w_bytes + i * a_limb, &tmA, kb * kBlockK, (int)(i * p.a_rows_per_limb) + a_row, full);
+                armed = it + 1;
+            }
+            if (*abort_flag) {
+                // leave no copy in flight: wait (bounded) for every stage that was armed and that no consumer waited for
+                for (int i = (armed > stages ? armed - stages : 0); i < armed; ++i)
+                    for (uint32_t it = 0; it < kSpinLimit; ++it)
+                        if (mbar_try(bar_full + 8 * (i % stages), (i / stages) & 1)) break;
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && some) {
+            const uint32_t idesc = (2u << 4)                               // int32 accumulators
+                                   | (1u << 7) | (1u << 10)                 // signed 8-bit A and B
+                                   | ((uint32_t)((La * R) >> 3) << 17)       // N
+                                   | ((uint32_t)(kTileM >> 4) << 24);        // M
+            bool ok = mbar_wait(bar_zeroed, 0, abort_flag);
+            tc_fence_after();
+            for (int kb = kb_begin; ok && kb < kb_end; ++kb) {
+                const int it = kb - kb_begin, s = it % stages;
+                ok = mbar_wait(bar_full + 8 * s, (it / stages) & 1, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t sw = smem_base + s * stage_bytes;
+                issue_k_block_n(p.Lb, tmem, (uint32_t)R, sw, sw + w_bytes, idesc, it ? 1u : 0u, kBlockK / 32);
+                umma_commit(bar_empty + 8 * s);
+            }
+            umma_commit(bar_accum);
+        }
+    } else {
+        const int q = warp & 3, col = q * 32 + lane;             // tensor-memory lane quarter, column of the tile
+        const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
+        bool ok = true;
+        if (some) {
+            // the first MMA overwrites its La * R columns; the later limbs' last columns start at zero
+            for (int c = La * R; c < D * R; c += 8) tmem_st8_zero(tq + (uint32_t)c);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_zeroed);
+            ok = mbar_wait(bar_accum, 0, abort_flag);
+            tc_fence_after();
+        }
+        EpilogueCtx ec;
+        ec.tq = tq; ec.D = D; ec.NT = R;
+        const int64_t n = n0 + col;
+        const int shift = p.group_shift ? p.group_shift[2 * group + (n >= p.n_split ? 1 : 0)] : p.shift;
+        const int64_t addend = share == 0 ? p.addend : 0;
+        for (int r0 = 0; r0 < rows; r0 += 8) {
+            int64_t s64[8];
+            i128w sum[8];
+            if (!some) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) sum[i] = make_i128(addend);
+            } else if (!p.fits64) {
+                gather_chunk<false>(ec, r0, addend, s64, sum);
+            } else {
+                if (!gather64<8>(D, tq + (uint32_t)r0, R, addend, s64, NoHook())) gather_chunk<true>(ec, r0, addend, s64, sum);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) sum[i] = make_i128(s64[i]);
+            }
+            if (!ok) continue;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (r0 + i >= rows) continue;
+                if (p.ksplit > 1) {
+                    red[(r0 + i) * kTileM + col] = sum[i].lo;
+                    if (!p.fits64) red[(rows + r0 + i) * kTileM + col] = (uint64_t)sum[i].hi;
+                } else if (n < p.N && m0 + r0 + i < p.M)
+                    rows_store(p, sum[i], shift, z, m0 + r0 + i, n);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc(tmem, p.tmem_cols);
+    if (p.ksplit > 1) {
+        cluster_barrier();
+        for (int i = share * kRowsThreads + threadIdx.x; i < rows * kTileM; i += p.ksplit * kRowsThreads) {
+            const int64_t m = m0 + (i >> 7), n = n0 + (i & 127);
+            if (m >= p.M || n >= p.N) continue;
+            const uint32_t at = smem_u32(red + i);
+            i128w sum{0, 0};
+            for (int s = 0; s < p.ksplit; ++s) {
+                const uint64_t lo = peer_u64(at, s);
+                if (p.fits64) sum.lo += lo;
+                else sum = add128(sum, i128w{lo, (int64_t)peer_u64(at + (uint32_t)rows * kTileM * 8, s)});
+            }
+            rows_store(p, sum, p.group_shift ? p.group_shift[2 * group + (n >= p.n_split ? 1 : 0)] : p.shift, z, m, n);
+        }
+        cluster_barrier();        // a peer may still be reading this CTA's sums
+    }
+    if (p.tile_group) {           // padding rows behind the box: the result of zero rows
+        for (int i = share * kRowsThreads + threadIdx.x; i < (kTileM - R) * kTileM; i += p.ksplit * kRowsThreads) {
+            const int64_t m = m0 + R + (i >> 7), n = n0 + (i & 127);
+            if (m < p.M && n < p.N)
+                rows_store(p, make_i128(p.addend), p.group_shift ? p.group_shift[2 * group + (n >= p.n_split ? 1 : 0)] : p.shift, z, m, n);
+        }
+    }
+    if (threadIdx.x == 0 && s_abort) *p.error_flag = 1;
+}
+
+// ------------------------------------------------------------------------------------
 // persistent variant for shallow K
 // ------------------------------------------------------------------------------------
 // When K is small (attention scores, per-head projections) a tile's MMAs take a few thousand
@@ -1916,7 +2135,7 @@ static int allow_big_smem(K kernel, bool (&done)[64])
     }
     return ZKDS_OK;
 }
-static bool g_attr_onetile[64], g_attr_p16[64], g_attr_p8[64];
+static bool g_attr_onetile[64], g_attr_rows[64], g_attr_p16[64], g_attr_p8[64];
 
 static cudaEvent_t* timing_events()
 {
@@ -2068,6 +2287,36 @@ static int launch_persistent(int ew, int ctas, size_t smem, cudaStream_t st, con
     return check_launch();
 }
 
+// profiling pass: wait for the kernel, add its duration and the int8 work it issued
+static int record_launch(const Contraction& p, int La, int Lb, const unsigned long long* d_absmax, cudaEvent_t* ev, int NT)
+{
+    if (!g_accumulate) return ZKDS_OK;
+    float ms = 0.f;
+    ZKDS_CUDA(cudaEventSynchronize(ev[1]));
+    ZKDS_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+    int la_used = La;
+    if (d_absmax) {
+        unsigned long long h = 0;
+        ZKDS_CUDA(cudaMemcpy(&h, d_absmax, sizeof(h), cudaMemcpyDeviceToHost));
+        int need = limbs_needed(h);
+        if (need < la_used) la_used = need;
+    }
+    if (switches().trace)
+        fprintf(stderr, "limb_gemm batches=%lld M=%lld N=%lld K=%lld La=%d(%d) Lb=%d NT=%d tail=%d: %.3f ms\n",
+                (long long)p.batches, (long long)p.M, (long long)p.N, (long long)p.K, la_used, La, Lb, NT,
+                (p.addin || p.ep_div || p.causal_H) ? 1 : 0, ms);
+    if (g_tot_launches < 256) {
+        LaunchRecord& r = g_records[g_tot_launches];
+        r.v[0] = (double)p.batches; r.v[1] = (double)p.M; r.v[2] = (double)p.N; r.v[3] = (double)p.K;
+        r.v[4] = la_used; r.v[5] = Lb; r.v[6] = ms; r.v[7] = (p.tile_group ? 1.0 : 0.0) + (p.b_sz ? 2.0 : 0.0);
+    }
+    g_tot_ms += ms;
+    g_tot_ops += 2.0 * (double)la_used * Lb * (double)p.batches * (double)p.M * (double)p.N * (double)p.K *
+                 issued_share(p.M, p.N, p.K, NT, p.skip_tiles, p.skip_k, p.skip_H, p.skip_start);
+    g_tot_launches += 1;
+    return ZKDS_OK;
+}
+
 int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* pre_b, cudaStream_t st)
 {
     if (pre_b) Lb = pre_b->L;
@@ -2199,6 +2448,71 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         if (rc != ZKDS_OK) return rc;
     }
 
+    // few rows: the weights take the MMA's 128 rows (limb_rows_kernel).  Up to 64 rows, or promised groups of up to 64, with
+    // a plain epilogue; wherever its diagonals fit tensor memory and two stages (or the sums of a split) shared memory
+    const int few = p.tile_group ? p.group_rows : p.M <= 64 ? (int)p.M : 0;
+    if (!persistent && few > 0 && few <= 64 && !p.skip_k && !p.skip_tiles && !p.addin && !p.ep_div && !p.causal_H) {
+        const int R = few <= 16 ? 16 : few <= 32 ? 32 : 64;
+        const size_t full = (size_t)Lb * kTileM * kBlockK + (size_t)La * R * kBlockK;
+        uint32_t tcols = 32;
+        while (tcols < (uint32_t)(D * R)) tcols <<= 1;
+        const int64_t tiles = (p.N + kTileM - 1) / kTileM, all = tiles * p.batches * (p.tile_group ? mt : 1);
+        const int64_t kb = (Kp + kBlockK - 1) / kBlockK;
+        const int fits64 = sum_fits64(La, Lb, p.K, p.addend);
+        if (tcols <= 512 && La * R <= 256 && 2 * full <= smem_max && all <= 0x7fffffffll / 8 && mt <= 65535) {
+            // shares of K: the fewest K blocks that an SM works through, four more for each CTA's start and end.  Row tiles
+            // of experts are mostly unused, so their number says nothing: no split there
+            int ks = 1;
+            int64_t best = 0;
+            for (int c = 1; c <= (p.tile_group ? 1 : 8); c *= 2) {
+                if (c > 1 && (kb < 2 * c || (size_t)(fits64 ? 1 : 2) * p.M * kTileM * 8 > 2 * full)) break;
+                const int64_t cost = (all * c + sm_count() - 1) / sm_count() * ((kb + c - 1) / c + 4);
+                if (c == 1 || cost < best) { best = cost; ks = c; }
+            }
+            // two CTAs to an SM where there is more than one for it: one starts or finishes while the other streams
+            const bool pair = all * ks > sm_count() && tcols <= 256 && 2 * full + 1024 <= 112 * 1024;
+            const size_t pipe = pair ? 111 * 1024 : smem_max;
+            CUtensorMap mapA, mapW;
+            const int64_t pitch = (pre_b && pre_b->pitch) ? pre_b->pitch : Kp;
+            if (pitch < Kp || (pitch & 15)) return ZKDS_ERR_ARG;
+            if (!make_plane_map(&mapA, pa, (int64_t)La * a_rows, Kp, R) ||
+                !make_plane_map(&mapW, pb, (int64_t)Lb * b_rows, Kp, kTileM, pitch))
+                return ZKDS_ERR_UNSUPPORTED;
+            LimbParams lp{};
+            lp.La = La; lp.Lb = Lb; lp.NT = R; lp.kblocks = (int)kb;
+            lp.ksplit = ks; lp.kb_per_split = (int)((kb + ks - 1) / ks);
+            lp.tmem_cols = tcols;
+            lp.M = p.M; lp.N = p.N; lp.batches = p.batches;
+            lp.a_rows_per_limb = a_rows; lp.b_rows_per_limb = b_rows; lp.b_batch_rows = p.N;
+            lp.b_batched = p.b_sz ? 1 : 0;
+            lp.C = p.C; lp.R = p.R; lp.c_sz = p.c_sz; lp.c_sm = p.c_sm;
+            lp.addend = p.addend; lp.shift = p.shift; lp.r_legacy = p.r_legacy;
+            lp.error_flag = fl->dev; lp.fits64 = fits64;
+            lp.a_absmax = d_absmax; lp.overflow_flag = fl->overflow_dev;
+            lp.tile_group = p.tile_group; lp.group_shift = p.group_shift; lp.n_split = p.n_split;
+            rc = allow_big_smem(limb_rows_kernel, g_attr_rows);
+            if (rc != ZKDS_OK) return rc;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(tiles * ks), (unsigned)(p.tile_group ? mt : 1), (unsigned)p.batches);
+            cfg.blockDim = dim3(kRowsThreads);
+            cfg.dynamicSmemBytes = pipe + 1024;
+            cfg.stream = st;
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)ks;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            cudaEvent_t* ev = timing_events();
+            if (ev) ZKDS_CUDA(cudaEventRecord(ev[0], st));
+            rc = set_cuda_error(cudaLaunchKernelEx(&cfg, limb_rows_kernel, mapA, mapW, lp, (uint32_t)pipe));
+            if (rc == ZKDS_OK) rc = check_launch();
+            if (ev) ZKDS_CUDA(cudaEventRecord(ev[1], st));
+            if (ev && rc == ZKDS_OK) return record_launch(p, La, Lb, d_absmax, ev, R);
+            return rc;
+        }
+    }
+
     // few rows (decode, the small-M GEMM): a smaller A box, more pipeline stages
     int a_box = kTileM;
     if (!persistent && (p.tile_group ? p.group_rows != 0 : p.M <= 64)) {
@@ -2310,32 +2624,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         }
     }
     if (ev) ZKDS_CUDA(cudaEventRecord(ev[1], st));
-    if (ev && g_accumulate && rc == ZKDS_OK) {
-        // profiling pass: wait for the kernel, add its duration and the int8 work it issued
-        float ms = 0.f;
-        ZKDS_CUDA(cudaEventSynchronize(ev[1]));
-        ZKDS_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-        int la_used = La;
-        if (d_absmax) {
-            unsigned long long h = 0;
-            ZKDS_CUDA(cudaMemcpy(&h, d_absmax, sizeof(h), cudaMemcpyDeviceToHost));
-            int need = limbs_needed(h);
-            if (need < la_used) la_used = need;
-        }
-        if (switches().trace)
-            fprintf(stderr, "limb_gemm batches=%lld M=%lld N=%lld K=%lld La=%d(%d) Lb=%d NT=%d stages=%d fits64=%d tail=%d: %.3f ms\n",
-                    (long long)p.batches, (long long)p.M, (long long)p.N, (long long)p.K, la_used, La, Lb, NT,
-                    stages, lp.fits64, (p.addin || p.ep_div || p.causal_H) ? 1 : 0, ms);
-        if (g_tot_launches < 256) {
-            LaunchRecord& r = g_records[g_tot_launches];
-            r.v[0] = (double)p.batches; r.v[1] = (double)p.M; r.v[2] = (double)p.N; r.v[3] = (double)p.K;
-            r.v[4] = la_used; r.v[5] = Lb; r.v[6] = ms; r.v[7] = (p.tile_group ? 1.0 : 0.0) + (p.b_sz ? 2.0 : 0.0);
-        }
-        g_tot_ms += ms;
-        g_tot_ops += 2.0 * (double)la_used * Lb * (double)p.batches * (double)p.M * (double)p.N * (double)p.K *
-                     issued_share(p.M, p.N, p.K, NT, p.skip_tiles, p.skip_k, p.skip_H, p.skip_start);
-        g_tot_launches += 1;
-    }
+    if (ev && rc == ZKDS_OK) return record_launch(p, La, Lb, d_absmax, ev, NT);
     return rc;
 }
 
