@@ -91,6 +91,9 @@ int zkds_device_status(int clear);
                                    reports, like a limb bound that did not hold, so a caller may also promise
                                    optimistically and repeat the call without the flag when it is told so;
                                    without row_index such a row is lost silently. */
+#define ZKDS_GROUP_LEAVE_PADDING 128  /* grouped entry points: rows of C that hold no group's data (unused tiles, rows
+                                   behind the promised ones) may stay unwritten, and zkds_glu_prepared does not read
+                                   them.  For callers that only use the rows of their tokens. */
 
 /* =============================================================================
  * Group 1 — the reference's symbols (same names, same argument lists)

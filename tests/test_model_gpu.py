@@ -694,3 +694,27 @@ def test_combine_over_column_parts(kmod, dev, slots, cols):
     for s in range(slots):
         want += np.where(pos[:, s:s + 1] >= 0, (out[pos[:, s]] * w[:, s:s + 1]) >> 23, 0)
     assert (got.cpu().numpy() == want).all()
+
+
+@pytest.mark.parametrize("few", [None, 32, 64])
+def test_padding_of_expert_tiles_left_out(kmod, dev, few):
+    """with leave_padding the rows of groups are those of the full call, and what lies in the padding rows between the two
+    products (here values beyond every bound) is neither read nor replaced"""
+    rng = np.random.default_rng(5)
+    E, I, D, counts = 3, 192, 256, [20, 0, 31]
+    w13, w2 = (kmod.WeightPlanes(t(rng.integers(-2**15, 2**15, (E, n, k)).astype(np.int32), dev)) for n, k in ((2 * I, D), (D, I)))
+    src = np.full(4 * 128, -1, np.int32)
+    src[:20], src[128:159] = np.arange(20), np.arange(31)
+    group = torch.tensor([0, 2, -1, -1], dtype=torch.int32, device=dev)
+    x, rows = t(rng.integers(-2**20, 2**20, (40, D)), dev), torch.from_numpy(src).to(dev)
+    r13 = kmod.grouped_prepared(x, w13, group, 16, a_limbs=3, dynamic=True, row_index=rows, max_group_rows=few)
+    want = kmod.glu_prepared(r13[:, :I], r13[:, I:], w2, 16, ld=2 * I, a_limbs=4, tile_group=group, max_group_rows=few)
+    got13 = kmod.grouped_prepared(x, w13, group, 16, a_limbs=3, dynamic=True, row_index=rows, max_group_rows=few, leave_padding=True)
+    used = torch.from_numpy(src >= 0).to(dev)
+    assert torch.equal(got13[used], r13[used])
+    r13[256:] = 2**62
+    if few:
+        r13[few:128], r13[128 + few:256] = 2**62, 2**62
+    got = kmod.glu_prepared(r13[:, :I], r13[:, I:], w2, 16, ld=2 * I, a_limbs=4, tile_group=group, max_group_rows=few, leave_padding=True)
+    assert torch.equal(got[used], want[used])
+    kmod.device_status()

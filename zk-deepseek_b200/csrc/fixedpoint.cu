@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(kThreads)
 glu_planes_kernel(const int64_t* __restrict__ r1, const int64_t* __restrict__ r2, int64_t ld,
                   const int64_t* __restrict__ lut_g, int8_t* __restrict__ planes, int L, int64_t rows, int64_t n,
                   int64_t Kp, int64_t plane_stride, unsigned* overflow, unsigned long long* absmax_out,
-                  int tpr_log2)
+                  int tpr_log2, const int* __restrict__ tile_group, int box)
 {
     __shared__ int64_t lut[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = lut_g[i];
@@ -1114,6 +1114,7 @@ glu_planes_kernel(const int64_t* __restrict__ r1, const int64_t* __restrict__ r2
     const int64_t rpb = kThreads >> tpr_log2;
     for (int64_t r = (int64_t)blockIdx.x * rpb + (threadIdx.x >> tpr_log2); r < rows;
          r += (int64_t)gridDim.x * rpb) {
+        if (tile_group && ((int)(r & 127) >= box || tile_group[r >> 7] < 0)) continue;
         const int64_t* a = r1 + r * ld;
         const int64_t* b = r2 + r * ld;
         int8_t* drow = planes + r * Kp;
@@ -1196,7 +1197,7 @@ bool glu_planes_supported(const int64_t* r1, const int64_t* r2, int64_t ld, int6
 
 int launch_glu_planes(const int64_t* r1, const int64_t* r2, int64_t ld, const int64_t* lut, int8_t* planes, int L,
                       int64_t rows, int64_t n, int64_t Kp, int64_t plane_stride, unsigned* overflow,
-                      unsigned long long* absmax_out, cudaStream_t st)
+                      unsigned long long* absmax_out, const int* tile_group, int box, cudaStream_t st)
 {
     if (rows == 0) return ZKDS_OK;
     if (!glu_planes_supported(r1, r2, ld, n) || L < 1 || L > 9 || (Kp & 3) || Kp < n) return ZKDS_ERR_UNSUPPORTED;
@@ -1208,7 +1209,7 @@ int launch_glu_planes(const int64_t* r1, const int64_t* r2, int64_t ld, const in
     if (grid > cap) grid = cap;
 #define ZKDS_GP(LL)                                                                                         \
     glu_planes_kernel<LL><<<(unsigned)grid, kThreads, 0, st>>>(r1, r2, ld, lut, planes, L, rows, n, Kp,     \
-                                                               plane_stride, overflow, absmax_out, tl)
+                                                               plane_stride, overflow, absmax_out, tl, tile_group, box)
     switch (L) {
     case 2: ZKDS_GP(2); break;
     case 3: ZKDS_GP(3); break;

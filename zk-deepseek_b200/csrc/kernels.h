@@ -54,9 +54,10 @@ int launch_glu(const int64_t* r1, const int64_t* r2, int64_t ld, int64_t* h, int
                const int64_t* lut, int64_t rows, int64_t n, cudaStream_t st);
 // (silu_q23(r1) * r2) >> 23 written as limb planes (see launch_softmax_planes for the layout)
 bool glu_planes_supported(const int64_t* r1, const int64_t* r2, int64_t ld, int64_t n);
+// tile_group, box: rows of 128-row tiles with a negative entry, and rows from `box` on of the others, are left out (null: none)
 int launch_glu_planes(const int64_t* r1, const int64_t* r2, int64_t ld, const int64_t* lut, int8_t* planes, int L,
                       int64_t rows, int64_t n, int64_t Kp, int64_t plane_stride, unsigned* overflow,
-                      unsigned long long* absmax_out, cudaStream_t st);
+                      unsigned long long* absmax_out, const int* tile_group, int box, cudaStream_t st);
 int launch_gather_rows(const int64_t* src, const int* index, int64_t* dst, int64_t rows, int64_t cols,
                        cudaStream_t st);
 // Gate.forward after the sigmoid (model.py:1140-1211): bias, grouped top-k selection, gathered and
@@ -113,6 +114,7 @@ struct Contraction {
     // hold data (no group has more rows than that); the kernel then loads only those rows of A and the other
     // rows of a tile come out as zero rows would
     int group_rows;
+    int leave_padding;        // grouped mode: rows of C that hold no group's data may stay as they are
     // limb kernel only: row m of A is source row a_row_index[m] (negative: a row of zeros), so a row
     // gather needs no pass of its own
     const int* a_row_index;

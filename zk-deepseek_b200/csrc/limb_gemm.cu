@@ -405,6 +405,7 @@ struct LimbParams {
     // n_split on (n_split a multiple of 8); null = the uniform shift above
     const int* group_shift;
     int64_t n_split;
+    int leave_padding;        // grouped mode: unused tiles, and rows behind the box of the others, are not stored
     // epilogue extension: v = quotient; v += addin[m][n]; v = floor(v * ep_mul / ep_div);
     // rows are (s, h) pairs with causal_H heads: v += mask_value where n > causal_start + s
     const int64_t* addin;
@@ -850,6 +851,7 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (group < 0) {
             // unused row tile (uniform for the CTA, before any barrier or allocation): its output
             // rows are defined as zero so that later passes over the whole buffer see clean data
+            if (p.leave_padding) return;
             const int64_t r0 = (int64_t)blockIdx.x * kTileM, c0 = (int64_t)blockIdx.y * p.NT;
             for (int i = threadIdx.x; i < kTileM * p.NT; i += kThreads) {
                 const int64_t r = r0 + i / p.NT, c = c0 + i % p.NT;
@@ -1015,8 +1017,8 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             ec.nc_begin = 8 * per * part < p.NT ? 8 * per * part : p.NT;
             ec.nc_end = 8 * per * (part + 1) < p.NT ? 8 * per * (part + 1) : p.NT;
         }
-        ec.crow = crow; ec.rrow = rrow; ec.row_ok = row_ok; ec.vec_ok = vec_ok;
-        if (beyond_box && ok) {
+        ec.crow = crow; ec.rrow = rrow; ec.row_ok = row_ok && !(beyond_box && p.leave_padding); ec.vec_ok = vec_ok;
+        if (beyond_box && ok && !p.leave_padding) {
             // padding rows of a grouped tile whose A box stops short of them: the MMAs summed whatever follows
             // the box in shared memory into these lanes.  Every warp clears the columns it is about to read.
             for (int d = 0; d < D; ++d)
@@ -1154,6 +1156,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int64_t n0 = (int64_t)(blockIdx.x / p.ksplit) * kTileM, z = blockIdx.z, m0 = (int64_t)blockIdx.y * kTileM;
     const int group = p.tile_group ? p.tile_group[blockIdx.y] : 0;
     if (group < 0) {              // unused row tile, the same for the whole cluster: zeros, as limb_gemm_kernel leaves them
+        if (p.leave_padding) return;
         for (int i = share * kRowsThreads + threadIdx.x; i < kTileM * kTileM; i += p.ksplit * kRowsThreads) {
             const int64_t r = m0 + (i >> 7), c = n0 + (i & 127);
             if (r < p.M && c < p.N) p.C[r * p.c_sm + c] = 0;
@@ -1305,7 +1308,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         cluster_barrier();        // a peer may still be reading this CTA's sums
     }
-    if (p.tile_group) {           // padding rows behind the box: the result of zero rows
+    if (p.tile_group && !p.leave_padding) {           // padding rows behind the box: the result of zero rows
         for (int i = share * kRowsThreads + threadIdx.x; i < (kTileM - R) * kTileM; i += p.ksplit * kRowsThreads) {
             const int64_t m = m0 + R + (i >> 7), n = n0 + (i & 127);
             if (m < p.M && n < p.N)
@@ -2424,7 +2427,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     } else if (p.glu_lut) {
         if (p.batches != 1 || p.a_div != 1 || p.a_row_index || !p.glu_r2) return ZKDS_ERR_ARG;
         rc = launch_glu_planes(p.A, p.glu_r2, p.a_sm, p.glu_lut, pa, La, a_rows, p.K, Kp, a_rows * Kp,
-                               fl->overflow_dev, d_absmax, st);
+                               fl->overflow_dev, d_absmax, p.leave_padding ? p.tile_group : nullptr,
+                               p.group_rows ? p.group_rows : kTileM, st);
     } else {
         RowParts parts{};
         if (p.a_n_parts > 0) {
@@ -2490,6 +2494,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
             lp.error_flag = fl->dev; lp.fits64 = fits64;
             lp.a_absmax = d_absmax; lp.overflow_flag = fl->overflow_dev;
             lp.tile_group = p.tile_group; lp.group_shift = p.group_shift; lp.n_split = p.n_split;
+            lp.leave_padding = p.tile_group ? p.leave_padding : 0;
             rc = allow_big_smem(limb_rows_kernel, g_attr_rows);
             if (rc != ZKDS_OK) return rc;
             cudaLaunchConfig_t cfg = {};
@@ -2554,6 +2559,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     lp.skip_tiles = p.skip_tiles; lp.skip_k = p.skip_k; lp.skip_H = p.skip_H; lp.skip_start = p.skip_start;
     lp.tile_group = p.tile_group;
     lp.group_shift = p.group_shift; lp.n_split = p.n_split;
+    lp.leave_padding = p.tile_group ? p.leave_padding : 0;
     lp.addin = p.addin; lp.ep_mul = p.ep_mul; lp.ep_div = p.ep_div;
     lp.causal_H = p.causal_H; lp.causal_start = p.causal_start; lp.mask_value = p.mask_value;
 

@@ -34,7 +34,7 @@ ALGO_AUTO, ALGO_EXACT, ALGO_LIMB = 0, 1, 2
 REMAINDER_LEGACY = 4
 LIMBS_DYNAMIC = 8
 CAUSAL_SKIP = 16
-GROUP_ROWS_32, GROUP_ROWS_64 = 32, 64
+GROUP_ROWS_32, GROUP_ROWS_64, GROUP_LEAVE_PADDING = 32, 64, 128
 
 # Remainder flavour of int64_bmm_broadcast.  True reproduces the reference binary:
 # exact for c_rescale <= 31, the low 32 bits of the sum above that
@@ -407,7 +407,7 @@ def _group_rows_flag(max_rows):
 
 
 def grouped_prepared(A, planes, tile_group, c_rescale, a_limbs=0, dynamic=False, group_shift=None,
-                     n_split=0, row_index=None, max_group_rows=None):
+                     n_split=0, row_index=None, max_group_rows=None, leave_padding=False):
     """Routed-expert linear layer: A flat (n_tiles*128, K), tile_group int32 (n_tiles,) on the
     device (expert of each 128-row tile, negative = unused) -> C (n_tiles*128, N).
     group_shift: optional int32 (experts, 2) device tensor of per-expert shifts for the output
@@ -417,8 +417,9 @@ def grouped_prepared(A, planes, tile_group, c_rescale, a_limbs=0, dynamic=False,
     index_select of model.py:1372-1378 happens inside the limb split (a_limbs must be given).
     max_group_rows: a bound on the rows of every group that the caller can prove (decode: a token names an
     expert at most once, so no expert has more rows than there are tokens); up to 64 the kernel then fetches
-    only the first 32 / 64 rows of every tile."""
-    gflag = _group_rows_flag(max_group_rows)
+    only the first 32 / 64 rows of every tile.
+    leave_padding: rows of C that hold no group's data (unused tiles, rows behind the bound) may stay undefined."""
+    gflag = _group_rows_flag(max_group_rows) | (GROUP_LEAVE_PADDING if leave_padding else 0)
     if group_shift is not None:
         assert group_shift.dtype == torch.int32 and group_shift.is_cuda and group_shift.is_contiguous()
     _dev_i64(A, "A")
@@ -445,11 +446,12 @@ def grouped_prepared(A, planes, tile_group, c_rescale, a_limbs=0, dynamic=False,
 
 
 def glu_prepared(r1, r2, planes, c_rescale, ld=None, a_limbs=3, dynamic=True, tile_group=None,
-                 group_shift=None, n_split=0, max_group_rows=None):
+                 group_shift=None, n_split=0, max_group_rows=None, leave_padding=False):
     """w2 of a gated MLP with the gate inside its limb split: C = (h @ W2^T) >> c_rescale with
     h = (silu_q23(r1) * r2) >> 23 (model.py:1034-1049, 1271-1281); h only ever exists as int8 limb
     planes.  r1, r2: (rows, K) views sharing the row stride ld (default K); planes: prepared W2, or
     the experts' stacked W2 together with tile_group (and group_shift) as in grouped_prepared.
+    leave_padding (with tile_group): as in grouped_prepared, and such rows of r1 and r2 are not read.
     Returns None when the kernel does not take the shape (use glu_q23 and the linear layer then)."""
     for t_, name in ((r1, "r1"), (r2, "r2")):     # strided row views of one buffer are the normal case
         assert t_.dtype == torch.int64 and t_.is_cuda and t_.dim() == 2 and t_.stride(1) == 1, name
@@ -469,7 +471,8 @@ def glu_prepared(r1, r2, planes, c_rescale, ld=None, a_limbs=3, dynamic=True, ti
                                    tile_group.data_ptr() if tile_group is not None else None, C.data_ptr(),
                                    int(c_rescale), group_shift.data_ptr() if group_shift is not None else None,
                                    int(n_split), a_limbs,
-                                   _a_flags(a_limbs, dynamic) | (_group_rows_flag(max_group_rows) if tile_group is not None else 0),
+                                   _a_flags(a_limbs, dynamic) | ((_group_rows_flag(max_group_rows) | (
+                                       GROUP_LEAVE_PADDING if leave_padding else 0)) if tile_group is not None else 0),
                                    _stream())
     if rc == 6:
         return None
@@ -743,7 +746,8 @@ def _ptr_array(ptrs):
 
 
 def grouped_gather_parts_prepared(part_ptrs, rows_per_part, row_index, planes, tile_group, c_rescale, a_limbs,
-                                  dynamic=True, group_shift=None, n_split=0, max_group_rows=None):
+                                  dynamic=True, group_shift=None, n_split=0, max_group_rows=None,
+                                  leave_padding=False):
     """grouped_prepared(row_index=...) whose source rows lie in len(part_ptrs) buffers of rows_per_part rows
     each (device addresses; the token rows of every GPU, read in place): row_index[m] = g names row
     g % rows_per_part of buffer g // rows_per_part.  The caller keeps the buffers alive and synchronised."""
@@ -759,7 +763,8 @@ def grouped_gather_parts_prepared(part_ptrs, rows_per_part, row_index, planes, t
             _ptr_array(part_ptrs), len(part_ptrs), int(rows_per_part), row_index.data_ptr(), planes.handle,
             tile_group.data_ptr(), n_tiles, C.data_ptr(), int(c_rescale),
             group_shift.data_ptr() if group_shift is not None else None, int(n_split), a_limbs,
-            _a_flags(a_limbs, dynamic) | _group_rows_flag(max_group_rows), _stream()), "grouped_gather_parts_prepared")
+            _a_flags(a_limbs, dynamic) | _group_rows_flag(max_group_rows) | (GROUP_LEAVE_PADDING if leave_padding else 0),
+            _stream()), "grouped_gather_parts_prepared")
     return C
 
 
