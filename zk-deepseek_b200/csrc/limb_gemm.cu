@@ -1112,7 +1112,7 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // on one SM cannot block one another.
 // 64 sequences through a dense and a routed block (decoding): all its contractions of this kind 2400 -> 1949 us, the whole
 // step 4239 -> 3823 us; one sequence 1116 -> 671 us with its per-head products left out, the step 1982 -> 1835 us.
-constexpr int kRowsEpiWarps = 4, kRowsThreads = 64 + 32 * kRowsEpiWarps;
+constexpr int kRowsEpiWarps = 8, kRowsThreads = 64 + 32 * kRowsEpiWarps;
 
 __device__ __forceinline__ uint64_t peer_u64(uint32_t own, uint32_t rank)
 {
@@ -1142,7 +1142,7 @@ __device__ __forceinline__ void rows_store(const LimbParams& p, i128w sum, int s
 }
 
 // p.NT = R rows of activations (tmA's box); tmW's box holds 128 weight rows.  grid (n_tiles * ksplit, row tiles, batches)
-__global__ void __launch_bounds__(kRowsThreads)
+__global__ void __launch_bounds__(kRowsThreads, 2)
 limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const LimbParams p,
                  const uint32_t pipe_bytes)
 {
@@ -1172,6 +1172,8 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     const int D = La + p.Lb - 1;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint32_t tmem_cols = 32;
+    while (tmem_cols < (uint32_t)(D * R)) tmem_cols <<= 1;
     const uint32_t w_bytes = (uint32_t)p.Lb * kTileM * kBlockK, a_limb = (uint32_t)R * kBlockK;
     const uint32_t stage_bytes = w_bytes + (uint32_t)La * a_limb;
     const int stages = min(8, (int)(pipe_bytes / stage_bytes));
@@ -1192,7 +1194,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(smem_u32(&s_tmem_base), p.tmem_cols);
+    if (warp == 1) tmem_alloc(smem_u32(&s_tmem_base), tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1250,7 +1252,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         bool ok = true;
         if (some) {
             // the first MMA overwrites its La * R columns; the later limbs' last columns start at zero
-            for (int c = La * R; c < D * R; c += 8) tmem_st8_zero(tq + (uint32_t)c);
+            for (int c = La * R + 8 * ((warp - 2) >> 2); c < D * R; c += 8 * (kRowsEpiWarps / 4)) tmem_st8_zero(tq + (uint32_t)c);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -1263,7 +1265,8 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int64_t n = n0 + col;
         const int shift = p.group_shift ? p.group_shift[2 * group + (n >= p.n_split ? 1 : 0)] : p.shift;
         const int64_t addend = share == 0 ? p.addend : 0;
-        for (int r0 = 0; r0 < rows; r0 += 8) {
+        // the two warps of a quarter take turns of eight rows
+        for (int r0 = 8 * ((warp - 2) >> 2); r0 < rows; r0 += 8 * (kRowsEpiWarps / 4)) {
             int64_t s64[8];
             i128w sum[8];
             if (!some) {
@@ -1291,18 +1294,24 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 1) tmem_dealloc(tmem, p.tmem_cols);
+    if (warp == 1) tmem_dealloc(tmem, tmem_cols);
     if (p.ksplit > 1) {
         cluster_barrier();
         for (int i = share * kRowsThreads + threadIdx.x; i < rows * kTileM; i += p.ksplit * kRowsThreads) {
             const int64_t m = m0 + (i >> 7), n = n0 + (i & 127);
             if (m >= p.M || n >= p.N) continue;
             const uint32_t at = smem_u32(red + i);
+            uint64_t lo[8], hi[8];        // of all peers at once: a round trip costs more than the additions
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                lo[s] = s < p.ksplit ? peer_u64(at, s) : 0;
+                hi[s] = s < p.ksplit && !p.fits64 ? peer_u64(at + (uint32_t)rows * kTileM * 8, s) : 0;
+            }
             i128w sum{0, 0};
-            for (int s = 0; s < p.ksplit; ++s) {
-                const uint64_t lo = peer_u64(at, s);
-                if (p.fits64) sum.lo += lo;
-                else sum = add128(sum, i128w{lo, (int64_t)peer_u64(at + (uint32_t)rows * kTileM * 8, s)});
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                if (p.fits64) sum.lo += lo[s];
+                else sum = add128(sum, i128w{lo[s], (int64_t)hi[s]});
             }
             rows_store(p, sum, p.group_shift ? p.group_shift[2 * group + (n >= p.n_split ? 1 : 0)] : p.shift, z, m, n);
         }
@@ -2374,7 +2383,17 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     // (wq_b, K = 1536: 0.70 against 0.85 ms; w2 of the shared expert, K = 2048: 0.68 against 0.93 ms)
     int64_t max_kb = 8;
     if (switches().persistent_max_kb >= 0) max_kb = switches().persistent_max_kb;
-    if (!p.R && !p.skip_k && (Kp + kBlockK - 1) / kBlockK <= max_kb && !switches().no_persistent &&
+    // few rows: the weights take the MMA's 128 rows (limb_rows_kernel).  Up to 64 rows at any depth, or promised groups of up
+    // to 64, with a plain epilogue; wherever its diagonals fit tensor memory and two stages (or the sums of a split) shared
+    // memory.  The persistent kernel, which took shallow K before, spends its time on 128-row MMAs of 96 columns there
+    // (128 heads, K = 128, 512 columns: 1 row 54 -> 16 us, 64 rows 54 -> 30 us)
+    const int few = p.tile_group ? p.group_rows : p.M <= 64 ? (int)p.M : 0, few_rows = few <= 16 ? 16 : few <= 32 ? 32 : 64;
+    const int64_t kb = (Kp + kBlockK - 1) / kBlockK, rows_tiles = (p.N + kTileM - 1) / kTileM;
+    const size_t rows_stage = (size_t)Lb * kTileM * kBlockK + (size_t)La * few_rows * kBlockK;
+    const bool by_rows = few > 0 && few <= 64 && !p.skip_k && !p.skip_tiles && !p.addin && !p.ep_div && !p.causal_H &&
+                         D * few_rows <= 512 && La * few_rows <= 256 && (kb < 2 ? kb : 2) * rows_stage <= smem_max && mt <= 65535 &&
+                         rows_tiles * p.batches * (p.tile_group ? mt : 1) <= 0x7fffffffll / 8;
+    if (!by_rows && !p.R && !p.skip_k && (Kp + kBlockK - 1) / kBlockK <= max_kb && !switches().no_persistent &&
         !(p.tile_group && switches().no_persistent_grouped)) {
         for (int cand : {64, 48, 32, 16}) {
             if (Lb * cand > 256 || 2 * D * cand > 512) continue;
@@ -2452,70 +2471,59 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         if (rc != ZKDS_OK) return rc;
     }
 
-    // few rows: the weights take the MMA's 128 rows (limb_rows_kernel).  Up to 64 rows, or promised groups of up to 64, with
-    // a plain epilogue; wherever its diagonals fit tensor memory and two stages (or the sums of a split) shared memory
-    const int few = p.tile_group ? p.group_rows : p.M <= 64 ? (int)p.M : 0;
-    if (!persistent && few > 0 && few <= 64 && !p.skip_k && !p.skip_tiles && !p.addin && !p.ep_div && !p.causal_H) {
-        const int R = few <= 16 ? 16 : few <= 32 ? 32 : 64;
-        const size_t full = (size_t)Lb * kTileM * kBlockK + (size_t)La * R * kBlockK;
-        uint32_t tcols = 32;
-        while (tcols < (uint32_t)(D * R)) tcols <<= 1;
-        const int64_t tiles = (p.N + kTileM - 1) / kTileM, all = tiles * p.batches * (p.tile_group ? mt : 1);
-        const int64_t kb = (Kp + kBlockK - 1) / kBlockK;
+    if (by_rows) {
+        const int64_t all = rows_tiles * p.batches * (p.tile_group ? mt : 1);
         const int fits64 = sum_fits64(La, Lb, p.K, p.addend);
-        if (tcols <= 512 && La * R <= 256 && 2 * full <= smem_max && all <= 0x7fffffffll / 8 && mt <= 65535) {
-            // shares of K: the fewest K blocks that an SM works through, four more for each CTA's start and end.  Row tiles
-            // of experts are mostly unused, so their number says nothing: no split there
-            int ks = 1;
-            int64_t best = 0;
-            for (int c = 1; c <= (p.tile_group ? 1 : 8); c *= 2) {
-                if (c > 1 && (kb < 2 * c || (size_t)(fits64 ? 1 : 2) * p.M * kTileM * 8 > 2 * full)) break;
-                const int64_t cost = (all * c + sm_count() - 1) / sm_count() * ((kb + c - 1) / c + 4);
-                if (c == 1 || cost < best) { best = cost; ks = c; }
-            }
-            // two CTAs to an SM where there is more than one for it: one starts or finishes while the other streams
-            const bool pair = all * ks > sm_count() && tcols <= 256 && 2 * full + 1024 <= 112 * 1024;
-            const size_t pipe = pair ? 111 * 1024 : smem_max;
-            CUtensorMap mapA, mapW;
-            const int64_t pitch = (pre_b && pre_b->pitch) ? pre_b->pitch : Kp;
-            if (pitch < Kp || (pitch & 15)) return ZKDS_ERR_ARG;
-            if (!make_plane_map(&mapA, pa, (int64_t)La * a_rows, Kp, R) ||
-                !make_plane_map(&mapW, pb, (int64_t)Lb * b_rows, Kp, kTileM, pitch))
-                return ZKDS_ERR_UNSUPPORTED;
-            LimbParams lp{};
-            lp.La = La; lp.Lb = Lb; lp.NT = R; lp.kblocks = (int)kb;
-            lp.ksplit = ks; lp.kb_per_split = (int)((kb + ks - 1) / ks);
-            lp.tmem_cols = tcols;
-            lp.M = p.M; lp.N = p.N; lp.batches = p.batches;
-            lp.a_rows_per_limb = a_rows; lp.b_rows_per_limb = b_rows; lp.b_batch_rows = p.N;
-            lp.b_batched = p.b_sz ? 1 : 0;
-            lp.C = p.C; lp.R = p.R; lp.c_sz = p.c_sz; lp.c_sm = p.c_sm;
-            lp.addend = p.addend; lp.shift = p.shift; lp.r_legacy = p.r_legacy;
-            lp.error_flag = fl->dev; lp.fits64 = fits64;
-            lp.a_absmax = d_absmax; lp.overflow_flag = fl->overflow_dev;
-            lp.tile_group = p.tile_group; lp.group_shift = p.group_shift; lp.n_split = p.n_split;
-            lp.leave_padding = p.tile_group ? p.leave_padding : 0;
-            rc = allow_big_smem(limb_rows_kernel, g_attr_rows);
-            if (rc != ZKDS_OK) return rc;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(tiles * ks), (unsigned)(p.tile_group ? mt : 1), (unsigned)p.batches);
-            cfg.blockDim = dim3(kRowsThreads);
-            cfg.dynamicSmemBytes = pipe + 1024;
-            cfg.stream = st;
-            cudaLaunchAttribute attr;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = (unsigned)ks;
-            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
-            cudaEvent_t* ev = timing_events();
-            if (ev) ZKDS_CUDA(cudaEventRecord(ev[0], st));
-            rc = set_cuda_error(cudaLaunchKernelEx(&cfg, limb_rows_kernel, mapA, mapW, lp, (uint32_t)pipe));
-            if (rc == ZKDS_OK) rc = check_launch();
-            if (ev) ZKDS_CUDA(cudaEventRecord(ev[1], st));
-            if (ev && rc == ZKDS_OK) return record_launch(p, La, Lb, d_absmax, ev, R);
-            return rc;
+        // shares of K: the fewest K blocks that an SM works through, four more for each CTA's start and end.  Row tiles
+        // of experts are mostly unused, so their number says nothing: no split there
+        int ks = 1;
+        int64_t best = 0;
+        for (int c = 1; c <= (p.tile_group ? 1 : 8); c *= 2) {
+            if (c > 1 && (kb < 2 * c || (size_t)(fits64 ? 1 : 2) * p.M * kTileM * 8 > 2 * rows_stage)) break;
+            const int64_t cost = (all * c + sm_count() - 1) / sm_count() * ((kb + c - 1) / c + 4);
+            if (c == 1 || cost < best) { best = cost; ks = c; }
         }
+        // two CTAs to an SM where there is more than one for it: one starts or finishes while the other streams
+        const bool pair = all * ks > sm_count() && (kb < 2 * ks ? 1 : 2) * rows_stage <= 111 * 1024;
+        const size_t pipe = pair ? 111 * 1024 : smem_max;
+        CUtensorMap mapA, mapW;
+        const int64_t pitch = (pre_b && pre_b->pitch) ? pre_b->pitch : Kp;
+        if (pitch < Kp || (pitch & 15)) return ZKDS_ERR_ARG;
+        if (!make_plane_map(&mapA, pa, (int64_t)La * a_rows, Kp, few_rows) ||
+            !make_plane_map(&mapW, pb, (int64_t)Lb * b_rows, Kp, kTileM, pitch))
+            return ZKDS_ERR_UNSUPPORTED;
+        LimbParams lp{};
+        lp.La = La; lp.Lb = Lb; lp.NT = few_rows; lp.kblocks = (int)kb;
+        lp.ksplit = ks; lp.kb_per_split = (int)((kb + ks - 1) / ks);
+        lp.M = p.M; lp.N = p.N; lp.batches = p.batches;
+        lp.a_rows_per_limb = a_rows; lp.b_rows_per_limb = b_rows; lp.b_batch_rows = p.N;
+        lp.b_batched = p.b_sz ? 1 : 0;
+        lp.C = p.C; lp.R = p.R; lp.c_sz = p.c_sz; lp.c_sm = p.c_sm;
+        lp.addend = p.addend; lp.shift = p.shift; lp.r_legacy = p.r_legacy;
+        lp.error_flag = fl->dev; lp.fits64 = fits64;
+        lp.a_absmax = d_absmax; lp.overflow_flag = fl->overflow_dev;
+        lp.tile_group = p.tile_group; lp.group_shift = p.group_shift; lp.n_split = p.n_split;
+        lp.leave_padding = p.tile_group ? p.leave_padding : 0;
+        rc = allow_big_smem(limb_rows_kernel, g_attr_rows);
+        if (rc != ZKDS_OK) return rc;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(rows_tiles * ks), (unsigned)(p.tile_group ? mt : 1), (unsigned)p.batches);
+        cfg.blockDim = dim3(kRowsThreads);
+        cfg.dynamicSmemBytes = pipe + 1024;
+        cfg.stream = st;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)ks;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        cudaEvent_t* ev = timing_events();
+        if (ev) ZKDS_CUDA(cudaEventRecord(ev[0], st));
+        rc = set_cuda_error(cudaLaunchKernelEx(&cfg, limb_rows_kernel, mapA, mapW, lp, (uint32_t)pipe));
+        if (rc == ZKDS_OK) rc = check_launch();
+        if (ev) ZKDS_CUDA(cudaEventRecord(ev[1], st));
+        if (ev && rc == ZKDS_OK) return record_launch(p, La, Lb, d_absmax, ev, few_rows);
+        return rc;
     }
 
     // few rows (decode, the small-M GEMM): a smaller A box, more pipeline stages
