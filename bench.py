@@ -661,6 +661,7 @@ class MlaWorkload:
         for lin in (attn.wkv_b_1, attn.wkv_b_2, attn.wo):
             lin.scale = torch.tensor(shift, dtype=torch.int32, device=dev)
         attn.score_limbs = self.score_limbs
+        attn.causal_skip = False          # this workload counts the full score matrix
         self.attn = attn
         gx = torch.Generator(device=dev).manual_seed(55)
         x_all = _normal_i(torch, gx, (1, self.T, a.dim), 2.0**xs, dev, torch.int64)

@@ -165,6 +165,37 @@ def test_mla_prefill_with_masked_half_skipped(M, mo, kmod, dev):
     kmod.device_status()
 
 
+@pytest.mark.parametrize("S,limbs,skip", [(6, (5, 4), None), (37, (5, 4), None), (63, (5, 4), None), (37, (5, 4), True), (64, (5, 4), True)])
+def test_mla_prefill_of_any_length(M, mo, kmod, dev, S, limbs, skip):
+    """prompts whose length is no multiple of four take the score, softmax and P . KV kernels with padding positions; with
+    and without the masked half, against the full computation; and the rule that leaves the masked half out by itself"""
+    a = small_args(M, kv_lora_rank=128, n_heads=8)
+    rng = np.random.default_rng(S)
+    attn = M.MLA(0, a).to(dev)
+    load_mla(attn, mla_weights(rng, a), dev)
+    attn.score_limbs = limbs
+    x, mask, freqs = np.rint(rng.standard_normal((1, S, a.dim)) * 2.0**21).astype(np.int64), t(mo.causal_mask(S), dev), freqs_table(M, a)
+    taken, plain = [], kmod.softmax_pv_fused
+
+    def counted(scores, *args, **kw):
+        out = plain(scores, *args, **kw)
+        taken.append(scores.shape[-1] if out is not None else None)
+        return out
+    kmod.softmax_pv_fused = counted
+    try:
+        attn.causal_skip = skip
+        got = attn(t(x, dev), 0, freqs[:S].to(dev), mask)
+        assert taken == [(S + 3) // 4 * 4]
+    finally:
+        kmod.softmax_pv_fused = plain
+    attn.causal_skip, attn.score_limbs = False, (0, 0)
+    want = attn(t(x, dev), 0, freqs[:S].to(dev), mask)
+    assert torch.equal(got, want)
+    kmod.device_status()
+    full = M.MLA(0, small_args(M, kv_lora_rank=512, qk_rope_head_dim=64))
+    assert full.causal_skip is None and full._masked_weigh_nothing(3, 3) and not full._masked_weigh_nothing(4, 4)
+
+
 def test_mla_decode_reads_resident_cache_planes(M, mo, kmod, dev):
     """Decode steps read the latent cache from resident limb planes (one new position split per step, score
     rows padded to four columns, the padding never read).  Against the oracle: a prefill, then single-token steps

@@ -34,6 +34,7 @@ ALGO_AUTO, ALGO_EXACT, ALGO_LIMB = 0, 1, 2
 REMAINDER_LEGACY = 4
 LIMBS_DYNAMIC = 8
 CAUSAL_SKIP = 16
+SOFTMAX_PLANES_COLUMNS = 8192      # columns that the softmax in front of P . KV takes (a row in a block's registers)
 GROUP_ROWS_32, GROUP_ROWS_64, GROUP_LEAVE_PADDING = 32, 64, 128
 
 # Remainder flavour of int64_bmm_broadcast.  True reproduces the reference binary:

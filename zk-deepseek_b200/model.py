@@ -372,8 +372,9 @@ class MLA(nn.Module):
         # Prefill with the causal mask: do not compute, write or read the masked half of the score
         # and probability tensors.  The layer's output is unchanged (a masked score always gets
         # weight 0, int64_gemm.cu:706-710); only the masked entries of the two tensors are left
-        # undefined, so it is switched off whenever they are dumped (snark).
-        self.causal_skip = False
+        # undefined, so it is switched off whenever they are dumped (snark).  None: where the promised limbs prove that no
+        # masked score can get a weight (_masked_weigh_nothing); True: always; False: never.
+        self.causal_skip = None
         # Decode (no mask) reads the latent cache from resident limb planes (K.CachePlanes): a step splits only
         # its new position instead of copying and re-splitting the whole cache twice.  Needs promised limb
         # bounds (score_limbs); the int64 caches stay the reference copy (dumps, prefill, measured reruns) and
@@ -397,6 +398,15 @@ class MLA(nn.Module):
             ent = (key, K.WeightPlanes(w, k_last=k_last))
             self._head_planes[id(lin)] = ent
         return ent[1]
+
+    def _masked_weigh_nothing(self, a_limbs, b_limbs):
+        """True when scores of such limbs cannot reach the mask's 2^42: a row always sees its own position, so a masked
+        score lies more than 64 * 2^19 below the largest one, where the softmax gives 0 (int64_gemm.cu:706-710)"""
+        def largest(limbs):
+            return 128 * (256 ** limbs - 1) // 255
+        both = largest(a_limbs) * largest(b_limbs)
+        score = (self.kv_lora_rank * both >> 23) + (self.qk_rope_head_dim * both >> 21) + 4
+        return 2 * (score * self.softmax_scale1 // self.softmax_scale2 + 1) + (64 << 19) < (64 << 36)
 
     def forward(self, x, start_pos, freqs_cis, mask):
         if self.seq_parallel and world_size > 1:
@@ -510,22 +520,37 @@ class MLA(nn.Module):
         causal = mask is not None and start_pos == 0 and _is_causal_mask(mask, seqlen)
         scores = None
         if K.ALGO != K.ALGO_EXACT:
-            skip = causal and self.causal_skip and not snark and dyn and bl > 0
-            scores = K.mla_scores_fused(q_abs, kv_all, q_pe.contiguous(), pe_all, 23, 21, self.softmax_scale1,
+            # a prompt whose length is no multiple of four gets padding positions (zeros, masked for every row and left out of
+            # the softmax by number), so that it takes the kernels that read and write whole 16-byte pieces too
+            pad = -end_pos % 4 if causal and not snark and dyn and bl > 0 and end_pos <= K.SOFTMAX_PLANES_COLUMNS else 0
+            kv_in, pe_in = (F.pad(kv_all, (0, 0, 0, pad)), F.pad(pe_all, (0, 0, 0, pad))) if pad else (kv_all, pe_all)
+            wanted = self.causal_skip
+            if wanted is None:
+                wanted = end_pos <= K.SOFTMAX_PLANES_COLUMNS and dyn and bl > 0 and self._masked_weigh_nothing(al, bl)
+            skip = causal and wanted and not snark and dyn and bl > 0
+            scores = K.mla_scores_fused(q_abs, kv_in, q_pe.contiguous(), pe_in, 23, 21, self.softmax_scale1,
                                         self.softmax_scale2, causal=causal, a_limbs=al, b_limbs=bl, dynamic=dyn,
                                         skip_masked=skip)
             if scores is not None and skip:
-                ctx = K.softmax_pv_fused(scores, kv_all, 23, causal_skip=True, start_pos=0, a_limbs=3, b_limbs=bl)
+                ctx = K.softmax_pv_fused(scores, kv_in, 23, causal_skip=True, start_pos=0, a_limbs=3, b_limbs=bl)
                 if ctx is not None:
                     del scores
                     return ctx
                 probs = torch.empty_like(scores)
                 if K.softmax_q19_causal(scores, probs, 0):
                     del scores
-                    ctx = K.einsum_bsht_btc_bshc_causal(probs, kv_all, 23, 0, a_limbs=3, b_limbs=bl)
+                    ctx = K.einsum_bsht_btc_bshc_causal(probs, kv_in, 23, 0, a_limbs=3, b_limbs=bl)
                     del probs
                     return ctx
-                # softmax shape not taken by the causal kernel: recompute the scores in full
+            elif scores is not None and pad:
+                # every row weighs the columns 0 .. end_pos - 1: the rows of all positions as those of one
+                rows = scores.view(bsz, 1, seqlen * scores.shape[2], end_pos + pad)
+                ctx = K.softmax_pv_fused(rows, kv_in, 23, causal_skip=True, start_pos=end_pos - 1, a_limbs=3, b_limbs=bl)
+                if ctx is not None:
+                    del scores, rows
+                    return ctx.view(bsz, seqlen, -1, ctx.shape[-1])
+            if scores is not None and (skip or pad):
+                # softmax shape not taken by these kernels: recompute the scores in full
                 scores = K.mla_scores_fused(q_abs, kv_all, q_pe.contiguous(), pe_all, 23, 21, self.softmax_scale1,
                                             self.softmax_scale2, causal=causal, a_limbs=al, b_limbs=bl,
                                             dynamic=dyn)
