@@ -41,6 +41,8 @@ typedef struct {
     float* out2;           /* may be null: columns from `split` (a multiple of 32) on go here, in 32-bit, unrotated */
     long long ldo2;
     long long split;
+    int early;             /* 1: W has been complete since before the launch in front of this one on the stream, so that its
+                              first rows may be requested while that one still runs */
 } zkfp_linear_args;
 
 int zkfp_linear(const zkfp_linear_args* a, void* stream);

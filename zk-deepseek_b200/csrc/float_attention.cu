@@ -577,6 +577,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid_c
 __global__ void __launch_bounds__(256)
 latent_combine_kernel(const LatentParams p, bf16* __restrict__ out, long long o_head)
 {
+    chain_enter();
     __shared__ float red[8][9][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.z, c0 = blockIdx.x * 8;
     const int rt = blockIdx.y >> 2, row = (blockIdx.y & 3) * 32 + lane, row0 = rt * kTile;
@@ -678,8 +679,7 @@ int launch_attention_decode_tc(const zkfp_attention_args& a, cudaStream_t st)
                                                                                                              k2, p);
     int rc = fp_launched();
     if (rc != ZKDS_OK) return rc;
-    latent_combine_kernel<<<dim3((unsigned)(p.c / 8), (unsigned)p.row_tiles * 4, (unsigned)a.batch), 256, 0, st>>>(
-        p, (bf16*)a.out, a.o_head);
+    fp_launch(latent_combine_kernel, dim3((unsigned)(p.c / 8), (unsigned)p.row_tiles * 4, (unsigned)a.batch), dim3(256), 0, st, p, (bf16*)a.out, a.o_head);
     return fp_launched();
 }
 

@@ -174,13 +174,25 @@ __device__ __forceinline__ float reduce8(float (&v)[8], int lane)
 template <typename T, int MT>
 __global__ void __launch_bounds__(256)
 linear_stream_kernel(const T* __restrict__ A, long long lda, const T* __restrict__ W, long long ldw, int M, int N, int K,
-                     int ksplit, const LinEpi e)
+                     int ksplit, int early, const LinEpi e)
 {
     __shared__ float part[8][MT][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int groups = 8 / ksplit, ks = warp % ksplit;
     const int n = (blockIdx.x * groups + warp / ksplit) * 8;
     const int m0 = blockIdx.y * MT;
+    if (early && n < N) {            // this warp's first weights on their way into L2 while the kernel in front ends
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int k = (ks + u * ksplit) * 256 + lane * 8;
+            if (k < K && (lane * 8 * (int)sizeof(T)) % 128 == 0) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (long long)(n + r) * ldw + k) : "memory");
+            }
+        }
+    }
+    chain_enter();
     float acc[MT][8] = {};
     if (n < N) {
         const T* w = W + (long long)n * ldw;
@@ -259,8 +271,9 @@ constexpr int kSkinnyK = 128;            // k of a block: four 16-byte loads a l
 template <int NT>                        // tiles of eight rows of A
 __global__ void __launch_bounds__(256, NT <= 2 ? 2 : 1)
 linear_skinny_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ W, long long ldw, int M, int N, int K,
-                     int ksplit, const LinEpi e)
+                     int ksplit, int early, const LinEpi e)
 {
+    if (!early) chain_enter();
     __shared__ float part[8][16][NT * 8 + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int groups = 8 / ksplit, ks = warp % ksplit;
@@ -285,6 +298,7 @@ linear_skinny_kernel(const bf16* __restrict__ A, long long lda, const bf16* __re
         const int step = ksplit * kSkinnyK;
         int k = ks * kSkinnyK;
         if (k < K) fetch(cur, k);
+        if (early) chain_enter();        // its first weights are on their way while the kernel in front ends
         for (int it = 0; k < K; k += step, ++it) {
             if (k + step < K) fetch(nxt, k + step);
 #pragma unroll
@@ -310,7 +324,7 @@ linear_skinny_kernel(const bf16* __restrict__ A, long long lda, const bf16* __re
                     }
             }
         }
-    }
+    } else if (early) chain_enter();
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -341,9 +355,9 @@ int linear_stream(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
     const unsigned gx = (unsigned)((a.N / 8 + groups - 1) / groups);
     const T *A = (const T*)a.A, *W = (const T*)a.W;
     const int M = (int)a.M, N = (int)a.N, K = (int)a.K;
-    if (M == 1) linear_stream_kernel<T, 1><<<dim3(gx, 1), 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
-    else if (M == 2) linear_stream_kernel<T, 2><<<dim3(gx, 1), 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
-    else linear_stream_kernel<T, 4><<<dim3(gx, (M + 3) / 4), 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
+    if (M == 1) fp_launch(linear_stream_kernel<T, 1>, dim3(gx, 1), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
+    else if (M == 2) fp_launch(linear_stream_kernel<T, 2>, dim3(gx, 1), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
+    else fp_launch(linear_stream_kernel<T, 4>, dim3(gx, (M + 3) / 4), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
     return fp_launched();
 }
 
@@ -370,9 +384,9 @@ int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, cudaStream_
     const unsigned grid = (unsigned)((tiles + groups - 1) / groups);
     const bf16 *A = (const bf16*)a.A, *W = (const bf16*)a.W;
     const int M = (int)a.M, N = (int)a.N, K = (int)a.K;
-    if (M <= 8) linear_skinny_kernel<1><<<grid, 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
-    else if (M <= 16) linear_skinny_kernel<2><<<grid, 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
-    else if (M <= kSkinnyRows) linear_skinny_kernel<4><<<grid, 256, 0, st>>>(A, a.lda, W, a.ldw, M, N, K, ksplit, e);
+    if (M <= 8) fp_launch(linear_skinny_kernel<1>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
+    else if (M <= 16) fp_launch(linear_skinny_kernel<2>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
+    else if (M <= kSkinnyRows) fp_launch(linear_skinny_kernel<4>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
     else return ZKDS_ERR_UNSUPPORTED;
     return fp_launched();
 }

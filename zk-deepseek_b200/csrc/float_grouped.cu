@@ -12,6 +12,7 @@ template <typename T, int LANES, int V>
 __global__ void __launch_bounds__(256)
 heads_post_kernel(const zkfp_heads_args a)
 {
+    chain_enter();
     const int lane = threadIdx.x % LANES, units = a.heads + a.kv_heads;
     const long long unit = (long long)blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
     if (unit >= a.rows * units) return;              // whole groups of lanes leave together
@@ -68,7 +69,7 @@ int heads_post(const zkfp_heads_args& a, cudaStream_t st)
 {
     const long long per = 256 / LANES, blocks = (a.rows * (a.heads + a.kv_heads) + per - 1) / per;
     if (blocks > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
-    heads_post_kernel<T, LANES, V><<<(unsigned)blocks, 256, 0, st>>>(a);
+    fp_launch(heads_post_kernel<T, LANES, V>, dim3((unsigned)blocks), dim3(256), 0, st, a);
     return fp_launched();
 }
 
@@ -112,6 +113,7 @@ template <typename T>
 __global__ void __launch_bounds__(kGroupedThreads)
 grouped_partial_kernel(const zkfp_grouped_args a, int chunk, int kpitch, int chunks)
 {
+    chain_enter();
     extern __shared__ __align__(16) uint8_t sm[];
     const int b = blockIdx.z, kv = blockIdx.y, tid = threadIdx.x, d = a.d, vecs = d / 8;
     const int start = a.start[b];
@@ -220,6 +222,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 grouped_combine_kernel(const zkfp_grouped_args a, int chunk, int chunks)
 {
+    chain_enter();
     extern __shared__ float red[];                          // [8][d] sums, then [8] sums of weights
     const long long all_rows = a.seq * a.heads, rh = blockIdx.x;          // (sequence, token, head)
     const int b = (int)(rh / all_rows), rest = (int)(rh - (long long)b * all_rows), t = rest / a.heads, h = rest - t * a.heads;
@@ -277,13 +280,12 @@ int grouped_attention(const zkfp_grouped_args& a, cudaStream_t st)
     const int chunks = grouped_chunks<T>(a);
     if (g.smem > 100 * 1024 || a.batch * a.seq * a.heads > 0x7fffffffll || a.kv_heads > 65535) return ZKDS_ERR_UNSUPPORTED;
     ZKDS_CUDA(cudaFuncSetAttribute(grouped_partial_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    grouped_partial_kernel<T><<<dim3((unsigned)chunks, (unsigned)a.kv_heads, (unsigned)a.batch), kGroupedThreads, g.smem, st>>>(
-        a, g.chunk, g.kpitch, chunks);
+    fp_launch(grouped_partial_kernel<T>, dim3((unsigned)chunks, (unsigned)a.kv_heads, (unsigned)a.batch), dim3(kGroupedThreads), g.smem, st, a, g.chunk, g.kpitch, chunks);
     const int rc = fp_launched();
     if (rc != ZKDS_OK) return rc;
     const size_t smem = sizeof(float) * (8 * (size_t)a.d + 8);
     if (smem > 48 * 1024) return ZKDS_ERR_UNSUPPORTED;
-    grouped_combine_kernel<T><<<(unsigned)(a.batch * a.seq * a.heads), 256, smem, st>>>(a, g.chunk, chunks);
+    fp_launch(grouped_combine_kernel<T>, dim3((unsigned)(a.batch * a.seq * a.heads)), dim3(256), smem, st, a, g.chunk, chunks);
     return fp_launched();
 }
 

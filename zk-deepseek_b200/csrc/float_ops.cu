@@ -12,6 +12,7 @@ __global__ void __launch_bounds__(256)
 embed_kernel(const long long* __restrict__ tokens, const T* __restrict__ table, long long ld_table, long long vocab,
              float* __restrict__ x, bf16* __restrict__ xb, long long ldx, float scale)
 {
+    chain_enter();
     const long long r = blockIdx.x, t = tokens[r];
     const bool ok = t >= 0 && t < vocab;
     for (long long c = threadIdx.x * 8; c < ldx; c += 256 * 8) {
@@ -40,6 +41,7 @@ add_norm_kernel(float* __restrict__ x, const float* __restrict__ y, const float*
                 const float* __restrict__ w2, T* __restrict__ h, long long ldx, long long ldy, int width, int padded,
                 float eps)
 {
+    chain_enter();
     __shared__ float red[8];
     const long long r = blockIdx.x;
     float* xr = x + r * ldx;
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(256)
 norm_rows_kernel(const float* __restrict__ x, long long ldx, const int* __restrict__ index, const float* __restrict__ w,
                  T* __restrict__ out, long long ldo, int width, int padded, float eps)
 {
+    chain_enter();
     __shared__ float red[8];
     const long long r = index ? index[blockIdx.x] : (long long)blockIdx.x;
     norm_row(x + r * ldx, w, out + blockIdx.x * ldo, width, padded, eps, red);
@@ -144,6 +147,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 latent_post_kernel(const zkfp_latent_args a)
 {
+    chain_enter();
     __shared__ float red[8];
     const long long r = blockIdx.x;
     const float* yr = a.y + r * a.ldy;
@@ -180,6 +184,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 perhead_absorb_kernel(const zkfp_perhead_args a)
 {
+    chain_enter();
     __shared__ float part[8][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.x, c = (blockIdx.y * 32 + lane) * 8;
@@ -229,6 +234,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 perhead_expand_kernel(const zkfp_perhead_args a)
 {
+    chain_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.y, v = blockIdx.x * 8 + warp;
     if (v >= a.n_out) return;
@@ -399,9 +405,9 @@ int zkfp_embed(const long long* tokens, const void* table, long long ld_table, l
     if (rows == 0) return ZKDS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == ZKFP_BF16)
-        embed_kernel<bf16><<<(unsigned)rows, 256, 0, st>>>(tokens, (const bf16*)table, ld_table, vocab, x, (bf16*)xb, ldx, scale);
+        fp_launch(embed_kernel<bf16>, dim3((unsigned)rows), dim3(256), 0, st, tokens, (const bf16*)table, ld_table, vocab, x, (bf16*)xb, ldx, scale);
     else
-        embed_kernel<float><<<(unsigned)rows, 256, 0, st>>>(tokens, (const float*)table, ld_table, vocab, x, (bf16*)xb, ldx, scale);
+        fp_launch(embed_kernel<float>, dim3((unsigned)rows), dim3(256), 0, st, tokens, (const float*)table, ld_table, vocab, x, (bf16*)xb, ldx, scale);
     return fp_launched();
 }
 
@@ -412,9 +418,9 @@ int zkfp_add_norm(float* x, const float* y, const float* w, const float* w2, voi
     if (rows == 0) return ZKDS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     if (h_dtype == ZKFP_BF16)
-        add_norm_kernel<bf16><<<(unsigned)rows, 256, 0, st>>>(x, y, w, w2, (bf16*)h, ldx, ldy, (int)width, (int)ldx, (float)eps);
+        fp_launch(add_norm_kernel<bf16>, dim3((unsigned)rows), dim3(256), 0, st, x, y, w, w2, (bf16*)h, ldx, ldy, (int)width, (int)ldx, (float)eps);
     else
-        add_norm_kernel<float><<<(unsigned)rows, 256, 0, st>>>(x, y, w, w2, (float*)h, ldx, ldy, (int)width, (int)ldx, (float)eps);
+        fp_launch(add_norm_kernel<float>, dim3((unsigned)rows), dim3(256), 0, st, x, y, w, w2, (float*)h, ldx, ldy, (int)width, (int)ldx, (float)eps);
     return fp_launched();
 }
 
@@ -425,9 +431,9 @@ int zkfp_norm_rows(const float* x, long long ldx, const int* index, const float*
     if (n == 0) return ZKDS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == ZKFP_BF16)
-        norm_rows_kernel<bf16><<<(unsigned)n, 256, 0, st>>>(x, ldx, index, w, (bf16*)out, ldo, (int)width, (int)ldx, (float)eps);
+        fp_launch(norm_rows_kernel<bf16>, dim3((unsigned)n), dim3(256), 0, st, x, ldx, index, w, (bf16*)out, ldo, (int)width, (int)ldx, (float)eps);
     else
-        norm_rows_kernel<float><<<(unsigned)n, 256, 0, st>>>(x, ldx, index, w, (float*)out, ldo, (int)width, (int)ldx, (float)eps);
+        fp_launch(norm_rows_kernel<float>, dim3((unsigned)n), dim3(256), 0, st, x, ldx, index, w, (float*)out, ldo, (int)width, (int)ldx, (float)eps);
     return fp_launched();
 }
 
@@ -438,8 +444,8 @@ int zkfp_latent_post(const zkfp_latent_args* a, void* stream)
     if (a->rows == 0) return ZKDS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid((unsigned)a->rows, a->own_kv ? 2u : 1u);
-    if (a->dtype == ZKFP_BF16) latent_post_kernel<bf16><<<grid, 256, 0, st>>>(*a);
-    else latent_post_kernel<float><<<grid, 256, 0, st>>>(*a);
+    if (a->dtype == ZKFP_BF16) fp_launch(latent_post_kernel<bf16>, grid, dim3(256), 0, st, *a);
+    else fp_launch(latent_post_kernel<float>, grid, dim3(256), 0, st, *a);
     return fp_launched();
 }
 
@@ -453,12 +459,12 @@ int zkfp_perhead(const zkfp_perhead_args* a, void* stream)
     const unsigned tz = (unsigned)((a->tokens + kPerHeadTokens - 1) / kPerHeadTokens);
     if (a->transposed) {
         const dim3 grid((unsigned)a->heads, (unsigned)((a->n_out + 255) / 256), tz);
-        if (a->dtype == ZKFP_BF16) perhead_absorb_kernel<bf16><<<grid, 256, 0, st>>>(*a);
-        else perhead_absorb_kernel<float><<<grid, 256, 0, st>>>(*a);
+        if (a->dtype == ZKFP_BF16) fp_launch(perhead_absorb_kernel<bf16>, grid, dim3(256), 0, st, *a);
+        else fp_launch(perhead_absorb_kernel<float>, grid, dim3(256), 0, st, *a);
     } else {
         const dim3 grid((unsigned)((a->n_out + 7) / 8), (unsigned)a->heads, tz);
-        if (a->dtype == ZKFP_BF16) perhead_expand_kernel<bf16><<<grid, 256, 0, st>>>(*a);
-        else perhead_expand_kernel<float><<<grid, 256, 0, st>>>(*a);
+        if (a->dtype == ZKFP_BF16) fp_launch(perhead_expand_kernel<bf16>, grid, dim3(256), 0, st, *a);
+        else fp_launch(perhead_expand_kernel<float>, grid, dim3(256), 0, st, *a);
     }
     return fp_launched();
 }

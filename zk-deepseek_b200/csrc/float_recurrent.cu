@@ -27,6 +27,7 @@ template <typename T, int TAPS>
 __global__ void __launch_bounds__(128)
 short_conv_kernel(const zkfp_conv_args a)
 {
+    chain_enter();
     const int c = (int)(blockIdx.x * 128 + threadIdx.x) * 8, b = blockIdx.z, t0 = blockIdx.y * kConvTokens;
     const int t1 = min(t0 + kConvTokens, (int)a.seq), taps = TAPS ? TAPS : a.taps;
     const long long slot = a.slots[b];
@@ -100,10 +101,10 @@ int short_conv(const zkfp_conv_args& a, cudaStream_t st)
     const dim3 grid((unsigned)((a.channels / 8 + 127) / 128), (unsigned)((a.seq + kConvTokens - 1) / kConvTokens), (unsigned)a.batch);
     if (grid.y > 65535u) return ZKDS_ERR_UNSUPPORTED;
     switch (a.taps) {
-    case 2: short_conv_kernel<T, 2><<<grid, 128, 0, st>>>(a); break;
-    case 3: short_conv_kernel<T, 3><<<grid, 128, 0, st>>>(a); break;
-    case 4: short_conv_kernel<T, 4><<<grid, 128, 0, st>>>(a); break;
-    default: short_conv_kernel<T, 0><<<grid, 128, 0, st>>>(a);
+    case 2: fp_launch(short_conv_kernel<T, 2>, grid, dim3(128), 0, st, a); break;
+    case 3: fp_launch(short_conv_kernel<T, 3>, grid, dim3(128), 0, st, a); break;
+    case 4: fp_launch(short_conv_kernel<T, 4>, grid, dim3(128), 0, st, a); break;
+    default: fp_launch(short_conv_kernel<T, 0>, grid, dim3(128), 0, st, a);
     }
     return fp_launched();
 }
@@ -117,6 +118,7 @@ template <typename T, int NR>
 __global__ void __launch_bounds__(256)
 scan_kernel(const zkfp_scan_args a)
 {
+    chain_enter();
     constexpr int N = 8 * NR;
     __shared__ float qs[kScanTokens][N], ks[kScanTokens][N], vs[kScanTokens][32], part[kScanTokens][8][32];
     __shared__ float as[kScanTokens], ws[kScanTokens];
@@ -202,11 +204,11 @@ template <typename T>
 int scan(const zkfp_scan_args& a, cudaStream_t st)
 {
     const dim3 grid((unsigned)((a.p + 31) / 32), (unsigned)a.heads, (unsigned)a.batch);
-    if (a.n <= 32) scan_kernel<T, 4><<<grid, 256, 0, st>>>(a);
-    else if (a.n <= 64) scan_kernel<T, 8><<<grid, 256, 0, st>>>(a);
-    else if (a.n <= 128) scan_kernel<T, 16><<<grid, 256, 0, st>>>(a);
-    else if (a.n <= 256) scan_kernel<T, 32><<<grid, 256, 0, st>>>(a);
-    else if (a.n <= 512) scan_kernel<T, 64><<<grid, 256, 0, st>>>(a);
+    if (a.n <= 32) fp_launch(scan_kernel<T, 4>, grid, dim3(256), 0, st, a);
+    else if (a.n <= 64) fp_launch(scan_kernel<T, 8>, grid, dim3(256), 0, st, a);
+    else if (a.n <= 128) fp_launch(scan_kernel<T, 16>, grid, dim3(256), 0, st, a);
+    else if (a.n <= 256) fp_launch(scan_kernel<T, 32>, grid, dim3(256), 0, st, a);
+    else if (a.n <= 512) fp_launch(scan_kernel<T, 64>, grid, dim3(256), 0, st, a);
     else return ZKDS_ERR_UNSUPPORTED;
     return fp_launched();
 }
@@ -218,6 +220,7 @@ template <typename T, int THREADS, int KEEP, bool FIRST>
 __global__ void __launch_bounds__(256)
 gated_norm_kernel(const zkfp_gated_norm_args a, int parts, int stride)
 {
+    chain_enter();
     __shared__ float red[8];
     const long long unit = (long long)blockIdx.x * (256 / THREADS) + threadIdx.x / THREADS;
     if (unit >= a.rows * parts) return;                  // whole warps, or the whole block
@@ -286,6 +289,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 gated_norm_any_kernel(const zkfp_gated_norm_args a, int parts)
 {
+    chain_enter();
     __shared__ float red[8];
     const long long r = blockIdx.x / parts;
     const int part = (int)(blockIdx.x - r * parts);
@@ -325,11 +329,11 @@ int gated_norm_packed(const zkfp_gated_norm_args& a, int parts, int stride, cuda
     const long long units = a.rows * parts;
     if (units > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
     const unsigned warps = (unsigned)((units + 7) / 8);
-    if (stride <= 256) gated_norm_kernel<T, 32, 1, FIRST><<<warps, 256, 0, st>>>(a, parts, stride);
-    else if (stride <= 512) gated_norm_kernel<T, 32, 2, FIRST><<<warps, 256, 0, st>>>(a, parts, stride);
-    else if (stride <= 1024) gated_norm_kernel<T, 32, 4, FIRST><<<warps, 256, 0, st>>>(a, parts, stride);
-    else if (stride <= 2048) gated_norm_kernel<T, 32, 8, FIRST><<<warps, 256, 0, st>>>(a, parts, stride);
-    else gated_norm_kernel<T, 256, 4, FIRST><<<(unsigned)units, 256, 0, st>>>(a, parts, stride);
+    if (stride <= 256) fp_launch(gated_norm_kernel<T, 32, 1, FIRST>, dim3(warps), dim3(256), 0, st, a, parts, stride);
+    else if (stride <= 512) fp_launch(gated_norm_kernel<T, 32, 2, FIRST>, dim3(warps), dim3(256), 0, st, a, parts, stride);
+    else if (stride <= 1024) fp_launch(gated_norm_kernel<T, 32, 4, FIRST>, dim3(warps), dim3(256), 0, st, a, parts, stride);
+    else if (stride <= 2048) fp_launch(gated_norm_kernel<T, 32, 8, FIRST>, dim3(warps), dim3(256), 0, st, a, parts, stride);
+    else fp_launch(gated_norm_kernel<T, 256, 4, FIRST>, dim3((unsigned)units), dim3(256), 0, st, a, parts, stride);
     return fp_launched();
 }
 
@@ -341,7 +345,7 @@ int gated_norm(const zkfp_gated_norm_args& a, cudaStream_t st)
     if (whole_head || (a.p == a.vdim && a.part % 8 == 0))
         return a.weight ? gated_norm_packed<T, true>(a, parts, stride, st) : gated_norm_packed<T, false>(a, parts, stride, st);
     if (a.rows * parts > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
-    gated_norm_any_kernel<T><<<(unsigned)(a.rows * parts), 256, 0, st>>>(a, parts);
+    fp_launch(gated_norm_any_kernel<T>, dim3((unsigned)(a.rows * parts)), dim3(256), 0, st, a, parts);
     return fp_launched();
 }
 
