@@ -130,7 +130,7 @@ def _check(status, what):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def device_status(sync=False):

@@ -734,6 +734,9 @@ class FloatTransformer(nn.Module):
         return self._recorded[B].run(tokens, start_pos, slots)
 
 
+STEPS_AHEAD = 4
+
+
 class RecordedStep:
     """The kernels of a one-token step of B sequences: the first run records the calls with their buffers, later runs
     issue them again.  Tokens, positions and slots are device inputs."""
@@ -743,18 +746,19 @@ class RecordedStep:
         self.model, self.calls = model, None
         self.tokens = torch.zeros(B, 1, dtype=torch.int64, device=dev)
         self.meta = torch.zeros(2, B, dtype=torch.int32, device=dev)
-        self.host = torch.zeros(2, B, dtype=torch.int32).pin_memory()
+        # several buffers for the inputs, so that the host may prepare steps while earlier ones still run
+        self.host = [torch.zeros(2, B, dtype=torch.int32).pin_memory() for _ in range(STEPS_AHEAD)]
         self.rows = torch.arange(B, dtype=torch.int32, device=dev)
-        self.copied = torch.cuda.Event()
+        self.copied, self.turn = [torch.cuda.Event() for _ in range(STEPS_AHEAD)], 0
 
     def run(self, tokens, start_pos, slots):
-        self.copied.synchronize()         # the previous step's inputs have left the pinned buffer
-        self.host[0].fill_(start_pos)
-        for b, s in enumerate(slots):
-            self.host[1, b] = s
-        self.meta.copy_(self.host, non_blocking=True)
+        host, copied = self.host[self.turn], self.copied[self.turn]
+        self.turn = (self.turn + 1) % STEPS_AHEAD
+        copied.synchronize()              # the inputs of the step that used this buffer have left it
+        host.copy_(torch.tensor([[start_pos] * len(slots), slots], dtype=torch.int32))
+        self.meta.copy_(host, non_blocking=True)
         self.tokens.copy_(tokens, non_blocking=True)
-        self.copied.record()
+        copied.record()
         if self.calls is not None:
             self.calls.replay()
             return self.logits.clone()

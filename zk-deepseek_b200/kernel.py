@@ -24,6 +24,7 @@ Differences from the reference module, all on the host side:
     reaches them.
 """
 import ctypes
+import functools
 import os
 
 import torch
@@ -142,7 +143,8 @@ def _check(status, what):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle alone: a Stream object for every call costs more than the call's other arguments together
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 class _NoSwitch:
@@ -304,6 +306,7 @@ def last_kernel_ms():
     return float(lib.zkds_last_kernel_ms())
 
 
+@functools.lru_cache(maxsize=4096)
 def limb_kernel_takes(K, a_limbs, b_limbs):
     """True when the tensor-core limb kernel handles a contraction of depth K with these limb
     counts (mirrors the launcher: int32 diagonal bound, tile and pipeline fit)."""
