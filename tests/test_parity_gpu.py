@@ -766,3 +766,21 @@ def test_few_rows_against_many_weights(kmod, orc, dev, M, K, N, abits, bbits, s)
     """the weights as the MMA's rows: edges of the boxes of 16, 32 and 64 rows and of 128 columns, ragged and empty shares of
     K, sums of one and of two words.  (Not 23 bits: three signed limbs end at 8355711, below 2^23.)"""
     test_small_m_gemm_split_over_k(kmod, orc, dev, M, K, N, abits, bbits, s)
+
+
+@pytest.mark.parametrize("M,K,N,wdtype,at", [(3, 2049, 5, np.int32, (2, 2048)), (1, 7, 4, np.int64, (0, 6)), (5, 4098, 3, np.int64, (4, 4097)),
+                                             (40, 2048, 2100, np.int32, (39, 0))])
+@pytest.mark.parametrize("skew", [0, 1])
+def test_measured_ranges(kmod, orc, dev, M, K, N, wdtype, at, skew):
+    """one extreme value in the last row of either operand decides its limbs: ends of segments, odd lengths, sources that are
+    only 8-byte aligned, divisors, the most negative number"""
+    rng = np.random.default_rng(K)
+    A, B = rand_i64(rng, (1, M, K), 10), rand_i64(rng, (N, K), 6).astype(wdtype)
+    for hi, div in ((2**29 + 1, 1), (-2**31, 1), (-2**40, 256), (-2**63, 1)):
+        A[0, at[0], at[1]], B[N - 1, K - 1] = hi, -2**28
+        flat = torch.zeros(A.size + skew, dtype=torch.int64, device=dev)
+        flat[skew:] = g(A, dev).flatten()
+        C, R = kmod.int64_bmm_broadcast(flat[skew:].view(1, M, K), g(B, dev), div, 1, 8)
+        Co, Ro = orc.gemm(A, B, div, 1, 8, orc.R_LEGACY)
+        same(C, Co, "C")
+        same(R, Ro, "R")
