@@ -977,10 +977,10 @@ class Block(nn.Module):
             saveTensor(f"{d}/attn_norm_y.bin", atten_normed)
             saveTensor(f"{d}/attn_norm_rms.bin", rms)
         attned = self.attn(atten_normed, start_pos, freqs_cis, mask)
-        x = x + attned * (2 ** 12)
+        x = torch.add(x, attned, alpha=2 ** 12)
         ffn_normed, rms = self.ffn_norm(x)
         ffned = self.ffn(start_pos, ffn_normed)
-        x = x + ffned * (2 ** 8)
+        x = torch.add(x, ffned, alpha=2 ** 8)
         if snark and CHECK_STATUS:      # dumps of a step whose limb bound did not hold must not be trusted
             K.device_status(sync=True)
         return x
