@@ -784,3 +784,18 @@ def test_measured_ranges(kmod, orc, dev, M, K, N, wdtype, at, skew):
         Co, Ro = orc.gemm(A, B, div, 1, 8, orc.R_LEGACY)
         same(C, Co, "C")
         same(R, Ro, "R")
+
+
+@pytest.mark.parametrize("S,H,T,start", [(300, 8, 300, 0), (150, 3, 152, 0), (40, 128, 400, 357), (9, 16, 1028, 1000)])
+def test_causal_probabilities_of_tiles_that_end_early(kmod, dev, S, H, T, start):
+    """tiles of 128 rows over several positions, blocks of 128 columns that they do not reach: after a full call has filled the
+    scratch with other probabilities, against the softmax over masked scores"""
+    rng = np.random.default_rng(T)
+    scores, kv = g(rand_i64(rng, (2, S, H, T), 21), dev), g(rand_i64(rng, (2, T, 64), 20), dev)
+    kmod.softmax_pv_fused(torch.zeros_like(scores), kv, 23, a_limbs=3, b_limbs=3)
+    beyond = torch.arange(T, device=dev)[None, None, None, :] > start + torch.arange(S, device=dev)[None, :, None, None]
+    want = kmod.softmax_pv_fused(torch.where(beyond, scores - (64 << 36), scores), kv, 23, a_limbs=3, b_limbs=3)
+    kmod.softmax_pv_fused(torch.zeros_like(scores), kv, 23, a_limbs=3, b_limbs=3)
+    got = kmod.softmax_pv_fused(scores, kv, 23, causal_skip=True, start_pos=start, a_limbs=3, b_limbs=3)
+    assert got is not None and torch.equal(got, want)
+    kmod.device_status()
