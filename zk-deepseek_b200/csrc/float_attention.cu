@@ -575,7 +575,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid_c
 
 // merges the chunks of 32 rows x 8 latent columns: the warps share the chunks.  grid (c / 8, row tiles * 4, batch)
 __global__ void __launch_bounds__(256)
-latent_combine_kernel(const LatentParams p, bf16* __restrict__ out, long long o_head)
+latent_combine_kernel(const LatentParams p, bf16* out, long long o_head)
 {
     chain_enter();
     __shared__ float red[8][9][32];

@@ -170,6 +170,9 @@ __device__ __forceinline__ void epilogue8(const LinEpi& e, int pos, long long m,
 // chain_enter, in front of everything that reads or writes what another kernel touches, waits until that one is complete
 // and its results are visible, and lets the next kernel's blocks come.  (A kernel waits for all before it that way: the
 // one in front has itself waited.)
+// Such a kernel is resident while another one still writes what it is going to read.  So none of its operands is
+// __restrict__ or loaded through the non-coherent path: both promise that nobody writes the data while the kernel runs, and
+// either lets the compiler move a load in front of the wait.  Plain loads stay behind the asm's "memory".
 // One sequence of Munalorn at width 4096 decoding: 34 launches, 469 -> 407 us; four sequences of Vifelix at width 2048, a prompt
 // of 150 and 16 tokens: 3789 -> 3093 us.  (Results are the same bits.)
 __device__ __forceinline__ void chain_enter()

@@ -173,8 +173,8 @@ __device__ __forceinline__ float reduce8(float (&v)[8], int lane)
 
 template <typename T, int MT>
 __global__ void __launch_bounds__(256)
-linear_stream_kernel(const T* __restrict__ A, long long lda, const T* __restrict__ W, long long ldw, int M, int N, int K,
-                     int ksplit, int early, const LinEpi e)
+linear_stream_kernel(const T* A, long long lda, const T* W, long long ldw, int M, int N, int K, int ksplit, int early,
+                     const LinEpi e)
 {
     __shared__ float part[8][MT][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -251,7 +251,7 @@ linear_stream_kernel(const T* __restrict__ A, long long lda, const T* __restrict
 __device__ __forceinline__ uint4 stream16(const bf16* p)
 {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
@@ -270,8 +270,8 @@ constexpr int kSkinnyK = 128;            // k of a block: four 16-byte loads a l
 
 template <int NT>                        // tiles of eight rows of A
 __global__ void __launch_bounds__(256, NT <= 2 ? 2 : 1)
-linear_skinny_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ W, long long ldw, int M, int N, int K,
-                     int ksplit, int early, const LinEpi e)
+linear_skinny_kernel(const bf16* A, long long lda, const bf16* W, long long ldw, int M, int N, int K, int ksplit, int early,
+                     const LinEpi e)
 {
     if (!early) chain_enter();
     __shared__ float part[8][16][NT * 8 + 1];

@@ -9,19 +9,27 @@ namespace {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-embed_kernel(const long long* __restrict__ tokens, const T* __restrict__ table, long long ld_table, long long vocab,
-             float* __restrict__ x, bf16* __restrict__ xb, long long ldx, float scale)
+embed_kernel(const long long* tokens, const T* table, long long ld_table, long long vocab, float* x, bf16* xb, long long ldx,
+             float scale)
 {
     chain_enter();
     const long long r = blockIdx.x, t = tokens[r];
     const bool ok = t >= 0 && t < vocab;
-    for (long long c = threadIdx.x * 8; c < ldx; c += 256 * 8) {
-        float v[8] = {};
-        if (ok) load8(table + t * ld_table + c, v);
+    constexpr int KEEP = 2;               // pieces of 2048 columns whose loads are in flight together
+    for (long long c0 = threadIdx.x * 8; c0 < ldx; c0 += KEEP * 2048) {
+        float v[KEEP][8] = {};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] *= scale;
-        store8(x + r * ldx + c, v);
-        if (xb) store8(xb + r * ldx + c, v);
+        for (int k = 0; k < KEEP; ++k)
+            if (ok && c0 + k * 2048 < ldx) load8(table + t * ld_table + c0 + k * 2048, v[k]);
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const long long c = c0 + k * 2048;
+            if (c >= ldx) break;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[k][i] *= scale;
+            store8(x + r * ldx + c, v[k]);
+            if (xb) store8(xb + r * ldx + c, v[k]);
+        }
     }
 }
 
@@ -37,9 +45,8 @@ __device__ __forceinline__ float sum_squares8(const float (&v)[8])
 // is found again in L1 / L2
 template <typename T>
 __global__ void __launch_bounds__(256)
-add_norm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w,
-                const float* __restrict__ w2, T* __restrict__ h, long long ldx, long long ldy, int width, int padded,
-                float eps)
+add_norm_kernel(float* x, const float* y, const float* w, const float* w2, T* h, long long ldx, long long ldy, int width,
+                int padded, float eps)
 {
     chain_enter();
     __shared__ float red[8];
@@ -66,45 +73,58 @@ add_norm_kernel(float* __restrict__ x, const float* __restrict__ y, const float*
     s = block_sum(s, red);
     const float rs = 1.0f / sqrtf(s / (float)width + eps);
     s = 0.f;
-    auto apply = [&](int c, float (&v)[8]) {          // leaves the new x in v
-        float a[8], g[8];
-        load8(xr + c, a);
-        load8(w + c, g);
+    auto apply = [&](int c, const float (&a)[8], const float (&g)[8], float (&v)[8]) {          // leaves the new x in v
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = a[i] + v[i] * rs * g[i];
         store8(xr + c, v);
         if (w2) s += sum_squares8(v);
         else if (h) store8(hr + c, v);
     };
+    // loads before stores: the compiler may not move one over the other (see chain_enter)
+    float a[KEEP][8], g[KEEP][8];
 #pragma unroll
     for (int k = 0; k < KEEP; ++k) {
         const int c = (k * 256 + threadIdx.x) * 8;
-        if (c < padded) apply(c, keep[k]);
+        if (c < padded) {
+            load8(xr + c, a[k]);
+            load8(w + c, g[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int c = (k * 256 + threadIdx.x) * 8;
+        if (c < padded) apply(c, a[k], g[k], keep[k]);
     }
     for (int c = (KEEP * 256 + threadIdx.x) * 8; c < padded; c += 256 * 8) {
         float v[8];
         load8(yr + c, v);
-        apply(c, v);
+        load8(xr + c, a[0]);
+        load8(w + c, g[0]);
+        apply(c, a[0], g[0], v);
     }
     if (!w2) return;
     s = block_sum(s, red);
     const float rx = 1.0f / sqrtf(s / (float)width + eps);
-    auto write = [&](int c, const float (&v)[8]) {
-        float g[8];
-        load8(w2 + c, g);
+    auto write = [&](int c, float (&f)[8], const float (&v)[8]) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) g[i] *= v[i] * rx;
-        store8(hr + c, g);
+        for (int i = 0; i < 8; ++i) f[i] *= v[i] * rx;
+        store8(hr + c, f);
     };
 #pragma unroll
     for (int k = 0; k < KEEP; ++k) {
         const int c = (k * 256 + threadIdx.x) * 8;
-        if (c < padded) write(c, keep[k]);
+        if (c < padded) load8(w2 + c, g[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int c = (k * 256 + threadIdx.x) * 8;
+        if (c < padded) write(c, g[k], keep[k]);
     }
     for (int c = (KEEP * 256 + threadIdx.x) * 8; c < padded; c += 256 * 8) {
         float v[8];
         load8(xr + c, v);                 // written by this thread above
-        write(c, v);
+        load8(w2 + c, g[0]);
+        write(c, g[0], v);
     }
 }
 
@@ -121,20 +141,32 @@ __device__ __forceinline__ void norm_row(const float* xr, const float* w, T* out
     }
     s = block_sum(s, red);
     const float rs = 1.0f / sqrtf(s / (float)width + eps);
-    for (int c = threadIdx.x * 8; c < padded; c += blockDim.x * 8) {
-        float v[8], g[8];
-        load8(xr + c, v);
-        load8(w + c, g);
+    constexpr int KEEP = 2;               // pieces of a column group whose loads are in flight together
+    for (int c0 = threadIdx.x * 8; c0 < padded; c0 += KEEP * blockDim.x * 8) {
+        float v[KEEP][8], g[KEEP][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = v[i] * rs * g[i];
-        store8(out + c, v);
+        for (int k = 0; k < KEEP; ++k) {
+            const int c = c0 + k * blockDim.x * 8;
+            if (c < padded) {
+                load8(xr + c, v[k]);
+                load8(w + c, g[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int c = c0 + k * blockDim.x * 8;
+            if (c >= padded) break;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[k][i] = v[k][i] * rs * g[k][i];
+            store8(out + c, v[k]);
+        }
     }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-norm_rows_kernel(const float* __restrict__ x, long long ldx, const int* __restrict__ index, const float* __restrict__ w,
-                 T* __restrict__ out, long long ldo, int width, int padded, float eps)
+norm_rows_kernel(const float* x, long long ldx, const int* index, const float* w, T* out, long long ldo, int width, int padded,
+                 float eps)
 {
     chain_enter();
     __shared__ float red[8];
