@@ -112,6 +112,28 @@ def test_linear_of_few_bfloat16_rows(K, M, N, Kd):
     test_linear_and_its_epilogues(K, "bfloat16", M, N, Kd)
 
 
+@pytest.mark.parametrize("kind", ["normal", "biased", "outliers"])
+@pytest.mark.parametrize("N,Kd", [(512, 7168), (2048, 2048), (2048, 4096), (4096, 512), (2120, 264)])
+def test_few_bfloat16_rows_are_as_exact_as_many(K, N, Kd, kind):
+    """the streamed products against the tiles that 33 rows take: the same rows, no larger distance from 64 bits.  An error is
+    the norm over 3 x N results that are rounded independently, so that equally exact sums differ by some per cent"""
+    A, W = rnd((33, Kd), "float32"), rnd((N, Kd), "float32", 1, Kd ** -0.5)
+    if kind == "biased":
+        A, W = A.abs(), W + 0.5 * Kd ** -0.5
+    if kind == "outliers":
+        A[:, ::97] *= 30
+    A, W = A.bfloat16(), W.bfloat16()
+    want = A.double() @ W.double().T
+
+    def distance(M):
+        out = torch.empty((M, N), device="cuda")
+        K.linear(A[:M], W, out)
+        return ((out.double() - want[:M])[:3].norm() / want[:3].norm()).item()
+    many = distance(33)
+    for M in (3, 8, 16, 32):
+        assert distance(M) <= 1.1 * many, (M, distance(M), many)
+
+
 @pytest.mark.parametrize("M,N,Kd", [(17, 24, 8), (32, 136, 24), (33, 128, 2056), (64, 264, 8192), (65, 2120, 40), (97, 16, 4104)])
 def test_linear_of_float32_tiles(K, M, N, Kd):
     """edges of the tiles of 32 and 64 rows and 128 columns, blocks of K, and shares of K of which some are empty"""

@@ -299,7 +299,7 @@ linear_skinny_kernel(const bf16* A, long long lda, const bf16* W, long long ldw,
         int k = ks * kSkinnyK;
         if (k < K) fetch(cur, k);
         if (early) chain_enter();        // its first weights are on their way while the kernel in front ends
-        for (int it = 0; k < K; k += step, ++it) {
+        for (; k < K; k += step) {
             if (k + step < K) fetch(nxt, k + step);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -313,22 +313,20 @@ linear_skinny_kernel(const bf16* A, long long lda, const bf16* W, long long ldw,
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) { cur[0][u] = nxt[0][u]; cur[1][u] = nxt[1][u]; }
-            // fresh accumulators every 512 k: a product's own additions are cut off rather than rounded
-            if ((it & 3) == 3) {
+            // fresh accumulators for every block of 128 k: a product's own additions are cut off rather than rounded
 #pragma unroll
-                for (int j = 0; j < NT; ++j)
+            for (int j = 0; j < NT; ++j)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        sum[j][i] += acc[j][i];
-                        acc[j][i] = 0.f;
-                    }
-            }
+                for (int i = 0; i < 4; ++i) {
+                    sum[j][i] += acc[j][i];
+                    acc[j][i] = 0.f;
+                }
         }
     } else if (early) chain_enter();
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) part[warp][g + (i >> 1) * 8][j * 8 + t * 2 + (i & 1)] = sum[j][i] + acc[j][i];
+        for (int i = 0; i < 4; ++i) part[warp][g + (i >> 1) * 8][j * 8 + t * 2 + (i & 1)] = sum[j][i];
     __syncthreads();
     // eight columns of one row an item, the shares of K added in a fixed order
     for (int it = threadIdx.x; it < groups * 2 * M; it += 256) {
