@@ -526,6 +526,37 @@ def test_a_step_must_follow_what_the_slot_holds(models):
         model.begin_batch(5)
 
 
+def busy():
+    """a few tens of milliseconds of work in front of whatever is launched next, so that the host is steps ahead"""
+    a = torch.ones(8192, 8192, device="cuda")
+    for _ in range(4):
+        a = a @ a * 1e-4
+    return a
+
+
+@pytest.mark.parametrize("buffers", [1, 2])
+@pytest.mark.parametrize("case", ["WIDE", "V_WIDE"])
+def test_pinned_tokens_may_be_overwritten_after_the_call(models, case, buffers):
+    cfg, W, model = models(case, "bfloat16")
+    toks = tokens_of(cfg, 10, 80)
+    want = run(model, toks, [2] + [1] * 8)
+    run(model, toks, [2] + [1] * 8)                  # recorded by now
+    held = [torch.zeros(1, 1, dtype=torch.int64).pin_memory() for _ in range(buffers)]
+    slots, out = model.begin_batch(1), []
+    out.append(model.step(torch.tensor([toks[:2]]), 0, slots, want=[0, 1])[0])
+    torch.cuda.synchronize()
+    keep = busy()
+    for i in range(2, 10):
+        held[i % buffers][0, 0] = toks[i]
+        out.append(model.step(held[i % buffers], i, slots)[0])
+    for h in held:
+        h.zero_()
+    got = torch.cat(out).cpu().numpy()
+    model.end_batch(slots)
+    del keep
+    assert np.array_equal(got, want)
+
+
 # ---- generation and command lines -----------------------------------------------------------------------------------
 def oracle_greedy(cfg, W, prompt, n):
     """greedy tokens and the smallest margin by which one was chosen"""

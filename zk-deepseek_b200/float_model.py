@@ -748,15 +748,18 @@ class RecordedStep:
         self.meta = torch.zeros(2, B, dtype=torch.int32, device=dev)
         # several buffers for the inputs, so that the host may prepare steps while earlier ones still run
         self.host = [torch.zeros(2, B, dtype=torch.int32).pin_memory() for _ in range(STEPS_AHEAD)]
+        self.host_tokens = [torch.zeros(B, 1, dtype=torch.int64).pin_memory() for _ in range(STEPS_AHEAD)]
         self.rows = torch.arange(B, dtype=torch.int32, device=dev)
         self.copied, self.turn = [torch.cuda.Event() for _ in range(STEPS_AHEAD)], 0
 
     def run(self, tokens, start_pos, slots):
-        host, copied = self.host[self.turn], self.copied[self.turn]
         self.turn = (self.turn + 1) % STEPS_AHEAD
-        copied.synchronize()              # the inputs of the step that used this buffer have left it
+        host, copied = self.host[self.turn], self.copied[self.turn]
+        copied.synchronize()              # the inputs of the step that used these buffers have left them
         host.copy_(torch.tensor([[start_pos] * len(slots), slots], dtype=torch.int32))
         self.meta.copy_(host, non_blocking=True)
+        if tokens.device.type == "cpu":   # the caller may overwrite its buffer, pinned or not, once this call returns
+            tokens = self.host_tokens[self.turn].copy_(tokens)
         self.tokens.copy_(tokens, non_blocking=True)
         copied.record()
         if self.calls is not None:
