@@ -786,6 +786,51 @@ def test_measured_ranges(kmod, orc, dev, M, K, N, wdtype, at, skew):
         same(R, Ro, "R")
 
 
+@pytest.mark.parametrize("Bn,S,H,Cd,D", [(1, 300, 8, 5, 3), (2, 17, 3, 64, 16), (3, 1, 5, 130, 4), (1, 2, 2, 1, 1)])
+@pytest.mark.parametrize("last", [False, True])
+def test_measured_ranges_of_short_rows(kmod, orc, dev, Bn, S, H, Cd, D, last):
+    """operands without gaps are measured as one row, heads inside rows too: the first or the last element decides"""
+    rng = np.random.default_rng(Cd)
+    at = -1 if last else 0
+    A, B, B2 = rand_i64(rng, (Bn, S, H, Cd), 10), rand_i64(rng, (H, D, Cd), 6).astype(np.int32), rand_i64(rng, (Bn, D, Cd), 6)
+    A.reshape(-1)[at], B.reshape(-1)[at], B2.reshape(-1)[at] = -2**40, -2**29, 2**33
+    same(kmod.einsum_bshc_hdc_bshd(g(A, dev), g(B, dev), 5), orc.einsum_bshc_hdc_bshd(A, B, 5), "heads")
+    same(kmod.einsum_bshc_btc_bsht(g(A, dev), g(B2, dev), 5), orc.einsum_bshc_btc_bsht(A, B2, 5), "scores")
+
+
+@pytest.mark.parametrize("rows,K,pitch", [(9, 24, 32), (5, 1024, 1100), (6, 1023, 1024), (3, 2050, 2064), (1, 40, 48)])
+def test_measured_ranges_of_rows_with_gaps(kmod, dev, rows, K, pitch):
+    """short ones and long ones, before prepared weights (which are not measured)"""
+    A = torch.randint(-1000, 1000, (rows, pitch), device=dev)
+    W = torch.randint(-100, 100, (16, K), device=dev, dtype=torch.int32)
+    A[:, K:] = 2**62
+    A[rows - 1, K - 1], W[15, K - 1] = -2**41, -2**20
+    planes, C = kmod.WeightPlanes(W), torch.empty(rows, 16, dtype=torch.int64, device=dev)
+    rc = kmod.lib.zkds_contraction_prepared(A.data_ptr(), 0, pitch, planes.handle, 0, C.data_ptr(), None, rows * 16, 16, 1, rows, 1, 0,
+                                            9, 0, 0, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    want = (A[:, None, :K] * W[None].long()).sum(-1) >> 9
+    assert torch.equal(C, want)
+
+
+def test_measuring_short_rows_takes_no_longer_than_their_bytes(kmod, dev):
+    """16.8 MB in rows of 8: measuring them costs the host's wait and some twenty microseconds, a row at a time it took 700"""
+    A, B = torch.randint(-30000, 30000, (1, 262144, 8), device=dev), torch.randint(-30000, 30000, (64, 8), device=dev)
+
+    def fastest(**limbs):
+        best = 1e9
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            kmod.int64_bmm_broadcast(A, B, 1, 1, 8, **limbs)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+    assert fastest() - fastest(a_limbs=2, b_limbs=2) < 250
+
+
 @pytest.mark.parametrize("S,H,T,start", [(300, 8, 300, 0), (150, 3, 152, 0), (40, 128, 400, 357), (9, 16, 1028, 1000)])
 def test_causal_probabilities_of_tiles_that_end_early(kmod, dev, S, H, T, start):
     """tiles of 128 rows over several positions, blocks of 128 columns that they do not reach: after a full call has filled the

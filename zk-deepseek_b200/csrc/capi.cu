@@ -162,7 +162,7 @@ static int run_contraction(const Contraction& p, int a_limbs, int b_limbs, int f
         if (apart) rc = launch_absmax(p.A, 64, p.batches, p.M, p.K, p.a_sz, p.a_sm, 1, p.a_div, d, st);
         if (rc != ZKDS_OK) return rc;
         // B may be shared by every batch (b_sz == 0)
-        if (apart) {
+        if (apart && b_limbs <= 0) {
             rc = launch_absmax(p.B, p.b_bits, p.b_sz ? p.batches : 1, p.N, p.K, p.b_sz, p.b_sn, p.b_sk,
                                p.b_div, d + 1, st);
             if (rc != ZKDS_OK) return rc;

@@ -2043,8 +2043,10 @@ int launch_split_t(const T* X, int8_t* planes, int L, int64_t nb, int64_t rows, 
 
 // Both operands' ranges in one launch: 2048 consecutive elements of a row a step of a block, its loads all in flight, one
 // atomic a block.  Bound by the bytes read.  32 x 7168 by 576 x 7168 int64, the whole product with its ranges measured:
-// 78.3 -> 60.8 us.  absmax_kernel (a 64-bit division and one load an element, an atomic a warp: 10.8 us each there) is left
-// for sources that are not contiguous along K and for the other entry points that measure.
+// 78.3 -> 60.8 us.  An operand without gaps is one long row, since a step of a short row would leave most of its threads without
+// work: 262144 x 8, row by row 1004 us for the product, as one row 278 (absmax_kernel 290).  absmax_kernel (a 64-bit division and one load
+// an element, an atomic a warp: 10.8 us each there) is left for short rows with gaps, for sources that are not contiguous along
+// K and for the other entry points that measure.
 struct RangeOf {
     const void* X;
     int64_t rows, cols, sz, sr, div, segs, steps;      // steps = batches * rows * segs, 0 = nothing to measure
@@ -2108,14 +2110,21 @@ range_kernel(const RangeOf a, const RangeOf b, uint64_t* out)
 
 }  // namespace
 
-// out_dev[0], out_dev[1] <- ranges of A and B as launch_absmax measures them (null: not measured); ZKDS_ERR_UNSUPPORTED for a B
-// that is not contiguous along K
+// out_dev[0], out_dev[1] <- ranges of A and B as launch_absmax measures them, of those that are wanted; ZKDS_ERR_UNSUPPORTED for
+// a B that is not contiguous along K, and for rows with gaps between them that fill less than half of a step
 int launch_ranges(const Contraction& p, bool want_a, bool want_b, uint64_t* out_dev, cudaStream_t st)
 {
     if (want_b && p.b_sk != 1) return ZKDS_ERR_UNSUPPORTED;
     auto range = [](const void* X, int bits, int64_t batches, int64_t rows, int64_t cols, int64_t sz, int64_t sr, int64_t div) {
         RangeOf o{};
         const int64_t per = 128 / bits;
+        const bool by_batch = (rows == 1 || sr == cols) && (batches == 1 || sz == rows * cols);
+        const bool by_row = (batches == 1 || sz == cols) && (rows == 1 || sr == batches * cols);
+        if (by_batch || by_row) {
+            cols *= rows * batches;
+            rows = batches = 1;
+            sz = sr = 0;
+        }
         o.X = X; o.rows = rows; o.cols = cols; o.sz = sz; o.sr = sr; o.div = div; o.bits = bits;
         o.segs = (cols + 2047) / 2048;
         o.steps = batches * rows * o.segs;
@@ -2127,6 +2136,8 @@ int launch_ranges(const Contraction& p, bool want_a, bool want_b, uint64_t* out_
     if (want_b) b = range(p.B, p.b_bits, p.b_sz ? p.batches : 1, p.N, p.K, p.b_sz, p.b_sn, p.b_div);
     int64_t grid = a.steps + b.steps;
     if (grid == 0) return ZKDS_OK;
+    for (const RangeOf& o : {a, b})
+        if (o.steps > o.segs && 2 * o.cols < o.segs * 2048) return ZKDS_ERR_UNSUPPORTED;
     if (grid > (int64_t)sm_count() * 8) grid = (int64_t)sm_count() * 8;
     range_kernel<<<(unsigned)grid, 256, 0, st>>>(a, b, out_dev);
     return check_launch();
