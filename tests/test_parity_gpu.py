@@ -813,6 +813,18 @@ def test_measured_ranges_of_rows_with_gaps(kmod, dev, rows, K, pitch):
     assert torch.equal(C, want)
 
 
+def test_more_batches_than_can_be_measured_are_refused(kmod, dev):
+    """whatever the order of the operands: 65535 are taken, one more is not"""
+    A = torch.ones(1, 1, 65536, 2, dtype=torch.int64, device=dev)
+    for call, W in ((kmod.einsum_bshc_hdc_bshd, torch.ones(65536, 3, 2, dtype=torch.int32, device=dev)),
+                    (kmod.einsum_bshd_hdc_bshc, torch.ones(65536, 2, 3, dtype=torch.int32, device=dev))):
+        got = call(A[:, :, 1:].contiguous(), W[1:].contiguous(), 0)
+        assert got.shape == (1, 1, 65535, 3) and bool((got == 2).all())
+        with pytest.raises(kmod.ZkdsError) as e:
+            call(A, W, 0)
+        assert e.value.status == kmod.ERR_RANGE
+
+
 def test_measuring_short_rows_takes_no_longer_than_their_bytes(kmod, dev):
     """16.8 MB in rows of 8: measuring them costs the host's wait and some twenty microseconds, a row at a time it took 700"""
     A, B = torch.randint(-30000, 30000, (1, 262144, 8), device=dev), torch.randint(-30000, 30000, (64, 8), device=dev)

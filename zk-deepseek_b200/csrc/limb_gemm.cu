@@ -2115,6 +2115,7 @@ range_kernel(const RangeOf a, const RangeOf b, uint64_t* out)
 int launch_ranges(const Contraction& p, bool want_a, bool want_b, uint64_t* out_dev, cudaStream_t st)
 {
     if (want_b && p.b_sk != 1) return ZKDS_ERR_UNSUPPORTED;
+    if (p.batches > 65535 && p.K > 0) return ZKDS_ERR_RANGE;       // as launch_absmax
     auto range = [](const void* X, int bits, int64_t batches, int64_t rows, int64_t cols, int64_t sz, int64_t sr, int64_t div) {
         RangeOf o{};
         const int64_t per = 128 / bits;
