@@ -441,7 +441,7 @@ int zkds_gate_select(const int64_t* sigma, const int32_t* bias, int64_t tokens, 
 /* Rows of the routed experts (replaces torch.where / bincount per expert, model.py:1366-1374): the (token, slot) pairs whose
  * expert lies in first_expert .. first_expert + experts - 1, sorted by expert, pairs of an expert in their own order, every
  * expert padded to tiles of 128 rows.  row_src [n_tiles * 128] = token of the row, -1 for padding; pos [tokens][slots] = row of
- * the pair, -1 for other experts (and past the last tile); tile_group [n_tiles] = expert of the tile, -1 = unused;
+ * the pair, -1 for other experts (and past the last tile, which raises the flag that zkds_device_status reports); tile_group [n_tiles] = expert of the tile, -1 = unused;
  * counts [experts] = pairs.  Returns ZKDS_ERR_UNSUPPORTED (silently) for experts > 512 or more than 131072 pairs. */
 int zkds_moe_route(const int64_t* indices, int64_t tokens, int slots, int64_t first_expert, int experts, int64_t n_tiles,
                    int* row_src, int* pos, int* tile_group, int64_t* counts, void* stream);

@@ -715,6 +715,27 @@ def test_route_kernel(M, kmod, dev, T, k, first, E, bound):
     assert (row_src == want_src).all() and (pos == want_pos).all() and (group == want_group).all()
 
 
+@pytest.mark.parametrize("T,k,E,n_tiles", [(300, 4, 8, 5), (40, 8, 16, 1), (3, 2, 4, 0), (4099, 2, 7, 60)])
+def test_more_pairs_than_promised_are_reported(kmod, dev, T, k, E, n_tiles):
+    """tiles for fewer pairs than there are: the surplus has no row, nothing is written behind the tiles, and the range flag
+    says so; with enough tiles it does not"""
+    idx = t(np.stack([np.random.default_rng(i).permutation(E)[:k] for i in range(T)]).astype(np.int64), dev)
+    full = [v.cpu().numpy() for v in kmod.moe_route(idx, 0, E, (T * k + E * 127) // 128)]
+    kmod.device_status(sync=True)
+    row_src, group = (torch.full((n + 64,), 77, dtype=torch.int32, device=dev) for n in (n_tiles * 128, n_tiles))
+    pos, counts = torch.empty(T, k, dtype=torch.int32, device=dev), torch.empty(E, dtype=torch.int64, device=dev)
+    assert kmod.lib.zkds_moe_route(idx.data_ptr(), T, k, 0, E, n_tiles, row_src.data_ptr(), pos.data_ptr(), group.data_ptr(),
+                                   counts.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    with pytest.raises(kmod.ZkdsError) as e:
+        kmod.device_status(sync=True)
+    assert e.value.status == kmod.ERR_RANGE
+    kmod.device_status(sync=True)                    # read once
+    assert bool((row_src[n_tiles * 128:] == 77).all()) and bool((group[n_tiles:] == 77).all())
+    assert (row_src[:n_tiles * 128].cpu().numpy() == full[0][:n_tiles * 128]).all()
+    assert (group[:n_tiles].cpu().numpy() == full[2][:n_tiles]).all() and (counts.cpu().numpy() == full[3]).all()
+    assert (pos.cpu().numpy() == np.where(full[1] < n_tiles * 128, full[1], -1)).all()
+
+
 @pytest.mark.parametrize("slots,cols", [(1, 2), (3, 514), (8, 7168), (9, 1030)])
 def test_combine_over_column_parts(kmod, dev, slots, cols):
     rng = np.random.default_rng(slots)

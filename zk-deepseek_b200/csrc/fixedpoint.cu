@@ -1584,7 +1584,8 @@ constexpr int64_t kRouteMaxPairs = 1 << 17;      // beyond, one CTA takes longer
 
 __global__ void __launch_bounds__(kRouteThreads)
 moe_route_kernel(const int64_t* __restrict__ indices, int pairs, int slots, int64_t first, int E, int n_tiles,
-                 int* __restrict__ row_src, int* __restrict__ pos, int* __restrict__ tile_group, int64_t* __restrict__ counts)
+                 int* __restrict__ row_src, int* __restrict__ pos, int* __restrict__ tile_group, int64_t* __restrict__ counts,
+                 unsigned* overflow)
 {
     extern __shared__ int route_smem[];
     int* place = route_smem;                             // [warp][E]: counts, then the next row of the warp's pairs
@@ -1641,7 +1642,10 @@ moe_route_kernel(const int64_t* __restrict__ indices, int pairs, int slots, int6
         __syncwarp();
         if (e < E && lane == __ffs(same) - 1) place[warp * E + e] += __popc(same);
         __syncwarp();
-        if (row >= rows) row = -1;                       // more pairs than the caller said there can be
+        if (row >= rows) {                               // more pairs than the caller said there can be: reported
+            row = -1;
+            *overflow = 1u;
+        }
         if (row >= 0) row_src[row] = (p + lane) / slots;
         if (in) pos[p + lane] = row;
     }
@@ -1654,11 +1658,13 @@ int launch_moe_route(const int64_t* indices, int64_t tokens, int slots, int64_t 
 {
     if (slots < 1 || experts < 1 || experts > kRouteMaxE || tokens > kRouteMaxPairs / slots || n_tiles > (1 << 23))
         return ZKDS_ERR_UNSUPPORTED;
+    unsigned* overflow = limb_range_flag();
+    if (!overflow) return ZKDS_ERR_WORKSPACE;
     const size_t smem = ((size_t)(kRouteWarps + 2) * experts + 1) * sizeof(int);
     ZKDS_CUDA(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(((kRouteWarps + 2) * kRouteMaxE + 1) * sizeof(int))));
     moe_route_kernel<<<1, kRouteThreads, smem, st>>>(indices, (int)(tokens * slots), slots, first_expert, experts, (int)n_tiles,
-                                                     row_src, pos, tile_group, counts);
+                                                     row_src, pos, tile_group, counts, overflow);
     return check_launch();
 }
 

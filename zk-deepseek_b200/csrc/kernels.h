@@ -213,6 +213,7 @@ int limb_timing_record(long long i, double* out8);
 // live in host-mapped memory: reading them needs no synchronisation, but they describe only
 // kernels that have finished.  clear != 0 resets them.
 int limb_device_status(int clear);
+unsigned* limb_range_flag();      // device view of the word behind ZKDS_ERR_RANGE of the current device; null: no memory
 
 // max |x / div| over a strided int64 / int32 operand, written to *out_dev (uint64)
 int launch_absmax(const void* X, int bits, int64_t batches, int64_t rows, int64_t cols,

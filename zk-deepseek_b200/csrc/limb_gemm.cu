@@ -2162,6 +2162,12 @@ int launch_absmax(const void* X, int bits, int64_t batches, int64_t rows, int64_
     return check_launch();
 }
 
+unsigned* limb_range_flag()
+{
+    DeviceFlags* f = flags_for_device();
+    return f ? f->overflow_dev : nullptr;
+}
+
 int limb_device_status(int clear)
 {
     DeviceFlags* f = flags_for_device();
