@@ -324,6 +324,22 @@ def test_moe_layer_small(M, mo, kmod, dev):
     kmod.device_status()
 
 
+@pytest.mark.parametrize("T", [1, 90])
+def test_experts_whose_second_product_takes_the_gate_apart(M, mo, kmod, dev, monkeypatch, T):
+    """the fused gate refused for a shape that it was expected to take: the same words through the gate by itself"""
+    a = small_args(M)
+    rng = np.random.default_rng(43)
+    moe = build_moe(M, a, moe_weights(rng, a, with_bias=False), dev)
+    x = t(np.rint(rng.standard_normal((1, T, a.dim)) * 2.0**23).astype(np.int64), dev)
+    want = moe(0, x)
+    fill = torch.full((1 << 24,), 2**62, dtype=torch.int64, device=dev)      # what unwritten memory may hold
+    del fill
+    monkeypatch.setattr(kmod, "glu_prepared", lambda *args, tile_group=None, real=kmod.glu_prepared, **kw: (
+        None if tile_group is not None else real(*args, **kw)))
+    assert torch.equal(moe(0, x), want)
+    kmod.device_status(sync=True)
+
+
 def test_optimistic_group_rows_are_checked_on_the_device(M, mo, kmod, dev):
     """72 tokens, 16 experts, top-4: 18 rows per expert on average, so the grouped GEMMs are launched with the
     optimistic 64-row bound (a bound is only certain up to 64 tokens).  Here every token names expert 0: 72 rows

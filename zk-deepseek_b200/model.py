@@ -893,14 +893,16 @@ class MoE(nn.Module):
             lambda out, pos: K.moe_combine(out, pos, weights.contiguous(), base))
         # nobody reads the tiles' padding rows between the three calls: neither written nor read (the dumps keep zeros)
         leave = not snark and I % 2 == 0 and K.limb_kernel_takes(I, lim, w2.limbs)
-        # the dispatch gather (model.py:1372-1378) runs inside the limb split of the first GEMM
-        if parts is not None:
-            r13 = K.grouped_gather_parts_prepared(parts[0], parts[1], row_src, w13, tile_group, 0, a_limbs=lim,
-                                                  dynamic=True, group_shift=s13, n_split=I, max_group_rows=few,
-                                                  leave_padding=leave)
-        else:
-            r13 = K.grouped_prepared(x.contiguous(), w13, tile_group, 0, a_limbs=lim, dynamic=True, group_shift=s13,
-                                     n_split=I, row_index=row_src, max_group_rows=few, leave_padding=leave)
+
+        def first(leave):
+            # the dispatch gather (model.py:1372-1378) runs inside the limb split of the first GEMM
+            if parts is not None:
+                return K.grouped_gather_parts_prepared(parts[0], parts[1], row_src, w13, tile_group, 0, a_limbs=lim,
+                                                       dynamic=True, group_shift=s13, n_split=I, max_group_rows=few,
+                                                       leave_padding=leave)
+            return K.grouped_prepared(x.contiguous(), w13, tile_group, 0, a_limbs=lim, dynamic=True, group_shift=s13,
+                                      n_split=I, row_index=row_src, max_group_rows=few, leave_padding=leave)
+        r13 = first(leave)
         if snark:
             h, sl = K.glu_q23(r13[:, :I], r13[:, I:], ld=2 * I, want_silu=True)
             self._dump_experts(start_pos, r13[:, :I], sl, counts)
@@ -910,7 +912,8 @@ class MoE(nn.Module):
                                  leave_padding=leave)
             if out is not None:
                 return finish(out, pos)
-            assert not leave
+            if leave:                                 # the gate by itself reads every row
+                r13 = first(False)
             h = K.glu_q23(r13[:, :I], r13[:, I:], ld=2 * I)
         out = K.grouped_prepared(h, w2, tile_group, 0, a_limbs=lim, dynamic=True, group_shift=s2, n_split=0,
                                  max_group_rows=few)
