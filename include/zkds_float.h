@@ -41,11 +41,12 @@ typedef struct {
     float* out2;           /* may be null: columns from `split` (a multiple of 32) on go here, in 32-bit, unrotated */
     long long ldo2;
     long long split;
-    int early;             /* 1: W has been complete since before the launch in front of this one on the stream, so that its
-                              first rows may be requested while that one still runs */
 } zkfp_linear_args;
 
 int zkfp_linear(const zkfp_linear_args* a, void* stream);
+/* The same for a W that has been complete since before the launch in front of this one on the stream: its first rows may be
+ * requested while that one still runs. */
+int zkfp_linear_early(const zkfp_linear_args* a, void* stream);
 
 /* x[r] = scale * table[tokens[r]] in 32-bit; xb (may be null) the same in bfloat16.  Ids outside [0, vocab) give zeros. */
 int zkfp_embed(const long long* tokens, const void* table, long long ld_table, long long vocab, float* x, void* xb,

@@ -1,9 +1,11 @@
 """The C-ABI library loads without a GPU and exports every symbol the header declares."""
 import ctypes
+import importlib
 import os
 import re
+import subprocess
 
-from conftest import ROOT
+from conftest import PKG, ROOT
 
 REFERENCE_SYMBOLS = [
     "int64_32_bmm_broadcast_launcher", "int64_64_bmm_broadcast_launcher", "bf16_to_int32_2d",
@@ -42,6 +44,16 @@ def test_float_library_exports_every_declared_symbol(float_libpath):
     missing = [n for n in names if not hasattr(lib, n)]
     assert not missing, missing
     assert sorted(os.listdir(os.path.join(ROOT, "include"))) == ["zkds_float.h", "zkds_int64.h"]
+
+
+def test_argument_structures_keep_their_size(float_libpath, tmp_path):
+    """a caller built against the header of an earlier library passes structures of this size; the ctypes ones match the header"""
+    fk = importlib.import_module(PKG + ".float_kernel")
+    src = tmp_path / "sizes.c"
+    src.write_text('#include <stdio.h>\n#include "zkds_float.h"\nint main(void) { printf("%zu", sizeof(zkfp_linear_args)); return 0; }\n')
+    subprocess.run(["gcc", "-I", os.path.join(ROOT, "include"), str(src), "-o", str(tmp_path / "sizes")], check=True)
+    size = int(subprocess.run([str(tmp_path / "sizes")], check=True, capture_output=True, text=True).stdout)
+    assert size == ctypes.sizeof(fk.LinearArgs) == 184
 
 
 def test_host_only_entry_points(libpath, orc):

@@ -112,6 +112,30 @@ def test_linear_of_few_bfloat16_rows(K, M, N, Kd):
     test_linear_and_its_epilogues(K, "bfloat16", M, N, Kd)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,N,Kd", [(1, 640, 328), (1, 24, 8), (2, 2120, 4104), (3, 16, 136), (8, 1000, 520), (9, 2120, 264), (16, 40, 7168),
+                                    (17, 72, 1032), (32, 9000, 136)])
+def test_weights_requested_before_the_wait_change_nothing(K, dtype, M, N, Kd):
+    """a recorded linear layer directly behind the kernel that makes its input: ragged tiles, warps without rows, empty shares
+    of K; its input changes from run to run, and the results are those of the layer by itself"""
+    x, w, W = rnd((M, Kd), "float32"), rnd((Kd,), "float32", 1), rnd((N, Kd), dtype, 2, Kd ** -0.5)
+    A, out, want = (torch.empty(s, dtype=d, device="cuda") for s, d in (((M, Kd), W.dtype), ((M, N), torch.float32), ((M, N), torch.float32)))
+    with K.Recording() as calls:
+        K.norm_rows(x, None, w, A, Kd, 1e-6)
+        K.linear(A, W, out)
+    got, wanted = [], []
+    for i in range(6):
+        x.copy_(rnd((M, Kd), "float32", 10 + i))
+        calls.replay()
+        calls.replay()
+        got.append(out.clone())
+        K.linear(A, W, want)
+        wanted.append(want.clone())
+    for a, b in zip(got, wanted):
+        assert torch.equal(a, b)
+    assert not torch.equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("kind", ["normal", "biased", "outliers"])
 @pytest.mark.parametrize("N,Kd", [(512, 7168), (2048, 2048), (2048, 4096), (4096, 512), (2120, 264)])
 def test_few_bfloat16_rows_are_as_exact_as_many(K, N, Kd, kind):
@@ -524,6 +548,40 @@ def test_a_step_must_follow_what_the_slot_holds(models):
     model.end_batch(slots)
     with pytest.raises(RuntimeError):
         model.begin_batch(5)
+
+
+def test_weights_changed_between_recorded_steps(models):
+    """in place and without a wait of the host: the next step has them, although its layers request weights early"""
+    cfg, W, model = models("WIDE", "bfloat16")
+    toks, layer = tokens_of(cfg, 12, 81), model.layers[-1]
+    weights = [t for t in layer.state_dict().values() if t is not None and t.dim() == 2 and t.dtype == torch.bfloat16] + [model.head]
+    old = [t.clone() for t in weights]
+    new = [t.flip(0) for t in old]
+
+    def logits(wait):
+        for t, v in zip(weights, old):               # both passes read the prompt with the same weights
+            t.copy_(v)
+        slots, out = model.begin_batch(1), []
+        out.append(model.step(torch.tensor([toks[:2]]), 0, slots)[0])
+        keep = None if wait else busy()
+        for i in range(2, 12):
+            if wait:
+                torch.cuda.synchronize()
+            for t, v in zip(weights, new if i % 2 else old):
+                t.copy_(v)
+            if wait:
+                torch.cuda.synchronize()
+            out.append(model.step(torch.tensor([toks[i:i + 1]]), i, slots)[0])
+        model.end_batch(slots)
+        del keep
+        return torch.cat(out).cpu()
+    try:
+        want, got = logits(True), logits(False)
+    finally:
+        for t, v in zip(weights, old):
+            t.copy_(v)
+    assert len(weights) > 2 and torch.equal(got, want)
+    assert not torch.equal(want, torch.from_numpy(run(model, toks, [2] + [1] * 10)[1:]))
 
 
 def busy():

@@ -101,7 +101,7 @@ int zkfp_linear_path(const zkfp_linear_args* a)
     return a->dtype == ZKFP_BF16 ? 1 : 0;
 }
 
-int zkfp_linear(const zkfp_linear_args* a, void* stream)
+static int linear(const zkfp_linear_args* a, bool early, void* stream)
 {
     if (!linear_ok(a)) return ZKDS_ERR_ARG;
     if (a->M == 0) return ZKDS_OK;
@@ -114,12 +114,15 @@ int zkfp_linear(const zkfp_linear_args* a, void* stream)
     e.bias = a->bias; e.out2 = a->out2; e.ldo2 = a->ldo2; e.split = a->out2 ? a->split : a->N;
     cudaStream_t st = (cudaStream_t)stream;
     switch (zkfp_linear_path(a)) {
-    case 3: return launch_linear_skinny(*a, e, st);
-    case 2: return launch_linear_stream(*a, e, st);
+    case 3: return launch_linear_skinny(*a, e, early, st);
+    case 2: return launch_linear_stream(*a, e, early, st);
     case 1: return launch_linear_tc(*a, e, st);
     default: return launch_linear_f32(*a, e, st);
     }
 }
+
+int zkfp_linear(const zkfp_linear_args* a, void* stream) { return linear(a, false, stream); }
+int zkfp_linear_early(const zkfp_linear_args* a, void* stream) { return linear(a, true, stream); }
 
 int zkfp_attention_path(const zkfp_attention_args* a)
 {

@@ -343,7 +343,7 @@ linear_skinny_kernel(const bf16* A, long long lda, const bf16* W, long long ldw,
 }
 
 template <typename T>
-int linear_stream(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
+int linear_stream(const zkfp_linear_args& a, const LinEpi& e, bool early, cudaStream_t st)
 {
     int ksplit = 1;
     while (ksplit < 8 && (long long)ksplit * 512 < a.K) ksplit *= 2;
@@ -353,9 +353,9 @@ int linear_stream(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
     const unsigned gx = (unsigned)((a.N / 8 + groups - 1) / groups);
     const T *A = (const T*)a.A, *W = (const T*)a.W;
     const int M = (int)a.M, N = (int)a.N, K = (int)a.K;
-    if (M == 1) fp_launch(linear_stream_kernel<T, 1>, dim3(gx, 1), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
-    else if (M == 2) fp_launch(linear_stream_kernel<T, 2>, dim3(gx, 1), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
-    else fp_launch(linear_stream_kernel<T, 4>, dim3(gx, (M + 3) / 4), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
+    if (M == 1) fp_launch(linear_stream_kernel<T, 1>, dim3(gx, 1), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, early, e);
+    else if (M == 2) fp_launch(linear_stream_kernel<T, 2>, dim3(gx, 1), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, early, e);
+    else fp_launch(linear_stream_kernel<T, 4>, dim3(gx, (M + 3) / 4), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, early, e);
     return fp_launched();
 }
 
@@ -370,7 +370,7 @@ bool linear_skinny_takes(const zkfp_linear_args& a)
     return a.M <= 8 || (a.M <= 16 && weights <= 140000000) || (a.M <= kSkinnyRows && weights <= 20000000);
 }
 
-int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
+int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, bool early, cudaStream_t st)
 {
     // warps on the same rows until every SM has a block.  More of them leave a last wave that is nearly empty and cost
     // more reductions (16384 x 2048, 4 rows: 2 shares 15.5 us, 4: 17.5, 8: 20.5), fewer leave SMs idle (4096 x 4096:
@@ -382,9 +382,9 @@ int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, cudaStream_
     const unsigned grid = (unsigned)((tiles + groups - 1) / groups);
     const bf16 *A = (const bf16*)a.A, *W = (const bf16*)a.W;
     const int M = (int)a.M, N = (int)a.N, K = (int)a.K;
-    if (M <= 8) fp_launch(linear_skinny_kernel<1>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
-    else if (M <= 16) fp_launch(linear_skinny_kernel<2>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
-    else if (M <= kSkinnyRows) fp_launch(linear_skinny_kernel<4>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, a.early, e);
+    if (M <= 8) fp_launch(linear_skinny_kernel<1>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, early, e);
+    else if (M <= 16) fp_launch(linear_skinny_kernel<2>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, early, e);
+    else if (M <= kSkinnyRows) fp_launch(linear_skinny_kernel<4>, dim3(grid), dim3(256), 0, st, A, a.lda, W, a.ldw, M, N, K, ksplit, early, e);
     else return ZKDS_ERR_UNSUPPORTED;
     return fp_launched();
 }
@@ -425,9 +425,9 @@ int launch_linear_f32(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t s
     return fp_launched();
 }
 
-int launch_linear_stream(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
+int launch_linear_stream(const zkfp_linear_args& a, const LinEpi& e, bool early, cudaStream_t st)
 {
-    return a.dtype == ZKFP_BF16 ? linear_stream<bf16>(a, e, st) : linear_stream<float>(a, e, st);
+    return a.dtype == ZKFP_BF16 ? linear_stream<bf16>(a, e, early, st) : linear_stream<float>(a, e, early, st);
 }
 
 }  // namespace zkds

@@ -29,7 +29,7 @@ class LinearArgs(ctypes.Structure):
     _fields_ = [("A", _vp), ("W", _vp), ("out", _vp), ("aux", _vp), ("table", _vp), ("start", _vp),
                 ("lda", _ll), ("ldw", _ll), ("ldo", _ll), ("ldaux", _ll), ("M", _ll), ("N", _ll), ("K", _ll),
                 ("seq", _ll), ("positions", _ll), ("dtype", _i), ("out_dtype", _i), ("epilogue", _i), ("pairs", _i), ("period", _i),
-                ("offset", _i), ("rot_begin", _i), ("rot_end", _i), ("bias", _vp), ("out2", _vp), ("ldo2", _ll), ("split", _ll), ("early", _i)]
+                ("offset", _i), ("rot_begin", _i), ("rot_end", _i), ("bias", _vp), ("out2", _vp), ("ldo2", _ll), ("split", _ll)]
 
 
 class LatentArgs(ctypes.Structure):
@@ -93,7 +93,7 @@ def _sig(name, argtypes, restype=_i):
     return fn
 
 
-_linear = _sig("zkfp_linear", [ctypes.POINTER(LinearArgs), _vp])
+_linear, _linear_early = (_sig(name, [ctypes.POINTER(LinearArgs), _vp]) for name in ("zkfp_linear", "zkfp_linear_early"))
 _latent = _sig("zkfp_latent_post", [ctypes.POINTER(LatentArgs), _vp])
 _perhead = _sig("zkfp_perhead", [ctypes.POINTER(PerHeadArgs), _vp])
 _attention = _sig("zkfp_attention", [ctypes.POINTER(AttentionArgs), _vp])
@@ -210,9 +210,9 @@ def linear(A, W, out, epilogue=STORE, aux=None, table=None, start=None, seq=1, p
                    W.stride(0), out.stride(0), aux.stride(0) if aux is not None else 0, A.shape[0], W.shape[0],
                    W.shape[1], seq, table.shape[0] if table is not None else 0, code(A.dtype), code(out.dtype),
                    epilogue, pairs, period, offset, rotated[0], rotated[1], ptr(bias), ptr(out2),
-                   out2.stride(0) if out2 is not None else 0, W.shape[0] - out2.shape[1] if out2 is not None else 0,
-                   Recording.active is not None)      # a recorded step starts with copies: weights are older than those
-    _call(_linear, (ctypes.byref(a),), "linear", A, W, out, aux, table, start, bias, out2)
+                   out2.stride(0) if out2 is not None else 0, W.shape[0] - out2.shape[1] if out2 is not None else 0)
+    # a recorded step starts with copies: weights are older than those
+    _call(_linear_early if Recording.active is not None else _linear, (ctypes.byref(a),), "linear", A, W, out, aux, table, start, bias, out2)
     return out
 
 
