@@ -747,8 +747,8 @@ class RecordedStep:
         self.tokens = torch.zeros(B, 1, dtype=torch.int64, device=dev)
         self.meta = torch.zeros(2, B, dtype=torch.int32, device=dev)
         # several buffers for the inputs, so that the host may prepare steps while earlier ones still run
-        self.host = [torch.zeros(2, B, dtype=torch.int32).pin_memory() for _ in range(STEPS_AHEAD)]
-        self.host_tokens = [torch.zeros(B, 1, dtype=torch.int64).pin_memory() for _ in range(STEPS_AHEAD)]
+        self.host = torch.zeros(STEPS_AHEAD, 2, B, dtype=torch.int32).pin_memory()
+        self.host_tokens = torch.zeros(STEPS_AHEAD, B, 1, dtype=torch.int64).pin_memory()
         self.rows = torch.arange(B, dtype=torch.int32, device=dev)
         self.copied, self.turn = [torch.cuda.Event() for _ in range(STEPS_AHEAD)], 0
 
