@@ -1,10 +1,13 @@
 """Kernels that may start before the kernel in front of them has ended (float_common.cuh, chain_enter): nothing in their source
 may promise that their operands stay as they are while they run, nor read or write before the wait what another kernel touches."""
 import glob
+import importlib
 import os
 import re
+import threading
 
 import pytest
+import torch
 
 from conftest import PKG, ROOT
 
@@ -51,3 +54,21 @@ def test_no_load_of_the_chain_goes_through_the_non_coherent_path():
         text = _code(path)
         if "chain_enter()" in text:
             assert "ld.global.nc" not in text and "__ldg" not in text and "ld.global.constant" not in text, path
+
+
+def test_a_thread_records_its_own_calls_only(float_libpath, monkeypatch):
+    """another thread's layer is neither recorded nor told that its weights are old"""
+    K = importlib.import_module(PKG + ".float_kernel")
+    seen = []
+    monkeypatch.setattr(K, "_stream", lambda: 0)
+    monkeypatch.setattr(K, "_linear", lambda *args: seen.append("plain") or 0)
+    monkeypatch.setattr(K, "_linear_early", lambda *args: seen.append("early") or 0)
+    A, W, out = torch.zeros(3, 8), torch.zeros(16, 8), torch.zeros(3, 16)
+    with K.Recording() as calls:
+        other = threading.Thread(target=K.linear, args=(A, W, out))
+        other.start()
+        other.join()
+        assert seen == ["plain"] and not calls.calls and not calls.held
+        K.linear(A, W, out)
+    K.linear(A, W, out)
+    assert seen == ["plain", "early", "plain"] and len(calls.calls) == 1 and calls.held[0] is A

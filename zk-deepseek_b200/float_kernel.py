@@ -5,6 +5,7 @@ There is no CPU or PyTorch fallback: a missing library raises at import, a faile
 """
 import ctypes
 import os
+import threading
 
 import torch
 
@@ -142,19 +143,25 @@ def device_status(sync=False):
 
 class Recording:
     """Calls made while recording, with their argument structures and the tensors they point to, to be issued again
-    without rebuilding anything: the host side of a one-token step is a loop over prepared calls."""
+    without rebuilding anything: the host side of a one-token step is a loop over prepared calls.  A thread records its
+    own calls only."""
 
-    active = None
+    _thread = threading.local()
 
     def __init__(self):
         self.calls, self.held = [], []
 
+    @classmethod
+    def current(cls):
+        """what this thread is recording, or None"""
+        return getattr(cls._thread, "active", None)
+
     def __enter__(self):
-        Recording.active = self
+        Recording._thread.active = self
         return self
 
     def __exit__(self, *exc):
-        Recording.active = None
+        Recording._thread.active = None
         return False
 
     def replay(self):
@@ -167,9 +174,10 @@ class Recording:
 
 def _call(fn, args, what, *tensors):
     _check(fn(*args, _stream()), what)
-    if Recording.active is not None:
-        Recording.active.calls.append((fn, args, what))
-        Recording.active.held.extend(tensors)
+    recording = Recording.current()
+    if recording is not None:
+        recording.calls.append((fn, args, what))
+        recording.held.extend(tensors)
 
 
 def code(dtype):
@@ -212,7 +220,7 @@ def linear(A, W, out, epilogue=STORE, aux=None, table=None, start=None, seq=1, p
                    epilogue, pairs, period, offset, rotated[0], rotated[1], ptr(bias), ptr(out2),
                    out2.stride(0) if out2 is not None else 0, W.shape[0] - out2.shape[1] if out2 is not None else 0)
     # a recorded step starts with copies: weights are older than those
-    _call(_linear_early if Recording.active is not None else _linear, (ctypes.byref(a),), "linear", A, W, out, aux, table, start, bias, out2)
+    _call(_linear_early if Recording.current() is not None else _linear, (ctypes.byref(a),), "linear", A, W, out, aux, table, start, bias, out2)
     return out
 
 
