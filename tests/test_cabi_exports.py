@@ -73,6 +73,20 @@ def test_host_only_entry_points(libpath, orc):
     assert lib.zkds_last_status() == 0
 
 
+def test_stream_handle_without_torch_s_private_call(kmod, float_libpath, monkeypatch):
+    import torch
+
+    class Stream:
+        cuda_stream = 77
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: Stream)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    for module in (kmod, importlib.import_module(PKG + ".float_kernel")):
+        monkeypatch.setattr(module, "_raw_stream", None)
+        assert module._stream() == 77
+        monkeypatch.setattr(module, "_raw_stream", lambda device: 78 + device)
+        assert module._stream() == 78
+
+
 def test_kernel_module_surface(kmod):
     """Every name the reference's model.py / generate.py import from `kernel` exists."""
     for name in ("act_quant", "weight_dequant", "fp8_gemm", "int64_bmm_broadcast",

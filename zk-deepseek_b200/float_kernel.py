@@ -130,8 +130,14 @@ def _check(status, what):
         raise FloatOpsError("%s: %s" % (what, text), status)
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # the handle alone where this torch gives it (no public call does without a Stream object)
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def device_status(sync=False):

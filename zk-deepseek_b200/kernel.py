@@ -142,9 +142,15 @@ def _check(status, what):
         raise ZkdsError("%s: %s" % (what, msg), status)
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    # the handle alone: a Stream object for every call costs more than the call's other arguments together
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # the handle alone where this torch gives it (no public call does): a Stream object for every call costs more than the
+    # call's other arguments together
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 class _NoSwitch:
