@@ -813,6 +813,42 @@ def test_measured_ranges_of_rows_with_gaps(kmod, dev, rows, K, pitch):
     assert torch.equal(C, want)
 
 
+@pytest.mark.parametrize("M,H,N,K,wbits", [(33, 2, 130, 264, 15), (64, 3, 40, 520, 30), (48, 1, 2048, 2064, 15), (63, 16, 128, 512, 15), (34, 5, 16, 16, 30),
+                                           (64, 1, 1000, 4100, 30)])
+def test_boxes_of_32_among_33_to_64_rows(kmod, dev, M, H, N, K, wbits):
+    """two boxes for the rows of a batch, the second one ragged, with and without a split, beside the rows of the next batch; the
+    same words as tiles of 128 rows, which 65 rows take"""
+    g_ = torch.Generator(device=dev).manual_seed(M * N)
+    A = torch.randint(-2**20, 2**20, (1, 130, H, K), device=dev, generator=g_)
+    W = torch.randint(-2**wbits, 2**wbits, (H, N, K), device=dev, generator=g_, dtype=torch.int32)
+    planes = kmod.WeightPlanes(W)
+    want = kmod.einsum_heads_prepared(A, planes, 9, True, a_limbs=3, dynamic=True)
+    got = kmod.einsum_heads_prepared(A[:, :M].contiguous(), planes, 9, True, a_limbs=3, dynamic=True)
+    assert torch.equal(got, want[:, :M])
+    kmod.device_status(sync=True)
+
+
+def test_clusters_beyond_those_that_the_gpu_holds_do_not_double_the_time(kmod, dev):
+    """64 rows by 2048 columns are sixteen tiles of columns, of whose clusters of eight the GPU holds fifteen: as a second round
+    they took 1.6 times what 1536 columns take (the weights: 1.33 times)"""
+    x = torch.randint(-2**20, 2**20, (1, 64, 7168), device=dev)
+
+    def fastest(N):
+        planes = kmod.WeightPlanes(torch.randint(-2**14, 2**14, (N, 7168), dtype=torch.int32, device=dev))
+        best = 1e9
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            for _ in range(10):
+                kmod.linear_prepared(x, planes, 16, a_limbs=3, dynamic=True)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+    assert fastest(2048) < 1.4 * fastest(1536)
+
+
 def test_more_batches_than_can_be_measured_are_refused(kmod, dev):
     """whatever the order of the operands: 65535 are taken, one more is not"""
     A = torch.ones(1, 1, 65536, 2, dtype=torch.int64, device=dev)

@@ -23,6 +23,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "tcgen05.cuh"
@@ -1141,7 +1143,8 @@ __device__ __forceinline__ void rows_store(const LimbParams& p, i128w sum, int s
     }
 }
 
-// p.NT = R rows of activations (tmA's box); tmW's box holds 128 weight rows.  grid (n_tiles * ksplit, row tiles, batches)
+// p.NT = R rows of activations (tmA's box); tmW's box holds 128 weight rows.  grid (n_tiles * ksplit, row tiles, batches); the
+// row tiles of a grouped call are 128 rows apart, others R
 __global__ void __launch_bounds__(kRowsThreads, 2)
 limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const LimbParams p,
                  const uint32_t pipe_bytes)
@@ -1153,7 +1156,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int share = blockIdx.x % p.ksplit, R = p.NT;
-    const int64_t n0 = (int64_t)(blockIdx.x / p.ksplit) * kTileM, z = blockIdx.z, m0 = (int64_t)blockIdx.y * kTileM;
+    const int64_t n0 = (int64_t)(blockIdx.x / p.ksplit) * kTileM, z = blockIdx.z, m0 = (int64_t)blockIdx.y * (p.tile_group ? kTileM : R);
     const int group = p.tile_group ? p.tile_group[blockIdx.y] : 0;
     if (group < 0) {              // unused row tile, the same for the whole cluster: zeros, as limb_gemm_kernel leaves them
         if (p.leave_padding) return;
@@ -1202,7 +1205,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     volatile int* abort_flag = &s_abort;
     // the sums of a split tile: [row][128 columns], one word or (a second plane behind it) two
     uint64_t* red = reinterpret_cast<uint64_t*>(smem_raw + (smem_base - smem_u32(smem_raw)));
-    const int rows = p.tile_group ? R : (int)p.M;
+    const int rows = p.tile_group ? R : (int)(p.M - m0 < R ? p.M - m0 : R);
 
     if (warp == 0) {
         if (lane == 0 && some) {
@@ -2436,6 +2439,33 @@ static int record_launch(const Contraction& p, int La, int Lb, const unsigned lo
     return ZKDS_OK;
 }
 
+// clusters of so many CTAs of limb_rows_kernel that the current device holds at a time with one CTA to an SM
+static int rows_clusters(int size, size_t smem)
+{
+    static std::atomic<int> known[64][4];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / size;
+    std::atomic<int>& held = known[dev][size == 1 ? 0 : size == 2 ? 1 : size == 4 ? 2 : 3];
+    int n = held.load(std::memory_order_relaxed);
+    if (n) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(size * sm_count()));
+    cfg.blockDim = dim3(kRowsThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, limb_rows_kernel, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = sm_count() / size;
+    }
+    held.store(n, std::memory_order_relaxed);
+    return n;
+}
+
 int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* pre_b, cudaStream_t st)
 {
     if (pre_b) Lb = pre_b->L;
@@ -2579,28 +2609,44 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     }
 
     if (by_rows) {
-        const int64_t all = rows_tiles * p.batches * (p.tile_group ? mt : 1);
+        rc = allow_big_smem(limb_rows_kernel, g_attr_rows);
+        if (rc != ZKDS_OK) return rc;
         const int fits64 = sum_fits64(La, Lb, p.K, p.addend);
-        // shares of K: the fewest K blocks that an SM works through, four more for each CTA's start and end.  Row tiles
-        // of experts are mostly unused, so their number says nothing: no split there
-        int ks = 1;
-        int64_t best = 0;
-        for (int c = 1; c <= (p.tile_group ? 1 : 8); c *= 2) {
-            if (c > 1 && (kb < 2 * c || (size_t)(fits64 ? 1 : 2) * p.M * kTileM * 8 > 2 * rows_stage)) break;
-            const int64_t cost = (all * c + sm_count() - 1) / sm_count() * ((kb + c - 1) / c + 4);
-            if (c == 1 || cost < best) { best = cost; ks = c; }
+        const int64_t column_tiles = rows_tiles * p.batches;
+        // Boxes of few_rows rows, or of 32 where that gives two, and shares of K, by the K blocks that an SM works through:
+        // a CTA's start and end take as long as one block and one more for eight rows, and as much again for the sums of a
+        // split.  Beyond the clusters that the GPU holds at a time (of eight CTAs no more than 15, not 18) there is another
+        // round, or two CTAs to an SM where they fit, of which one starts or finishes while the other streams.
+        // 64 rows, against 64-row boxes and rounds counted in SMs: 2048 x 7168 44 -> 30 us (four limbs 64 -> 40), 24576 x 1536
+        // 69 -> 44, 4096 x 512 of four limbs 33 -> 24; the tiles of limb_gemm_kernel take 38, 51, 59 and 28.
+        // Row tiles of experts are mostly unused, so their number says nothing: one box and no split there.
+        int ks = 1, box = few_rows;
+        bool pair = false;
+        double best = 0.0;
+        for (int r = few_rows; r >= (p.tile_group || few_rows <= 32 ? few_rows : 32); r -= 32) {
+            const size_t r_stage = (size_t)Lb * kTileM * kBlockK + (size_t)La * r * kBlockK;
+            const int64_t tiles = column_tiles * (p.tile_group ? mt : (p.M + r - 1) / r), rows = p.tile_group || p.M > r ? r : p.M;
+            for (int c = 1; c <= (p.tile_group ? 1 : 8); c *= 2) {
+                if (c > 1 && (kb < 2 * c || (size_t)(fits64 ? 1 : 2) * rows * kTileM * 8 > 2 * r_stage)) break;
+                const int held = rows_clusters(c, smem_max + 1024);
+                const bool two = tiles > held && (kb < 2 * c ? 1 : 2) * r_stage <= 111 * 1024;
+                const double share = (double)((kb + c - 1) / c), ends = (1.0 + rows / 8.0) * (c > 1 ? 2 : 1);
+                const double load = (double)tiles / held;
+                const double cost = tiles <= held ? share + ends
+                                    : two ? load * share + (double)((tiles + 2 * held - 1) / (2 * held)) * ends
+                                          : (double)((tiles + held - 1) / held) * (share + ends);
+                if (best == 0.0 || cost < best) { best = cost; ks = c; box = r; pair = two; }
+            }
         }
-        // two CTAs to an SM where there is more than one for it: one starts or finishes while the other streams
-        const bool pair = all * ks > sm_count() && (kb < 2 * ks ? 1 : 2) * rows_stage <= 111 * 1024;
         const size_t pipe = pair ? 111 * 1024 : smem_max;
         CUtensorMap mapA, mapW;
         const int64_t pitch = (pre_b && pre_b->pitch) ? pre_b->pitch : Kp;
         if (pitch < Kp || (pitch & 15)) return ZKDS_ERR_ARG;
-        if (!make_plane_map(&mapA, pa, (int64_t)La * a_rows, Kp, few_rows) ||
+        if (!make_plane_map(&mapA, pa, (int64_t)La * a_rows, Kp, box) ||
             !make_plane_map(&mapW, pb, (int64_t)Lb * b_rows, Kp, kTileM, pitch))
             return ZKDS_ERR_UNSUPPORTED;
         LimbParams lp{};
-        lp.La = La; lp.Lb = Lb; lp.NT = few_rows; lp.kblocks = (int)kb;
+        lp.La = La; lp.Lb = Lb; lp.NT = box; lp.kblocks = (int)kb;
         lp.ksplit = ks; lp.kb_per_split = (int)((kb + ks - 1) / ks);
         lp.M = p.M; lp.N = p.N; lp.batches = p.batches;
         lp.a_rows_per_limb = a_rows; lp.b_rows_per_limb = b_rows; lp.b_batch_rows = p.N;
@@ -2611,10 +2657,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         lp.a_absmax = d_absmax; lp.overflow_flag = fl->overflow_dev;
         lp.tile_group = p.tile_group; lp.group_shift = p.group_shift; lp.n_split = p.n_split;
         lp.leave_padding = p.tile_group ? p.leave_padding : 0;
-        rc = allow_big_smem(limb_rows_kernel, g_attr_rows);
-        if (rc != ZKDS_OK) return rc;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(rows_tiles * ks), (unsigned)(p.tile_group ? mt : 1), (unsigned)p.batches);
+        cfg.gridDim = dim3((unsigned)(rows_tiles * ks), (unsigned)(p.tile_group ? mt : (p.M + box - 1) / box), (unsigned)p.batches);
         cfg.blockDim = dim3(kRowsThreads);
         cfg.dynamicSmemBytes = pipe + 1024;
         cfg.stream = st;
@@ -2629,7 +2673,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         rc = set_cuda_error(cudaLaunchKernelEx(&cfg, limb_rows_kernel, mapA, mapW, lp, (uint32_t)pipe));
         if (rc == ZKDS_OK) rc = check_launch();
         if (ev) ZKDS_CUDA(cudaEventRecord(ev[1], st));
-        if (ev && rc == ZKDS_OK) return record_launch(p, La, Lb, d_absmax, ev, few_rows);
+        if (ev && rc == ZKDS_OK) return record_launch(p, La, Lb, d_absmax, ev, box);
         return rc;
     }
 
