@@ -172,6 +172,15 @@ def test_linear_takes_the_kernel_meant_for_the_shape(K):
     assert path(1, K.BF16) == 2 and path(1, K.F32) == 2 and path(100, K.BF16) == 1 and path(100, K.F32) == 0
 
 
+@pytest.mark.parametrize("M,N,Kd,want", [(16, 65536, 256, 3), (17, 16384, 512, 3), (32, 8192, 2048, 3), (32, 4096, 4096, 3), (17, 12288, 1024, 1),
+                                         (32, 65536, 256, 1), (32, 32768, 512, 1), (32, 10304, 2048, 1), (33, 64, 64, 1)])
+def test_few_rows_take_the_faster_kernel(K, M, N, Kd, want):
+    """the sides of the line as they were measured"""
+    a = K.LinearArgs()
+    a.M, a.N, a.K, a.dtype = M, N, Kd, K.BF16
+    assert K.linear_path(ctypes.byref(a)) == want
+
+
 @pytest.mark.parametrize("width", [52, 328, 9000])
 def test_norms_and_embedding(K, width):
     pitch = K.pad8(width)

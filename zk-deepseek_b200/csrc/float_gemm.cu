@@ -365,9 +365,12 @@ bool linear_skinny_takes(const zkfp_linear_args& a)
 {
     // Up to eight rows always.  Beyond, every eight rows cost a product and a load of A per sixteen bytes of weights, and
     // the tcgen05 tiles win once the weights are large enough to hide their start and split sums (16 rows: 7168 x 18432
-    // 60 against 65 us, 36864 x 7168 104 against 96; 32 rows: 2048 x 8192 20 against 30, 10304 x 2048 26 against 19).
+    // 60 against 65 us, 36864 x 7168 104 against 96; 32 rows: 2048 x 8192 20 against 30, 10304 x 2048 26 against 19).  Beyond
+    // 8192 columns the tiles fill the SMs without a split and win sooner (32 rows: 16384 x 512 13.3 against 13.5, 12288 x 1024
+    // 18.7 against 15.6, 65536 x 256 28.2 against 23.8).
     const long long weights = a.N * a.K;
-    return a.M <= 8 || (a.M <= 16 && weights <= 140000000) || (a.M <= kSkinnyRows && weights <= 20000000);
+    return a.M <= 8 || (a.M <= 16 && weights <= 140000000) ||
+           (a.M <= kSkinnyRows && weights <= (a.N <= 8192 ? 20000000 : 10000000));
 }
 
 int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, bool early, cudaStream_t st)
