@@ -164,6 +164,12 @@ def test_linear_of_float32_tiles(K, M, N, Kd):
     test_linear_and_its_epilogues(K, "float32", M, N, Kd)
 
 
+@pytest.mark.parametrize("M,N,Kd", [(33, 2048, 16), (1000, 136, 128), (64, 16, 112), (300, 520, 8)])
+def test_linear_of_shallow_float32_tiles(K, M, N, Kd):
+    """tiles of 32 rows for a K that is not shared"""
+    test_linear_and_its_epilogues(K, "float32", M, N, Kd)
+
+
 def test_linear_takes_the_kernel_meant_for_the_shape(K):
     def path(M, dtype):
         a = K.LinearArgs()

@@ -394,8 +394,11 @@ int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, bool early,
 
 int launch_linear_f32(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st)
 {
-    // 32-row tiles for the rows that would leave half of a 64-row tile empty, while there are few tiles of rows
-    const bool small = a.M <= 32 || (a.M > 64 && a.M <= 96);
+    // 32-row tiles for the rows that would leave half of a 64-row tile empty, while there are few tiles of rows, and for a K
+    // that is too shallow to be shared, where a CTA's start and end are the time (64 x 2048, K = 16: 4.9 us, in
+    // 64-row tiles 6.9)
+    const bool small = a.M <= 32 || (a.M > 64 && a.M <= 96) ||
+                       (a.K <= 128 && (a.M + 63) / 64 * ((a.N + kFN - 1) / kFN) <= fp_sm_count());
     const long long bm = small ? 32 : 64, kb = (a.K + kFK - 1) / kFK;
     const long long tiles = (a.M + bm - 1) / bm * ((a.N + kFN - 1) / kFN);
     // shares of K: the fewest blocks of K that an SM works through one after the other, with 6 more for a CTA's start and
