@@ -752,7 +752,7 @@ def test_more_pairs_than_promised_are_reported(kmod, dev, T, k, E, n_tiles):
     assert (pos.cpu().numpy() == np.where(full[1] < n_tiles * 128, full[1], -1)).all()
 
 
-@pytest.mark.parametrize("slots,cols", [(1, 2), (3, 514), (8, 7168), (9, 1030)])
+@pytest.mark.parametrize("slots,cols", [(1, 2), (2, 514), (3, 514), (8, 7168), (9, 1030)])
 def test_combine_over_column_parts(kmod, dev, slots, cols):
     rng = np.random.default_rng(slots)
     out, w = rng.integers(-2**40, 2**40, (20, cols)), rng.integers(0, 2**22, (5, slots))

@@ -1259,6 +1259,8 @@ int launch_gather_rows(const int64_t* src, const int* index, int64_t* dst, int64
 // wrapping int64 product, floor division by 2^23, order-free integer sum); pos < 0 skips a slot
 // One block per token and 256 column pairs, four slots' rows in flight: bound by the bytes of the rows.  One token x 8 slots
 // x 7168 columns 55 -> 5 us (it was one block walking the columns, a chain of two loads per slot), 1001 tokens 99 -> 94 us.
+// One or two slots take as many at a time (STEP): 1001 tokens x 7168 columns of one slot 31 us four at a time, 23 us one.
+template <int STEP>
 __global__ void __launch_bounds__(kThreads)
 moe_combine_kernel(const longlong2* __restrict__ out, const int* __restrict__ pos,
                    const int64_t* __restrict__ w, const longlong2* __restrict__ base,
@@ -1267,17 +1269,17 @@ moe_combine_kernel(const longlong2* __restrict__ out, const int* __restrict__ po
     const int64_t t = blockIdx.x;
     for (int64_t c = (int64_t)blockIdx.y * kThreads + threadIdx.x; c < cols2; c += (int64_t)gridDim.y * kThreads) {
         longlong2 acc = base ? base[t * cols2 + c] : make_longlong2(0, 0);
-        for (int s0 = 0; s0 < slots; s0 += 4) {
-            longlong2 v[4];
-            int64_t ws[4];
+        for (int s0 = 0; s0 < slots; s0 += STEP) {
+            longlong2 v[STEP];
+            int64_t ws[STEP];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < STEP; ++i) {
                 const int r = s0 + i < slots ? pos[t * slots + s0 + i] : -1;
                 ws[i] = r < 0 ? 0 : w[t * slots + s0 + i];
                 v[i] = r < 0 ? make_longlong2(0, 0) : out[(int64_t)r * cols2 + c];
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < STEP; ++i) {
                 acc.x = (int64_t)((uint64_t)acc.x + (uint64_t)((int64_t)((uint64_t)v[i].x * (uint64_t)ws[i]) >> 23));
                 acc.y = (int64_t)((uint64_t)acc.y + (uint64_t)((int64_t)((uint64_t)v[i].y * (uint64_t)ws[i]) >> 23));
             }
@@ -1294,7 +1296,8 @@ int launch_moe_combine(const int64_t* out, const int* pos, const int64_t* w, con
         ((((uintptr_t)out | (uintptr_t)base | (uintptr_t)y) & 15) != 0))
         return ZKDS_ERR_ARG;
     const int64_t parts = (cols / 2 + kThreads - 1) / kThreads;
-    moe_combine_kernel<<<dim3((unsigned)tokens, (unsigned)(parts < 65535 ? parts : 65535)), kThreads, 0, st>>>(
+    auto* kernel = slots == 1 ? moe_combine_kernel<1> : slots == 2 ? moe_combine_kernel<2> : moe_combine_kernel<4>;
+    kernel<<<dim3((unsigned)tokens, (unsigned)(parts < 65535 ? parts : 65535)), kThreads, 0, st>>>(
         reinterpret_cast<const longlong2*>(out), pos, w, reinterpret_cast<const longlong2*>(base),
         reinterpret_cast<longlong2*>(y), slots, cols / 2);
     return check_launch();
