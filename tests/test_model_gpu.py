@@ -196,6 +196,49 @@ def test_mla_prefill_of_any_length(M, mo, kmod, dev, S, limbs, skip):
     assert full.causal_skip is None and full._masked_weigh_nothing(3, 3) and not full._masked_weigh_nothing(4, 4)
 
 
+@pytest.mark.parametrize("S", [37, 64])
+@pytest.mark.parametrize("al,bl", [(3, 3), (4, 3), (3, 4)])
+def test_masked_half_left_out_by_the_rule(M, mo, kmod, dev, monkeypatch, S, al, bl):
+    """limbs for which the rule proves that no masked score can weigh anything, with operands at the ends of those limbs and
+    signs that make a masked score the largest of its row: the call skips, and gives the words of the full computation with
+    the same limbs and with measured ones"""
+    a = small_args(M, kv_lora_rank=128, n_heads=8)
+    rng = np.random.default_rng(S + 8 * al + bl)
+    attn = M.MLA(0, a).to(dev)
+    load_mla(attn, mla_weights(rng, a), dev)
+    assert attn.causal_skip is None and attn._masked_weigh_nothing(al, bl)
+    top = lambda limbs: 127 * (256 ** limbs - 1) // 255          # digits reach from -128 to 127: both signs end here
+    near = lambda limbs, *shape: top(limbs) - rng.integers(0, 1000, shape)
+    C, R, H = a.kv_lora_rank, a.qk_rope_head_dim, a.n_heads
+    signs_c, signs_r = rng.choice([-1, 1], C), rng.choice([-1, 1], R)
+    later = np.where(np.arange(S) % 2, 1, -1)[None, :, None]     # every other position as far up or down as scores go
+    # (the rotary part enters the common sum two bits up: its share of the limbs ends at a quarter)
+    q_abs, q_pe = t(near(al, 1, S, H, C) * signs_c, dev), t((near(al, 1, S, H, R) >> 2) * signs_r, dev)
+    kv, pe = t(near(bl, 1, S, C) * signs_c * later, dev), t(near(bl, 1, S, R) * signs_r * later, dev)
+    nope = torch.zeros(1, S, H, a.qk_nope_head_dim, dtype=torch.int64, device=dev)
+    monkeypatch.setattr(kmod, "einsum_heads_prepared", lambda *args, **kw: q_abs)
+    monkeypatch.setattr(kmod, "einsum_bshd_hdc_bshc", lambda *args, **kw: q_abs)
+    skipped, served, scores, softmax = [], [], kmod.mla_scores_fused, kmod.softmax_pv_fused
+    monkeypatch.setattr(kmod, "mla_scores_fused", lambda *args, skip_masked=False, **kw: (
+        skipped.append(skip_masked), scores(*args, skip_masked=skip_masked, **kw))[1])
+
+    def counted(*args, **kw):
+        out = softmax(*args, **kw)
+        served.append(out is not None)
+        return out
+    monkeypatch.setattr(kmod, "softmax_pv_fused", counted)
+
+    def core(limbs, skip):
+        attn.score_limbs, attn.causal_skip = limbs, skip
+        got = attn._core(nope, q_pe, kv, pe, 1, S, 0, t(mo.causal_mask(S), dev), None)
+        kmod.device_status(sync=True)
+        return got
+    got = core((al, bl), None)
+    assert skipped == [True] and served == [True]
+    assert torch.equal(got, core((al, bl), False)) and torch.equal(got, core((0, 0), None))
+    assert skipped == [True, False, False]
+
+
 def test_mla_decode_reads_resident_cache_planes(M, mo, kmod, dev):
     """Decode steps read the latent cache from resident limb planes (one new position split per step, score
     rows padded to four columns, the padding never read).  Against the oracle: a prefill, then single-token steps
@@ -729,6 +772,20 @@ def test_route_kernel(M, kmod, dev, T, k, first, E, bound):
         want_group[row // 128:row // 128 + tiles] = e
         row += tiles * 128
     assert (row_src == want_src).all() and (pos == want_pos).all() and (group == want_group).all()
+
+
+@pytest.mark.parametrize("T,k,first,E,bound", [(1, 8, 0, 32, None), (64, 8, 16, 16, 300), (1001, 8, 0, 64, None), (4099, 2, 3, 7, None)])
+def test_tensor_operations_route_like_the_kernel(M, kmod, dev, monkeypatch, T, k, first, E, bound):
+    """what serves more pairs than the kernel takes, at sizes that the kernel takes"""
+    class Layer:
+        n_local_experts, experts_start_idx = E, first
+    rng = np.random.default_rng(T)
+    idx = t(np.stack([rng.permutation(first + E + 5)[:k] for _ in range(T)]).astype(np.int64), dev)
+    want = M.MoE.route(Layer, idx, bound)
+    monkeypatch.setattr(kmod, "moe_route", lambda *args: None)
+    got = M.MoE.route(Layer, idx, bound)
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and torch.equal(a, b)
 
 
 @pytest.mark.parametrize("T,k,E,n_tiles", [(300, 4, 8, 5), (40, 8, 16, 1), (3, 2, 4, 0), (4099, 2, 7, 60)])
