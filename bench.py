@@ -370,7 +370,7 @@ class GemmSmallMWorkload:
         pp = paths["prepared_planes"]
         alg = 8 * self.M * self.K + 4 * self.N * self.K + 16 * self.M * self.N
         gbs = alg / pp["us"] / 1e3
-        return {"bound": "hbm", "kernel": "split_rows_kernel + limb_gemm_kernel (split over K)",
+        return {"bound": "hbm", "kernel": "split_rows_kernel + limb_rows_kernel (K shared by a cluster)",
                 "achieved": round(gbs, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": round(gbs / peaks["hbm_gbs"], 4), "traffic": 15200000, "kernel_us": pp["us"],
                 "traffic_note": "ncu dram__bytes_read + dram__bytes_write of one call: 13.3 MB tensor-core kernel "

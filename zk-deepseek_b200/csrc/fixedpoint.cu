@@ -1583,7 +1583,9 @@ namespace {
 
 constexpr int kRouteThreads = 1024, kRouteWarps = 32;
 constexpr int kRouteMaxE = 512;
-constexpr int64_t kRouteMaxPairs = 1 << 17;      // beyond, one CTA takes longer than a sort over the whole GPU
+// Beyond, one CTA takes longer than a sort over the whole GPU: 131072 pairs of 256 experts 192 us against 188 us of the tensor
+// operations' kernels (382 us of their call), 262144 pairs 404 against 220 (378).  16 experts: 131072 pairs 119 against 195.
+constexpr int64_t kRouteMaxPairs = 1 << 17;
 
 __global__ void __launch_bounds__(kRouteThreads)
 moe_route_kernel(const int64_t* __restrict__ indices, int pairs, int slots, int64_t first, int E, int n_tiles,

@@ -352,7 +352,7 @@ struct LimbParams {
     int La, Lb, NT, stages;
     int kblocks;
     int64_t k_extent;         // K bytes per plane row (0 = unknown): a partial last K block issues fewer MMAs
-    uint32_t tmem_cols;       // power of two >= (La + Lb - 1) * NT
+    uint32_t tmem_cols;       // power of two >= (La + Lb - 1) * NT (limb_rows_kernel: taken from the limbs in use, not set)
     int64_t M, N, batches;
     int64_t a_rows_per_limb;  // batches * M
     int64_t b_rows_per_limb;  // nbB * b_batch_rows
@@ -1112,8 +1112,8 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // slice through distributed shared memory, so a split needs neither a workspace nor atomics.  A CTA gives its tensor memory
 // back before it waits for its cluster: what holds tensor memory never waits for another CTA, so CTAs of several launches
 // on one SM cannot block one another.
-// 64 sequences through a dense and a routed block (decoding): all its contractions of this kind 2400 -> 1949 us, the whole
-// step 4239 -> 3823 us; one sequence 1116 -> 671 us with its per-head products left out, the step 1982 -> 1835 us.
+// 64 sequences through a dense and a routed block and the head (decoding): the 24 contractions of this kind 2648 -> 1686 us,
+// the two of the routed experts among them; one sequence 1264 -> 706 us.
 constexpr int kRowsEpiWarps = 8, kRowsThreads = 64 + 32 * kRowsEpiWarps;
 
 __device__ __forceinline__ uint64_t peer_u64(uint32_t own, uint32_t rank)
