@@ -372,8 +372,8 @@ class GemmSmallMWorkload:
         gbs = alg / pp["us"] / 1e3
         return {"bound": "hbm", "kernel": "split_rows_kernel + limb_rows_kernel (K shared by a cluster)",
                 "achieved": round(gbs, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                "frac": round(gbs / peaks["hbm_gbs"], 4), "traffic": 15200000, "kernel_us": pp["us"],
-                "traffic_note": "ncu dram__bytes_read + dram__bytes_write of one call: 13.3 MB tensor-core kernel "
+                "frac": round(gbs / peaks["hbm_gbs"], 4), "traffic": 15050000, "kernel_us": pp["us"],
+                "traffic_note": "ncu dram__bytes_read + dram__bytes_write of one call: 13.2 MB tensor-core kernel "
                                 "(weight and activation planes) + 1.9 MB activation split; the outputs stay in L2",
                 "algorithmic_bytes": alg, "paths": paths,
                 "note": "algorithmic bytes = 8MK + 4NK + 16MN (int32 W) / GPU time of one call replayed from a CUDA "
