@@ -829,7 +829,7 @@ def test_boxes_of_32_among_33_to_64_rows(kmod, dev, M, H, N, K, wbits):
 
 
 def test_clusters_beyond_those_that_the_gpu_holds_do_not_double_the_time(kmod, dev):
-    """64 rows by 2048 columns are sixteen tiles of columns, of whose clusters of eight the GPU holds fifteen: as a second round
+    """64 rows by 2048 columns are sixteen tiles of columns, of whose clusters of eight the GPU holds fifteen: as a second wave
     they took 1.6 times what 1536 columns take (the weights: 1.33 times)"""
     x = torch.randint(-2**20, 2**20, (1, 64, 7168), device=dev)
 

@@ -2047,9 +2047,9 @@ int launch_split_t(const T* X, int8_t* planes, int L, int64_t nb, int64_t rows, 
 // Both operands' ranges in one launch: 2048 consecutive elements of a row a step of a block, its loads all in flight, one
 // atomic a block.  Bound by the bytes read.  32 x 7168 by 576 x 7168 int64, the whole product with its ranges measured:
 // 78.3 -> 60.8 us.  An operand without gaps is one long row, since a step of a short row would leave most of its threads without
-// work: 262144 x 8, row by row 1004 us for the product, as one row 278 (absmax_kernel 290).  absmax_kernel (a 64-bit division and one load
-// an element, an atomic a warp: 10.8 us each there) is left for short rows with gaps, for sources that are not contiguous along
-// K and for the other entry points that measure.
+// work: 262144 x 8, row by row 1004 us for the product, as one row 278 (absmax_kernel 290).  absmax_kernel (a 64-bit division and
+// one load an element, an atomic a warp: 10.8 us each for 32 and 576 rows of 7168) is left for short rows with gaps, for sources
+// that are not contiguous along K and for the other entry points that measure.
 struct RangeOf {
     const void* X;
     int64_t rows, cols, sz, sr, div, segs, steps;      // steps = batches * rows * segs, 0 = nothing to measure
@@ -2616,8 +2616,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         // Boxes of few_rows rows, or of 32 where that gives two, and shares of K, by the K blocks that an SM works through:
         // a CTA's start and end take as long as one block and one more for eight rows, and as much again for the sums of a
         // split.  Beyond the clusters that the GPU holds at a time (of eight CTAs no more than 15, not 18) there is another
-        // round, or two CTAs to an SM where they fit, of which one starts or finishes while the other streams.
-        // 64 rows, against 64-row boxes and rounds counted in SMs: 2048 x 7168 44 -> 30 us (four limbs 64 -> 40), 24576 x 1536
+        // wave, or two CTAs to an SM where they fit, of which one starts or finishes while the other streams.
+        // 64 rows, against 64-row boxes and waves counted in SMs: 2048 x 7168 44 -> 30 us (four limbs 64 -> 40), 24576 x 1536
         // 69 -> 44, 4096 x 512 of four limbs 33 -> 24; the tiles of limb_gemm_kernel take 38, 51, 59 and 28.
         // Row tiles of experts are mostly unused, so their number says nothing: one box and no split there.
         int ks = 1, box = few_rows;
