@@ -892,3 +892,36 @@ def test_causal_probabilities_of_tiles_that_end_early(kmod, dev, S, H, T, start)
     got = kmod.softmax_pv_fused(scores, kv, 23, causal_skip=True, start_pos=start, a_limbs=3, b_limbs=3)
     assert got is not None and torch.equal(got, want)
     kmod.device_status()
+
+
+@pytest.mark.parametrize("T", [4, 128, 508, 512, 516, 1024, 1028, 2048, 2052, 4096, 4100, 8176])
+def test_softmax_to_limbs_over_ranges_and_row_lengths(kmod, orc, dev, T):
+    """rows whose scores lie beyond 32 bits above or below, at the edges of both, all equal, and differences from the maximum
+    around those where a weight becomes zero: every row against the oracle's softmax"""
+    rng, S = np.random.default_rng(T), 14
+    scores = np.rint(rng.standard_normal((1, S, 3, T)) * 2.0 ** 20).astype(np.int64)
+    scores[0, 0] += 1 << 31                                   # above 32 bits
+    scores[0, 1] += (1 << 31) - (1 << 20)                     # partly
+    scores[0, 2] -= 1 << 31                                   # below, partly
+    scores[0, 3] -= 1 << 42                                   # all masked
+    scores[0, 4, :, 1:] = -(64 << 36)                         # one that is not
+    scores[0, 5] = np.iinfo(np.int64).min
+    scores[0, 6] = np.iinfo(np.int64).max
+    scores[0, 7, :, 0], scores[0, 7, :, 1:] = np.iinfo(np.int64).max, np.iinfo(np.int64).min
+    scores[0, 8] = 5
+    edges = np.array([0, 1, (1 << 23) - 2, (1 << 23) - 1, 1 << 23, (1 << 23) + 1, 64 << 19, (64 << 19) + 1, 1 << 31, 1 << 40])
+    for s, top in ((9, 0), (10, (1 << 31) - 1), (11, -(1 << 31)), (12, -(1 << 31) + (1 << 26)), (13, 1 << 50)):
+        scores[0, s] = top - edges[rng.integers(0, len(edges), (3, T))]
+        scores[0, s, :, T // 2] = top
+    kv = np.zeros((1, T, 16), np.int64)                       # column c of the context is the probability of key picked[c]
+    picked = rng.integers(0, T, 15)
+    kv[0, picked, np.arange(15)] = 1 << 20
+    kv[0, :, 15] = 1 + np.arange(T)
+    want = orc.einsum_bsht_btc_bshc(orc.softmax(scores, 19), kv, 20)
+    kmod.softmax_init_q19()
+    sd = g(scores, dev)
+    for dynamic in (False, True):
+        got = kmod.softmax_pv_fused(sd, g(kv, dev), 20, a_limbs=3, b_limbs=3, dynamic=dynamic)
+        same(got, want, "dynamic=%s" % dynamic)
+    same(sd, scores, "scores untouched")
+    kmod.device_status(sync=True)

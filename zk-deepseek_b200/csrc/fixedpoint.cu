@@ -5,10 +5,12 @@
 // bit for bit (inference/int64_gemm.cu:223-385, 605-768, 775-1017) with the slow
 // integer divisions replaced by a double-precision estimate plus an exact
 // integer correction.
+#include <limits.h>
 #include <stdlib.h>
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tcgen05.cuh"
 
 namespace zkds {
 
@@ -422,48 +424,212 @@ static int launch_softmax_q19_reg(const int64_t* X, int64_t* Wout, int64_t* C, c
 // The same Q19 softmax, but the probabilities leave the kernel as signed 8-bit limb planes (the A
 // operand of the tensor-core contraction that consumes them) instead of int64 words: plane l of row
 // r lives at planes + l * plane_stride + r * Kp.  Balanced radix-256 digits as in the limb split;
-// columns from `valid` up to what the row's tile needs, or from T up to Kp, are written as zero.  E = groups of four columns per thread.
-// MINB: CTAs per SM the kernel is compiled for.  The 4096-column case (E = 4, three limbs) asks for eight: 32
-// registers and 68 bytes of spills instead of 48 registers and five CTAs, 6.95 against 7.48 ms on the 17 GB
-// score tensor of the 4096-token prefill (six CTAs: 7.13 ms).
-template <int E, int LL, int MINB, bool FULL>      // LL: limb count known at compile time, 0 = use L; FULL as above
-__global__ void __launch_bounds__(kThreads, MINB)
+// columns from `valid` up to what the row's tile needs, or from T up to Kp, are written as zero.
+struct PlanesRow {
+    int valid, quads_valid, quads_all;
+};
+
+__device__ __forceinline__ PlanesRow planes_row(unsigned row, int T, int64_t Kp, int valid_H, int valid_S, int valid_start)
+{
+    PlanesRow r;
+    r.valid = T;
+    r.quads_all = (int)(Kp >> 2);
+    if (valid_H) {
+        const unsigned rows = (unsigned)valid_H * (unsigned)valid_S, at = row % rows;
+        const int sidx = (int)(at / (unsigned)valid_H);
+        r.valid = valid_start + sidx + 1 < T ? valid_start + sidx + 1 : T;
+        if (valid_S > 1) {
+            // the contraction reads a tile of 128 rows up to the block of 128 columns that its last row ends in: zeros that
+            // far (4096 tokens: 4.76 -> 4.48 ms; one position has nothing to leave out)
+            const unsigned last = min(at | 127u, rows - 1);
+            const int64_t end = ((int64_t)valid_start + last / (unsigned)valid_H + 1 + 127) & ~(int64_t)127;
+            if (end < Kp) r.quads_all = (int)(end >> 2);
+        }
+    }
+    r.quads_valid = (r.valid + 3) >> 2;
+    return r;
+}
+
+// Three limbs, what probabilities need.  Bound by issue slots (about 30 instructions an element) and by the latency of a row's
+// chain: load, maximum, weights, sum, quotients.  So blocks are small and stay: each walks rows, NT threads on one, and the
+// next row is on its way into shared memory (one bulk copy) as soon as this one is in registers.  Everything behind the
+// load runs in 32 bits: scores are clamped from below, and a row that has one above 2^31, or none above the clamp, is read
+// again in 64; a difference from the maximum is cut below 2^23, where the weight is zero; the quotient comes from a 32-bit
+// reciprocal that is never above, and is then itself or one below.  E: groups of four columns a thread.
+// 4096 tokens of 128 heads, causal (5.9 GB): 4.48 -> 2.72 ms against a block of 256 threads a row; the attention layer around it
+// 25.19 -> 23.43 ms, a dense block of 777 tokens 9.48 -> 9.30, decoding of 64 sequences 3.18 -> 3.11.
+template <int NT, int E, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+softmax_q19_rows_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, int8_t* __restrict__ planes, unsigned rows, int T,
+                        int64_t Kp, int64_t plane_stride, unsigned long long* absmax_out, int valid_H, int valid_S,
+                        int valid_start, int* error_flag)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int kWarps = NT / 32, kTooHigh = 1, kGaveUp = 2;
+    constexpr uint32_t kCut = (1u << 23) - 1;
+    __shared__ uint32_t lut[256];
+    __shared__ int red_max[kWarps], red_flags[kWarps];
+    __shared__ uint32_t red_sum[kWarps], red_top[kWarps];
+    __shared__ int64_t red64[32];
+    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ int s_abort;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t bar = smem_u32(&s_bar);
+    const longlong2* buf = reinterpret_cast<const longlong2*>(smem_raw);
+    for (int i = tid; i < 256; i += NT) lut[i] = (uint32_t)lut_g[i];
+    auto request = [&](unsigned row) {
+        const uint32_t bytes = (uint32_t)planes_row(row, T, Kp, valid_H, valid_S, valid_start).quads_valid * 32u;
+        mbar_expect_tx(bar, bytes);
+        bulk_load(smem_u32(smem_raw), X + (int64_t)row * T, bytes, bar);
+    };
+    if (tid == 0) {
+        s_abort = 0;
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        request(blockIdx.x);
+    }
+    __syncthreads();
+    uint32_t parity = 0, seen = 0;
+    for (unsigned row = blockIdx.x; row < rows; row += gridDim.x, parity ^= 1u) {
+        const PlanesRow r = planes_row(row, T, Kp, valid_H, valid_S, valid_start);
+        int flags = mbar_wait(bar, parity, &s_abort) ? 0 : kGaveUp;
+        int v[4 * E], mx = INT_MIN;
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const int q = tid + j * NT;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) v[4 * j + h] = INT_MIN;
+            if (q < r.quads_valid) {
+                const longlong2 a = buf[2 * q], b = buf[2 * q + 1];
+                const int64_t x[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const int lo = (int)x[h], hi = (int)(x[h] >> 32), sign = lo >> 31;
+                    if (4 * q + h < r.valid) {
+                        v[4 * j + h] = hi < sign ? INT_MIN : lo;
+                        flags |= hi > sign ? kTooHigh : 0;
+                    }
+                    mx = max(mx, v[4 * j + h]);
+                }
+            }
+        }
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        flags = __reduce_or_sync(0xffffffffu, flags);
+        if (lane == 0) { red_max[warp] = mx; red_flags[warp] = flags; }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) { mx = max(mx, red_max[w]); flags |= red_flags[w]; }
+        if (flags & kGaveUp) break;
+        if (flags || mx < INT_MIN + (1 << 26)) {             // the same for the whole block
+            int64_t top = INT64_MIN;
+#pragma unroll 1
+            for (int q = tid; q < r.quads_valid; q += NT)
+                for (int h = 0; h < 4; ++h)
+                    if (4 * q + h < r.valid) {
+                        const int64_t x = reinterpret_cast<const int64_t*>(smem_raw)[4 * q + h];
+                        top = x > top ? x : top;
+                    }
+            top = block_max_i64(top, red64);
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const int c = 4 * (tid + j * NT) + h;
+                    v[4 * j + h] = INT_MIN;
+                    if (c < r.valid) {
+                        const uint64_t d = (uint64_t)top - (uint64_t)reinterpret_cast<const int64_t*>(smem_raw)[c];
+                        v[4 * j + h] = -(int)(d < kCut ? d : kCut);
+                    }
+                }
+            mx = 0;
+            __syncthreads();
+        }
+        if (tid == 0 && row + gridDim.x < rows) request(row + gridDim.x);      // everybody has read this row
+
+        uint32_t w[4 * E], sum32 = 0, top_w = 0;              // at most 32 weights of at most 2^19 + 1 each
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) w[4 * j + h] = 0;
+            if (tid + j * NT < r.quads_valid) {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const uint32_t d = min((uint32_t)mx - (uint32_t)v[4 * j + h], kCut);
+                    const uint32_t y = __umulhi(d << 9, 756388u << 4);           // (d * 756388) >> 19
+                    w[4 * j + h] = lut[(y >> 11) & 255u] >> (y >> 19);
+                    sum32 += w[4 * j + h];
+                    top_w = max(top_w, w[4 * j + h]);
+                }
+            }
+        }
+        sum32 = __reduce_add_sync(0xffffffffu, sum32);
+        top_w = __reduce_max_sync(0xffffffffu, top_w);
+        if (lane == 0) { red_sum[warp] = sum32; red_top[warp] = top_w; }
+        __syncthreads();
+        uint64_t sum = 0;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) { sum += red_sum[i]; top_w = max(top_w, red_top[i]); }
+
+        // m <= 2^63 / (sum << z) < m * (1 + 2^-22) + 1: w * 2^19 / sum = w * m * 2^(z - 44) or less than one more
+        const uint32_t s32 = (uint32_t)sum;
+        const int z = __clz((int)s32);
+        const bool small = sum != 0 && sum <= (1ull << 31) && z <= 24;
+        const uint32_t m = __float2uint_rd(__frcp_rd(__uint2float_ru(s32 << (z & 31))) * 9223372036854775808.0f);
+        auto quotient = [&](uint32_t wi) -> uint32_t {
+            if (!small) return sum ? (uint32_t)(((uint64_t)wi << 19) / sum) : 0u;
+            const uint32_t q = __umulhi(wi << 12, m) >> ((24 - z) & 31);
+            return q + ((wi << 19) - q * s32 >= s32 ? 1u : 0u);       // the remainder is below 2 * sum <= 2^32
+        };
+        int8_t* drow = planes + (int64_t)row * Kp;
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const int q = tid + j * NT;
+            if (q >= r.quads_all) continue;
+            uint32_t t[4] = {0x00808080u, 0x00808080u, 0x00808080u, 0x00808080u};
+            // balanced digits of a value below 2^23 - 2^15 (these are at most 2^19): the bytes of u + 0x808080, each with
+            // its top bit flipped (digit + 128 is what the biased sum holds at every position)
+            if (q < r.quads_valid) {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) t[h] += quotient(w[4 * j + h]);
+            }
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                const uint32_t sel = 0x0040u + 0x0011u * (uint32_t)l;     // byte l of both operands
+                const uint32_t lo = __byte_perm(t[0], t[1], sel), hi = __byte_perm(t[2], t[3], sel);
+                *reinterpret_cast<uint32_t*>(drow + 4 * q + l * plane_stride) = __byte_perm(lo, hi, 0x5410u) ^ 0x80808080u;
+            }
+        }
+        if (absmax_out && tid == 0) seen = max(seen, quotient(top_w));
+    }
+    if (tid == 0) {
+        if (s_abort) *(volatile int*)error_flag = 1;
+        if (absmax_out && seen) atomicMax(absmax_out, (unsigned long long)seen);
+    }
+}
+
+// any other number of limbs: a block a row
+template <int E>
+__global__ void __launch_bounds__(kThreads)
 softmax_q19_planes_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, int8_t* __restrict__ planes,
                           int L, int T, int64_t Kp, int64_t plane_stride, unsigned* overflow,
                           unsigned long long* absmax_out, int valid_H, int valid_S, int valid_start)
 {
-    __shared__ uint32_t lut[256];
     __shared__ int64_t red[32];
-    __shared__ uint64_t s_magic;
-    for (int i = threadIdx.x; i < 256; i += kThreads) lut[i] = (uint32_t)lut_g[i];
     const longlong2* xv = reinterpret_cast<const longlong2*>(X + (int64_t)blockIdx.x * T);
     int8_t* drow = planes + (int64_t)blockIdx.x * Kp;
-    int valid = T;
-    if (!FULL && valid_H) {
-        const int sidx = (int)((blockIdx.x / (unsigned)valid_H) % (unsigned)valid_S);
-        valid = valid_start + sidx + 1 < T ? valid_start + sidx + 1 : T;
-    }
-    const int quads_valid = (valid + 3) >> 2;
-    int quads_all = (int)(Kp >> 2);
-    if (!FULL && valid_H && valid_S > 1) {
-        // the contraction reads a tile of 128 rows up to the block of 128 columns that its last row ends in: zeros that far
-        // (4096 tokens: 4.76 -> 4.48 ms; one position has nothing to leave out)
-        const unsigned rows = (unsigned)valid_H * (unsigned)valid_S, last = min((blockIdx.x % rows) | 127u, rows - 1);
-        const int64_t end = ((int64_t)valid_start + last / (unsigned)valid_H + 1 + 127) & ~(int64_t)127;
-        if (end < Kp) quads_all = (int)(end >> 2);
-    }
+    const PlanesRow r = planes_row(blockIdx.x, T, Kp, valid_H, valid_S, valid_start);
 
     int64_t v[4 * E];
     int64_t mx = INT64_MIN;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         const int q = threadIdx.x + j * kThreads;
-        if (q < quads_valid) {
+        if (q < r.quads_valid) {
             const longlong2 a = xv[2 * q], b = xv[2 * q + 1];
             v[4 * j] = a.x; v[4 * j + 1] = a.y; v[4 * j + 2] = b.x; v[4 * j + 3] = b.y;
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                if (!FULL && 4 * q + h >= valid) v[4 * j + h] = INT64_MIN;
+                if (4 * q + h >= r.valid) v[4 * j + h] = INT64_MIN;
                 mx = v[4 * j + h] > mx ? v[4 * j + h] : mx;
             }
         }
@@ -477,96 +643,41 @@ softmax_q19_planes_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, i
         const int q = threadIdx.x + j * kThreads;
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
-            uint32_t wi = 0;
-            if (q < quads_valid && (FULL || 4 * q + h < valid)) {
-                const uint64_t d = (uint64_t)mx - (uint64_t)v[4 * j + h];
-                if (d <= (uint64_t)(64 << 19)) {
-                    const uint32_t y = (uint32_t)(((uint64_t)(uint32_t)d * 756388u) >> 19);
-                    const uint32_t k = y >> 19;
-                    const uint32_t t = lut[(y & 0x7FFFFu) >> 11];
-                    wi = k >= 32u ? 0u : (t >> k);
-                }
-            }
-            w[4 * j + h] = wi;
-            sum32 += wi;
+            w[4 * j + h] = 0;
+            if (q < r.quads_valid && 4 * q + h < r.valid) w[4 * j + h] = (uint32_t)softmax_weight<19>(v[4 * j + h], mx, lut_g);
+            sum32 += w[4 * j + h];
         }
     }
     const uint64_t sumW = (uint64_t)block_sum_i64((int64_t)sum32, red);
-    if (threadIdx.x == 0) s_magic = sumW ? 0xFFFFFFFFFFFFFFFFull / sumW : 0;
-    __syncthreads();
-    const uint64_t magic = s_magic;
-    const uint32_t m_lo = (uint32_t)magic, m_hi = (uint32_t)(magic >> 32);
-    const bool small = sumW < (1ull << 32);
-    const uint32_t s32 = (uint32_t)sumW;
 
     uint32_t seen = 0;
     bool ovf = false;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         const int q = threadIdx.x + j * kThreads;
-        if (q >= quads_all) continue;
-        uint32_t u[4] = {0, 0, 0, 0};
-        if (q < quads_valid) {
+        if (q >= r.quads_all) continue;
+        uint32_t pl[9] = {};
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const uint32_t wi = w[4 * j + h];
-                const uint64_t num = (uint64_t)wi << 19;
-                uint64_t qt = ((uint64_t)wi * m_hi + (((uint64_t)wi * m_lo) >> 32)) >> 13;
-                if (small) {
-                    const uint64_t rem = num - qt * s32;      // qt is the quotient or one below it (see above)
-                    qt += rem >= sumW ? 1 : 0;
-                } else if (sumW) {
-                    qt = num / sumW;
+        for (int h = 0; h < 4; ++h) {
+            const uint32_t u = q < r.quads_valid && sumW ? (uint32_t)(((uint64_t)w[4 * j + h] << 19) / sumW) : 0u;
+            seen = u > seen ? u : seen;
+            int32_t x = (int32_t)u;
+#pragma unroll
+            for (int l = 0; l < 9; ++l) {
+                if (l < L) {
+                    pl[l] |= (uint32_t)(x & 0xFF) << (h * 8);
+                    x = (x >> 8) + ((x >> 7) & 1);
                 }
-                u[h] = (uint32_t)qt;                 // 0 .. 2^19
-                seen = u[h] > seen ? u[h] : seen;
             }
+            ovf |= (x != 0);
         }
-        if (LL == 3) {
-            // balanced digits of a value below 2^23 - 2^15: the bytes of u + 0x808080, each with its
-            // top bit flipped (digit + 128 is what the biased sum holds at every position)
-            uint32_t t[4];
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                t[h] = u[h] + 0x00808080u;
-                ovf |= (t[h] >> 24) != 0;
-            }
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-                const uint32_t sel = 0x0040u + 0x0011u * (uint32_t)l;     // byte l of both operands
-                const uint32_t lo = __byte_perm(t[0], t[1], sel), hi = __byte_perm(t[2], t[3], sel);
-                *reinterpret_cast<uint32_t*>(drow + 4 * q + l * plane_stride) =
-                    __byte_perm(lo, hi, 0x5410u) ^ 0x80808080u;
-            }
-        } else {
-            constexpr int LMAX = LL ? LL : 9;
-            uint32_t pl[LMAX];
-#pragma unroll
-            for (int l = 0; l < LMAX; ++l) pl[l] = 0;
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                int32_t x = (int32_t)u[h];
-#pragma unroll
-                for (int l = 0; l < LMAX; ++l) {
-                    if (LL || l < L) {
-                        pl[l] |= (uint32_t)(x & 0xFF) << (h * 8);
-                        x = (x >> 8) + ((x >> 7) & 1);
-                    }
-                }
-                ovf |= (x != 0);
-            }
-#pragma unroll
-            for (int l = 0; l < LMAX; ++l)
-                if (LL || l < L) *reinterpret_cast<uint32_t*>(drow + 4 * q + l * plane_stride) = pl[l];
-        }
+        for (int l = 0; l < 9; ++l)
+            if (l < L) *reinterpret_cast<uint32_t*>(drow + 4 * q + l * plane_stride) = pl[l];
     }
     if (ovf) *overflow = 1u;
     if (absmax_out) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const uint32_t other = __shfl_xor_sync(0xffffffffu, seen, o);
-            seen = other > seen ? other : seen;
-        }
+        seen = __reduce_max_sync(0xffffffffu, seen);
         if ((threadIdx.x & 31) == 0 && seen) atomicMax(absmax_out, (unsigned long long)seen);
     }
 }
@@ -579,29 +690,34 @@ bool softmax_planes_supported(const int64_t* X, int64_t rows, int64_t T, int64_t
 
 int launch_softmax_planes(const int64_t* X, const int64_t* lut, int8_t* planes, int L, int64_t rows, int64_t T,
                           int64_t Kp, int64_t plane_stride, unsigned* overflow, unsigned long long* absmax_out,
-                          int64_t valid_H, int64_t valid_S, int64_t valid_start, cudaStream_t st)
+                          int64_t valid_H, int64_t valid_S, int64_t valid_start, int* error_flag, cudaStream_t st)
 {
     if (!softmax_planes_supported(X, rows, T, Kp) || L < 1 || L > 9 || valid_H > 0x7fffffff ||
         valid_S > 0x7fffffff || valid_start > 0x7fffffff)
         return ZKDS_ERR_UNSUPPORTED;
-    const int per = (int)(((Kp >> 2) + kThreads - 1) / kThreads);
-    const unsigned g = (unsigned)rows;
     const int vS = valid_S > 0 ? (int)valid_S : 1;
-#define ZKDS_SP(E)                                                                                        \
-    do {                                                                                                  \
-        if (L == 3 && valid_H == 0)                                                                       \
-            softmax_q19_planes_kernel<E, 3, (E == 4 ? 6 : 1), true><<<g, kThreads, 0, st>>>(              \
-                X, lut, planes, L, (int)T, Kp, plane_stride, overflow, absmax_out, (int)valid_H, vS,      \
-                (int)valid_start);                                                                        \
-        else if (L == 3)                                                                                  \
-            softmax_q19_planes_kernel<E, 3, (E == 4 ? 8 : 1), false><<<g, kThreads, 0, st>>>(             \
-                X, lut, planes, L, (int)T, Kp, plane_stride, overflow, absmax_out, (int)valid_H, vS,      \
-                (int)valid_start);                                                                        \
-        else                                                                                              \
-            softmax_q19_planes_kernel<E, 0, 1, false><<<g, kThreads, 0, st>>>(X, lut, planes, L, (int)T, Kp, \
-                                                                    plane_stride, overflow, absmax_out,   \
-                                                                    (int)valid_H, vS, (int)valid_start);  \
-    } while (0)
+    if (L == 3) {
+        // 128 threads hold rows of up to 4096 columns, 32 a thread; as many blocks to an SM as registers and rows in shared memory
+        // leave, so that the chains of several rows overlap
+        const int64_t quads = Kp >> 2;
+        auto run = [&](auto kernel, int threads, int per_sm) {
+            const size_t smem = (size_t)T * 8;
+            const int64_t fit = (int64_t)(227 * 1024 / (smem + 3072)), blocks = sm_count() * (fit < per_sm ? fit : per_sm);
+            ZKDS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+            kernel<<<(unsigned)(rows < blocks ? rows : blocks), threads, smem, st>>>(
+                X, lut, planes, (unsigned)rows, (int)T, Kp, plane_stride, absmax_out, (int)valid_H, vS, (int)valid_start, error_flag);
+            return check_launch();
+        };
+        if (quads <= 128) return run(softmax_q19_rows_kernel<128, 1, 12>, 128, 12);
+        if (quads <= 256) return run(softmax_q19_rows_kernel<128, 2, 12>, 128, 12);
+        if (quads <= 512) return run(softmax_q19_rows_kernel<128, 4, 10>, 128, 10);
+        if (quads <= 1024) return run(softmax_q19_rows_kernel<128, 8, 6>, 128, 6);
+        return run(softmax_q19_rows_kernel<256, 8, 3>, 256, 3);
+    }
+    const int per = (int)(((Kp >> 2) + kThreads - 1) / kThreads);
+#define ZKDS_SP(E)                                                                                                    \
+    softmax_q19_planes_kernel<E><<<(unsigned)rows, kThreads, 0, st>>>(X, lut, planes, L, (int)T, Kp, plane_stride,    \
+                                                                     overflow, absmax_out, (int)valid_H, vS, (int)valid_start)
     if (per <= 1) ZKDS_SP(1);
     else if (per <= 2) ZKDS_SP(2);
     else if (per <= 4) ZKDS_SP(4);
