@@ -925,3 +925,51 @@ def test_softmax_to_limbs_over_ranges_and_row_lengths(kmod, orc, dev, T):
         same(got, want, "dynamic=%s" % dynamic)
     same(sd, scores, "scores untouched")
     kmod.device_status(sync=True)
+
+
+@pytest.mark.parametrize("M,N,K,limbs", [(1, 128, 16, 3), (1, 576, 7168, 4), (15, 130, 1000, 3), (16, 2112, 1536, 5), (17, 64, 129, 3),
+                                         (31, 16500, 8, 2), (32, 300, 2056, 5), (33, 300, 2056, 4), (2, 4000, 250, 6)])
+def test_few_rows_are_cut_into_limbs_by_the_product(kmod, orc, dev, M, N, K, limbs):
+    """edges of the tiles of 16 and 32 rows, ragged K (also odd, where rows are not aligned), every number of limbs; a value
+    beyond the promise raises the flag"""
+    rng = np.random.default_rng(M * N + K)
+    X, W = rand_i64(rng, (1, M, K), 8 * limbs - 2), rand_i64(rng, (N, K), 13).astype(np.int32)
+    top = 128 * (256 ** limbs - 1) // 255
+    ones = (256 ** limbs - 1) // 255
+    X[0, 0, 0], X[0, -1, -1] = -top if M <= 32 else ones - top, top - ones          # the largest that digits of -128 .. 127 hold
+    planes = kmod.WeightPlanes(g(W, dev))
+    want = orc.gemm(X, W, 1, 1, 9, orc.R_LEGACY)
+    for dynamic in (False, True):
+        got = kmod.linear_prepared(g(X, dev), planes, 9, a_limbs=limbs, want_remainder=True, dynamic=dynamic)
+        same(got[0], want[0], "C")
+        same(got[1], want[1], "R")
+    kmod.device_status(sync=True)
+    X[0, M // 2, K // 2] = top + 1
+    kmod.linear_prepared(g(X, dev), planes, 9, a_limbs=limbs, dynamic=True)
+    with pytest.raises(kmod.ZkdsError) as e:
+        kmod.device_status(sync=True)
+    assert e.value.status == kmod.ERR_RANGE
+
+
+def test_few_rows_of_experts_behind_an_index(kmod, orc, dev):
+    """rows gathered by index, tiles of padding in between; an expert with more rows than were promised raises the flag"""
+    rng, E, N, K, T = np.random.default_rng(3), 3, 200, 520, 9
+    X, W = rand_i64(rng, (1, T, K), 20), rand_i64(rng, (E, N, K), 13).astype(np.int32)
+    index = np.full((4, 128), -1, np.int32)
+    index[0, :5], index[2, :9], index[3, :1] = rng.integers(0, T, 5), np.arange(9), 4
+    group = np.array([1, -1, 0, 2], np.int32)
+    planes, gi = kmod.WeightPlanes(g(W, dev)), g(index.reshape(-1), dev)
+    got = kmod.grouped_prepared(g(X[0], dev), planes, g(group, dev), 7, a_limbs=3, dynamic=True, row_index=gi, max_group_rows=32)
+    want = np.zeros((512, N), np.int64)
+    for t, e in enumerate(group):
+        rows = index[t][index[t] >= 0]
+        if len(rows):
+            want[t * 128:t * 128 + len(rows)] = orc.gemm(X[:, rows], W[e], 1, 1, 7, orc.R_LEGACY)[0][0]
+    same(got, want)
+    kmod.device_status(sync=True)
+    index[2, 32] = 1
+    kmod.grouped_prepared(g(X[0], dev), planes, g(group, dev), 7, a_limbs=3, dynamic=True, row_index=g(index.reshape(-1), dev),
+                          max_group_rows=32)
+    with pytest.raises(kmod.ZkdsError) as e:
+        kmod.device_status(sync=True)
+    assert e.value.status == kmod.ERR_RANGE

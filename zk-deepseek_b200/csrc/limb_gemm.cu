@@ -427,6 +427,11 @@ struct LimbParams {
     // lands in accumulator rows nobody stores (M <= 64) or that are zeroed before the epilogue reads them
     // (grouped tiles: their padding rows are stored, as the result of zero rows).  0 = 128.
     int a_box_rows;
+    // limb_rows_kernel<true>: the activations as they are, row (z, m) at a_src + z * a_sz + m * a_sm (m through a_row_index
+    // when given, a negative entry a row of zeros), K of them
+    const int64_t* a_src;
+    int64_t a_sz, a_sm, K;
+    const int* a_row_index;
 };
 
 __device__ __forceinline__ int limbs_needed_dev(unsigned long long maxabs)
@@ -1114,6 +1119,7 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // on one SM cannot block one another.
 // 64 sequences through a dense and a routed block and the head (decoding): the 24 contractions of this kind 2648 -> 1686 us,
 // the two of the routed experts among them; one sequence 1264 -> 706 us.
+constexpr int kDirectRows = 32;         // up to so many activation rows are cut into limbs by the kernel itself (two a thread)
 constexpr int kRowsEpiWarps = 8, kRowsThreads = 64 + 32 * kRowsEpiWarps;
 
 __device__ __forceinline__ uint64_t peer_u64(uint32_t own, uint32_t rank)
@@ -1143,8 +1149,43 @@ __device__ __forceinline__ void rows_store(const LimbParams& p, i128w sum, int s
     }
 }
 
+// balanced digits of eight consecutive words, L <= 7: digit + 128 is what v + 0x80..80 holds at every position.  Eight bytes a
+// limb, `step` apart; false when a word does not fit
+__device__ __forceinline__ bool put_digits(const int64_t (&v)[8], int L, uint32_t dst, uint32_t step)
+{
+    const uint64_t bias = 0x80808080808080ull & ((1ull << (8 * L)) - 1ull);
+    uint32_t lo[8], hi[8];
+    uint64_t beyond = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint64_t t = (uint64_t)v[i] + bias;
+        beyond |= t >> (8 * L);
+        lo[i] = (uint32_t)t;
+        hi[i] = (uint32_t)(t >> 32);
+    }
+    auto put = [&](const uint32_t (&w)[8], int l, uint32_t at) {
+        const uint32_t sel = 0x0040u + 0x0011u * (uint32_t)l;     // byte l of both operands
+        const uint32_t a = __byte_perm(__byte_perm(w[0], w[1], sel), __byte_perm(w[2], w[3], sel), 0x5410u) ^ 0x80808080u;
+        const uint32_t b = __byte_perm(__byte_perm(w[4], w[5], sel), __byte_perm(w[6], w[7], sel), 0x5410u) ^ 0x80808080u;
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
+    };
+#pragma unroll
+    for (int l = 0; l < 4; ++l)
+        if (l < L) put(lo, l, dst + (uint32_t)l * step);
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+        if (l + 4 < L) put(hi, l, dst + (uint32_t)(l + 4) * step);
+    return beyond == 0;
+}
+
 // p.NT = R rows of activations (tmA's box); tmW's box holds 128 weight rows.  grid (n_tiles * ksplit, row tiles, batches); the
 // row tiles of a grouped call are 128 rows apart, others R
+// DIRECT (up to 32 rows): the epilogue warps, which have nothing to do until the sums are complete, read the activations and cut
+// them into limbs on their way into the stages, so that a call is one launch: no pass that writes planes, no range to measure
+// and to clear before.  Every column tile reads and cuts the rows anew, which at 32 rows is half of what the weights move and at 64
+// would be as much.  One sequence through two blocks and the head: 114 -> 72 launches, 1401 -> 1272 us; 64 sequences, whose routed
+// experts take it: 3174 -> 3126.
+template <bool DIRECT>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const LimbParams p,
                  const uint32_t pipe_bytes)
@@ -1189,7 +1230,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int s = 0; s < stages; ++s) {
-            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_full + 8 * s, DIRECT ? 1 + kRowsEpiWarps : 1);
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_zeroed, kRowsEpiWarps);
@@ -1216,10 +1257,10 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const int it = kb - kb_begin, s = it % stages;
                 if (!mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag)) break;
                 const uint32_t full = bar_full + 8 * s, sw = smem_base + s * stage_bytes;
-                mbar_expect_tx(full, stage_bytes);
+                mbar_expect_tx(full, DIRECT ? w_bytes : stage_bytes);
                 for (int j = 0; j < p.Lb; ++j)
                     tma_load_2d(sw + j * (kTileM * kBlockK), &tmW, kb * kBlockK, (int)(j * p.b_rows_per_limb) + w_row, full);
-                for (int i = 0; i < La; ++i)
+                for (int i = 0; i < La && !DIRECT; ++i)
                     tma_load_2d(sw + w_bytes + i * a_limb, &tmA, kb * kBlockK, (int)(i * p.a_rows_per_limb) + a_row, full);
                 armed = it + 1;
             }
@@ -1253,6 +1294,67 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int q = warp & 3, col = q * 32 + lane;             // tensor-memory lane quarter, column of the tile
         const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
         bool ok = true;
+        // DIRECT: sixteen threads a row, eight words of a K block each, up to two rows a thread
+        auto cut_rows = [&]() {
+            const int et = (int)threadIdx.x - 64, unit = et & 15;
+            const bool wide = (((uintptr_t)p.a_src & 15) | (uintptr_t)((p.a_sm | p.a_sz) & 1)) == 0;
+            const int64_t* src[2];
+            uint32_t dst[2];
+            bool fits = true;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int r = (et >> 4) + 16 * u;
+                src[u] = nullptr;
+                if (r < R && m0 + r < p.M) {
+                    const int64_t from = p.a_row_index ? p.a_row_index[m0 + r] : m0 + r;
+                    if (from >= 0) src[u] = p.a_src + z * p.a_sz + from * p.a_sm + unit * 8;
+                }
+                dst[u] = smem_base + w_bytes + (uint32_t)(r * kBlockK + (((unit >> 1) ^ (r & 7)) << 4) + (unit & 1) * 8);
+                if (r < R && !src[u])
+                    for (int s = 0; s < stages; ++s)
+                        for (int i = 0; i < La; ++i)
+                            asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(dst[u] + s * stage_bytes + i * a_limb), "r"(0u)
+                                         : "memory");
+            }
+            // a row with data behind the promised rows of a group would be dropped
+            if (p.tile_group && p.a_row_index && et < kTileM - R && m0 + R + et < p.M) fits = p.a_row_index[m0 + R + et] < 0;
+            auto fetch = [&](int64_t (&v)[2][8], int kb) {
+                const int64_t k = (int64_t)kb * kBlockK + unit * 8;
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (!src[u] || kb >= kb_end) continue;
+                    const int64_t* x = src[u] + (int64_t)kb * kBlockK;
+                    if (wide && k + 8 <= p.K) {
+#pragma unroll
+                        for (int i = 0; i < 8; i += 2) {
+                            const longlong2 t = *reinterpret_cast<const longlong2*>(x + i);
+                            v[u][i] = t.x; v[u][i + 1] = t.y;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[u][i] = k + i < p.K ? x[i] : 0;
+                    }
+                }
+            };
+            int64_t cur[2][8] = {}, nxt[2][8] = {};
+            fetch(cur, kb_begin);
+            for (int kb = kb_begin; kb < kb_end; ++kb) {
+                const int it = kb - kb_begin, s = it % stages;
+                fetch(nxt, kb + 1);
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag))) return false;
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (src[u]) fits &= put_digits(cur[u], La, dst[u] + s * stage_bytes, a_limb);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) cur[u][i] = nxt[u][i];
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * s);
+            }
+            if (!fits) *p.overflow_flag = 1u;
+            return true;
+        };
         if (some) {
             // the first MMA overwrites its La * R columns; the later limbs' last columns start at zero
             for (int c = La * R + 8 * ((warp - 2) >> 2); c < D * R; c += 8 * (kRowsEpiWarps / 4)) tmem_st8_zero(tq + (uint32_t)c);
@@ -1260,7 +1362,8 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_zeroed);
-            ok = mbar_wait(bar_accum, 0, abort_flag);
+            if (DIRECT) ok = cut_rows();
+            if (ok) ok = mbar_wait(bar_accum, 0, abort_flag);
             tc_fence_after();
         }
         EpilogueCtx ec;
@@ -2257,7 +2360,7 @@ static int allow_big_smem(K kernel, bool (&done)[64])
     }
     return ZKDS_OK;
 }
-static bool g_attr_onetile[64], g_attr_rows[64], g_attr_p16[64], g_attr_p8[64];
+static bool g_attr_onetile[64], g_attr_rows[64], g_attr_direct[64], g_attr_p16[64], g_attr_p8[64];
 
 static cudaEvent_t* timing_events()
 {
@@ -2458,7 +2561,7 @@ static int rows_clusters(int size, size_t smem)
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, limb_rows_kernel, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, limb_rows_kernel<false>, &cfg) != cudaSuccess || n < 1) {
         cudaGetLastError();
         n = sm_count() / size;
     }
@@ -2565,18 +2668,21 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
 
     DeviceFlags* fl = flags_for_device();
     if (!fl) return ZKDS_ERR_WORKSPACE;
-    int8_t* pa = (int8_t*)workspace((size_t)La * a_rows * Kp + 1024, 0);
-    if (!pa) return ZKDS_ERR_WORKSPACE;
+    const bool direct = by_rows && few <= kDirectRows && La <= 7 && p.a_div == 1 && !p.softmax_lut && !p.glu_lut && p.a_n_parts == 0;
+    int8_t* pa = direct ? nullptr : (int8_t*)workspace((size_t)La * a_rows * Kp + 1024, 0);
+    if (!pa && !direct) return ZKDS_ERR_WORKSPACE;
     unsigned long long* d_absmax = nullptr;
-    if (p.dynamic_a) {
+    if (p.dynamic_a && !direct) {
         unsigned long long* words = (unsigned long long*)workspace(8 * sizeof(uint64_t), 5);
         if (!words) return ZKDS_ERR_WORKSPACE;
         d_absmax = words + 2;
         ZKDS_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(uint64_t), st));
     }
     const int64_t Kp16 = Kp;
-    int rc;
-    if (p.softmax_lut) {
+    int rc = ZKDS_OK;
+    if (direct) {
+        // limb_rows_kernel reads the activations itself
+    } else if (p.softmax_lut) {
         if (p.a_sm != p.K || p.a_sz != p.M * p.K || p.a_div != 1) return ZKDS_ERR_ARG;
         rc = launch_softmax_planes(p.A, p.softmax_lut, pa, La, a_rows, p.K, Kp, a_rows * Kp, fl->overflow_dev,
                                    d_absmax, p.skip_k ? p.skip_H : 0, p.softmax_S, p.skip_start, fl->dev, st);
@@ -2609,7 +2715,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     }
 
     if (by_rows) {
-        rc = allow_big_smem(limb_rows_kernel, g_attr_rows);
+        rc = allow_big_smem(limb_rows_kernel<false>, g_attr_rows);
+        if (rc == ZKDS_OK) rc = allow_big_smem(limb_rows_kernel<true>, g_attr_direct);
         if (rc != ZKDS_OK) return rc;
         const int fits64 = sum_fits64(La, Lb, p.K, p.addend);
         const int64_t column_tiles = rows_tiles * p.batches;
@@ -2639,10 +2746,10 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
             }
         }
         const size_t pipe = pair ? 111 * 1024 : smem_max;
-        CUtensorMap mapA, mapW;
+        CUtensorMap mapA{}, mapW;
         const int64_t pitch = (pre_b && pre_b->pitch) ? pre_b->pitch : Kp;
         if (pitch < Kp || (pitch & 15)) return ZKDS_ERR_ARG;
-        if (!make_plane_map(&mapA, pa, (int64_t)La * a_rows, Kp, box) ||
+        if ((!direct && !make_plane_map(&mapA, pa, (int64_t)La * a_rows, Kp, box)) ||
             !make_plane_map(&mapW, pb, (int64_t)Lb * b_rows, Kp, kTileM, pitch))
             return ZKDS_ERR_UNSUPPORTED;
         LimbParams lp{};
@@ -2657,6 +2764,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         lp.a_absmax = d_absmax; lp.overflow_flag = fl->overflow_dev;
         lp.tile_group = p.tile_group; lp.group_shift = p.group_shift; lp.n_split = p.n_split;
         lp.leave_padding = p.tile_group ? p.leave_padding : 0;
+        lp.a_src = p.A; lp.a_sz = p.a_sz; lp.a_sm = p.a_sm; lp.K = p.K; lp.a_row_index = p.a_row_index;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(rows_tiles * ks), (unsigned)(p.tile_group ? mt : (p.M + box - 1) / box), (unsigned)p.batches);
         cfg.blockDim = dim3(kRowsThreads);
@@ -2670,7 +2778,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         cfg.numAttrs = 1;
         cudaEvent_t* ev = timing_events();
         if (ev) ZKDS_CUDA(cudaEventRecord(ev[0], st));
-        rc = set_cuda_error(cudaLaunchKernelEx(&cfg, limb_rows_kernel, mapA, mapW, lp, (uint32_t)pipe));
+        rc = set_cuda_error(direct ? cudaLaunchKernelEx(&cfg, limb_rows_kernel<true>, mapA, mapW, lp, (uint32_t)pipe)
+                                   : cudaLaunchKernelEx(&cfg, limb_rows_kernel<false>, mapA, mapW, lp, (uint32_t)pipe));
         if (rc == ZKDS_OK) rc = check_launch();
         if (ev) ZKDS_CUDA(cudaEventRecord(ev[1], st));
         if (ev && rc == ZKDS_OK) return record_launch(p, La, Lb, d_absmax, ev, box);
