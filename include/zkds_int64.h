@@ -95,6 +95,12 @@ int zkds_device_status(int clear);
                                    behind the promised ones) may stay unwritten, and zkds_glu_prepared does not read
                                    them.  For callers that only use the rows of their tokens. */
 
+#define ZKDS_SCORES_32 256       /* zkds_mla_scores with ZKDS_CAUSAL_SKIP, zkds_softmax_pv with causal_skip: the scores are
+                                   int32 words, half the bytes of the largest tensor of a prompt.  Only where the limb
+                                   counts prove every score below 2^31 (both positive; three on three at 23 / 21 bits do):
+                                   otherwise, and for shapes that the kernel does not take, ZKDS_ERR_UNSUPPORTED.  Columns
+                                   that a row does not see are not masked. */
+
 /* =============================================================================
  * Group 1 — the reference's symbols (same names, same argument lists)
  * ========================================================================== */

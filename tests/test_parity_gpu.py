@@ -973,3 +973,51 @@ def test_few_rows_of_experts_behind_an_index(kmod, orc, dev):
     with pytest.raises(kmod.ZkdsError) as e:
         kmod.device_status(sync=True)
     assert e.value.status == kmod.ERR_RANGE
+
+
+@pytest.mark.parametrize("dims", [(1, 4, 128, 4), (1, 5, 128, 68), (2, 130, 8, 132), (1, 300, 16, 300), (1, 33, 48, 1000), (1, 700, 2, 704)])
+@pytest.mark.parametrize("bits,limbs", [((22, 21), (3, 3)), ((30, 21), (4, 3)), ((14, 20), (3, 3))])
+def test_scores_of_several_row_tiles(kmod, orc, dev, dims, bits, limbs):
+    """several row tiles a batch, column tiles that end early or lie beyond the last visible column, fewer limbs in use than
+    promised, scores around the 2^30 up to which their scale is taken in 32 bits"""
+    (Bn, S, H, T), C1, C2 = dims, 512, 64
+    rng = np.random.default_rng(S + T)
+    qa, kv = rand_i64(rng, (Bn, S, H, C1), bits[0]), rand_i64(rng, (Bn, T, C1), bits[1])
+    qp, pe = rand_i64(rng, (Bn, S, H, C2), bits[0] - 2), rand_i64(rng, (Bn, T, C2), bits[1])
+    qa[0, 0, :, :], kv[0, 0, :] = (1 << bits[0]) - 1, (1 << bits[1]) - 1          # the largest
+    want = (orc.einsum_bshc_btc_bsht(qa, kv, 23) + orc.einsum_bshc_btc_bsht(qp, pe, 21)) * 94 // 695
+    mask = np.where(np.arange(T)[None, :] > np.arange(S)[:, None], -(64 << 36), 0).astype(np.int64)[None, :, None, :]
+    args = (g(qa, dev), g(kv, dev), g(qp, dev), g(pe, dev))
+    for dyn in (False, True):
+        kw = dict(a_limbs=limbs[0], b_limbs=limbs[1], dynamic=dyn)
+        same(kmod.mla_scores_fused(*args, **kw), want, "all")
+        same(kmod.mla_scores_fused(*args, causal=True, **kw), want + mask, "masked")
+        got = kmod.mla_scores_fused(*args, causal=True, skip_masked=True, **kw).cpu().numpy()
+        own = np.broadcast_to(mask == 0, got.shape)
+        assert np.array_equal(got[own], want[own])
+    kmod.device_status(sync=True)
+
+
+@pytest.mark.parametrize("dims", [(1, 5, 128, 8), (2, 130, 8, 132), (1, 300, 16, 300), (1, 700, 2, 704)])
+def test_scores_in_32_bits(kmod, dev, dims):
+    """the largest operands that three limbs hold: the same words as in 64 bits in the columns that a row sees, the same context;
+    limbs that prove nothing give 64-bit words"""
+    (Bn, S, H, T), C1, C2 = dims, 512, 64
+    rng = np.random.default_rng(S)
+    top = 128 * (256 ** 3 - 1) // 255
+    qa, kv = (rng.integers(-top, top - 65792, s, dtype=np.int64) for s in ((Bn, S, H, C1), (Bn, T, C1)))
+    qp, pe = rng.integers(-top // 4, top // 4 - 65792, (Bn, S, H, C2), dtype=np.int64), rng.integers(-top, top - 65792, (Bn, T, C2), dtype=np.int64)
+    for s, sign in ((0, 1), (1, -1)):             # sums as large as they get
+        qa[:, s], qp[:, s] = -top * sign if sign > 0 else top - 65793, -top // 4 if sign > 0 else top // 4 - 65793
+    kv[:, 0], pe[:, 0] = -top, -top
+    args, kw = (g(qa, dev), g(kv, dev), g(qp, dev), g(pe, dev)), dict(causal=True, a_limbs=3, b_limbs=3, skip_masked=True)
+    wide, narrow = kmod.mla_scores_fused(*args, **kw), kmod.mla_scores_fused(*args, narrow=True, **kw)
+    assert narrow.dtype == torch.int32
+    own = (torch.arange(T, device=dev)[None, :] <= torch.arange(S, device=dev)[:, None])[None, :, None, :].expand_as(wide)
+    assert torch.equal(narrow.long()[own], wide[own]) and int(wide[own].abs().max()) > 1 << 29
+    kmod.softmax_init_q19()
+    a, b = (kmod.softmax_pv_fused(x, args[1], 23, causal_skip=True, start_pos=0, a_limbs=3, b_limbs=3) for x in (wide, narrow))
+    assert a is not None and torch.equal(a, b)
+    for other in (dict(a_limbs=4), dict(skip_masked=False), dict(a_limbs=0)):
+        assert kmod.mla_scores_fused(*args, narrow=True, **dict(kw, **other)).dtype == torch.int64
+    kmod.device_status(sync=True)

@@ -379,6 +379,17 @@ int zkds_einsum_bshc_btc_bsht_ex(const int64_t* A, const int64_t* KV, int64_t* o
                   "zkds_einsum_bshc_btc_bsht_ex");
 }
 
+// every score that operands of so many limbs can give lies strictly within 32 bits
+static bool scores_fit32(int a_limbs, int b_limbs, int64_t C1, int64_t C2, int64_t rescale1, int64_t rescale2, int64_t mul, int64_t div)
+{
+    if (a_limbs < 1 || b_limbs < 1 || a_limbs > 4 || b_limbs > 4 || C1 > 65536 || C2 > 65536 || mul < 0 || mul > 65536 || div < 0)
+        return false;
+    auto largest = [](int limbs) { return (__int128)128 * ((((int64_t)1 << (8 * limbs)) - 1) / 255); };
+    const __int128 both = largest(a_limbs) * largest(b_limbs);
+    const __int128 sum = (C1 * both >> rescale1) + (C2 * both >> rescale2) + 4;
+    return (div ? sum * mul / div + 1 : sum) < ((int64_t)1 << 31);
+}
+
 int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe, const int64_t* pe,
                     int64_t* out, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C1, int64_t C2,
                     int64_t rescale1, int64_t rescale2, int64_t ep_mul, int64_t ep_div, int causal,
@@ -390,6 +401,12 @@ int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe
     if (B == 0 || S == 0 || H == 0 || T == 0) return finish(ZKDS_OK, "zkds_mla_scores");
     if (!q_abs || !kv || !q_pe || !pe || !out) return finish(ZKDS_ERR_ARG, "zkds_mla_scores");
     cudaStream_t st = ST(stream);
+    const bool narrow = (flags & ZKDS_SCORES_32) != 0;
+    if (narrow && !(causal && (flags & ZKDS_CAUSAL_SKIP) &&
+                    scores_fit32(a_limbs, b_limbs, C1, C2, rescale1, rescale2, ep_mul, ep_div))) {
+        t_status = ZKDS_ERR_UNSUPPORTED;
+        return t_status;
+    }
     if (a_limbs <= 0 || b_limbs <= 0) {
         uint64_t* d = (uint64_t*)workspace(8 * sizeof(uint64_t), 5);
         if (!d) return finish(ZKDS_ERR_WORKSPACE, "zkds_mla_scores");
@@ -420,6 +437,7 @@ int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe
     f.causal_H = causal ? H : 0; f.causal_start = start_pos; f.mask_value = mask_value;
     f.dynamic_a = (flags & ZKDS_LIMBS_DYNAMIC) ? 1 : 0;
     f.skip_tiles = (flags & ZKDS_CAUSAL_SKIP) ? 1 : 0;
+    f.out_bits = narrow ? 32 : 64;
     // ZKDS_ERR_UNSUPPORTED is an expected answer here (the caller then runs the two contractions
     // separately), so it is returned without the stderr line
     int rc = launch_scores_fused(f, a_limbs, b_limbs, st);
@@ -529,6 +547,8 @@ int zkds_softmax_pv(const int64_t* scores, const int64_t* KV, int64_t* out, cons
     cudaStream_t st = ST(stream);
     Contraction p = einsum_problem(2, scores, KV, out, rescale, B, S, H, T, C);
     p.softmax_lut = lut; p.softmax_S = S;
+    p.softmax_bits = flags & ZKDS_SCORES_32 ? 32 : 64;
+    if (p.softmax_bits == 32 && !causal_skip) { t_status = ZKDS_ERR_UNSUPPORTED; return t_status; }
     if (causal_skip) { p.skip_k = 1; p.skip_H = H; p.skip_start = start_pos; }
     p.dynamic_a = ((flags & ZKDS_LIMBS_DYNAMIC) && a_limbs > 0) ? 1 : 0;
     if (a_limbs <= 0) a_limbs = 3;

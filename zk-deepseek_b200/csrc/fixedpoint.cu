@@ -455,12 +455,12 @@ __device__ __forceinline__ PlanesRow planes_row(unsigned row, int T, int64_t Kp,
 // next row is on its way into shared memory (one bulk copy) as soon as this one is in registers.  Everything behind the
 // load runs in 32 bits: scores are clamped from below, and a row that has one above 2^31, or none above the clamp, is read
 // again in 64; a difference from the maximum is cut below 2^23, where the weight is zero; the quotient comes from a 32-bit
-// reciprocal that is never above, and is then itself or one below.  E: groups of four columns a thread.
+// reciprocal that is never above, and is then itself or one below.  E: groups of four columns a thread; S: the scores' words.
 // 4096 tokens of 128 heads, causal (5.9 GB): 4.48 -> 2.72 ms against a block of 256 threads a row; the attention layer around it
 // 25.19 -> 23.43 ms, a dense block of 777 tokens 9.48 -> 9.30, decoding of 64 sequences 3.18 -> 3.11.
-template <int NT, int E, int MINB>
+template <typename S, int NT, int E, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
-softmax_q19_rows_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, int8_t* __restrict__ planes, unsigned rows, int T,
+softmax_q19_rows_kernel(const S* X, const int64_t* __restrict__ lut_g, int8_t* __restrict__ planes, unsigned rows, int T,
                         int64_t Kp, int64_t plane_stride, unsigned long long* absmax_out, int valid_H, int valid_S,
                         int valid_start, int* error_flag)
 {
@@ -475,10 +475,10 @@ softmax_q19_rows_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, int
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar = smem_u32(&s_bar);
-    const longlong2* buf = reinterpret_cast<const longlong2*>(smem_raw);
+    const S* buf = reinterpret_cast<const S*>(smem_raw);
     for (int i = tid; i < 256; i += NT) lut[i] = (uint32_t)lut_g[i];
     auto request = [&](unsigned row) {
-        const uint32_t bytes = (uint32_t)planes_row(row, T, Kp, valid_H, valid_S, valid_start).quads_valid * 32u;
+        const uint32_t bytes = (uint32_t)planes_row(row, T, Kp, valid_H, valid_S, valid_start).quads_valid * (uint32_t)(4 * sizeof(S));
         mbar_expect_tx(bar, bytes);
         bulk_load(smem_u32(smem_raw), X + (int64_t)row * T, bytes, bar);
     };
@@ -500,14 +500,20 @@ softmax_q19_rows_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, int
 #pragma unroll
             for (int h = 0; h < 4; ++h) v[4 * j + h] = INT_MIN;
             if (q < r.quads_valid) {
-                const longlong2 a = buf[2 * q], b = buf[2 * q + 1];
-                const int64_t x[4] = {a.x, a.y, b.x, b.y};
+                S x[4];
+#pragma unroll
+                for (int h = 0; h < 4; h += 16 / (int)sizeof(S))
+                    *reinterpret_cast<int4*>(x + h) = *reinterpret_cast<const int4*>(buf + 4 * q + h);
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
-                    const int lo = (int)x[h], hi = (int)(x[h] >> 32), sign = lo >> 31;
+                    const int lo = (int)x[h];
                     if (4 * q + h < r.valid) {
-                        v[4 * j + h] = hi < sign ? INT_MIN : lo;
-                        flags |= hi > sign ? kTooHigh : 0;
+                        v[4 * j + h] = lo;
+                        if (sizeof(S) == 8) {
+                            const int hi = (int)((int64_t)x[h] >> 32), sign = lo >> 31;
+                            if (hi < sign) v[4 * j + h] = INT_MIN;
+                            flags |= hi > sign ? kTooHigh : 0;
+                        }
                     }
                     mx = max(mx, v[4 * j + h]);
                 }
@@ -526,7 +532,7 @@ softmax_q19_rows_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, int
             for (int q = tid; q < r.quads_valid; q += NT)
                 for (int h = 0; h < 4; ++h)
                     if (4 * q + h < r.valid) {
-                        const int64_t x = reinterpret_cast<const int64_t*>(smem_raw)[4 * q + h];
+                        const int64_t x = buf[4 * q + h];
                         top = x > top ? x : top;
                     }
             top = block_max_i64(top, red64);
@@ -537,7 +543,7 @@ softmax_q19_rows_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, int
                     const int c = 4 * (tid + j * NT) + h;
                     v[4 * j + h] = INT_MIN;
                     if (c < r.valid) {
-                        const uint64_t d = (uint64_t)top - (uint64_t)reinterpret_cast<const int64_t*>(smem_raw)[c];
+                        const uint64_t d = (uint64_t)top - (uint64_t)(int64_t)buf[c];
                         v[4 * j + h] = -(int)(d < kCut ? d : kCut);
                     }
                 }
@@ -682,42 +688,54 @@ softmax_q19_planes_kernel(const int64_t* X, const int64_t* __restrict__ lut_g, i
     }
 }
 
-bool softmax_planes_supported(const int64_t* X, int64_t rows, int64_t T, int64_t Kp)
+bool softmax_planes_supported(const void* X, int64_t rows, int64_t T, int64_t Kp)
 {
     return rows > 0 && rows <= 0x7fffffffll && T >= 4 && (T & 3) == 0 && Kp >= T && (Kp & 3) == 0 &&
            Kp <= 8 * 4 * kThreads && ((uintptr_t)X & 15) == 0;
 }
 
-int launch_softmax_planes(const int64_t* X, const int64_t* lut, int8_t* planes, int L, int64_t rows, int64_t T,
+template <typename S>
+static int softmax_rows(const S* X, const int64_t* lut, int8_t* planes, int64_t rows, int64_t T, int64_t Kp, int64_t plane_stride,
+                        unsigned long long* absmax_out, int64_t valid_H, int64_t valid_S, int64_t valid_start, int* error_flag,
+                        cudaStream_t st)
+{
+    auto run = [&](auto kernel, int threads, int per_sm) {
+        const size_t smem = (size_t)T * sizeof(S);
+        const int64_t fit = (int64_t)(227 * 1024 / (smem + 3072)), blocks = sm_count() * (fit < per_sm ? fit : per_sm);
+        ZKDS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+        kernel<<<(unsigned)(rows < blocks ? rows : blocks), threads, smem, st>>>(
+            X, lut, planes, (unsigned)rows, (int)T, Kp, plane_stride, absmax_out, (int)valid_H, (int)valid_S, (int)valid_start, error_flag);
+        return check_launch();
+    };
+    // 128 threads hold rows of up to 4096 columns, 32 a thread; as many blocks to an SM as registers and rows in shared memory
+    // leave, so that the chains of several rows overlap
+    const int64_t quads = Kp >> 2;
+    if (quads <= 128) return run(softmax_q19_rows_kernel<S, 128, 1, 12>, 128, 12);
+    if (quads <= 256) return run(softmax_q19_rows_kernel<S, 128, 2, 12>, 128, 12);
+    if (quads <= 512) return run(softmax_q19_rows_kernel<S, 128, 4, 10>, 128, 10);
+    if (quads <= 1024) return run(softmax_q19_rows_kernel<S, 128, 8, 7>, 128, 7);
+    return run(softmax_q19_rows_kernel<S, 256, 8, 3>, 256, 3);
+}
+
+int launch_softmax_planes(const void* X, int x_bits, const int64_t* lut, int8_t* planes, int L, int64_t rows, int64_t T,
                           int64_t Kp, int64_t plane_stride, unsigned* overflow, unsigned long long* absmax_out,
                           int64_t valid_H, int64_t valid_S, int64_t valid_start, int* error_flag, cudaStream_t st)
 {
     if (!softmax_planes_supported(X, rows, T, Kp) || L < 1 || L > 9 || valid_H > 0x7fffffff ||
-        valid_S > 0x7fffffff || valid_start > 0x7fffffff)
+        valid_S > 0x7fffffff || valid_start > 0x7fffffff || (x_bits == 32 && L != 3))
         return ZKDS_ERR_UNSUPPORTED;
-    const int vS = valid_S > 0 ? (int)valid_S : 1;
-    if (L == 3) {
-        // 128 threads hold rows of up to 4096 columns, 32 a thread; as many blocks to an SM as registers and rows in shared memory
-        // leave, so that the chains of several rows overlap
-        const int64_t quads = Kp >> 2;
-        auto run = [&](auto kernel, int threads, int per_sm) {
-            const size_t smem = (size_t)T * 8;
-            const int64_t fit = (int64_t)(227 * 1024 / (smem + 3072)), blocks = sm_count() * (fit < per_sm ? fit : per_sm);
-            ZKDS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-            kernel<<<(unsigned)(rows < blocks ? rows : blocks), threads, smem, st>>>(
-                X, lut, planes, (unsigned)rows, (int)T, Kp, plane_stride, absmax_out, (int)valid_H, vS, (int)valid_start, error_flag);
-            return check_launch();
-        };
-        if (quads <= 128) return run(softmax_q19_rows_kernel<128, 1, 12>, 128, 12);
-        if (quads <= 256) return run(softmax_q19_rows_kernel<128, 2, 12>, 128, 12);
-        if (quads <= 512) return run(softmax_q19_rows_kernel<128, 4, 10>, 128, 10);
-        if (quads <= 1024) return run(softmax_q19_rows_kernel<128, 8, 6>, 128, 6);
-        return run(softmax_q19_rows_kernel<256, 8, 3>, 256, 3);
-    }
+    const int64_t vS = valid_S > 0 ? valid_S : 1;
+    if (x_bits == 32)
+        return softmax_rows((const int32_t*)X, lut, planes, rows, T, Kp, plane_stride, absmax_out, valid_H, vS, valid_start,
+                            error_flag, st);
+    if (L == 3)
+        return softmax_rows((const int64_t*)X, lut, planes, rows, T, Kp, plane_stride, absmax_out, valid_H, vS, valid_start,
+                            error_flag, st);
     const int per = (int)(((Kp >> 2) + kThreads - 1) / kThreads);
-#define ZKDS_SP(E)                                                                                                    \
-    softmax_q19_planes_kernel<E><<<(unsigned)rows, kThreads, 0, st>>>(X, lut, planes, L, (int)T, Kp, plane_stride,    \
-                                                                     overflow, absmax_out, (int)valid_H, vS, (int)valid_start)
+#define ZKDS_SP(E)                                                                                                          \
+    softmax_q19_planes_kernel<E><<<(unsigned)rows, kThreads, 0, st>>>((const int64_t*)X, lut, planes, L, (int)T, Kp,        \
+                                                                     plane_stride, overflow, absmax_out, (int)valid_H,     \
+                                                                     (int)vS, (int)valid_start)
     if (per <= 1) ZKDS_SP(1);
     else if (per <= 2) ZKDS_SP(2);
     else if (per <= 4) ZKDS_SP(4);

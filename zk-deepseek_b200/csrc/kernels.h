@@ -40,8 +40,9 @@ int launch_softmax_causal(const int64_t* X, int64_t* C, const int64_t* lut, int6
                           int64_t T, int64_t start, cudaStream_t st);
 // Q19 softmax whose probabilities are written as signed 8-bit limb planes (row pitch Kp, limb l at
 // planes + l * plane_stride); valid_H > 0 restricts row (b, s, h) to columns <= valid_start + s
-bool softmax_planes_supported(const int64_t* X, int64_t rows, int64_t T, int64_t Kp);
-int launch_softmax_planes(const int64_t* X, const int64_t* lut, int8_t* planes, int L, int64_t rows, int64_t T,
+bool softmax_planes_supported(const void* X, int64_t rows, int64_t T, int64_t Kp);
+// x_bits: 64, or 32 with L == 3
+int launch_softmax_planes(const void* X, int x_bits, const int64_t* lut, int8_t* planes, int L, int64_t rows, int64_t T,
                           int64_t Kp, int64_t plane_stride, unsigned* overflow, unsigned long long* absmax_out,
                           int64_t valid_H, int64_t valid_S, int64_t valid_start, int* error_flag, cudaStream_t st);
 int launch_rope(const int64_t* A, const int64_t* Tb, int64_t* C, int64_t batch, int64_t S,
@@ -140,6 +141,7 @@ struct Contraction {
     // (limb kernel only; softmax_S = sequence positions per batch when skip_k is set)
     const int64_t* softmax_lut;
     int64_t softmax_S;
+    int softmax_bits;         // words of the scores: 0 = 64, 32
     // A is r1 of a gated MLP (rows of K words, row stride a_sm): the limb planes are produced from
     // (silu_q23(A) * glu_r2) >> 23, glu_r2 with the same row stride, and the gated product never reaches
     // memory as int64 (limb kernel only, batches == 1)
@@ -176,6 +178,7 @@ struct FusedScores {
     int64_t ep_mul, ep_div, causal_H, causal_start, mask_value;
     int dynamic_a;
     int skip_tiles;   // with causal_H: tiles whose every column is masked are neither computed nor written
+    int out_bits;     // 32: out is int32 (with skip_tiles; limbs that prove every score below 2^31), what a row does not see is not masked
     // B1 | B2 already split (resident cache planes): [Lb][batches][b_batch_rows][K1 + round16(K2)] int8, of
     // which rows [0, N) of every batch are in use; B1 and B2 are then ignored
     const int8_t* b_planes;

@@ -385,6 +385,7 @@ struct LimbParams {
     // epilogue on one plain set in a single 64-column buffer measured slower than the one-tile kernel
     // with 80-column tiles on P.KV: 8.6 against 8.0 ms.)
     int fold_epilogue;
+    int out32;                // merged scores: C holds 32-bit words
     unsigned backoff;         // 1: waiting warps sleep between polls (see mbar_wait), 0: they poll back to back
     // optional wait accounting (null = off): [0] MMA warp cycles waiting for operand stages, [1] for
     // free accumulators, [2] MMA warp total, [3] first epilogue warp cycles waiting for accumulators,
@@ -1651,6 +1652,22 @@ __device__ __forceinline__ void epilogue_part(const LimbParams& p, uint32_t tq, 
     __syncwarp();
 }
 
+// The scores' scale 94 / 695 for quotients that fit 31 bits, once the accumulators have been folded: the addend carries kTailOffset (a
+// multiple of 695 above 2^30) quotients, so that a quotient u is positive; q = floor(u * ceil(94 * 2^32 / 695) / 2^32) is the
+// floor or one above it, and the remainder, exact modulo 2^32, tells which.  About 25 instructions a score where 64-bit quotients,
+// checks and branches were 118.  With 32-bit scores behind it, 4096 tokens of 128 heads: scores 9.05 -> 8.62 ms, the softmax that
+// reads them 2.72 -> 2.32.
+constexpr int kTailTimes = 1544985;
+constexpr uint32_t kTailOffset = 695u * kTailTimes;
+constexpr int kTailScaled = 94 * kTailTimes;
+
+__device__ __forceinline__ int32_t scale_94_695_offset(uint32_t u)
+{
+    const uint32_t q = __umulhi(u, 580902052u);
+    const int32_t r = (int32_t)(u * 94u - q * 695u);
+    return (int32_t)q + (r >> 31) - kTailScaled;
+}
+
 // Epilogue of the merged dual accumulation (one warp: rows 32 q .. 32 q + 31, its CW columns of the
 // tile, CW = 8 or 16).  The diagonals are folded into two running values per column as they arrive
 // (T' = main sum + both addends in 64 bits, r2 = extra sum + scaled second addend modulo 2^32), one
@@ -1666,6 +1683,11 @@ __device__ __forceinline__ void epilogue_merged(const LimbParams& p, uint32_t tq
 {
     int64_t T[CW];
     uint32_t R[EE ? CW : 1];
+    const int sh = p.shift >= 63 ? 63 : p.shift;
+    // scaled scores: see scale_94_695_offset.  The extra set is kept where the quotient's remainder would be (its low `shift`
+    // bits at the top of the word), so that the comparison of the two is a subtraction's borrow.
+    const bool scaled = EE && p.ep_mul == 94 && p.ep_div == 695;
+    const int64_t addend = scaled ? p.addend + ((int64_t)kTailOffset << sh) : p.addend;
     // Fewer, fuller round trips to tensor memory while few values are live: the extra diagonals all at
     // once (nothing else is held yet), then main diagonals 0 and 1 together, then one per wait.
     if (EE) {
@@ -1688,7 +1710,7 @@ __device__ __forceinline__ void epilogue_merged(const LimbParams& p, uint32_t tq
         tmem_ld_wait();
 #pragma unroll
         for (int c = 0; c < CW; ++c) {
-            T[c] = mad_wide(a0[c], 1, p.addend);
+            T[c] = mad_wide(a0[c], 1, addend);
             if (DD > 1) T[c] = mad_wide(a1[c], 1 << 8, T[c]);
         }
     }
@@ -1715,14 +1737,76 @@ __device__ __forceinline__ void epilogue_merged(const LimbParams& p, uint32_t tq
     }
 
     const int64_t m = tc.m0 + q * 32 + lane;
-    const int64_t srow = p.causal_H ? seq_row(m, p.causal_H) : 0;
     const int64_t nbase = tc.n0 + c0;
-    const int sh = p.shift >= 63 ? 63 : p.shift;
+    if (EE && scaled) {
+        // 64 bits only until the quotient.  `high` and `sign` tell whether every quotient of the warp was one of 31 bits
+        uint32_t u[CW], high = 0, sign = 0;
+#pragma unroll
+        for (int c = 0; c < CW; ++c) {
+            const uint32_t lo = (uint32_t)T[c], hi = (uint32_t)((uint64_t)T[c] >> 32);
+            const uint32_t v = __funnelshift_r(lo, hi, sh);
+            asm("{\n\t.reg .u32 t;\n\tsub.cc.u32 t, %1, %2;\n\tsubc.u32 %0, %3, 0;\n\t}"
+                : "=r"(u[c]) : "r"(lo << (32 - sh)), "r"(R[EE ? c : 0] << (32 - sh)), "r"(v));
+            high |= hi;
+            sign |= u[c];
+        }
+        // columns that this row sees, of CW; all of them except at the diagonal
+        int seen = CW;
+        if (p.causal_H) {
+            const int64_t left = p.causal_start + seq_row(m, p.causal_H) + 1 - nbase;
+            seen = left < CW ? (left < 0 ? 0 : (int)left) : CW;
+        }
+        if (__all_sync(0xffffffffu, (high >> sh) == 0 && (int32_t)sign >= 0)) {
+            if (m >= p.M) return;
+            const int64_t at = tc.z * p.c_sz + m * p.c_sm + nbase;
+            if (p.out32) {
+                int32_t* crow = reinterpret_cast<int32_t*>(p.C) + at;
+                const bool wide = (((uintptr_t)p.C & 15) | (uintptr_t)((p.c_sm | p.c_sz) & 3)) == 0 && nbase + CW <= p.N;
+#pragma unroll
+                for (int c = 0; c < CW; c += 4) {
+                    int32_t o[4];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) o[h] = scale_94_695_offset(u[c + h]);
+                    if (wide) *reinterpret_cast<int4*>(crow + c) = make_int4(o[0], o[1], o[2], o[3]);
+                    else
+#pragma unroll
+                        for (int h = 0; h < 4; ++h)
+                            if (nbase + c + h < p.N) crow[c + h] = o[h];
+                }
+                return;
+            }
+            int64_t* crow = p.C + at;
+            const bool wide = (((uintptr_t)p.C & 31) | (uintptr_t)((p.c_sm | p.c_sz) & 3)) == 0 && nbase + CW <= p.N;
+#pragma unroll
+            for (int c = 0; c < CW; c += 4) {
+                int64_t o[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    o[h] = scale_94_695_offset(u[c + h]);
+                    if (c + h >= seen) o[h] = (int64_t)((uint64_t)o[h] + (uint64_t)p.mask_value);
+                }
+                if (wide)
+                    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(crow + c), "l"(o[0]), "l"(o[1]),
+                                 "l"(o[2]), "l"(o[3])
+                                 : "memory");
+                else
+#pragma unroll
+                    for (int h = 0; h < 4; ++h)
+                        if (nbase + c + h < p.N) crow[c + h] = o[h];
+            }
+            return;
+        }
+#pragma unroll
+        for (int c = 0; c < CW; ++c) T[c] -= (int64_t)kTailOffset << sh;
+    }
+
+    const int64_t srow = p.causal_H ? seq_row(m, p.causal_H) : 0;
     const uint32_t mask = EE ? (1u << p.shift) - 1u : 0u;
     const bool tail = p.ep_div || p.causal_H;
     // each thread owns CW consecutive words of one output row: 32-byte stores (one full sector each)
     int64_t* crow = p.C + tc.z * p.c_sz + m * p.c_sm + nbase;
-    const bool wide_ok = ((((uintptr_t)p.C) & 31) == 0) && ((p.c_sm & 3) == 0) && ((p.c_sz & 3) == 0) &&
+    int32_t* crow32 = p.out32 ? reinterpret_cast<int32_t*>(p.C) + tc.z * p.c_sz + m * p.c_sm + nbase : nullptr;
+    const bool wide_ok = !crow32 && ((((uintptr_t)p.C) & 31) == 0) && ((p.c_sm & 3) == 0) && ((p.c_sz & 3) == 0) &&
                          nbase + CW <= p.N;
     if (m < p.M) {
 #pragma unroll
@@ -1742,7 +1826,10 @@ __device__ __forceinline__ void epilogue_merged(const LimbParams& p, uint32_t tq
             } else {
 #pragma unroll
                 for (int h = 0; h < 4; ++h)
-                    if (nbase + c + h < p.N) crow[c + h] = o[h];
+                    if (nbase + c + h < p.N) {
+                        if (crow32) crow32[c + h] = (int32_t)o[h];
+                        else crow[c + h] = o[h];
+                    }
             }
         }
     }
@@ -2684,7 +2771,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         // limb_rows_kernel reads the activations itself
     } else if (p.softmax_lut) {
         if (p.a_sm != p.K || p.a_sz != p.M * p.K || p.a_div != 1) return ZKDS_ERR_ARG;
-        rc = launch_softmax_planes(p.A, p.softmax_lut, pa, La, a_rows, p.K, Kp, a_rows * Kp, fl->overflow_dev,
+        rc = launch_softmax_planes(p.A, p.softmax_bits ? p.softmax_bits : 64, p.softmax_lut, pa, La, a_rows, p.K, Kp, a_rows * Kp, fl->overflow_dev,
                                    d_absmax, p.skip_k ? p.skip_H : 0, p.softmax_S, p.skip_start, fl->dev, st);
     } else if (p.glu_lut) {
         if (p.batches != 1 || p.a_div != 1 || p.a_row_index || !p.glu_r2) return ZKDS_ERR_ARG;
@@ -2960,7 +3047,7 @@ int launch_scores_fused(const FusedScores& f, int La, int Lb, cudaStream_t st)
         }
         if (NT) break;
     }
-    if (!NT) return ZKDS_ERR_UNSUPPORTED;
+    if (!NT || (f.out_bits == 32 && !E)) return ZKDS_ERR_UNSUPPORTED;
     const int64_t Kp2 = (f.K2 + 15) & ~(int64_t)15;
     const int64_t pitch = f.K1 + Kp2;
     if (f.b_planes && (f.b_batch_rows < f.N || (((uintptr_t)f.b_planes) & 15))) return ZKDS_ERR_ARG;
@@ -3011,6 +3098,7 @@ int launch_scores_fused(const FusedScores& f, int La, int Lb, cudaStream_t st)
     lp.split_release = (nbuf == 1 && (E || !switches().no_split_release)) ? 1 : 0;
     lp.merged_E = E;
     lp.fold_epilogue = E ? 1 : 0;
+    lp.out32 = f.out_bits == 32 ? 1 : 0;
     lp.M = f.M; lp.N = f.N; lp.batches = f.batches;
     lp.a_rows_per_limb = a_rows; lp.b_rows_per_limb = b_rows; lp.b_batch_rows = f.b_planes ? f.b_batch_rows : f.N;
     lp.b_batched = 1;
@@ -3028,7 +3116,7 @@ int launch_scores_fused(const FusedScores& f, int La, int Lb, cudaStream_t st)
     lp.a_absmax = d_absmax;
     lp.overflow_flag = fl->overflow_dev;
     lp.ep_mul = f.ep_mul; lp.ep_div = f.ep_div;
-    lp.causal_H = f.causal_H; lp.causal_start = f.causal_start; lp.mask_value = f.mask_value;
+    lp.causal_H = f.out_bits == 32 ? 0 : f.causal_H; lp.causal_start = f.causal_start; lp.mask_value = f.mask_value;
     lp.skip_tiles = (f.skip_tiles && f.causal_H) ? 1 : 0; lp.skip_H = f.causal_H; lp.skip_start = f.causal_start;
     int64_t panel = (32ll << 20) / ((int64_t)La * kTileM * pitch);
     if (panel < 1) panel = 1;

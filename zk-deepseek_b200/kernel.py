@@ -35,6 +35,7 @@ ALGO_AUTO, ALGO_EXACT, ALGO_LIMB = 0, 1, 2
 REMAINDER_LEGACY = 4
 LIMBS_DYNAMIC = 8
 CAUSAL_SKIP = 16
+SCORES_32 = 256
 SOFTMAX_PLANES_COLUMNS = 8192      # columns that the softmax in front of P . KV takes (a row in a block's registers)
 GROUP_ROWS_32, GROUP_ROWS_64, GROUP_LEAVE_PADDING = 32, 64, 128
 
@@ -514,28 +515,38 @@ def attention_scores_fused(A, KV, rescale, addin=None, mul=0, div=0, causal=Fals
     return C
 
 
+def _scores_fit32(a_limbs, b_limbs, C1, C2, rescale1, rescale2, mul, div):
+    """every score of operands of so many limbs lies within 32 bits (the library checks the same)"""
+    if not (1 <= a_limbs <= 4 and 1 <= b_limbs <= 4 and div > 0):
+        return False
+    both = (128 * (256 ** a_limbs - 1) // 255) * (128 * (256 ** b_limbs - 1) // 255)
+    return ((C1 * both >> rescale1) + (C2 * both >> rescale2) + 4) * mul // div + 1 < 1 << 31
+
+
 def mla_scores_fused(q_abs, kv, q_pe, pe, rescale1=23, rescale2=21, mul=94, div=695, causal=False,
                      start_pos=0, mask_value=-(64 << 36), a_limbs=0, b_limbs=0, dynamic=False,
-                     skip_masked=False):
+                     skip_masked=False, narrow=False):
     """scores = ((score1 + score2) * mul // div) (+ causal mask) with score1 = einsum(q_abs, kv) at
     rescale1 and score2 = einsum(q_pe, pe) at rescale2, in one tensor-core pass (model.py:884-905).
-    Returns None when the fused kernel does not take the shape (caller falls back)."""
+    narrow (with causal and skip_masked): int32 scores where the limbs prove them to fit.  Returns None when the fused
+    kernel does not take the shape (caller falls back)."""
     for t, n in ((q_abs, "q_abs"), (kv, "kv"), (q_pe, "q_pe"), (pe, "pe")):
         _dev_i64(t, n)
     Bn, S, H, C1 = q_abs.shape
     T, C2 = kv.shape[1], q_pe.shape[3]
     assert kv.shape == (Bn, T, C1) and q_pe.shape == (Bn, S, H, C2) and pe.shape == (Bn, T, C2)
-    out = torch.empty((Bn, S, H, T), dtype=torch.int64, device=q_abs.device)
-    with _on(q_abs.device):
-        rc = lib.zkds_mla_scores(q_abs.data_ptr(), kv.data_ptr(), q_pe.data_ptr(), pe.data_ptr(), out.data_ptr(),
-                                 Bn, S, H, T, C1, C2, int(rescale1), int(rescale2), int(mul), int(div),
-                                 1 if causal else 0, int(start_pos), int(mask_value), a_limbs, b_limbs,
-                                 _a_flags(a_limbs, dynamic) | (CAUSAL_SKIP if (skip_masked and causal) else 0),
-                                 _stream())
-    if rc == 6:          # ZKDS_ERR_UNSUPPORTED
-        return None
-    _check(rc, "mla_scores_fused")
-    return out
+    flags = _a_flags(a_limbs, dynamic) | (CAUSAL_SKIP if (skip_masked and causal) else 0)
+    narrow = narrow and skip_masked and causal and _scores_fit32(a_limbs, b_limbs, C1, C2, rescale1, rescale2, mul, div)
+    for dtype, f in ((torch.int32, flags | SCORES_32), (torch.int64, flags)) if narrow else ((torch.int64, flags),):
+        out = torch.empty((Bn, S, H, T), dtype=dtype, device=q_abs.device)
+        with _on(q_abs.device):
+            rc = lib.zkds_mla_scores(q_abs.data_ptr(), kv.data_ptr(), q_pe.data_ptr(), pe.data_ptr(), out.data_ptr(),
+                                     Bn, S, H, T, C1, C2, int(rescale1), int(rescale2), int(mul), int(div),
+                                     1 if causal else 0, int(start_pos), int(mask_value), a_limbs, b_limbs, f, _stream())
+        if rc != 6:          # ZKDS_ERR_UNSUPPORTED
+            _check(rc, "mla_scores_fused")
+            return out
+    return None
 
 
 class CachePlanes:
@@ -669,16 +680,18 @@ def softmax_pv_fused(scores, kv, rescale=23, causal_skip=False, start_pos=0, a_l
     """einsum_bsht_btc_bshc(softmax_q19(scores), kv, rescale) in one call: scores [B, S, H, T], kv
     [B, T, C] -> [B, S, H, C] (model.py:911-926).  The probabilities go from the softmax kernel straight
     into the limb planes of the contraction and are never stored as int64; `scores` is not modified.
-    causal_skip: only columns t <= start_pos + s of a row are read.  Returns None when the kernel does
-    not take the shape (use softmax_q19 and the einsum then)."""
-    _dev_i64(scores, "scores")
+    causal_skip: only columns t <= start_pos + s of a row are read; scores may then be int32.  Returns None when the
+    kernel does not take the shape (use softmax_q19 and the einsum then)."""
+    narrow = causal_skip and scores.dtype == torch.int32
+    if not (narrow and scores.is_cuda and scores.is_contiguous()):
+        _dev_i64(scores, "scores")
     _dev_i64(kv, "kv")
     Bn, S, H, T = scores.shape
     Cd = kv.shape[2]
     assert Bn == kv.shape[0] and T == kv.shape[1]
     lut = _lut_on(EXP2_FRAC_LUT_Q19, scores.device, "softmax_init_q19")
     out = torch.empty((Bn, S, H, Cd), dtype=torch.int64, device=scores.device)
-    flags = ALGO_LIMB | (LIMBS_DYNAMIC if dynamic else 0)
+    flags = ALGO_LIMB | (LIMBS_DYNAMIC if dynamic else 0) | (SCORES_32 if narrow else 0)
     with _on(scores.device):
         rc = lib.zkds_softmax_pv(scores.data_ptr(), kv.data_ptr(), out.data_ptr(), lut.data_ptr(), int(rescale),
                                  Bn, S, H, T, Cd, 1 if causal_skip else 0, int(start_pos), a_limbs, b_limbs,

@@ -530,12 +530,13 @@ class MLA(nn.Module):
             skip = causal and wanted and not snark and dyn and bl > 0
             scores = K.mla_scores_fused(q_abs, kv_in, q_pe.contiguous(), pe_in, 23, 21, self.softmax_scale1,
                                         self.softmax_scale2, causal=causal, a_limbs=al, b_limbs=bl, dynamic=dyn,
-                                        skip_masked=skip)
+                                        skip_masked=skip, narrow=skip)
             if scores is not None and skip:
                 ctx = K.softmax_pv_fused(scores, kv_in, 23, causal_skip=True, start_pos=0, a_limbs=3, b_limbs=bl)
                 if ctx is not None:
                     del scores
                     return ctx
+                scores = scores.long()
                 probs = torch.empty_like(scores)
                 if K.softmax_q19_causal(scores, probs, 0):
                     del scores
