@@ -2114,6 +2114,287 @@ limb_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
 }
 
 // ------------------------------------------------------------------------------------
+// plain contractions: tile after tile, the epilogue under the next tile's MMAs
+// ------------------------------------------------------------------------------------
+// A tile's sums fill most of tensor memory, so a CTA of limb_gemm_kernel multiplies, then stores, and nothing of the one runs
+// under the other: at K = 1536 half of its time, at K = 2048 a third.  Here a CTA stays and walks tiles.  Sixteen epilogue warps
+// fold the diagonals of their columns into 64 or 128 bits as they read them, hand tensor memory back as soon as the last are in
+// registers, and shift and store while the next tile's MMAs run; narrow tiles have two buffers.  About 20 instructions an
+// output, stored from registers in whole 32-byte sectors.
+// Contractions of the attention layer, 4096 tokens: 9.4 -> 7.7 ms; 32 routed experts of 1001 tokens 3154 -> 2762 us, a dense block of
+// 777 tokens at the reference's magnitudes 9.30 -> 8.86 ms.
+constexpr int kTileWarps = 16, kTileThreads = 64 + 32 * kTileWarps;
+
+struct TileStore {
+    int64_t* c;               // this lane's row of C at the tile's first column
+    int64_t n0;               // that column
+    int shift;
+    bool row_ok, wide;        // wide: 32-byte stores stay aligned
+};
+
+template <int W>
+__device__ __forceinline__ void tile_store(const LimbParams& p, const TileStore& t, int col, const int64_t (&q)[W])
+{
+#pragma unroll
+    for (int c = 0; c < W; c += 4) {
+        if (t.wide && t.n0 + col + c + 4 <= p.N) {
+            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(t.c + col + c), "l"(q[c]), "l"(q[c + 1]), "l"(q[c + 2]),
+                         "l"(q[c + 3])
+                         : "memory");
+        } else {
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+                if (t.n0 + col + c + h < p.N) t.c[col + c + h] = q[c + h];
+        }
+    }
+}
+
+// W columns from `col` on of a tile whose sums fit 64 bits, DD diagonals.  `loaded` runs once they are in registers
+template <int DD, int W, typename F>
+__device__ __forceinline__ void tile_columns(const LimbParams& p, const TileStore& t, uint32_t tq, int col, const F& loaded)
+{
+    int64_t T[W];
+#pragma unroll
+    for (int d = 0; d < DD; d += 2) {
+        int32_t a[W], b[W];
+        tmem_ldn(tq + (uint32_t)(d * p.NT + col), a);
+        if (d + 1 < DD) tmem_ldn(tq + (uint32_t)((d + 1) * p.NT + col), b);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < W; ++c) {
+            if (d == 0) T[c] = mad_wide(a[c], 1, p.addend);
+            else if (d == 2) T[c] = mad_wide(a[c], 1 << 16, T[c]);
+            else T[c] = (int64_t)((uint64_t)T[c] + ((uint64_t)(uint32_t)a[c] << 32));     // only reaches the upper word
+            if (d + 1 < DD) {
+                if (d == 0) T[c] = mad_wide(b[c], 1 << 8, T[c]);
+                else if (d == 2) T[c] = mad_wide(b[c], 1 << 24, T[c]);
+                else T[c] = (int64_t)((uint64_t)T[c] + ((uint64_t)(uint32_t)b[c] << 40));
+            }
+        }
+    }
+    loaded();
+    if (!t.row_ok) return;
+    const int sh = t.shift >= 63 ? 63 : t.shift;
+#pragma unroll
+    for (int c = 0; c < W; ++c) T[c] >>= sh;
+    tile_store(p, t, col, T);
+}
+
+// four columns of any other sum, up to eight diagonals: two words of four diagonals each
+template <typename F>
+__device__ __forceinline__ void tile_columns_128(const LimbParams& p, const TileStore& t, uint32_t tq, int D, int col, const F& loaded)
+{
+    int64_t low[4], high[4] = {};
+    int32_t a[8][4];
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+        if (d < D) tmem_ldn(tq + (uint32_t)(d * p.NT + col), a[d]);
+        else a[d][0] = a[d][1] = a[d][2] = a[d][3] = 0;
+    }
+    tmem_ld_wait();
+    loaded();
+    if (!t.row_ok) return;
+    int64_t q[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        low[c] = four_diagonals(a[0][c], a[1][c], a[2][c], a[3][c]);
+        high[c] = four_diagonals(a[4][c], a[5][c], a[6][c], a[7][c]);
+        i128w v = add128(make_i128(low[c]), make_i128(p.addend));
+        v = add128(v, i128w{(uint64_t)high[c] << 32, high[c] >> 32});
+        q[c] = sar128_lo(v, t.shift);
+    }
+    tile_store(p, t, col, q);
+}
+
+template <int W, typename F>
+__device__ __forceinline__ void tile_columns_64(const LimbParams& p, const TileStore& t, uint32_t tq, int D, int col, const F& loaded)
+{
+    switch (D) {              // as many as a 62-bit sum can have
+    case 1: tile_columns<1, W>(p, t, tq, col, loaded); break;
+    case 2: tile_columns<2, W>(p, t, tq, col, loaded); break;
+    case 3: tile_columns<3, W>(p, t, tq, col, loaded); break;
+    case 4: tile_columns<4, W>(p, t, tq, col, loaded); break;
+    case 5: tile_columns<5, W>(p, t, tq, col, loaded); break;
+    default: tile_columns<6, W>(p, t, tq, col, loaded); break;
+    }
+}
+
+__global__ void __launch_bounds__(kTileThreads, 1)
+limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LimbParams p)
+{
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * 8 + 4];
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int La = p.La;
+    if (p.a_absmax) {
+        const int need = limbs_needed_dev(*p.a_absmax);
+        if (need > La) {
+            if (threadIdx.x == 0 && blockIdx.x == 0) *p.overflow_flag = 1u;
+        } else La = need;
+    }
+    const int D = La + p.Lb - 1;
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t a_bytes = (uint32_t)p.La * kTileM * kBlockK, b_bytes = (uint32_t)p.Lb * p.NT * kBlockK;
+    const uint32_t stage_bytes = a_bytes + b_bytes;
+    const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = smem_u32(&bars[8]);
+    const uint32_t bar_tfull = smem_u32(&bars[16]), bar_tempty = smem_u32(&bars[18]);      // [2]: sums complete; read and cleared
+    const int buf_cols = (p.La + p.Lb - 1) * p.NT;
+    const int64_t total = p.batches * p.m_tiles * p.n_tiles;
+    volatile int* abort_flag = &s_abort;
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < p.stages; ++s) {
+            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_tfull + 8 * b, 1);
+            mbar_init(bar_tempty + 8 * b, kTileWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&s_tmem_base), p.tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem_base;
+
+    // K blocks of a tile: under skip_k its rows see nothing beyond column skip_start + s_max
+    auto blocks_of = [&](const TileCoord& tc) {
+        if (!p.skip_k) return p.kblocks;
+        const int64_t last = tc.m0 + kTileM - 1 < p.M - 1 ? tc.m0 + kTileM - 1 : p.M - 1;
+        const int64_t need = (p.skip_start + seq_row(last, p.skip_H) + 1 + kBlockK - 1) / kBlockK;
+        return need < 1 ? 1 : need < p.kblocks ? (int)need : p.kblocks;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint32_t tx_bytes = (uint32_t)La * kTileM * kBlockK + b_bytes;
+            int s = 0, armed = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int64_t tile = blockIdx.x; ok && tile < total; tile += gridDim.x) {
+                const TileCoord tc = decode_tile(p, tile);
+                if (tc.group < 0) continue;
+                const int64_t zb = p.tile_group ? tc.group : (p.b_batched ? tc.z : 0);
+                const int a_row = (int)(tc.z * p.M + tc.m0), b_row = (int)(zb * p.b_batch_rows + tc.n0), n_blocks = blocks_of(tc);
+                for (int kb = 0; kb < n_blocks; ++kb) {
+                    if (!(ok = mbar_wait(bar_empty + 8 * s, phase ^ 1u, abort_flag, 96u * p.backoff))) break;
+                    const uint32_t full = bar_full + 8 * s, sa = smem_base + s * stage_bytes, sb = sa + a_bytes;
+                    mbar_expect_tx(full, tx_bytes);
+                    for (int i = 0; i < La; ++i)
+                        tma_load_2d(sa + i * (kTileM * kBlockK), &tmA, kb * kBlockK, (int)(i * p.a_rows_per_limb) + a_row, full);
+                    for (int j = 0; j < p.Lb; ++j)
+                        tma_load_2d(sb + j * (p.NT * kBlockK), &tmB, kb * kBlockK, (int)(j * p.b_rows_per_limb) + b_row, full);
+                    armed |= 1 << s;
+                    if (++s == p.stages) { s = 0; phase ^= 1u; }
+                }
+            }
+            if (*abort_flag)
+                // leave no copy in flight: wait (bounded) for what was armed last in every stage
+                for (int i = 0; i < p.stages; ++i)
+                    for (uint32_t it = 0; (armed >> i & 1) && it < kSpinLimit; ++it)
+                        if (mbar_try(bar_full + 8 * i, i < s ? phase : phase ^ 1u)) break;
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((p.Lb * p.NT) >> 3) << 17) |
+                                   ((uint32_t)(kTileM >> 4) << 24);
+            int s = 0, buf = 0;
+            uint32_t phase = 0, turn = 0;
+            bool ok = true;
+            for (int64_t tile = blockIdx.x; ok && tile < total; tile += gridDim.x) {
+                const TileCoord tc = decode_tile(p, tile);
+                if (tc.group < 0) continue;
+                const int n_blocks = blocks_of(tc);
+                if (!(ok = mbar_wait(bar_tempty + 8 * buf, turn, abort_flag, 24u * p.backoff))) break;
+                tc_fence_after();
+                const uint32_t acc = tmem + (uint32_t)(buf * buf_cols);
+                for (int kb = 0; kb < n_blocks; ++kb) {
+                    if (!(ok = mbar_wait(bar_full + 8 * s, phase, abort_flag, 24u * p.backoff))) break;
+                    tc_fence_after();
+                    const uint32_t sa = smem_base + s * stage_bytes;
+                    int ks_n = kBlockK / 32;          // a partial last block: the copy fills it with zeros, which need no products
+                    const int64_t left = p.k_extent - (int64_t)kb * kBlockK;
+                    if (left < kBlockK) ks_n = (int)((left + 31) >> 5);
+                    issue_k_block_n(La, acc, (uint32_t)p.NT, sa, sa + a_bytes, idesc, kb ? 1u : 0u, ks_n);
+                    umma_commit(bar_empty + 8 * s);
+                    if (++s == p.stages) { s = 0; phase ^= 1u; }
+                }
+                if (ok) umma_commit(bar_tfull + 8 * buf);
+                if (++buf == p.nbuf) { buf = 0; turn ^= 1u; }
+            }
+        }
+    } else {
+        const int ew = warp - 2, q = warp & 3, CW = p.NT / (kTileWarps / 4), c0 = (ew >> 2) * CW;
+        const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
+        // clears the columns that no first MMA overwrites, of W columns from col on
+        auto clear = [&](uint32_t tq, int col, int W) {
+            for (int d = p.Lb; d < D; ++d)
+                for (int c = 0; c < W; c += 4) tmem_st4_zero(tq + (uint32_t)(d * p.NT + col + c));
+        };
+        auto hand_back = [&](int buf) {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+        };
+        for (int b = 0; b < p.nbuf; ++b) {
+            clear(lanes + (uint32_t)(b * buf_cols), c0, CW);
+            hand_back(b);
+        }
+        int buf = 0;
+        uint32_t turn = 0;
+        const bool wide = ((uintptr_t)p.C & 31) == 0 && ((p.c_sm | p.c_sz) & 3) == 0;
+        for (int64_t tile = blockIdx.x; tile < total; tile += gridDim.x) {
+            const TileCoord tc = decode_tile(p, tile);
+            if (tc.group < 0) {
+                // unused row tile: its output is defined as zero unless nobody reads it
+                if (!p.leave_padding)
+                    for (int i = ew * 32 + lane; i < kTileM * p.NT; i += kTileWarps * 32) {
+                        const int64_t r = tc.m0 + i / p.NT, c = tc.n0 + i % p.NT;
+                        if (r < p.M && c < p.N) p.C[r * p.c_sm + c] = 0;
+                    }
+                continue;
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * buf, turn, abort_flag, 48u * p.backoff))) break;
+            tc_fence_after();
+            const uint32_t tq = lanes + (uint32_t)(buf * buf_cols);
+            const int64_t m = tc.m0 + q * 32 + lane, at = tc.z * p.c_sz + m * p.c_sm + tc.n0;
+            TileStore t;
+            t.c = p.C + at;
+            t.n0 = tc.n0; t.row_ok = m < p.M; t.wide = wide;
+            for (int col = c0; col < c0 + CW;) {
+                // the shift belongs to the group and to the side of n_split (a multiple of 8) that the columns lie on
+                t.shift = p.group_shift ? p.group_shift[2 * tc.group + (tc.n0 + col >= p.n_split ? 1 : 0)] : p.shift;
+                const int left = c0 + CW - col;
+                const bool split_ahead = p.group_shift && tc.n0 + col < p.n_split && tc.n0 + col + 16 > p.n_split;
+                const int W = !p.fits64 ? 4 : left >= 16 && !split_ahead ? 16 : left >= 8 && !(col & 7) ? 8 : 4;
+                auto loaded = [&]() {
+                    clear(tq, col, W);
+                    if (col + W >= c0 + CW) hand_back(buf);
+                };
+                if (!p.fits64) tile_columns_128(p, t, tq, D, col, loaded);
+                else if (W == 16) tile_columns_64<16>(p, t, tq, D, col, loaded);
+                else if (W == 8) tile_columns_64<8>(p, t, tq, D, col, loaded);
+                else tile_columns_64<4>(p, t, tq, D, col, loaded);
+                col += W;
+            }
+            if (++buf == p.nbuf) { buf = 0; turn ^= 1u; }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc(tmem, p.tmem_cols);
+    if (threadIdx.x == 0 && s_abort) *p.error_flag = 1;
+}
+
+// ------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------
 
@@ -2447,7 +2728,7 @@ static int allow_big_smem(K kernel, bool (&done)[64])
     }
     return ZKDS_OK;
 }
-static bool g_attr_onetile[64], g_attr_rows[64], g_attr_direct[64], g_attr_p16[64], g_attr_p8[64];
+static bool g_attr_onetile[64], g_attr_rows[64], g_attr_tiles[64], g_attr_direct[64], g_attr_p16[64], g_attr_p8[64];
 
 static cudaEvent_t* timing_events()
 {
@@ -2750,6 +3031,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
             }
         }
     }
+    // plain epilogues: limb_tiles_kernel, at shallow K in two buffers where they fit.  What is left to the other two: fewer than half
+    // as many tiles as SMs with a K that can be shared, boxes of few rows, remainders, element-wise tails, more than eight diagonals.
     if (persistent) NT = pNT;
     const int64_t nt_eff = (p.N + NT - 1) / NT;
 
@@ -2943,6 +3226,17 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
         }
     }
 
+    const bool tiles = !by_rows && !p.R && lp.ksplit == 1 && a_box == kTileM && !p.skip_tiles && !p.addin && !p.ep_div && !p.causal_H &&
+                       (lp.fits64 ? D <= 6 : D <= 8) && !switches().no_persistent;
+    if (tiles) {
+        lp.backoff = switches().no_backoff ? 0u : 1u;
+        lp.nbuf = 2 * D * NT <= 512 ? 2 : 1;
+        lp.stages = stages = (int)(smem_max / ((size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK));
+        if (stages > 8) lp.stages = stages = 8;
+        stage_bytes = (size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK;
+        lp.tmem_cols = 32;
+        while (lp.tmem_cols < (uint32_t)(lp.nbuf * D * NT)) lp.tmem_cols <<= 1;
+    }
     size_t smem = stage_bytes * stages + 1024;
     // more than half the shared memory per CTA keeps one CTA per SM, so its tensor-memory
     // allocation can never wait for a co-resident CTA
@@ -2958,7 +3252,14 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
                              : dim3((unsigned)(mt * nt_eff * lp.ksplit), 1, (unsigned)p.batches);
     cudaEvent_t* ev = timing_events();
     if (ev) ZKDS_CUDA(cudaEventRecord(ev[0], st));
-    if (persistent) {
+    if (tiles) {
+        const int64_t total_tiles = p.batches * mt * nt_eff;
+        if (total_tiles > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
+        rc = allow_big_smem(limb_tiles_kernel, g_attr_tiles);
+        if (rc != ZKDS_OK) return rc;
+        limb_tiles_kernel<<<(unsigned)(total_tiles < sm_count() ? total_tiles : sm_count()), kTileThreads, smem, st>>>(tmA, tmB, lp);
+        rc = check_launch();
+    } else if (persistent) {
         if (psmem < 120 * 1024) psmem = 120 * 1024;
         int64_t total_tiles = p.batches * mt * nt_eff;
         if (total_tiles > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
