@@ -283,7 +283,7 @@ split_rows_kernel(const T* __restrict__ X, int8_t* __restrict__ planes, int L, i
 // for the K block that opens a set of accumulators (its very first MMA then overwrites).
 template <int LA>
 __device__ __forceinline__ void issue_k_block(uint32_t acc, uint32_t nt_cols, uint32_t sa, uint32_t sb,
-                                              uint32_t idesc, uint32_t first_accumulates, int ks_n,
+                                              uint32_t idesc, uint32_t first_accumulates, int ks_n, uint32_t one,
                                               uint32_t a_stride16 = (128 * 128) >> 4)
 {
     const uint64_t hi = smem_desc_sw128(0) & 0xFFFFFFFF00000000ull;
@@ -297,34 +297,33 @@ __device__ __forceinline__ void issue_k_block(uint32_t acc, uint32_t nt_cols, ui
             for (int i = 0; i < LA; ++i) {
                 const uint64_t adesc = hi | (uint64_t)(a_lo + (uint32_t)i * a_stride16 + (uint32_t)(ks * 2));
                 const uint64_t bdesc = hi | (uint64_t)(b_lo + (uint32_t)(ks * 2));
-                if (ks == 0 && i == 0) umma_i8(acc, adesc, bdesc, idesc, first_accumulates);
-                else umma_i8_acc(acc + (uint32_t)i * nt_cols, adesc, bdesc, idesc);
+                umma_i8(acc + (uint32_t)i * nt_cols, adesc, bdesc, idesc, ks == 0 && i == 0 ? first_accumulates : 1u, one);
             }
         }
     }
 }
 
 __device__ __forceinline__ void issue_k_block_n(int La, uint32_t acc, uint32_t nt_cols, uint32_t sa, uint32_t sb,
-                                                uint32_t idesc, uint32_t first_accumulates, int ks_n,
+                                                uint32_t idesc, uint32_t first_accumulates, int ks_n, uint32_t one,
                                                 uint32_t a_stride16 = (128 * 128) >> 4)
 {
     switch (La) {
-    case 1: issue_k_block<1>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    case 2: issue_k_block<2>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    case 3: issue_k_block<3>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    case 4: issue_k_block<4>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    case 5: issue_k_block<5>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    case 6: issue_k_block<6>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    case 7: issue_k_block<7>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    case 8: issue_k_block<8>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
-    default: issue_k_block<9>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, a_stride16); break;
+    case 1: issue_k_block<1>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    case 2: issue_k_block<2>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    case 3: issue_k_block<3>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    case 4: issue_k_block<4>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    case 5: issue_k_block<5>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    case 6: issue_k_block<6>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    case 7: issue_k_block<7>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    case 8: issue_k_block<8>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
+    default: issue_k_block<9>(acc, nt_cols, sa, sb, idesc, first_accumulates, ks_n, one, a_stride16); break;
     }
 }
 
 // Merged dual accumulation, second part only: limb i of A against the lowest E - i limb tiles of the B
 // stack lands on diagonals i .. E-1 of the extra set (a handful of MMAs per tile, so a plain loop).
 __device__ __forceinline__ void issue_extra_block(int La, int E, uint32_t acc_extra, uint32_t nt_cols, uint32_t sa,
-                                                  uint32_t sb, uint32_t idesc, bool opens_set, int ks_n)
+                                                  uint32_t sb, uint32_t idesc, bool opens_set, int ks_n, uint32_t one)
 {
     for (int ks = 0; ks < ks_n; ++ks) {
         for (int i = 0; i < La && i < E; ++i) {
@@ -332,7 +331,7 @@ __device__ __forceinline__ void issue_extra_block(int La, int E, uint32_t acc_ex
             const uint32_t idesc_i = (idesc & ~(0x3Fu << 17)) | ((n_i >> 3) << 17);
             const uint64_t adesc = smem_desc_sw128(sa + (uint32_t)i * (128u * 128u)) + (uint64_t)(ks * 2);
             const uint64_t bdesc = smem_desc_sw128(sb) + (uint64_t)(ks * 2);
-            umma_i8(acc_extra + (uint32_t)i * nt_cols, adesc, bdesc, idesc_i, (opens_set && ks == 0 && i == 0) ? 0u : 1u);
+            umma_i8(acc_extra + (uint32_t)i * nt_cols, adesc, bdesc, idesc_i, (opens_set && ks == 0 && i == 0) ? 0u : 1u, one);
         }
     }
 }
@@ -941,28 +940,30 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
     if (warp == 0) {
         // ---- TMA producer -------------------------------------------------------------
-        if (lane == 0) {
+        const uint32_t one = elect_one();
+        const int la = (int)uniform((uint32_t)La);
+        {
             const int64_t zb = p.tile_group ? group : (p.b_batched ? z : 0);
-            const uint32_t tx_bytes = (uint32_t)La * a_limb_bytes + b_bytes;
+            const uint32_t tx_bytes = (uint32_t)la * a_limb_bytes + b_bytes;
             int armed = 0;
             for (int kb = kb_begin; kb < kb_end; ++kb) {
                 const int it = kb - kb_begin;
                 const int s = it % p.stages;
                 const uint32_t par = ((it / p.stages) & 1) ^ 1;
-                if (!mbar_wait(bar_empty + 8 * s, par, abort_flag)) break;
+                if (!mbar_wait_warp(bar_empty + 8 * s, par, abort_flag)) break;
                 const uint32_t full = bar_full + 8 * s;
-                mbar_expect_tx(full, tx_bytes);
+                mbar_expect_tx(full, tx_bytes, one);
                 const uint32_t sa = smem_base + s * stage_bytes;
                 const uint32_t sb = sa + a_bytes;
-                for (int i = 0; i < La; ++i)
+                for (int i = 0; i < la; ++i)
                     tma_load_2d(sa + i * a_limb_bytes, &tmA, kb * kBlockK,
-                                (int)(i * p.a_rows_per_limb + z * p.M + m0), full);
+                                (int)(i * p.a_rows_per_limb + z * p.M + m0), full, one);
                 for (int j = 0; j < p.Lb; ++j)
                     tma_load_2d(sb + j * (p.NT * kBlockK), &tmB, kb * kBlockK,
-                                (int)(j * p.b_rows_per_limb + zb * p.b_batch_rows + n0), full);
+                                (int)(j * p.b_rows_per_limb + zb * p.b_batch_rows + n0), full, one);
                 armed = it + 1;
             }
-            if (*abort_flag) {
+            if (__any_sync(0xffffffffu, *abort_flag)) {
                 // leave no copy in flight: wait (bounded) for every stage that was armed and
                 // that no consumer waited for
                 for (int i = (armed > p.stages ? armed - p.stages : 0); i < armed; ++i)
@@ -972,25 +973,27 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---- MMA issuer ---------------------------------------------------------------
-        if (lane == 0) {
+        const uint32_t one = elect_one(), tm = uniform(tmem);
+        const int la = (int)uniform((uint32_t)La);
+        {
             const uint32_t idesc = (2u << 4)                               // int32 accumulators
                                    | (1u << 7) | (1u << 10)                 // signed 8-bit A and B
                                    | ((uint32_t)((p.Lb * p.NT) >> 3) << 17)  // N
                                    | ((uint32_t)(kTileM >> 4) << 24);        // M
-            bool ok = mbar_wait(bar_zeroed, 0, abort_flag);
+            bool ok = mbar_wait_warp(bar_zeroed, 0, abort_flag);
             tc_fence_after();
             for (int kb = kb_begin; ok && kb < kb_end; ++kb) {
                 const int it = kb - kb_begin;
                 const int s = it % p.stages;
-                ok = mbar_wait(bar_full + 8 * s, (it / p.stages) & 1, abort_flag);
+                ok = mbar_wait_warp(bar_full + 8 * s, (it / p.stages) & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t sa = smem_base + s * stage_bytes;
-                issue_k_block_n(La, tmem, (uint32_t)p.NT, sa, sa + a_bytes, idesc, it ? 1u : 0u, kBlockK / 32,
+                issue_k_block_n(la, tm, (uint32_t)p.NT, sa, sa + a_bytes, idesc, it ? 1u : 0u, kBlockK / 32, one,
                                 a_limb_bytes >> 4);
-                umma_commit(bar_empty + 8 * s);
+                umma_commit(bar_empty + 8 * s, one);
             }
-            umma_commit(bar_accum);
+            umma_commit(bar_accum, one);
         }
     } else {
         // ---- accumulator zeroing, then epilogue -------------------------------------------
@@ -1250,22 +1253,24 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int rows = p.tile_group ? R : (int)(p.M - m0 < R ? p.M - m0 : R);
 
     if (warp == 0) {
-        if (lane == 0 && some) {
+        const uint32_t one = elect_one();
+        const int la = (int)uniform((uint32_t)La);
+        if (some) {
             const int64_t zb = p.tile_group ? group : (p.b_batched ? z : 0);
             const int a_row = (int)(z * p.M + m0), w_row = (int)(zb * p.b_batch_rows + n0);
             int armed = 0;
             for (int kb = kb_begin; kb < kb_end; ++kb) {
                 const int it = kb - kb_begin, s = it % stages;
-                if (!mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait_warp(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag)) break;
                 const uint32_t full = bar_full + 8 * s, sw = smem_base + s * stage_bytes;
-                mbar_expect_tx(full, DIRECT ? w_bytes : stage_bytes);
+                mbar_expect_tx(full, DIRECT ? w_bytes : stage_bytes, one);
                 for (int j = 0; j < p.Lb; ++j)
-                    tma_load_2d(sw + j * (kTileM * kBlockK), &tmW, kb * kBlockK, (int)(j * p.b_rows_per_limb) + w_row, full);
-                for (int i = 0; i < La && !DIRECT; ++i)
-                    tma_load_2d(sw + w_bytes + i * a_limb, &tmA, kb * kBlockK, (int)(i * p.a_rows_per_limb) + a_row, full);
+                    tma_load_2d(sw + j * (kTileM * kBlockK), &tmW, kb * kBlockK, (int)(j * p.b_rows_per_limb) + w_row, full, one);
+                for (int i = 0; i < la && !DIRECT; ++i)
+                    tma_load_2d(sw + w_bytes + i * a_limb, &tmA, kb * kBlockK, (int)(i * p.a_rows_per_limb) + a_row, full, one);
                 armed = it + 1;
             }
-            if (*abort_flag) {
+            if (__any_sync(0xffffffffu, *abort_flag)) {
                 // leave no copy in flight: wait (bounded) for every stage that was armed and that no consumer waited for
                 for (int i = (armed > stages ? armed - stages : 0); i < armed; ++i)
                     for (uint32_t it = 0; it < kSpinLimit; ++it)
@@ -1273,23 +1278,24 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && some) {
+        const uint32_t one = elect_one(), tm = uniform(tmem);
+        if (some) {
             const uint32_t idesc = (2u << 4)                               // int32 accumulators
                                    | (1u << 7) | (1u << 10)                 // signed 8-bit A and B
                                    | ((uint32_t)((La * R) >> 3) << 17)       // N
                                    | ((uint32_t)(kTileM >> 4) << 24);        // M
-            bool ok = mbar_wait(bar_zeroed, 0, abort_flag);
+            bool ok = mbar_wait_warp(bar_zeroed, 0, abort_flag);
             tc_fence_after();
             for (int kb = kb_begin; ok && kb < kb_end; ++kb) {
                 const int it = kb - kb_begin, s = it % stages;
-                ok = mbar_wait(bar_full + 8 * s, (it / stages) & 1, abort_flag);
+                ok = mbar_wait_warp(bar_full + 8 * s, (it / stages) & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t sw = smem_base + s * stage_bytes;
-                issue_k_block_n(p.Lb, tmem, (uint32_t)R, sw, sw + w_bytes, idesc, it ? 1u : 0u, kBlockK / 32);
-                umma_commit(bar_empty + 8 * s);
+                issue_k_block_n(p.Lb, tm, (uint32_t)R, sw, sw + w_bytes, idesc, it ? 1u : 0u, kBlockK / 32, one);
+                umma_commit(bar_empty + 8 * s, one);
             }
-            umma_commit(bar_accum);
+            umma_commit(bar_accum, one);
         }
     } else {
         const int q = warp & 3, col = q * 32 + lane;             // tensor-memory lane quarter, column of the tile
@@ -1912,33 +1918,36 @@ limb_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
 
     if (warp == 0) {
         // ---- TMA producer: one continuous pipeline over all of this CTA's tiles ---------------
-        if (lane == 0) {
-            const uint32_t tx_bytes = (uint32_t)La * kTileM * kBlockK + b_bytes;
+        const uint32_t one = elect_one();
+        const int la = (int)uniform((uint32_t)La);
+        {
+            const uint32_t tx_bytes = (uint32_t)la * kTileM * kBlockK + b_bytes;
             int64_t it = 0, armed = 0;
             bool ok = true;
             for (int64_t tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x) {
-                const TileCoord tc = decode_tile(p, tile);
+                TileCoord tc = decode_tile(p, tile);
+                tc.group = __reduce_max_sync(0xffffffffu, tc.group);
                 if (p.skip_tiles && tile_masked(p, tc)) continue;
                 if (tc.group < 0) continue;
                 const int64_t zb = p.tile_group ? tc.group : (p.b_batched ? tc.z : 0);
                 for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
                     const int s = (int)(it % p.stages);
                     const uint32_t par = (uint32_t)((it / p.stages) & 1) ^ 1u;
-                    if (!mbar_wait(bar_empty + 8 * s, par, abort_flag, 96u * p.backoff)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_empty + 8 * s, par, abort_flag, 96u * p.backoff)) { ok = false; break; }
                     const uint32_t full = bar_full + 8 * s;
-                    mbar_expect_tx(full, tx_bytes);
+                    mbar_expect_tx(full, tx_bytes, one);
                     const uint32_t sa = smem_base + s * stage_bytes;
                     const uint32_t sb = sa + a_bytes;
-                    for (int i = 0; i < La; ++i)
+                    for (int i = 0; i < la; ++i)
                         tma_load_2d(sa + i * (kTileM * kBlockK), &tmA, kb * kBlockK,
-                                    (int)(i * p.a_rows_per_limb + tc.z * p.M + tc.m0), full);
+                                    (int)(i * p.a_rows_per_limb + tc.z * p.M + tc.m0), full, one);
                     for (int j = 0; j < p.Lb; ++j)
                         tma_load_2d(sb + j * (p.NT * kBlockK), &tmB, kb * kBlockK,
-                                    (int)(j * p.b_rows_per_limb + zb * p.b_batch_rows + tc.n0), full);
+                                    (int)(j * p.b_rows_per_limb + zb * p.b_batch_rows + tc.n0), full, one);
                     armed = it + 1;
                 }
             }
-            if (*abort_flag) {
+            if (__any_sync(0xffffffffu, *abort_flag)) {
                 // leave no copy in flight: wait (bounded) for the stages armed last
                 for (int64_t j = (armed > p.stages ? armed - p.stages : 0); j < armed; ++j)
                     for (uint32_t w = 0; w < kSpinLimit; ++w)
@@ -1947,7 +1956,9 @@ limb_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
         }
     } else if (warp == 1) {
         // ---- MMA issuer ---------------------------------------------------------------------
-        if (lane == 0) {
+        const uint32_t one = elect_one(), tm = uniform(tmem);
+        const int la = (int)uniform((uint32_t)La);
+        {
             const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) |
                                    ((uint32_t)((p.Lb * p.NT) >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
             int64_t it = 0, t = 0;
@@ -1956,30 +1967,31 @@ limb_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
             long long w_full = 0, w_empty = 0, t_begin = prof ? clock64() : 0, t0 = 0;
             for (int64_t tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x) {
                 if (p.skip_tiles || p.tile_group) {
-                    const TileCoord tcm = decode_tile(p, tile);
+                    TileCoord tcm = decode_tile(p, tile);
+                    tcm.group = __reduce_max_sync(0xffffffffu, tcm.group);
                     if (tcm.group < 0 || (p.skip_tiles && tile_masked(p, tcm))) continue;
                 }
                 const int b = (int)(t % p.nbuf);
                 const uint32_t tpar = (uint32_t)((t / p.nbuf) & 1);
                 if (prof) t0 = clock64();
-                ok = mbar_wait(bar_tempty + 8 * b, tpar, abort_flag, 24u * p.backoff);
+                ok = mbar_wait_warp(bar_tempty + 8 * b, tpar, abort_flag, 24u * p.backoff);
                 if (prof) w_empty += clock64() - t0;
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc = tmem + (uint32_t)(b * buf_cols);
+                const uint32_t acc = tm + (uint32_t)(b * buf_cols);
                 for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
                     const int s = (int)(it % p.stages);
                     const bool second = p.k_switch && kb >= p.k_switch;
                     if (split && kb == p.k_switch) {
                         // the second set is still being drained by the previous tile's epilogue
                         if (prof) t0 = clock64();
-                        ok = mbar_wait(bar_tempty + 8, tpar, abort_flag, 24u * p.backoff);
+                        ok = mbar_wait_warp(bar_tempty + 8, tpar, abort_flag, 24u * p.backoff);
                         if (prof) w_empty += clock64() - t0;
                         if (!ok) break;
                         tc_fence_after();
                     }
                     if (prof) t0 = clock64();
-                    ok = mbar_wait(bar_full + 8 * s, (uint32_t)((it / p.stages) & 1), abort_flag, 24u * p.backoff);
+                    ok = mbar_wait_warp(bar_full + 8 * s, (uint32_t)((it / p.stages) & 1), abort_flag, 24u * p.backoff);
                     if (prof) w_full += clock64() - t0;
                     if (!ok) break;
                     tc_fence_after();
@@ -1993,17 +2005,17 @@ limb_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
                         const int64_t left = p.k_extent - (int64_t)kb * kBlockK;
                         if (left < kBlockK) ks_n = (int)((left + 31) >> 5);
                     }
-                    issue_k_block_n(La, acc_set, (uint32_t)p.NT, sa, sa + a_bytes, idesc,
-                                    kb != kb_first ? 1u : 0u, ks_n);
+                    issue_k_block_n(la, acc_set, (uint32_t)p.NT, sa, sa + a_bytes, idesc,
+                                    kb != kb_first ? 1u : 0u, ks_n, one);
                     if (merged && second)
-                        issue_extra_block(La, p.merged_E, acc + (uint32_t)set_cols, (uint32_t)p.NT, sa, sa + a_bytes,
-                                          idesc, kb == p.k_switch, ks_n);
-                    umma_commit(bar_empty + 8 * s);
+                        issue_extra_block(la, p.merged_E, acc + (uint32_t)set_cols, (uint32_t)p.NT, sa, sa + a_bytes,
+                                          idesc, kb == p.k_switch, ks_n, one);
+                    umma_commit(bar_empty + 8 * s, one);
                 }
-                if (ok) umma_commit(bar_tfull + 8 * b);
+                if (ok) umma_commit(bar_tfull + 8 * b, one);
                 ++t;
             }
-            if (prof) {
+            if (prof && one) {
                 atomicAdd(p.wait_cycles + 0, (unsigned long long)w_full);
                 atomicAdd(p.wait_cycles + 1, (unsigned long long)w_empty);
                 atomicAdd(p.wait_cycles + 2, (unsigned long long)(clock64() - t_begin));
@@ -2272,60 +2284,66 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     };
 
     if (warp == 0) {
-        if (lane == 0) {
-            const uint32_t tx_bytes = (uint32_t)La * kTileM * kBlockK + b_bytes;
+        const uint32_t one = elect_one();
+        const int la = (int)uniform((uint32_t)La);
+        {
+            const uint32_t tx_bytes = (uint32_t)la * kTileM * kBlockK + b_bytes;
             int s = 0, armed = 0;
             uint32_t phase = 0;
             bool ok = true;
             for (int64_t tile = blockIdx.x; ok && tile < total; tile += gridDim.x) {
-                const TileCoord tc = decode_tile(p, tile);
+                TileCoord tc = decode_tile(p, tile);
+                tc.group = __reduce_max_sync(0xffffffffu, tc.group);
                 if (tc.group < 0) continue;
                 const int64_t zb = p.tile_group ? tc.group : (p.b_batched ? tc.z : 0);
                 const int a_row = (int)(tc.z * p.M + tc.m0), b_row = (int)(zb * p.b_batch_rows + tc.n0), n_blocks = blocks_of(tc);
                 for (int kb = 0; kb < n_blocks; ++kb) {
-                    if (!(ok = mbar_wait(bar_empty + 8 * s, phase ^ 1u, abort_flag, 96u * p.backoff))) break;
+                    if (!(ok = mbar_wait_warp(bar_empty + 8 * s, phase ^ 1u, abort_flag, 96u * p.backoff))) break;
                     const uint32_t full = bar_full + 8 * s, sa = smem_base + s * stage_bytes, sb = sa + a_bytes;
-                    mbar_expect_tx(full, tx_bytes);
-                    for (int i = 0; i < La; ++i)
-                        tma_load_2d(sa + i * (kTileM * kBlockK), &tmA, kb * kBlockK, (int)(i * p.a_rows_per_limb) + a_row, full);
+                    mbar_expect_tx(full, tx_bytes, one);
+                    for (int i = 0; i < la; ++i)
+                        tma_load_2d(sa + i * (kTileM * kBlockK), &tmA, kb * kBlockK, (int)(i * p.a_rows_per_limb) + a_row, full, one);
                     for (int j = 0; j < p.Lb; ++j)
-                        tma_load_2d(sb + j * (p.NT * kBlockK), &tmB, kb * kBlockK, (int)(j * p.b_rows_per_limb) + b_row, full);
+                        tma_load_2d(sb + j * (p.NT * kBlockK), &tmB, kb * kBlockK, (int)(j * p.b_rows_per_limb) + b_row, full, one);
                     armed |= 1 << s;
                     if (++s == p.stages) { s = 0; phase ^= 1u; }
                 }
             }
-            if (*abort_flag)
+            if (__any_sync(0xffffffffu, *abort_flag))
                 // leave no copy in flight: wait (bounded) for what was armed last in every stage
                 for (int i = 0; i < p.stages; ++i)
                     for (uint32_t it = 0; (armed >> i & 1) && it < kSpinLimit; ++it)
                         if (mbar_try(bar_full + 8 * i, i < s ? phase : phase ^ 1u)) break;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        const uint32_t one = elect_one(), tm = uniform(tmem);
+        const int la = (int)uniform((uint32_t)La);
+        {
             const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((p.Lb * p.NT) >> 3) << 17) |
                                    ((uint32_t)(kTileM >> 4) << 24);
             int s = 0, buf = 0;
             uint32_t phase = 0, turn = 0;
             bool ok = true;
             for (int64_t tile = blockIdx.x; ok && tile < total; tile += gridDim.x) {
-                const TileCoord tc = decode_tile(p, tile);
+                TileCoord tc = decode_tile(p, tile);
+                tc.group = __reduce_max_sync(0xffffffffu, tc.group);
                 if (tc.group < 0) continue;
                 const int n_blocks = blocks_of(tc);
-                if (!(ok = mbar_wait(bar_tempty + 8 * buf, turn, abort_flag, 24u * p.backoff))) break;
+                if (!(ok = mbar_wait_warp(bar_tempty + 8 * buf, turn, abort_flag, 24u * p.backoff))) break;
                 tc_fence_after();
-                const uint32_t acc = tmem + (uint32_t)(buf * buf_cols);
+                const uint32_t acc = tm + (uint32_t)(buf * buf_cols);
                 for (int kb = 0; kb < n_blocks; ++kb) {
-                    if (!(ok = mbar_wait(bar_full + 8 * s, phase, abort_flag, 24u * p.backoff))) break;
+                    if (!(ok = mbar_wait_warp(bar_full + 8 * s, phase, abort_flag, 24u * p.backoff))) break;
                     tc_fence_after();
                     const uint32_t sa = smem_base + s * stage_bytes;
                     int ks_n = kBlockK / 32;          // a partial last block: the copy fills it with zeros, which need no products
                     const int64_t left = p.k_extent - (int64_t)kb * kBlockK;
                     if (left < kBlockK) ks_n = (int)((left + 31) >> 5);
-                    issue_k_block_n(La, acc, (uint32_t)p.NT, sa, sa + a_bytes, idesc, kb ? 1u : 0u, ks_n);
-                    umma_commit(bar_empty + 8 * s);
+                    issue_k_block_n(la, acc, (uint32_t)p.NT, sa, sa + a_bytes, idesc, kb ? 1u : 0u, ks_n, one);
+                    umma_commit(bar_empty + 8 * s, one);
                     if (++s == p.stages) { s = 0; phase ^= 1u; }
                 }
-                if (ok) umma_commit(bar_tfull + 8 * buf);
+                if (ok) umma_commit(bar_tfull + 8 * buf, one);
                 if (++buf == p.nbuf) { buf = 0; turn ^= 1u; }
             }
         }
