@@ -1021,3 +1021,30 @@ def test_scores_in_32_bits(kmod, dev, dims):
     for other in (dict(a_limbs=4), dict(skip_masked=False), dict(a_limbs=0)):
         assert kmod.mla_scores_fused(*args, narrow=True, **dict(kw, **other)).dtype == torch.int64
     kmod.device_status(sync=True)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 18432), (3, 1028), (40, 4102), (147, 2050)])
+def test_gated_product_of_few_long_rows(kmod, orc, dev, rows, n):
+    """rows whose columns several blocks share: ragged last segments, and a value beyond the promise in any segment raises the flag"""
+    rng, N = np.random.default_rng(rows + n), 24
+    r12 = np.rint(rng.standard_normal((rows, 2 * n)) * 2.0**22).astype(np.int64)
+    W = rand_i64(rng, (N, n), 13).astype(np.int32)
+    planes = kmod.WeightPlanes(g(W, dev))
+    kmod.silu_init_q23()
+
+    def run():
+        d = g(r12, dev)
+        return kmod.glu_prepared(d[:, :n], d[:, n:], planes, 9, ld=2 * n, a_limbs=4, dynamic=True)
+
+    r12[0, n - 1], r12[0, 2 * n - 1] = 30 << 23, 1 << 25                    # the largest in the last segment: four limbs
+    h = (orc.act(np.ascontiguousarray(r12[:, :n]), "silu", 23) * r12[:, n:]) >> 23
+    same(run(), orc.gemm(h[None], W, 1, 1, 9)[0][0], "gate + down projection")
+    kmod.device_status(sync=True)
+    for k in (0, n // 2, n - 1):
+        old = r12[-1, [k, n + k]].copy()
+        r12[-1, [k, n + k]] = 60 << 23, 1 << 32          # their product still fits 64 bits
+        run()
+        with pytest.raises(kmod.ZkdsError) as e:
+            kmod.device_status(sync=True)
+        assert e.value.status == kmod.ERR_RANGE
+        r12[-1, [k, n + k]] = old

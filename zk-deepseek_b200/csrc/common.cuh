@@ -120,4 +120,18 @@ __device__ __forceinline__ uint64_t warp_max_u64(uint64_t v)
     return v;
 }
 
+// The largest of a block's values into *out, all threads of the block together: one atomic a block, and none where the word
+// already holds as much.  (One a warp, the blocks of a large launch took 40 us and more for them, of a small one 4 us.)
+__device__ __forceinline__ void block_report_max(uint64_t v, unsigned long long* out)
+{
+    __shared__ uint64_t most[32];
+    v = warp_max_u64(v);
+    if ((threadIdx.x & 31) == 0) most[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        v = warp_max_u64(threadIdx.x < (blockDim.x + 31) >> 5 ? most[threadIdx.x] : 0);
+        if (threadIdx.x == 0 && v > *(volatile unsigned long long*)out) atomicMax(out, (unsigned long long)v);
+    }
+}
+
 }  // namespace zkds

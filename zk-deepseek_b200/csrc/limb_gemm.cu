@@ -58,8 +58,7 @@ absmax_kernel(const T* X, int64_t rows, int64_t cols, int64_t sz, int64_t sr, in
         if (v < 0 && a) a -= 1;
         best = a > best ? a : best;
     }
-    best = warp_max_u64(best);
-    if ((threadIdx.x & 31) == 0 && best) atomicMax((unsigned long long*)out, (unsigned long long)best);
+    block_report_max(best, (unsigned long long*)out);
 }
 
 // planes[l][z][r][Kp] (int8) <- limb l of X[z*sz + r*sr + k*sk] / div.  One thread converts four
@@ -127,10 +126,7 @@ split_kernel(const T* __restrict__ X, int8_t* __restrict__ planes, int L, int64_
             if (l < L) *reinterpret_cast<uint32_t*>(dst + l * plane_stride) = w[l];
     }
     if (ovf) *overflow = 1u;
-    if (absmax_out) {
-        seen = warp_max_u64(seen);
-        if ((threadIdx.x & 31) == 0 && seen) atomicMax(absmax_out, (unsigned long long)seen);
-    }
+    if (absmax_out) block_report_max(seen, absmax_out);
 }
 
 // The k-contiguous case of split_kernel without any integer division: a CTA of 256 threads is a
@@ -271,10 +267,7 @@ split_rows_kernel(const T* __restrict__ X, int8_t* __restrict__ planes, int L, i
     }
     seen = seen32 > seen ? seen32 : seen;
     if (ovf) *overflow = 1u;
-    if (absmax_out) {
-        seen = warp_max_u64(seen);
-        if ((threadIdx.x & 31) == 0 && seen) atomicMax(absmax_out, (unsigned long long)seen);
-    }
+    if (absmax_out) block_report_max(seen, absmax_out);
 }
 
 // The MMAs of one K block (up to four K steps of 32 bytes, LA limb tiles of A against the stacked B
