@@ -1048,3 +1048,26 @@ def test_gated_product_of_few_long_rows(kmod, orc, dev, rows, n):
             kmod.device_status(sync=True)
         assert e.value.status == kmod.ERR_RANGE
         r12[-1, [k, n + k]] = old
+
+
+@pytest.mark.parametrize("steps", [5, 1183, 1184, 1185, 2500])
+def test_measured_ranges_of_more_steps_than_blocks(kmod, orc, dev, steps):
+    """a block a step, blocks of several steps (eight blocks an SM), the largest in A's last step; a small range
+    behind a large one; behind work that outlasts the host's polling"""
+    rng, K = np.random.default_rng(steps), 2048
+    W = rand_i64(rng, (4, K), 9)
+    big = rand_i64(rng, (1, steps - 4, K), 9)                # a step is 2048 numbers; W has four
+    big[0, -1, -1] = 1 << 37
+    small = rand_i64(rng, big.shape, 9)
+    want = {id(x): orc.gemm(x, W, 1, 1, 3)[0] for x in (big, small)}
+    gw = g(W, dev)
+    for x in (big, small, big):
+        same(kmod.int64_bmm_broadcast(g(x, dev), gw, 1, 1, 3)[0], want[id(x)], "idle stream")
+    busy = torch.ones((4096, 4096), device=dev)
+    for x in (big, small):
+        gx = g(x, dev)
+        torch.cuda.synchronize()
+        for _ in range(40):
+            busy = busy @ busy
+        same(kmod.int64_bmm_broadcast(gx, gw, 1, 1, 3)[0], want[id(x)], "busy stream")
+    kmod.device_status(sync=True)

@@ -154,22 +154,21 @@ static int run_contraction(const Contraction& p, int a_limbs, int b_limbs, int f
 
     if (p.skip_k && a_limbs <= 0) return ZKDS_ERR_ARG;   // the unread part of A may hold anything
     if (a_limbs <= 0 || b_limbs <= 0) {
-        uint64_t* d = (uint64_t*)workspace(2 * sizeof(uint64_t), 5);
-        if (!d) return ZKDS_ERR_WORKSPACE;
-        ZKDS_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof(uint64_t), st));
-        int rc = launch_ranges(p, true, b_limbs <= 0, d, st);
-        const bool apart = rc == ZKDS_ERR_UNSUPPORTED;
-        if (apart) rc = launch_absmax(p.A, 64, p.batches, p.M, p.K, p.a_sz, p.a_sm, 1, p.a_div, d, st);
-        if (rc != ZKDS_OK) return rc;
-        // B may be shared by every batch (b_sz == 0)
-        if (apart && b_limbs <= 0) {
-            rc = launch_absmax(p.B, p.b_bits, p.b_sz ? p.batches : 1, p.N, p.K, p.b_sz, p.b_sn, p.b_sk,
-                               p.b_div, d + 1, st);
-            if (rc != ZKDS_OK) return rc;
-        }
         uint64_t h[2];
-        ZKDS_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, st));
-        ZKDS_CUDA(cudaStreamSynchronize(st));
+        int rc = measure_ranges(p, true, b_limbs <= 0, h, st);
+        if (rc == ZKDS_ERR_UNSUPPORTED) {
+            uint64_t* d = (uint64_t*)workspace(2 * sizeof(uint64_t), 5);
+            if (!d) return ZKDS_ERR_WORKSPACE;
+            ZKDS_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof(uint64_t), st));
+            rc = launch_absmax(p.A, 64, p.batches, p.M, p.K, p.a_sz, p.a_sm, 1, p.a_div, d, st);
+            // B may be shared by every batch (b_sz == 0)
+            if (rc == ZKDS_OK && b_limbs <= 0)
+                rc = launch_absmax(p.B, p.b_bits, p.b_sz ? p.batches : 1, p.N, p.K, p.b_sz, p.b_sn, p.b_sk, p.b_div, d + 1, st);
+            if (rc != ZKDS_OK) return rc;
+            ZKDS_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, st));
+            ZKDS_CUDA(cudaStreamSynchronize(st));
+        }
+        if (rc != ZKDS_OK) return rc;
         if (a_limbs <= 0) a_limbs = limbs_needed(h[0]);
         if (b_limbs <= 0) b_limbs = limbs_needed(h[1]);
     }

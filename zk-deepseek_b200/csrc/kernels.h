@@ -222,7 +222,7 @@ unsigned* limb_range_flag();      // device view of the word behind ZKDS_ERR_RAN
 int launch_absmax(const void* X, int bits, int64_t batches, int64_t rows, int64_t cols,
                   int64_t sz, int64_t sr, int64_t sc, int64_t div, uint64_t* out_dev,
                   cudaStream_t st);
-int launch_ranges(const Contraction& p, bool want_a, bool want_b, uint64_t* out_dev, cudaStream_t st);
+int measure_ranges(const Contraction& p, bool want_a, bool want_b, uint64_t* out, cudaStream_t st);
 
 // dead-code converters kept for ABI completeness (converters.cu)
 int launch_bf16_to_int32(const uint16_t* in, int32_t* out, int rows, int cols, int rescale,
