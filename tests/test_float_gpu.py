@@ -715,3 +715,39 @@ def test_trace_and_generate_programs(float_libpath, tmp_path, case, dtype):
                            timeout=300)
         assert r.returncode == 0, r.stderr[-2000:]
         assert json.loads(r.stdout.strip().split("\n")[-1]) == oracle_greedy(cfg, W, prompt, 6)[0]
+
+
+@pytest.mark.parametrize("M,N,Kd", [(17, 16, 136), (31, 136, 256), (64, 1000, 520), (160, 10000, 136), (161, 264, 1032), (320, 10000, 200),
+                                    (321, 2056, 4104), (33, 20000, 264)])
+def test_float32_layers_from_thirds(K, M, N, Kd):
+    """the tensor-core products of bfloat16 thirds: edges of the tiles of 160 rows and 128 columns, ragged blocks of K, shares.
+    The limit is that of 32-bit sums in chunks of 64 and then one by one: (64 / 16 + Kd / 64 + 4) roundings of 2^-24 of the sum of
+    absolute products, a few times what they add up to by chance"""
+    for scale in (1.0, 2.0 ** -60, 2.0 ** 60):
+        A, W = rnd((M, Kd), "float32", 3) * scale, rnd((N, Kd), "float32", 4, Kd ** -0.5)
+        out = torch.full((M, N), 7.0, device="cuda")
+        K.linear(A, W, out)
+        want, bound = A.double() @ W.double().T, A.double().abs() @ W.double().abs().T
+        assert ((out - want).abs() <= (8 + Kd / 64) * 2.0 ** -24 * bound).all()
+        assert (out - want).norm() <= 6e-7 * want.norm()
+    test_linear_and_its_epilogues(K, "float32", M, N, Kd)
+
+
+def test_float32_layers_keep_infinities_where_they_are(K):
+    """rows and weights with infinities, NaN, products and sums beyond the range: the outputs that see them, and no others"""
+    M, N, Kd = 170, 2056, 328          # (200 columns go to the other kernel, whose shares of K overflow each by itself: inf - inf)
+    A, W = rnd((M, Kd), "float32", 5), rnd((N, Kd), "float32", 6)
+    A[3, 7], A[5, 9], A[7, 100], W[11, 20], W[13, 7] = float("inf"), float("-inf"), float("nan"), float("inf"), 0.0
+    A[20, 300], W[17, 300] = 3e38, 3e38          # one product beyond the range
+    A[21], W[18] = 1e18, 1e19                    # only the sum (3.3e39) is
+    A[22, :2] = torch.tensor([1e-40, 3e-39])     # below the smallest normal number
+    out = torch.empty((M, N), device="cuda")
+    K.linear(A, W, out)
+    want = A.double() @ W.double().T
+    big = want.abs() > 3.4028235e38
+    want = torch.where(big, want.sign() * float("inf"), want).float()
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+    fine = torch.isfinite(want)
+    assert torch.equal(out[torch.isinf(want)], want[torch.isinf(want)])
+    bound = torch.nan_to_num(A, 0, 0, 0).double().abs() @ torch.nan_to_num(W, 0, 0, 0).double().abs().T
+    assert ((out - want)[fine].abs() <= (16 * 2.0 ** -24 * bound + 1e-38)[fine]).all()

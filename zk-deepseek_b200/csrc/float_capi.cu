@@ -117,7 +117,7 @@ static int linear(const zkfp_linear_args* a, bool early, void* stream)
     case 3: return launch_linear_skinny(*a, e, early, st);
     case 2: return launch_linear_stream(*a, e, early, st);
     case 1: return launch_linear_tc(*a, e, st);
-    default: return launch_linear_f32(*a, e, st);
+    default: return linear_split_takes(*a) ? launch_linear_split(*a, e, st) : launch_linear_f32(*a, e, st);
     }
 }
 

@@ -198,6 +198,8 @@ inline void fp_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, 
 
 // ---- launchers (float_ops.cu, float_gemm.cu, float_attention.cu) -------------------------------------------
 int launch_linear_f32(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
+bool linear_split_takes(const zkfp_linear_args& a);
+int launch_linear_split(const zkfp_linear_args& a, const LinEpi& e, cudaStream_t st);
 int launch_linear_stream(const zkfp_linear_args& a, const LinEpi& e, bool early, cudaStream_t st);
 bool linear_skinny_takes(const zkfp_linear_args& a);
 int launch_linear_skinny(const zkfp_linear_args& a, const LinEpi& e, bool early, cudaStream_t st);

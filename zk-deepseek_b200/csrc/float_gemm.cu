@@ -2,7 +2,8 @@
 //   few rows (decode)   linear_stream_kernel: every weight is read once, sixteen bytes a lane
 //   up to 32, bfloat16  linear_skinny_kernel: the same with warp-level tensor-core products
 //   many rows, bfloat16 linear_tc_kernel (float_gemm_tc.cu): tcgen05 tiles fed by TMA
-//   many rows, float32  linear_f32_kernel: true 32-bit products on the CUDA cores
+//   many rows, float32  linear_split_kernel (float_gemm_f32.cu): tcgen05 products of bfloat16 thirds; what that leaves,
+//                       linear_f32_kernel: 32-bit products on the CUDA cores
 #include "float_common.cuh"
 
 namespace zkds {
