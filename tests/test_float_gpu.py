@@ -751,3 +751,36 @@ def test_float32_layers_keep_infinities_where_they_are(K):
     assert torch.equal(out[torch.isinf(want)], want[torch.isinf(want)])
     bound = torch.nan_to_num(A, 0, 0, 0).double().abs() @ torch.nan_to_num(W, 0, 0, 0).double().abs().T
     assert ((out - want)[fine].abs() <= (16 * 2.0 ** -24 * bound + 1e-38)[fine]).all()
+
+
+@pytest.mark.parametrize("S,start,H,G,D,R,V,window", [
+    (1, 0, 1, 1, 8, 0, 8, 0), (31, 0, 2, 1, 64, 0, 64, 0), (32, 31, 4, 2, 64, 64, 128, 33), (33, 0, 3, 3, 72, 8, 120, 32),
+    (64, 63, 2, 2, 128, 64, 128, 64), (65, 64, 2, 1, 128, 0, 128, 65), (97, 200, 8, 2, 320, 64, 40, 100)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_float32_attention_of_prompts(K, S, start, H, G, D, R, V, window, gated):
+    """edges of the tiles of 32 tokens, 64 keys and 64 elements, several heads on a key head, gate and output pitch; a key and a
+    value that are not finite reach the tokens that see them and no others"""
+    base = max(0, start - window + 1) if window else 0
+    keys, bad = start + S - base, start + S // 2
+    q, kv, kr = rnd((S, H, D + R), "float32"), rnd((keys, G * (D + V)), "float32", 1), rnd((keys, R + 8), "float32", 2)
+    gate, out, st = rnd((S, H * V), "float32", 3), torch.zeros((S, H * V + 8), device="cuda"), torch.tensor([start], dtype=torch.int32, device="cuda")
+    a = attention_args(K, q, kv.data_ptr(), kr.data_ptr(), kv.data_ptr() + G * D * 4, out, st, q_head=D + R, o_head=V,
+                       k1_tok=kv.stride(0), k1_head=D, k2_tok=kr.stride(0), v_tok=kv.stride(0), v_head=V, base=base, keys=keys,
+                       batch=1, seq=S, heads=H, d1=D, d2=R, dv=V, window=window, shared=0, dtype=K.F32, scale=(D + R) ** -0.5,
+                       max_keys=keys, heads_per_kv=H // G, o_tok=H * V + 8)
+    if gated:
+        a.gate, a.gate_tok, a.gate_head, a.out_scale = gate.data_ptr(), H * V, V, 0.5
+    kv64, heads = kv.double().cpu().numpy(), [h // (H // G) for h in range(H)]
+    k = np.concatenate([kv64[:, :G * D].reshape(keys, G, D)[:, heads], np.repeat(kr.double().cpu().numpy()[:, None, :R], H, 1)], 2)
+    want = plain_attention(q.double().cpu().numpy(), k, kv64[:, G * D:].reshape(keys, G, V)[:, heads], start, base, window, (D + R) ** -0.5)
+    if gated:
+        want = want * (0.5 / (1 + np.exp(-gate.double().cpu().numpy().reshape(S, H, V))))
+    K.attention(a)
+    assert np.abs(out[:, :H * V].double().cpu().numpy().reshape(S, H, V) - want).max() < 2e-5
+    assert not out[:, H * V:].any()
+    kv[bad - base, G * D:] = float("nan")
+    K.attention(a)
+    got = out[:, :H * V].double().cpu().numpy().reshape(S, H, V)
+    sees = np.array([start + s >= bad and (not window or start + s - bad < window) for s in range(S)])
+    assert np.isnan(got[sees]).all() and np.abs(got[~sees] - want[~sees]).max(initial=0) < 2e-5
+    K.device_status(sync=True)

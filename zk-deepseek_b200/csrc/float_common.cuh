@@ -59,6 +59,19 @@ __device__ __forceinline__ void store8(bf16* p, const float (&v)[8])
                                               pack_bf16(v[6], v[7]));
 }
 
+// two products of 32-bit numbers an instruction, each rounded like fmaf
+__device__ __forceinline__ uint64_t twice(float v)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
 __device__ __forceinline__ float warp_sum(float v)
 {
 #pragma unroll

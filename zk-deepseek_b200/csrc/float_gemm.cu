@@ -20,18 +20,6 @@ namespace {
 // 8192 295 against 918, 2048 x 2048 86 against 235; 17 rows, 2048 x 8192: 96 against 704.
 constexpr int kFN = 128, kFK = 16, kFPitch = kFN + 4;
 
-__device__ __forceinline__ uint64_t twice(float v)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-    return r;
-}
-
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b)
-{
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-
 __device__ __forceinline__ float4 peer_float4(uint32_t own, unsigned rank)
 {
     float4 v;

@@ -403,6 +403,201 @@ attention_plain_kernel(const zkfp_attention_args a)
     }
 }
 
+// ---- float32 attention over per-head keys ---------------------------------------------------------------------------
+// A block handles 32 consecutive tokens of a head, a warp four of them from scores to output; keys come in tiles of 64.  Scores:
+// a lane has two keys and four tokens, output: four columns and four tokens, products two an instruction; the keys pass through
+// shared memory by 64 of their elements, transposed, and the next piece is on its way into registers under the products
+// of the current one.  Bound by the CUDA cores' multiply-adds (24 TFLOP/s on a prompt of 300, 16 heads of 192 and 128: 155 us in
+// attention_plain_kernel, which stages 32 keys at a time element by element between barriers and multiplies one by one, 77 us here; one
+// token behind 999: 427 and 151 us; error against 64 bits the same, 3.6e-7 and 7.3e-7).
+constexpr int kAttnTokens = 32, kAttnKeys = 64, kAttnPiece = 64, kAttnPitch = kAttnKeys + 4;
+
+__global__ void __launch_bounds__(256, 2)
+attention_f32_kernel(const zkfp_attention_args a)
+{
+    extern __shared__ __align__(16) float sm[];
+    const int dk = a.d1 + a.d2, dv = a.dv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.y;
+    float* Q = sm;                                             // [dk][kAttnTokens]
+    float* Ks = Q + dk * kAttnTokens;                          // [kAttnPiece][kAttnPitch]
+    float* V = Ks + kAttnPiece * kAttnPitch;                   // [kAttnKeys][dv]
+    float* P = V + kAttnKeys * dv + warp * kAttnKeys * 4;      // [kAttnKeys][4 tokens] of this warp
+    const int start = a.start[0];
+    if (start < 0 || start + a.seq > a.base + a.keys) return;      // not a step of these keys
+    const long long slot = a.slots ? a.slots[0] : 0;
+    const int kv_head = a.heads_per_kv > 1 ? head / a.heads_per_kv : head;
+    const int row0 = (int)(gridDim.x - 1 - blockIdx.x) * kAttnTokens;      // the longest blocks first
+    const int nrow = min(kAttnTokens, (int)a.seq - row0);
+    const float* q = (const float*)a.q;
+    const float* k1 = (const float*)a.k1 + slot * a.slot_stride + kv_head * a.k1_head;
+    const float* k2 = (const float*)a.k2 + slot * a.slot_stride;
+    const float* v = (const float*)a.v + slot * a.slot_stride + kv_head * a.v_head;
+    const int first = start + row0, last = first + nrow - 1;
+    int lo = a.window > 0 ? max(first - a.window + 1, 0) : 0;
+    if (lo < (int)a.base) lo = (int)a.base;
+    for (int i = threadIdx.x; i < kAttnTokens * (dk / 4); i += 256) {
+        const int r = i % kAttnTokens, d = i / kAttnTokens * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < nrow) x = *reinterpret_cast<const float4*>(q + ((long long)(row0 + r) * a.heads + head) * a.q_head + d);
+        Q[d * kAttnTokens + r] = x.x; Q[(d + 1) * kAttnTokens + r] = x.y;
+        Q[(d + 2) * kAttnTokens + r] = x.z; Q[(d + 3) * kAttnTokens + r] = x.w;
+    }
+    const int key = threadIdx.x & 63, part = (threadIdx.x >> 6) * 16, dv4 = dv / 4;
+    float4 kr[4], vr[8];
+    auto fetch_keys = [&](int j0, int d0) {
+        const long long p = (long long)j0 + key - a.base;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int d = d0 + part + 4 * i;
+            kr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j0 + key <= last && d < dk)
+                kr[i] = *reinterpret_cast<const float4*>(d < a.d1 ? k1 + p * a.k1_tok + d : k2 + p * a.k2_tok + (d - a.d1));
+        }
+    };
+    auto put_keys = [&]() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float* s = Ks + (part + 4 * i) * kAttnPitch + key;
+            s[0] = kr[i].x; s[kAttnPitch] = kr[i].y; s[2 * kAttnPitch] = kr[i].z; s[3 * kAttnPitch] = kr[i].w;
+        }
+    };
+    auto fetch_values = [&](int j0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int at = threadIdx.x + i * 256, r = at / dv4;
+            vr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < kAttnKeys && j0 + r <= last)
+                vr[i] = *reinterpret_cast<const float4*>(v + ((long long)j0 + r - a.base) * a.v_tok + (at - r * dv4) * 4);
+        }
+    };
+    auto put_values = [&]() {                      // true when one of them is not finite
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (threadIdx.x + i * 256 < kAttnKeys * dv4) reinterpret_cast<float4*>(V)[threadIdx.x + i * 256] = vr[i];
+            sum = fmaf(0.f, vr[i].x, fmaf(0.f, vr[i].y, fmaf(0.f, vr[i].z, fmaf(0.f, vr[i].w, sum))));
+        }
+        return sum != 0.f;                         // zeros stay zero, anything else times zero is no number
+    };
+    const int col = lane * 4 < dv ? lane * 4 : 0;  // this lane's columns; lanes behind the last repeat the first
+    float m[4], l[4] = {};
+    uint64_t acc[4][2] = {};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) m[r] = -INFINITY;
+    fetch_keys(lo, 0);
+    for (int j0 = lo; j0 <= last; j0 += kAttnKeys) {
+        uint64_t s[4] = {};
+        for (int d0 = 0; d0 < dk; d0 += kAttnPiece) {
+            __syncthreads();                       // the piece in front has been read (and, at first, Q is complete)
+            put_keys();
+            __syncthreads();
+            if (d0 + kAttnPiece < dk) fetch_keys(j0, d0 + kAttnPiece);
+            else fetch_values(j0);
+            const int nd = min(kAttnPiece, dk - d0);
+#pragma unroll 8
+            for (int d = 0; d < nd; ++d) {
+                const float4 x = *reinterpret_cast<const float4*>(Q + (d0 + d) * kAttnTokens + warp * 4);
+                const uint64_t kk = *reinterpret_cast<const uint64_t*>(Ks + d * kAttnPitch + 2 * lane);
+                fma2(s[0], twice(x.x), kk); fma2(s[1], twice(x.y), kk);
+                fma2(s[2], twice(x.z), kk); fma2(s[3], twice(x.w), kk);
+            }
+        }
+        float w[4][2];
+        bool seen[4][2];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int i = first + warp * 4 + r;
+            float sc[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = j0 + 2 * lane + h;
+                seen[r][h] = warp * 4 + r < nrow && j <= i && (a.window <= 0 || i - j < a.window);
+                sc[h] = seen[r][h] ? __uint_as_float((uint32_t)(s[r] >> (32 * h))) * a.scale : -INFINITY;
+            }
+            const float m_new = fmaxf(m[r], warp_max(fmaxf(sc[0], sc[1])));
+            const float f = m[r] == -INFINITY ? 0.f : expf(m[r] - m_new);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) w[r][h] = seen[r][h] ? expf(sc[h] - m_new) : 0.f;
+            l[r] = l[r] * f + warp_sum(w[r][0] + w[r][1]);
+            m[r] = m_new;
+            uint64_t t0 = 0, t1 = 0;
+            fma2(t0, twice(f), acc[r][0]);
+            fma2(t1, twice(f), acc[r][1]);
+            acc[r][0] = t0; acc[r][1] = t1;
+        }
+        // the readers of the values in front passed the barriers of this tile's keys.  Weights of keys that a token does not see
+        // are zeros, which would still spread what is not finite: such tiles mark them instead and leave them out
+        const bool odd = __syncthreads_or(put_values());
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float4*>(P + (2 * lane + h) * 4) = make_float4(
+                seen[0][h] ? w[0][h] : odd ? -1.f : 0.f, seen[1][h] ? w[1][h] : odd ? -1.f : 0.f,
+                seen[2][h] ? w[2][h] : odd ? -1.f : 0.f, seen[3][h] ? w[3][h] : odd ? -1.f : 0.f);
+        __syncwarp();
+        if (j0 + kAttnKeys <= last) fetch_keys(j0 + kAttnKeys, 0);
+        const int nk = min(kAttnKeys, last - j0 + 1);
+        if (odd) {
+#pragma unroll 1
+            for (int kk = 0; kk < nk; ++kk) {
+                const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(V + kk * dv + col);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float x = P[kk * 4 + r];
+                    if (x == -1.f) continue;
+                    fma2(acc[r][0], twice(x), y.x);
+                    fma2(acc[r][1], twice(x), y.y);
+                }
+            }
+            continue;
+        }
+#pragma unroll 4
+        for (int kk = 0; kk < nk; ++kk) {
+            const float4 x = *reinterpret_cast<const float4*>(P + kk * 4);
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(V + kk * dv + col);
+            fma2(acc[0][0], twice(x.x), y.x); fma2(acc[0][1], twice(x.x), y.y);
+            fma2(acc[1][0], twice(x.y), y.x); fma2(acc[1][1], twice(x.y), y.y);
+            fma2(acc[2][0], twice(x.z), y.x); fma2(acc[2][1], twice(x.z), y.y);
+            fma2(acc[3][0], twice(x.w), y.x); fma2(acc[3][1], twice(x.w), y.y);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int t = row0 + warp * 4 + r;
+        if (warp * 4 + r >= nrow) continue;
+        float* out = (float*)a.out + (a.o_tok ? t * a.o_tok + head * a.o_head : ((long long)t * a.heads + head) * a.o_head);
+        const float* gate = a.gate ? (const float*)a.gate + t * a.gate_tok + head * a.gate_head : nullptr;
+        if (lane * 4 >= dv) continue;
+        float o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = __uint_as_float((uint32_t)(acc[r][i >> 1] >> (32 * (i & 1)))) / l[r];
+        if (gate) {
+            const float4 z = *reinterpret_cast<const float4*>(gate + col);
+            o[0] *= sigmoid_f(z.x) * a.out_scale; o[1] *= sigmoid_f(z.y) * a.out_scale;
+            o[2] *= sigmoid_f(z.z) * a.out_scale; o[3] *= sigmoid_f(z.w) * a.out_scale;
+        }
+        *reinterpret_cast<float4*>(out + col) = make_float4(o[0], o[1], o[2], o[3]);
+    }
+}
+
+// what the kernel above takes: per-head keys of one sequence, values of up to 128 columns, rows of whole 16-byte pieces.  Not a few
+// tokens over a few keys, where only its start counts (3 over 3: 7.0 us in attention_plain_kernel, 8.6 here; 16 over 16: 17.4 and 13.1)
+bool attention_f32_takes(const zkfp_attention_args& a)
+{
+    const uintptr_t at = (uintptr_t)a.q | (uintptr_t)a.k1 | (uintptr_t)a.k2 | (uintptr_t)a.v | (uintptr_t)a.out;
+    const long long steps = a.q_head | a.o_head | a.k1_tok | a.k1_head | a.k2_tok | a.v_tok | a.v_head | a.slot_stride | a.o_tok;
+    return a.dtype == ZKFP_F32 && !a.shared && (a.seq >= 8 || a.keys > 64) && a.dv <= 128 && a.d1 + a.d2 <= 512 && !(at & 15) && !(steps & 3) && a.seq <= 0x7fffffff;
+}
+
+int attention_f32(const zkfp_attention_args& a, cudaStream_t st)
+{
+    const size_t smem = sizeof(float) * ((size_t)(a.d1 + a.d2) * kAttnTokens + kAttnPiece * kAttnPitch + (size_t)kAttnKeys * a.dv +
+                                         8 * kAttnKeys * 4);
+    ZKDS_CUDA(cudaFuncSetAttribute(attention_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedMax - 1024));
+    const dim3 grid((unsigned)((a.seq + kAttnTokens - 1) / kAttnTokens), (unsigned)a.heads);
+    attention_f32_kernel<<<grid, 256, smem, st>>>(a);
+    return fp_launched();
+}
+
+
 }  // namespace
 
 template <typename T>
@@ -421,6 +616,7 @@ static int attention_plain(const zkfp_attention_args& a, cudaStream_t st)
 
 int launch_attention_plain(const zkfp_attention_args& a, cudaStream_t st)
 {
+    if (attention_f32_takes(a)) return attention_f32(a, st);
     return a.dtype == ZKFP_BF16 ? attention_plain<bf16>(a, st) : attention_plain<float>(a, st);
 }
 
