@@ -2385,9 +2385,10 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             for (int col = c0; col < c0 + CW;) {
                 // the shift belongs to the group and to the side of n_split (a multiple of 8) that the columns lie on
                 t.shift = p.group_shift ? p.group_shift[2 * tc.group + (tc.n0 + col >= p.n_split ? 1 : 0)] : p.shift;
+                // the odd eight and four first: what is left once the last sixteen are in registers runs under the next products
                 const int left = c0 + CW - col;
                 const bool split_ahead = p.group_shift && tc.n0 + col < p.n_split && tc.n0 + col + 16 > p.n_split;
-                const int W = !p.fits64 ? 4 : left >= 16 && !split_ahead ? 16 : left >= 8 && !(col & 7) ? 8 : 4;
+                const int W = !p.fits64 || (left & 4) ? 4 : (left & 8) || split_ahead ? (p.group_shift && (col & 7) ? 4 : 8) : 16;
                 auto loaded = [&]() {
                     clear(tq, col, W);
                     if (col + W >= c0 + CW) hand_back(buf);
