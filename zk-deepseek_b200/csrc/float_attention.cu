@@ -135,38 +135,48 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid
     const uint32_t tmem = s.tmem;
 
     if (warp == 0) {
-        if (lane == 0) {
+        const uint32_t one = elect_one();
+        const int n_keys = __reduce_max_sync(0xffffffffu, kt.n), lo = __reduce_max_sync(0xffffffffu, kt.lo);
+        {
             const int tiles_q = t0 + kTile < p.seq ? 2 : 1;
-            mbar_expect_tx(smem_u32(&s.q_full), (uint32_t)tiles_q * bytesQ);
+            mbar_expect_tx(smem_u32(&s.q_full), (uint32_t)tiles_q * bytesQ, one);
             for (int g = 0; g < tiles_q; ++g) {
                 for (int c = 0; c < p.seg1; ++c)
-                    tma_load_3d(sQ + g * bytesQ + c * kSeg, &tmQ1, c * 64, head, t0 + g * kTile, smem_u32(&s.q_full));
+                    tma_load_3d(sQ + g * bytesQ + c * kSeg, &tmQ1, c * 64, head, t0 + g * kTile, smem_u32(&s.q_full), one);
                 for (int c = 0; c < p.seg2; ++c)
                     tma_load_3d(sQ + g * bytesQ + (p.seg1 + c) * kSeg, &tmQ2, c * 64, head, t0 + g * kTile,
-                                smem_u32(&s.q_full));
+                                smem_u32(&s.q_full), one);
             }
             int ks = 0, vs = 0;
             uint32_t kp = 0, vp = 0;
             bool ok = true;
-            for (int j = 0; j < kt.n && ok; ++j) {
-                const int y = kt.lo - p.base + j * kTile;
+            for (int j = 0; j < n_keys && ok; ++j) {
+                const int y = lo - p.base + j * kTile;
                 for (int c = 0; c < segq; ++c) {
-                    if (!(ok = mbar_wait(smem_u32(&s.k_empty[ks]), kp ^ 1u, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(smem_u32(&s.k_empty[ks]), kp ^ 1u, abort_flag))) break;
                     const uint32_t bar = smem_u32(&s.k_full[ks]), dst = sK + (uint32_t)ks * kSeg;
-                    mbar_expect_tx(bar, kSeg);
-                    if (c < p.seg1) tma_load_3d(dst, &tmK1, c * 64, kv_head, y, bar);
-                    else tma_load_2d(dst, &tmK2, (c - p.seg1) * 64, y, bar);
+                    mbar_expect_tx(bar, kSeg, one);
+                    if (c < p.seg1) tma_load_3d(dst, &tmK1, c * 64, kv_head, y, bar, one);
+                    else tma_load_2d(dst, &tmK2, (c - p.seg1) * 64, y, bar, one);
                     if (++ks == p.k_slots) { ks = 0; kp ^= 1u; }
                 }
-                if (!ok || !mbar_wait(smem_u32(&s.v_empty[vs]), vp ^ 1u, abort_flag)) break;
+                if (!ok || !mbar_wait_warp(smem_u32(&s.v_empty[vs]), vp ^ 1u, abort_flag)) break;
                 const uint32_t bar = smem_u32(&s.v_full[vs]), dst = sV + (uint32_t)vs * bytesV;
-                mbar_expect_tx(bar, bytesV);
-                for (int c = 0; c < p.segv; ++c) tma_load_3d(dst + c * kSeg, &tmV, c * 64, kv_head, y, bar);
+                mbar_expect_tx(bar, bytesV, one);
+                for (int c = 0; c < p.segv; ++c) tma_load_3d(dst + c * kSeg, &tmV, c * 64, kv_head, y, bar, one);
                 if (++vs == p.v_stages) { vs = 0; vp ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        const uint32_t one = elect_one(), tm = uniform(tmem);
+        KeyTiles ku = kt;
+        ku.n = __reduce_max_sync(0xffffffffu, kt.n);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            ku.first[g] = __reduce_max_sync(0xffffffffu, kt.first[g]);
+            ku.last[g] = __reduce_max_sync(0xffffffffu, kt.last[g]);
+        }
+        {
             const uint32_t idesc_s = idesc_bf16(kTile, kTile), idesc_o = idesc_bf16(kTile, (p.dv + 15) & ~15, true);
             uint32_t pp[2] = {0, 0};
             int ks = 0, vs = 0;                           // ring slot of the key tile's first segment, value stage
@@ -174,12 +184,12 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid
             // the score product of query tile g with the key tile at (ks, kp); `load` waits for its segments,
             // `release` hands each back after use
             auto scores = [&](int g, bool use, bool load, bool release) {
-                const uint32_t a = sQ + (uint32_t)g * bytesQ, d = tmem + (uint32_t)g * kTile;
+                const uint32_t a = sQ + (uint32_t)g * bytesQ, d = tm + (uint32_t)g * kTile;
                 int slot = ks;
                 uint32_t phase = kp;
                 for (int c = 0; c < segq; ++c) {
                     if (load) {
-                        if (!mbar_wait(smem_u32(&s.k_full[slot]), phase, abort_flag)) return false;
+                        if (!mbar_wait_warp(smem_u32(&s.k_full[slot]), phase, abort_flag)) return false;
                         tc_fence_after();
                     }
                     if (use) {
@@ -187,37 +197,37 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid
                         const uint64_t ad = smem_desc_sw128(a + (uint32_t)c * kSeg), bd = smem_desc_sw128(sK + (uint32_t)slot * kSeg);
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
-                            if (k * 16 < cols) umma_bf16(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc_s, (c | k) ? 1u : 0u);
+                            if (k * 16 < cols) umma_bf16(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc_s, (c | k) ? 1u : 0u, one);
                     }
-                    if (release) umma_commit(smem_u32(&s.k_empty[slot]));
+                    if (release) umma_commit(smem_u32(&s.k_empty[slot]), one);
                     if (++slot == p.k_slots) { slot = 0; phase ^= 1u; }
                 }
-                if (use) umma_commit(smem_u32(&s.s_full[g]));
+                if (use) umma_commit(smem_u32(&s.s_full[g]), one);
                 if (release) { ks = slot; kp = phase; }
                 return true;
             };
             auto active = [&](int g, int j) {
-                return g ? j >= kt.first[1] && j <= kt.last[1] : j >= kt.first[0] && j <= kt.last[0];
+                return g ? j >= ku.first[1] && j <= ku.last[1] : j >= ku.first[0] && j <= ku.last[0];
             };
-            bool ok = mbar_wait(smem_u32(&s.q_full), 0, abort_flag);
-            for (int j = -1; j < kt.n && ok; ++j) {
-                if (j >= 0 && !(ok = mbar_wait(smem_u32(&s.v_full[vs]), vp, abort_flag))) break;
+            bool ok = mbar_wait_warp(smem_u32(&s.q_full), 0, abort_flag);
+            for (int j = -1; j < ku.n && ok; ++j) {
+                if (j >= 0 && !(ok = mbar_wait_warp(smem_u32(&s.v_full[vs]), vp, abort_flag))) break;
                 for (int g = 0; g < 2 && ok; ++g) {
                     if (j >= 0 && active(g, j)) {
-                        if (!(ok = mbar_wait(smem_u32(&s.p_full[g]), pp[g], abort_flag))) break;
+                        if (!(ok = mbar_wait_warp(smem_u32(&s.p_full[g]), pp[g], abort_flag))) break;
                         pp[g] ^= 1u;
                         tc_fence_after();
-                        const uint32_t a = tmem + (uint32_t)g * kTile, d = tmem + 256u + (uint32_t)g * kTile;
+                        const uint32_t a = tm + (uint32_t)g * kTile, d = tm + 256u + (uint32_t)g * kTile;
                         const uint64_t vd = smem_desc_mn_sw128(sV + (uint32_t)vs * bytesV, kSeg);
-                        const bool opens = j == (g ? kt.first[1] : kt.first[0]);
+                        const bool opens = j == (g ? ku.first[1] : ku.first[0]);
 #pragma unroll
                         for (int k = 0; k < kTile / 16; ++k)
-                            umma_bf16_ts(d, a + (uint32_t)k * 8u, vd + (uint64_t)(k * 128), idesc_o, (!opens || k) ? 1u : 0u);
-                        if (j == (g ? kt.last[1] : kt.last[0])) umma_commit(smem_u32(&s.o_full[g]));
+                            umma_bf16_ts(d, a + (uint32_t)k * 8u, vd + (uint64_t)(k * 128), idesc_o, (!opens || k) ? 1u : 0u, one);
+                        if (j == (g ? ku.last[1] : ku.last[0])) umma_commit(smem_u32(&s.o_full[g]), one);
                     }
-                    if (j >= 0 && g == 1) umma_commit(smem_u32(&s.v_empty[vs]));
+                    if (j >= 0 && g == 1) umma_commit(smem_u32(&s.v_empty[vs]), one);
                     // every segment is waited for once and handed back once, also when no query tile uses it
-                    if (j + 1 < kt.n) ok = scores(g, active(g, j + 1), g == 0, g == 1);
+                    if (j + 1 < ku.n) ok = scores(g, active(g, j + 1), g == 0, g == 1);
                 }
                 if (!ok) break;
                 if (j >= 0 && ++vs == p.v_stages) { vs = 0; vp ^= 1u; }

@@ -9,6 +9,8 @@
 //              shared memory so that global accesses are whole row segments
 // Shapes with few tiles and a deep K split K over several pairs: each leaves its 32-bit sums in a workspace, and the
 // epilogue warp that arrives last at its part of a tile adds them up in a fixed order.
+// Warps 0 and 1 stay together and one elected lane issues (see elect_one): descriptors then live in uniform registers.  With
+// `if (lane == 0)` every MMA was preceded by moves out of the lane's registers: layers of a 4096-token prompt 8.5 -> 8.05 ms.
 // Every wait is bounded; one that runs out sets a host-visible flag and the CTAs leave through the normal path.
 #include <cuda.h>
 
@@ -196,7 +198,8 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const uint32_t tmem = s.tmem;
 
     if (warp == 0) {
-        if (lane == 0) {
+        const uint32_t one = elect_one();
+        {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -206,38 +209,39 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const int kb0 = (t % p.ksplit) * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.kblocks);
                 const int row_a = mt * 256 + (int)rank * kTM, row_w = nt * p.NT + (int)rank * (p.NT / 2);
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    if (!mbar_wait(smem_u32(&s.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(smem_u32(&s.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
                     const uint32_t full = smem_u32(&s.full[stage]), dst = smem0 + (uint32_t)stage * stage_bytes;
-                    if (rank == 0) mbar_expect_tx(full, 2 * stage_bytes);
-                    tma_load_2d_pair(dst, &tmA, kb * kBK, row_a, full);
-                    tma_load_2d_pair(dst + kBytesA, &tmW, kb * kBK, row_w, full);
+                    if (rank == 0) mbar_expect_tx(full, 2 * stage_bytes, one);
+                    tma_load_2d_pair(dst, &tmA, kb * kBK, row_a, full, one);
+                    tma_load_2d_pair(dst + kBytesA, &tmW, kb * kBK, row_w, full, one);
                     if (++stage == p.stages) { stage = 0; phase ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        if (rank == 0 && lane == 0) {
+        if (rank == 0) {
+            const uint32_t one = elect_one(), tm = uniform(tmem);
             const uint32_t idesc = idesc_bf16(256, p.NT);
             int stage = 0, buf = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
             for (int t = first; t < total && ok; t += pairs) {
-                if (!mbar_wait(smem_u32(&s.acc_empty[buf]), acc_phase ^ 1u, abort_flag)) break;
+                if (!mbar_wait_warp(smem_u32(&s.acc_empty[buf]), acc_phase ^ 1u, abort_flag)) break;
                 tc_fence_after();
-                const uint32_t acc = tmem + (uint32_t)buf * 256u;
+                const uint32_t acc = tm + (uint32_t)buf * 256u;
                 const int kb0 = (t % p.ksplit) * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.kblocks);
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    if (!mbar_wait(smem_u32(&s.full[stage]), phase, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(smem_u32(&s.full[stage]), phase, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t sa = smem0 + (uint32_t)stage * stage_bytes;
                     const uint64_t ad = smem_desc_sw128(sa), wd = smem_desc_sw128(sa + kBytesA);
 #pragma unroll
                     for (int k = 0; k < kBK / 16; ++k)
-                        umma_bf16_pair(acc, ad + (uint64_t)(k * 2), wd + (uint64_t)(k * 2), idesc, (kb > kb0 || k) ? 1u : 0u);
-                    umma_commit_pair(smem_u32(&s.empty[stage]));
+                        umma_bf16_pair(acc, ad + (uint64_t)(k * 2), wd + (uint64_t)(k * 2), idesc, (kb > kb0 || k) ? 1u : 0u, one);
+                    umma_commit_pair(smem_u32(&s.empty[stage]), one);
                     if (++stage == p.stages) { stage = 0; phase ^= 1u; }
                 }
-                if (ok) umma_commit_pair(smem_u32(&s.acc_full[buf]));
+                if (ok) umma_commit_pair(smem_u32(&s.acc_full[buf]), one);
                 if (++buf == 2) { buf = 0; acc_phase ^= 1u; }
             }
         }
