@@ -233,6 +233,15 @@ int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe
                     int64_t rescale1, int64_t rescale2, int64_t ep_mul, int64_t ep_div, int causal,
                     int64_t start_pos, int64_t mask_value, int a_limbs, int b_limbs, int flags, void* stream);
 
+/* The same with q_abs = (uk_rescale/2 + q_nope[b,s,h,:] . W_uk[h]) >> uk_rescale taken on the way: uk_planes holds the heads'
+ * weights [H][C1][D] (D = q_nope's width), uk_limbs > 0 promises q_nope's limbs and a_limbs (1..4) those of q_abs and q_pe, which
+ * stay limb planes between the two products.  Also ZKDS_ERR_UNSUPPORTED (silently) for up to 64 rows B * S, b_limbs <= 0, and where
+ * there is no room for the planes. */
+int zkds_mla_scores_heads(const int64_t* q_nope, const void* uk_planes, int64_t uk_rescale, int uk_limbs, const int64_t* kv,
+                          const int64_t* q_pe, const int64_t* pe, int64_t* out, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C1,
+                          int64_t C2, int64_t rescale1, int64_t rescale2, int64_t ep_mul, int64_t ep_div, int causal, int64_t start_pos,
+                          int64_t mask_value, int a_limbs, int b_limbs, int flags, void* stream);
+
 /* Causal counterparts for prefill attention whose masked scores were skipped (ZKDS_CAUSAL_SKIP).
  * Row (b, s, h) owns columns t <= start_pos + s only.  The results equal what softmax_q19 and
  * einsum_bsht_btc_bshc give on fully written masked scores, because a masked score (-(64<<36) added)
@@ -259,6 +268,14 @@ int zkds_einsum_bsht_btc_bshc_causal(const int64_t* P, const int64_t* KV, int64_
 int zkds_softmax_pv(const int64_t* scores, const int64_t* KV, int64_t* out, const int64_t* lut,
                     int64_t rescale, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C, int causal_skip,
                     int64_t start_pos, int a_limbs, int b_limbs, int flags, void* stream);
+
+/* The same followed by the heads' output weights: out [B,S,H,V] = ctx[b,s,h,:] . W_uv[h] >> uv_rescale with ctx the result above,
+ * which stays limb planes between the two products.  uv_planes: [heads][V][C], where H may hold the heads of several positions
+ * (S * H a multiple of the heads, out [B][S * H / heads][heads][V]); ctx_limbs (1..4) promises ctx's limbs.
+ * ZKDS_ERR_UNSUPPORTED (silently) also for b_limbs <= 0 and where there is no room for the planes. */
+int zkds_softmax_pv_heads(const int64_t* scores, const int64_t* KV, const void* uv_planes, int64_t uv_rescale, int ctx_limbs, int64_t* out,
+                          const int64_t* lut, int64_t rescale, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C, int causal_skip,
+                          int64_t start_pos, int a_limbs, int b_limbs, int flags, void* stream);
 
 /* ---- the latent cache kept as limb planes (decode) ---------------------------------------------------------
  * The reference's attention reads the whole int64 latent cache every step (model.py:884-926); split into limb

@@ -843,3 +843,27 @@ def test_padding_of_expert_tiles_left_out(kmod, dev, few):
     got = kmod.glu_prepared(r13[:, :I], r13[:, I:], w2, 16, ld=2 * I, a_limbs=4, tile_group=group, max_group_rows=few, leave_padding=True)
     assert torch.equal(got[used], want[used])
     kmod.device_status()
+
+
+@pytest.mark.parametrize("S,skip", [(129, None), (132, None), (130, False), (132, False), (131, True)])
+def test_mla_prefill_with_limbs_between_the_products(M, mo, kmod, dev, monkeypatch, S, skip):
+    """prompts whose queries and context stay limb planes, with and without padding positions and the masked half, against the layer
+    with measured limbs, which passes words"""
+    a = small_args(M, kv_lora_rank=128, n_heads=64, max_seq_len=160)
+    rng = np.random.default_rng(S)
+    attn = M.MLA(0, a).to(dev)
+    load_mla(attn, mla_weights(rng, a), dev)
+    x, mask, freqs = np.rint(rng.standard_normal((1, S, a.dim)) * 2.0**21).astype(np.int64), t(mo.causal_mask(S), dev), freqs_table(M, a)
+    through, plain = [], kmod.softmax_pv_fused
+
+    def counted(*args, heads=None, **kw):
+        out = plain(*args, heads=heads, **kw)
+        through.append(heads is not None and out is not None)
+        return out
+    monkeypatch.setattr(kmod, "softmax_pv_fused", counted)
+    attn.score_limbs, attn.causal_skip = (4, 4), skip
+    got = attn(t(x, dev), 0, freqs[:S].to(dev), mask)
+    kmod.device_status(sync=True)
+    assert through == [True]
+    attn.score_limbs, attn.causal_skip = (0, 0), False
+    assert torch.equal(got, attn(t(x, dev), 0, freqs[:S].to(dev), mask))

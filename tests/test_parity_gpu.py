@@ -1071,3 +1071,61 @@ def test_measured_ranges_of_more_steps_than_blocks(kmod, orc, dev, steps):
             busy = busy @ busy
         same(kmod.int64_bmm_broadcast(gx, gw, 1, 1, 3)[0], want[id(x)], "busy stream")
     kmod.device_status(sync=True)
+
+
+@pytest.mark.parametrize("B,S,H,D,C,R,T,limbs", [(1, 65, 40, 24, 128, 16, 68, 3), (2, 40, 24, 128, 256, 8, 44, 4), (1, 129, 16, 40, 512, 64, 132, 2),
+                                                 (1, 300, 8, 128, 512, 64, 304, 3)])
+def test_queries_that_stay_limbs_between_their_products(kmod, dev, B, S, H, D, C, R, T, limbs):
+    """the heads' product as limb planes of the scores against the same through words: ragged row tiles, batches, columns behind the
+    last tile; a query beyond its promise raises the flag"""
+    rng = np.random.default_rng(S + H)
+    q, q_pe = g(rand_i64(rng, (B, S, H, D), 20), dev), g(rand_i64(rng, (B, S, H, R), 8 * limbs - 5), dev)
+    kv, pe = g(rand_i64(rng, (B, T, C), 20), dev), g(rand_i64(rng, (B, T, R), 20), dev)
+    planes = kmod.WeightPlanes(g(rand_i64(rng, (H, C, D), 13).astype(np.int32), dev))
+    for beyond in (False, True):
+        heads = kmod.HeadsProduct(q, planes, 33 + 8 - 8 * limbs if beyond else 33 + 10 - 8 * limbs + (D > 64), 3)
+        if beyond:
+            q[-1, -1, -1] = (1 << 20) - 1
+            planes = kmod.WeightPlanes(torch.full((H, C, D), (1 << 13) - 1, dtype=torch.int32, device=dev))
+            heads = kmod.HeadsProduct(q, planes, 33 - 8 * limbs, 3)
+        words, heads.tensor = heads.tensor(), None                      # the planes or nothing
+        for how in (dict(), dict(causal=True), dict(causal=True, skip_masked=True), dict(causal=True, skip_masked=True, narrow=True)):
+            kw = dict(rescale1=23, rescale2=21, a_limbs=limbs, b_limbs=3, dynamic=True, **how)
+            got = kmod.mla_scores_fused(heads, kv, q_pe, pe, **kw)
+            if beyond:
+                with pytest.raises(kmod.ZkdsError) as e:
+                    kmod.device_status(sync=True)
+                assert e.value.status == kmod.ERR_RANGE
+                continue
+            want = kmod.mla_scores_fused(words, kv, q_pe, pe, **kw)
+            seen = torch.ones_like(want, dtype=torch.bool)
+            if "skip_masked" in how:
+                seen = (torch.arange(T, device=dev)[None] <= torch.arange(S, device=dev)[:, None])[None, :, None].expand_as(want)
+            assert got.dtype == want.dtype and torch.equal(got[seen], want[seen])
+            kmod.device_status(sync=True)
+
+
+@pytest.mark.parametrize("B,S,H,C,V,T,limbs", [(1, 129, 16, 512, 128, 132, 3), (2, 350, 5, 256, 24, 352, 4), (1, 1300, 16, 48, 40, 1300, 2),
+                                               (1, 65, 130, 144, 16, 68, 3)])
+def test_context_that_stays_limbs_between_its_products(kmod, dev, B, S, H, C, V, T, limbs):
+    """P . KV as limb planes of the heads' product against the same through words: several batches, heads that are no multiple of a tile,
+    a last column tile that is not full, the heads of all positions in one row; a context beyond its promise raises the flag"""
+    rng = np.random.default_rng(S + C)
+    scores = torch.randint(-9 << 19, 9 << 19, (B, S, H, T), device=dev, generator=torch.Generator(device=dev).manual_seed(S))
+    kv = g(rand_i64(rng, (B, T, C), 8 * limbs - 2), dev)
+    planes = kmod.WeightPlanes(g(rand_i64(rng, (H, V, C), 13).astype(np.int32), dev))
+    kmod.softmax_init_q19()
+    kw = dict(a_limbs=3, b_limbs=limbs)
+    for how in (dict(), dict(causal_skip=True, start_pos=T - S)):
+        ctx = kmod.softmax_pv_fused(scores, kv, 19, **kw, **how)
+        got = kmod.softmax_pv_fused(scores, kv, 19, **kw, **how, heads=(planes, 9, limbs))
+        assert torch.equal(got, kmod.einsum_heads_prepared(ctx, planes, 9, False, a_limbs=limbs, dynamic=True))
+    rows = scores.view(B, 1, S * H, T)
+    ctx = kmod.softmax_pv_fused(rows, kv, 19, causal_skip=True, start_pos=T - 2, **kw).view(B, S, H, C)
+    got = kmod.softmax_pv_fused(rows, kv, 19, causal_skip=True, start_pos=T - 2, **kw, heads=(planes, 9, limbs))
+    assert torch.equal(got, kmod.einsum_heads_prepared(ctx, planes, 9, False, a_limbs=limbs, dynamic=True))
+    kmod.device_status(sync=True)
+    kmod.softmax_pv_fused(scores, kv, 19, **kw, heads=(planes, 9, 1))
+    with pytest.raises(kmod.ZkdsError) as e:
+        kmod.device_status(sync=True)
+    assert e.value.status == kmod.ERR_RANGE

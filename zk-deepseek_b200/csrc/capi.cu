@@ -389,7 +389,37 @@ static bool scores_fit32(int a_limbs, int b_limbs, int64_t C1, int64_t C2, int64
     return (div ? sum * mul / div + 1 : sum) < ((int64_t)1 << 31);
 }
 
-int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe, const int64_t* pe,
+// q_abs, or where it is the product of the next three: q_nope [B,S,H,D] . W_uk, one weight a head
+struct HeadsProduct {
+    const int64_t* A;
+    const PlanesHandle* weights;
+    int64_t rescale, addend;
+    int limbs, dynamic;
+};
+
+static Contraction heads_problem(const HeadsProduct& h, int64_t rows, int64_t H)
+{
+    const int64_t K = h.weights->pl.K, N = h.weights->pl.rows;
+    Contraction p{};
+    p.A = h.A; p.b_bits = h.weights->b_bits;
+    p.batches = H; p.M = rows; p.N = N; p.K = K;
+    p.a_sz = K; p.a_sm = H * K;
+    p.b_sz = 1;
+    p.c_sz = N; p.c_sm = H * N;
+    p.a_div = 1; p.b_div = 1;
+    p.addend = h.addend; p.shift = (int)h.rescale;
+    p.dynamic_a = h.dynamic;
+    return p;
+}
+
+// the words behind a contraction's own, of slot 5, that a product left as limb planes is measured into
+static unsigned long long* planes_most()
+{
+    unsigned long long* words = (unsigned long long*)workspace(8 * sizeof(uint64_t), 5);
+    return words ? words + 4 : nullptr;
+}
+
+static int mla_scores(const int64_t* q_abs, const HeadsProduct* heads, const int64_t* kv, const int64_t* q_pe, const int64_t* pe,
                     int64_t* out, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C1, int64_t C2,
                     int64_t rescale1, int64_t rescale2, int64_t ep_mul, int64_t ep_div, int causal,
                     int64_t start_pos, int64_t mask_value, int a_limbs, int b_limbs, int flags, void* stream)
@@ -398,7 +428,7 @@ int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe
         rescale2 < 0 || rescale2 > 127)
         return finish(ZKDS_ERR_ARG, "zkds_mla_scores");
     if (B == 0 || S == 0 || H == 0 || T == 0) return finish(ZKDS_OK, "zkds_mla_scores");
-    if (!q_abs || !kv || !q_pe || !pe || !out) return finish(ZKDS_ERR_ARG, "zkds_mla_scores");
+    if ((!q_abs && !heads) || !kv || !q_pe || !pe || !out) return finish(ZKDS_ERR_ARG, "zkds_mla_scores");
     cudaStream_t st = ST(stream);
     const bool narrow = (flags & ZKDS_SCORES_32) != 0;
     if (narrow && !(causal && (flags & ZKDS_CAUSAL_SKIP) &&
@@ -437,11 +467,45 @@ int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe
     f.dynamic_a = (flags & ZKDS_LIMBS_DYNAMIC) ? 1 : 0;
     f.skip_tiles = (flags & ZKDS_CAUSAL_SKIP) ? 1 : 0;
     f.out_bits = narrow ? 32 : 64;
+    if (heads) {
+        const int64_t pitch = C1 + ((C2 + 15) & ~(int64_t)15), step = B * S * H * pitch;
+        f.a1_most = planes_most();
+        if (!f.a1_most) return finish(ZKDS_ERR_WORKSPACE, "zkds_mla_scores");
+        f.a1_planes = (int8_t*)workspace((size_t)a_limbs * step + 1024, 2);
+        if (!f.a1_planes) { t_status = ZKDS_ERR_UNSUPPORTED; return t_status; }       // words need less at a time
+        Contraction p = heads_problem(*heads, B * S, H);
+        p.to_planes = LimbOut{f.a1_planes, a_limbs, step, pitch, 1, H, 0, 1, f.a1_most};
+        int rc = launch_contraction_limb(p, heads->limbs, 0, &heads->weights->pl, st);
+        if (rc == ZKDS_ERR_UNSUPPORTED) { t_status = rc; return rc; }
+        if (rc != ZKDS_OK) return finish(rc, "zkds_mla_scores");
+    }
     // ZKDS_ERR_UNSUPPORTED is an expected answer here (the caller then runs the two contractions
     // separately), so it is returned without the stderr line
     int rc = launch_scores_fused(f, a_limbs, b_limbs, st);
     if (rc == ZKDS_ERR_UNSUPPORTED) { t_status = rc; return rc; }
     return finish(rc, "zkds_mla_scores");
+}
+
+int zkds_mla_scores(const int64_t* q_abs, const int64_t* kv, const int64_t* q_pe, const int64_t* pe, int64_t* out, int64_t B, int64_t S,
+                    int64_t H, int64_t T, int64_t C1, int64_t C2, int64_t rescale1, int64_t rescale2, int64_t ep_mul, int64_t ep_div,
+                    int causal, int64_t start_pos, int64_t mask_value, int a_limbs, int b_limbs, int flags, void* stream)
+{
+    return mla_scores(q_abs, nullptr, kv, q_pe, pe, out, B, S, H, T, C1, C2, rescale1, rescale2, ep_mul, ep_div, causal, start_pos,
+                      mask_value, a_limbs, b_limbs, flags, stream);
+}
+
+int zkds_mla_scores_heads(const int64_t* q_nope, const void* uk_planes, int64_t uk_rescale, int uk_limbs, const int64_t* kv,
+                          const int64_t* q_pe, const int64_t* pe, int64_t* out, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C1,
+                          int64_t C2, int64_t rescale1, int64_t rescale2, int64_t ep_mul, int64_t ep_div, int causal, int64_t start_pos,
+                          int64_t mask_value, int a_limbs, int b_limbs, int flags, void* stream)
+{
+    const PlanesHandle* w = (const PlanesHandle*)uk_planes;
+    if (!q_nope || !w || w->pl.nb != H || w->pl.rows != C1 || uk_rescale < 0 || uk_rescale > 127 || uk_limbs <= 0)
+        return finish(ZKDS_ERR_ARG, "zkds_mla_scores_heads");
+    if (a_limbs <= 0 || a_limbs > 4 || b_limbs <= 0) { t_status = ZKDS_ERR_UNSUPPORTED; return t_status; }
+    const HeadsProduct h{q_nope, w, uk_rescale, uk_rescale / 2, uk_limbs, (flags & ZKDS_LIMBS_DYNAMIC) ? 1 : 0};
+    return mla_scores(nullptr, &h, kv, q_pe, pe, out, B, S, H, T, C1, C2, rescale1, rescale2, ep_mul, ep_div, causal, start_pos, mask_value,
+                      a_limbs, b_limbs, flags, stream);
 }
 
 static int grouped_prepared(const int64_t* A, const int* row_index, const void* planes, const int* tile_group,
@@ -533,7 +597,7 @@ int zkds_einsum_bsht_btc_bshc_causal(const int64_t* P, const int64_t* KV, int64_
     return finish(run_contraction(p, a_limbs, b_limbs, f, ST(stream)), "zkds_einsum_bsht_btc_bshc_causal");
 }
 
-int zkds_softmax_pv(const int64_t* scores, const int64_t* KV, int64_t* out, const int64_t* lut,
+static int softmax_pv(const HeadsProduct* heads, const int64_t* scores, const int64_t* KV, int64_t* out, const int64_t* lut,
                     int64_t rescale, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C, int causal_skip,
                     int64_t start_pos, int a_limbs, int b_limbs, int flags, void* stream)
 {
@@ -562,9 +626,45 @@ int zkds_softmax_pv(const int64_t* scores, const int64_t* KV, int64_t* out, cons
         if (rc != ZKDS_OK) return finish(rc, "zkds_softmax_pv");
         b_limbs = limbs_needed(h);
     }
+    if (!heads) {
+        int rc = launch_contraction_limb(p, a_limbs, b_limbs, nullptr, st);
+        if (rc == ZKDS_ERR_UNSUPPORTED) { t_status = rc; return rc; }
+        return finish(rc, "zkds_softmax_pv");
+    }
+    // (a row may hold several positions' heads: the weights know how many heads there are)
+    const int64_t Hw = heads->weights->pl.nb, rows = B * S * H / Hw, step = rows * Hw * C;
+    unsigned long long* most = planes_most();
+    if (!most) return finish(ZKDS_ERR_WORKSPACE, "zkds_softmax_pv");
+    int8_t* ctx = (int8_t*)workspace((size_t)heads->limbs * step + 1024, 2);
+    if (!ctx) { t_status = ZKDS_ERR_UNSUPPORTED; return t_status; }
+    p.to_planes = LimbOut{ctx, heads->limbs, step, C, Hw, 1, rows, S * H / Hw, most};
     int rc = launch_contraction_limb(p, a_limbs, b_limbs, nullptr, st);
+    if (rc == ZKDS_OK) {
+        Contraction q = heads_problem(*heads, rows, Hw);
+        q.C = out;
+        q.a_planes = ctx; q.a_most = most;
+        rc = launch_contraction_limb(q, heads->limbs, 0, &heads->weights->pl, st);
+    }
     if (rc == ZKDS_ERR_UNSUPPORTED) { t_status = rc; return rc; }
     return finish(rc, "zkds_softmax_pv");
+}
+
+int zkds_softmax_pv(const int64_t* scores, const int64_t* KV, int64_t* out, const int64_t* lut, int64_t rescale, int64_t B, int64_t S,
+                    int64_t H, int64_t T, int64_t C, int causal_skip, int64_t start_pos, int a_limbs, int b_limbs, int flags, void* stream)
+{
+    return softmax_pv(nullptr, scores, KV, out, lut, rescale, B, S, H, T, C, causal_skip, start_pos, a_limbs, b_limbs, flags, stream);
+}
+
+int zkds_softmax_pv_heads(const int64_t* scores, const int64_t* KV, const void* uv_planes, int64_t uv_rescale, int ctx_limbs, int64_t* out,
+                          const int64_t* lut, int64_t rescale, int64_t B, int64_t S, int64_t H, int64_t T, int64_t C, int causal_skip,
+                          int64_t start_pos, int a_limbs, int b_limbs, int flags, void* stream)
+{
+    const PlanesHandle* w = (const PlanesHandle*)uv_planes;
+    if (!w || w->pl.nb <= 0 || H < 0 || S < 0 || (S * H) % w->pl.nb || w->pl.K != C || uv_rescale < 0 || uv_rescale > 127 || ctx_limbs <= 0)
+        return finish(ZKDS_ERR_ARG, "zkds_softmax_pv_heads");
+    if (ctx_limbs > 4 || a_limbs <= 0 || b_limbs <= 0) { t_status = ZKDS_ERR_UNSUPPORTED; return t_status; }
+    const HeadsProduct h{nullptr, w, uv_rescale, 0, ctx_limbs, 1};
+    return softmax_pv(&h, scores, KV, out, lut, rescale, B, S, H, T, C, causal_skip, start_pos, a_limbs, b_limbs, flags, stream);
 }
 
 int zkds_cache_planes_append(const int64_t* kv_new, const int64_t* pe_new, int8_t* score_planes,

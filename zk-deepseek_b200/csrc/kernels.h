@@ -84,6 +84,16 @@ int launch_peer_barrier(unsigned long long* const* flag_bases, int n_parts, int 
 // with the sum held in 128 bits.  A is int64 with unit k-stride; B is int32 or int64
 // with arbitrary n- and k-strides (so the MLA einsums map onto it without copies).
 // a_div / b_div are C truncating divisors applied to each element before the product.
+// Where a contraction leaves its results as limb planes for the next one instead of as words: row m of batch z at
+// data[l * step + ((m / div) * rq + (m % div) * rr + z * rz) * pitch], one byte a column and limb l < L <= 4; most <- the largest
+// magnitude (as a split measures it; zeroed by the launch).  A result that L limbs do not hold raises the limb flag.
+struct LimbOut {
+    int8_t* data;             // null = words
+    int L;
+    int64_t step, pitch, div, rq, rr, rz;
+    unsigned long long* most;
+};
+
 struct Contraction {
     const int64_t* A;
     const void* B;
@@ -142,6 +152,10 @@ struct Contraction {
     const int64_t* softmax_lut;
     int64_t softmax_S;
     int softmax_bits;         // words of the scores: 0 = 64, 32
+    LimbOut to_planes;        // ZKDS_ERR_UNSUPPORTED where limb_tiles_kernel does not take the call
+    // A is there as limb planes already, [La][batches][M][K rounded up to 16], with the range that was measured
+    const int8_t* a_planes;
+    const unsigned long long* a_most;
     // A is r1 of a gated MLP (rows of K words, row stride a_sm): the limb planes are produced from
     // (silu_q23(A) * glu_r2) >> 23, glu_r2 with the same row stride, and the gated product never reaches
     // memory as int64 (limb kernel only, batches == 1)
@@ -183,6 +197,9 @@ struct FusedScores {
     // which rows [0, N) of every batch are in use; B1 and B2 are then ignored
     const int8_t* b_planes;
     int64_t b_batch_rows;
+    // A1 is there as limb planes: columns [0, K1) of rows of K1 + round16(K2) bytes, [La][batches][M]; A2 is split beside them
+    int8_t* a1_planes;
+    unsigned long long* a1_most;
 };
 // new cache rows as limb planes in both layouts the attention contractions read (see zkds_cache_planes_append)
 int launch_cache_planes_append(const int64_t* kv_new, const int64_t* pe_new, int8_t* score_planes,

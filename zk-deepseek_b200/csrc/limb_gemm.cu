@@ -28,6 +28,8 @@
 
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "tcgen05.cuh"
@@ -409,6 +411,7 @@ struct LimbParams {
     const int64_t* addin;
     int64_t ep_mul, ep_div;
     int64_t causal_H, causal_start, mask_value;
+    LimbOut out;              // limb_tiles_kernel: results as the next contraction's limb planes
     // split-K (one-tile kernel, few output tiles, deep K: the weight-streaming shapes of decode).
     // ksplit CTAs share an output tile, each accumulates kb_per_split K blocks; they add their shares of
     // the sums (integers: exact in any order) to partial[tile][word][column][row], and the CTA that
@@ -2139,6 +2142,61 @@ struct TileStore {
     int shift;
     bool row_ok, wide;        // wide: 32-byte stores stay aligned
 };
+template <bool STAGED>          // through shared memory
+struct PlaneStore {
+    int8_t* planes;           // this lane's row of the limb planes at the tile's first column
+    uint32_t stage, limb;     // shared memory: this lane's row of the warps' limb tiles, bytes between limbs
+    int64_t n0;
+    int shift;
+    bool row_ok;
+    uint32_t *bits, *beyond;  // what this lane has met: bits of the magnitudes, words beyond L limbs
+};
+
+// W results as bytes of p.out's planes: the digits of v are the bytes of v + 0x80..80 with their top bits flipped, as in put_digits
+template <int W, bool STAGED>
+__device__ __forceinline__ void tile_store(const LimbParams& p, const PlaneStore<STAGED>& t, int col, const int64_t (&q)[W])
+{
+    const uint32_t bias = 0x80808080u >> (8 * (4 - p.out.L));
+    uint32_t low[W], bits = *t.bits, beyond = *t.beyond, any = 0;
+    const int left = (int)(p.N - t.n0) - col;
+#pragma unroll
+    for (int c = 0; c < W; ++c) {
+        const uint64_t v = (uint64_t)q[c] + bias;
+        low[c] = (uint32_t)v;
+        if ((c & ~3) >= left) continue;            // columns behind the last, fours of them: nobody's
+        beyond |= (uint32_t)(v >> 32);
+        any |= low[c];
+        const int32_t x = (int32_t)q[c];           // all of it, unless the word is beyond
+        bits |= (uint32_t)(x ^ (x >> 31));
+    }
+    *t.bits = bits;
+    *t.beyond = beyond | (p.out.L < 4 ? any >> (8 * p.out.L) : 0u);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        if (l >= p.out.L) break;
+        const uint32_t sel = 0x0040u + 0x0011u * (uint32_t)l;     // byte l of both operands
+        uint32_t w[W / 4];
+#pragma unroll
+        for (int i = 0; i < W / 4; ++i)
+            w[i] = __byte_perm(__byte_perm(low[4 * i], low[4 * i + 1], sel), __byte_perm(low[4 * i + 2], low[4 * i + 3], sel), 0x5410u) ^
+                   0x80808080u;
+        if constexpr (!STAGED) {
+            int8_t* at = t.planes + l * p.out.step + col;
+            // (N is a multiple of 16 and pieces of 8 and 16 start at multiples of 8: eights are inside or outside)
+            if (W == 16 && !(col & 8) && left >= 16)
+                asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(at), "r"(w[0]), "r"(w[1]), "r"(w[W / 4 - 2]), "r"(w[W / 4 - 1]) : "memory");
+            else if constexpr (W >= 8) {
+#pragma unroll
+                for (int i = 0; i < W / 4; i += 2)
+                    if (4 * i < left) asm volatile("st.global.v2.b32 [%0], {%1, %2};" ::"l"(at + 4 * i), "r"(w[i]), "r"(w[i + 1]) : "memory");
+            } else if (left > 0) asm volatile("st.global.b32 [%0], %1;" ::"l"(at), "r"(w[0]) : "memory");
+        } else {
+#pragma unroll
+            for (int i = 0; i < W / 4; ++i)
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(t.stage + (uint32_t)l * t.limb + (uint32_t)(col + 4 * i)), "r"(w[i]) : "memory");
+        }
+    }
+}
 
 template <int W>
 __device__ __forceinline__ void tile_store(const LimbParams& p, const TileStore& t, int col, const int64_t (&q)[W])
@@ -2158,8 +2216,8 @@ __device__ __forceinline__ void tile_store(const LimbParams& p, const TileStore&
 }
 
 // W columns from `col` on of a tile whose sums fit 64 bits, DD diagonals.  `loaded` runs once they are in registers
-template <int DD, int W, typename F>
-__device__ __forceinline__ void tile_columns(const LimbParams& p, const TileStore& t, uint32_t tq, int col, const F& loaded)
+template <int DD, int W, typename S, typename F>
+__device__ __forceinline__ void tile_columns(const LimbParams& p, const S& t, uint32_t tq, int col, const F& loaded)
 {
     int64_t T[W];
 #pragma unroll
@@ -2189,8 +2247,8 @@ __device__ __forceinline__ void tile_columns(const LimbParams& p, const TileStor
 }
 
 // four columns of any other sum, up to eight diagonals: two words of four diagonals each
-template <typename F>
-__device__ __forceinline__ void tile_columns_128(const LimbParams& p, const TileStore& t, uint32_t tq, int D, int col, const F& loaded)
+template <typename S, typename F>
+__device__ __forceinline__ void tile_columns_128(const LimbParams& p, const S& t, uint32_t tq, int D, int col, const F& loaded)
 {
     int64_t low[4], high[4] = {};
     int32_t a[8][4];
@@ -2214,8 +2272,8 @@ __device__ __forceinline__ void tile_columns_128(const LimbParams& p, const Tile
     tile_store(p, t, col, q);
 }
 
-template <int W, typename F>
-__device__ __forceinline__ void tile_columns_64(const LimbParams& p, const TileStore& t, uint32_t tq, int D, int col, const F& loaded)
+template <int W, typename S, typename F>
+__device__ __forceinline__ void tile_columns_64(const LimbParams& p, const S& t, uint32_t tq, int D, int col, const F& loaded)
 {
     switch (D) {              // as many as a 62-bit sum can have
     case 1: tile_columns<1, W>(p, t, tq, col, loaded); break;
@@ -2227,11 +2285,12 @@ __device__ __forceinline__ void tile_columns_64(const LimbParams& p, const TileS
     }
 }
 
+template <bool PLANES, bool STAGED>          // results as the limb planes of p.out, directly or through shared memory; else as words
 __global__ void __launch_bounds__(kTileThreads, 1)
 limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LimbParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * 8 + 4];
+    __shared__ __align__(8) uint64_t bars[2 * 8 + 4 + 4];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2262,6 +2321,7 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             mbar_init(bar_tfull + 8 * b, 1);
             mbar_init(bar_tempty + 8 * b, kTileWarps);
         }
+        for (int g = 0; STAGED && g < 4; ++g) mbar_init(smem_u32(&bars[20 + g]), kTileWarps / 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -2344,7 +2404,13 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             }
         }
     } else {
-        const int ew = warp - 2, q = warp & 3, CW = p.NT / (kTileWarps / 4), c0 = (ew >> 2) * CW;
+        // a quarter of the columns to a warp; whole eights where a lane stores their limbs itself
+        const int ew = warp - 2, q = warp & 3, part = ew >> 2, fine = PLANES && !STAGED ? 8 : 4, pieces = p.NT / fine;
+        const int c0 = pieces * part / 4 * fine, CW = pieces * (part + 1) / 4 * fine - c0;
+        // PLANES: the limb tiles of the four warps with the same rows, [limb][row][NT + 4] behind the stages
+        [[maybe_unused]] const uint32_t row_bytes = (uint32_t)p.NT + 4, staged = smem_base + (uint32_t)p.stages * stage_bytes +
+                                                                                 (uint32_t)(q * p.out.L * 32) * row_bytes;
+        [[maybe_unused]] const uint32_t bar_rows = smem_u32(&bars[20 + q]);      // even phases: written, odd ones: read
         const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
         // clears the columns that no first MMA overwrites, of W columns from col on
         auto clear = [&](uint32_t tq, int col, int W) {
@@ -2363,6 +2429,7 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
         int buf = 0;
         uint32_t turn = 0;
+        [[maybe_unused]] uint32_t bits = 0, beyond = 0;
         const bool wide = ((uintptr_t)p.C & 31) == 0 && ((p.c_sm | p.c_sz) & 3) == 0;
         for (int64_t tile = blockIdx.x; tile < total; tile += gridDim.x) {
             const TileCoord tc = decode_tile(p, tile);
@@ -2379,9 +2446,22 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             tc_fence_after();
             const uint32_t tq = lanes + (uint32_t)(buf * buf_cols);
             const int64_t m = tc.m0 + q * 32 + lane, at = tc.z * p.c_sz + m * p.c_sm + tc.n0;
-            TileStore t;
-            t.c = p.C + at;
-            t.n0 = tc.n0; t.row_ok = m < p.M; t.wide = wide;
+            [[maybe_unused]] int64_t row = 0;
+            std::conditional_t<PLANES, PlaneStore<STAGED>, TileStore> t;
+            t.n0 = tc.n0; t.row_ok = m < p.M;
+            if constexpr (PLANES) {
+                const int64_t whole = (uint32_t)m / (uint32_t)p.out.div, rest = m - whole * p.out.div;
+                row = (whole * p.out.rq + rest * p.out.rr + tc.z * p.out.rz) * p.out.pitch + tc.n0;
+                t.planes = p.out.data + row;
+                t.stage = staged + (uint32_t)lane * row_bytes;
+                t.limb = 32 * row_bytes;
+                // the rows in front have left shared memory
+                if (STAGED && !__all_sync(0xffffffffu, mbar_wait(bar_rows, 1u, abort_flag))) break;
+                t.bits = &bits; t.beyond = &beyond;
+            } else {
+                t.c = p.C + at;
+                t.wide = wide;
+            }
             for (int col = c0; col < c0 + CW;) {
                 // the shift belongs to the group and to the side of n_split (a multiple of 8) that the columns lie on
                 t.shift = p.group_shift ? p.group_shift[2 * tc.group + (tc.n0 + col >= p.n_split ? 1 : 0)] : p.shift;
@@ -2399,7 +2479,33 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 else tile_columns_64<4>(p, t, tq, D, col, loaded);
                 col += W;
             }
+            if constexpr (STAGED) {
+                // eight of the rows a warp, whole rows of the tile a store: NT bytes of every limb side by side
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_rows);
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_rows, 0u, abort_flag))) break;
+                const int words = p.NT / 4;
+                for (int r = part * 8; r < part * 8 + 8; ++r) {
+                    int8_t* at = p.out.data + __shfl_sync(0xffffffffu, row, r) + 4 * lane;
+                    if (tc.m0 + q * 32 + r >= p.M || lane >= words || tc.n0 + 4 * lane >= p.N) continue;
+                    for (int l = 0; l < p.out.L; ++l) {
+                        uint32_t w;
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w) : "r"(staged + (uint32_t)(l * 32 + r) * row_bytes + 4u * lane) : "memory");
+                        asm volatile("st.global.b32 [%0], %1;" ::"l"(at + l * p.out.step), "r"(w) : "memory");
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_rows);
+            }
             if (++buf == p.nbuf) { buf = 0; turn ^= 1u; }
+        }
+        if constexpr (PLANES) {
+            // the bits of all magnitudes together tell the limbs they need, but no more than were promised
+            bits = __reduce_or_sync(0xffffffffu, bits);
+            beyond = __reduce_or_sync(0xffffffffu, beyond);
+            const uint32_t top = 0x7F7F7F7Fu >> (8 * (4 - p.out.L));
+            const unsigned long long most = beyond ? ~0ull >> 1 : bits < top ? bits : top;
+            if (lane == 0 && most > *(volatile unsigned long long*)p.out.most) atomicMax(p.out.most, most);
         }
     }
     tc_fence_before();
@@ -2848,7 +2954,7 @@ static int allow_big_smem(K kernel, bool (&done)[64])
     }
     return ZKDS_OK;
 }
-static bool g_attr_onetile[64], g_attr_rows[64], g_attr_tiles[64], g_attr_direct[64], g_attr_p16[64], g_attr_p8[64];
+static bool g_attr_onetile[64], g_attr_rows[64], g_attr_tiles[64], g_attr_tile_planes[64], g_attr_tile_staged[64], g_attr_direct[64], g_attr_p16[64], g_attr_p8[64];
 
 static cudaEvent_t* timing_events()
 {
@@ -3155,23 +3261,33 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     // as many tiles as SMs with a K that can be shared, boxes of few rows, remainders, element-wise tails, more than eight diagonals.
     if (persistent) NT = pNT;
     const int64_t nt_eff = (p.N + NT - 1) / NT;
+    const size_t plane_rows = p.to_planes.data ? (size_t)kTileM * p.to_planes.L * (NT + 4) : 0;       // see limb_tiles_kernel
+    if (p.to_planes.data && (by_rows || p.R || p.tile_group || p.skip_tiles || p.addin || p.ep_div || p.causal_H || switches().no_persistent ||
+                             p.M <= 64 || p.M > 0x7fffffffll || (p.N & 15) || NT < 32 || smem_max < plane_rows ||
+                             (smem_max - plane_rows) / ((size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK) < 2 || p.to_planes.L > 4 ||
+                             p.batches * mt * nt_eff * 2 <= sm_count() || (sum_fits64(La, Lb, p.K, p.addend) ? D > 6 : D > 8)))
+        return ZKDS_ERR_UNSUPPORTED;
 
     DeviceFlags* fl = flags_for_device();
     if (!fl) return ZKDS_ERR_WORKSPACE;
-    const bool direct = by_rows && few <= kDirectRows && La <= 7 && p.a_div == 1 && !p.softmax_lut && !p.glu_lut && p.a_n_parts == 0;
-    int8_t* pa = direct ? nullptr : (int8_t*)workspace((size_t)La * a_rows * Kp + 1024, 0);
+    const bool direct = by_rows && few <= kDirectRows && La <= 7 && p.a_div == 1 && !p.softmax_lut && !p.glu_lut && p.a_n_parts == 0 &&
+                        !p.a_planes;
+    int8_t* pa = p.a_planes ? const_cast<int8_t*>(p.a_planes) : direct ? nullptr : (int8_t*)workspace((size_t)La * a_rows * Kp + 1024, 0);
     if (!pa && !direct) return ZKDS_ERR_WORKSPACE;
     unsigned long long* d_absmax = nullptr;
-    if (p.dynamic_a && !direct) {
+    if (p.a_planes) {
+        d_absmax = const_cast<unsigned long long*>(p.a_most);
+    } else if (p.dynamic_a && !direct) {
         unsigned long long* words = (unsigned long long*)workspace(8 * sizeof(uint64_t), 5);
         if (!words) return ZKDS_ERR_WORKSPACE;
         d_absmax = words + 2;
         ZKDS_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(uint64_t), st));
     }
+    if (p.to_planes.data) ZKDS_CUDA(cudaMemsetAsync(p.to_planes.most, 0, sizeof(uint64_t), st));
     const int64_t Kp16 = Kp;
     int rc = ZKDS_OK;
-    if (direct) {
-        // limb_rows_kernel reads the activations itself
+    if (direct || p.a_planes) {
+        // limb_rows_kernel reads the activations itself, or they are limbs already
     } else if (p.softmax_lut) {
         if (p.a_sm != p.K || p.a_sz != p.M * p.K || p.a_div != 1) return ZKDS_ERR_ARG;
         rc = launch_softmax_planes(p.A, p.softmax_bits ? p.softmax_bits : 64, p.softmax_lut, pa, La, a_rows, p.K, Kp, a_rows * Kp, fl->overflow_dev,
@@ -3318,6 +3434,12 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     lp.tile_group = p.tile_group;
     lp.group_shift = p.group_shift; lp.n_split = p.n_split;
     lp.leave_padding = p.tile_group ? p.leave_padding : 0;
+    // A lane's own row in global memory is 32 pieces of 16 bytes a store instruction; rows that pass through shared memory cost the
+    // warps two waits for each other a tile.  One K block (128 heads of 4096 tokens, K = 128): 785 us directly, 1175 staged, 718 with
+    // words; deeper ones: P . KV of 4096 tokens 4177, 3712, 3631, of 777 tokens (four limbs) 669, 616, 547.  The pass over those words
+    // that is saved takes 718, 712 and 195 us.
+    lp.out = p.to_planes;
+    const bool staged = lp.kblocks > 1;
     lp.addin = p.addin; lp.ep_mul = p.ep_mul; lp.ep_div = p.ep_div;
     lp.causal_H = p.causal_H; lp.causal_start = p.causal_start; lp.mask_value = p.mask_value;
 
@@ -3351,13 +3473,13 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     if (tiles) {
         lp.backoff = switches().no_backoff ? 0u : 1u;
         lp.nbuf = 2 * D * NT <= 512 ? 2 : 1;
-        lp.stages = stages = (int)(smem_max / ((size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK));
+        lp.stages = stages = (int)((smem_max - plane_rows) / ((size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK));
         if (stages > 8) lp.stages = stages = 8;
         stage_bytes = (size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK;
         lp.tmem_cols = 32;
         while (lp.tmem_cols < (uint32_t)(lp.nbuf * D * NT)) lp.tmem_cols <<= 1;
     }
-    size_t smem = stage_bytes * stages + 1024;
+    size_t smem = stage_bytes * stages + plane_rows + 1024;
     // more than half the shared memory per CTA keeps one CTA per SM, so its tensor-memory
     // allocation can never wait for a co-resident CTA
     if (smem < 120 * 1024) smem = 120 * 1024;
@@ -3375,9 +3497,10 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     if (tiles) {
         const int64_t total_tiles = p.batches * mt * nt_eff;
         if (total_tiles > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
-        rc = allow_big_smem(limb_tiles_kernel, g_attr_tiles);
+        auto kernel = !p.to_planes.data ? limb_tiles_kernel<false, false> : staged ? limb_tiles_kernel<true, true> : limb_tiles_kernel<true, false>;
+        rc = allow_big_smem(kernel, !p.to_planes.data ? g_attr_tiles : staged ? g_attr_tile_staged : g_attr_tile_planes);
         if (rc != ZKDS_OK) return rc;
-        limb_tiles_kernel<<<(unsigned)(total_tiles < sm_count() ? total_tiles : sm_count()), kTileThreads, smem, st>>>(tmA, tmB, lp);
+        kernel<<<(unsigned)(total_tiles < sm_count() ? total_tiles : sm_count()), kTileThreads, smem, st>>>(tmA, tmB, lp);
         rc = check_launch();
     } else if (persistent) {
         if (psmem < 120 * 1024) psmem = 120 * 1024;
@@ -3479,18 +3602,22 @@ int launch_scores_fused(const FusedScores& f, int La, int Lb, cudaStream_t st)
 
     DeviceFlags* fl = flags_for_device();
     if (!fl) return ZKDS_ERR_WORKSPACE;
-    int8_t* pa = (int8_t*)workspace((size_t)La * a_rows * pitch + 1024, 0);
+    int8_t* pa = f.a1_planes ? f.a1_planes : (int8_t*)workspace((size_t)La * a_rows * pitch + 1024, 0);
     int8_t* pb = f.b_planes ? const_cast<int8_t*>(f.b_planes)
                             : (int8_t*)workspace((size_t)Lb * b_rows * pitch + 1024, 1);
     if (!pa || !pb) return ZKDS_ERR_WORKSPACE;
     unsigned long long* d_absmax = nullptr;
-    if (f.dynamic_a) {
+    if (f.a1_planes) {
+        d_absmax = f.a1_most;
+    } else if (f.dynamic_a) {
         unsigned long long* words = (unsigned long long*)workspace(8 * sizeof(uint64_t), 5);
         if (!words) return ZKDS_ERR_WORKSPACE;
         d_absmax = words + 2;
         ZKDS_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(uint64_t), st));
     }
-    int rc = launch_split_t<int64_t>(f.A1, pa, La, f.batches, f.M, f.K1, f.K1, f.M * f.K1, f.K1, 1, 1,
+    int rc = ZKDS_OK;
+    if (!f.a1_planes)
+        rc = launch_split_t<int64_t>(f.A1, pa, La, f.batches, f.M, f.K1, f.K1, f.M * f.K1, f.K1, 1, 1,
                                      fl->overflow_dev, st, d_absmax, pitch);
     if (rc == ZKDS_OK)
         rc = launch_split_t<int64_t>(f.A2, pa + f.K1, La, f.batches, f.M, f.K2, Kp2, f.M * f.K2, f.K2, 1, 1,

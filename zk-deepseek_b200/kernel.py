@@ -101,8 +101,10 @@ _sig("zkds_einsum_bshc_btc_bsht_ex", [_vp, _vp, _vp, _ll, _ll, _ll, _ll, _ll, _l
                                       _ll, _i, _i, _i, _vp])
 _sig("zkds_mla_scores", [_vp, _vp, _vp, _vp, _vp, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _i, _ll, _ll,
                          _i, _i, _i, _vp])
+_sig("zkds_mla_scores_heads", [_vp, _vp, _ll, _i] + [_vp] * 4 + [_ll] * 10 + [_i, _ll, _ll, _i, _i, _i, _vp])
 _sig("zkds_softmax_causal", [_vp, _vp, _vp, _ll, _ll, _ll, _ll, _ll, _vp])
 _sig("zkds_softmax_pv", [_vp, _vp, _vp, _vp, _ll, _ll, _ll, _ll, _ll, _ll, _i, _ll, _i, _i, _i, _vp])
+_sig("zkds_softmax_pv_heads", [_vp] * 3 + [_ll, _i, _vp, _vp] + [_ll] * 6 + [_i, _ll, _i, _i, _i, _vp])
 _sig("zkds_einsum_bsht_btc_bshc_causal", [_vp, _vp, _vp, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _i, _i, _i, _vp])
 _sig("zkds_grouped_prepared", [_vp, _vp, _vp, _ll, _vp, _ll, _ll, _ll, _vp, _ll, _i, _i, _vp])
 _sig("zkds_glu_prepared", [_vp, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _ll, _vp, _ll, _i, _i, _vp])
@@ -523,14 +525,29 @@ def _scores_fit32(a_limbs, b_limbs, C1, C2, rescale1, rescale2, mul, div):
     return ((C1 * both >> rescale1) + (C2 * both >> rescale2) + 4) * mul // div + 1 < 1 << 31
 
 
+class HeadsProduct:
+    """einsum_heads_prepared(A, planes, rescale, True, a_limbs, True) that has not been taken: mla_scores_fused leaves it as limb planes
+    between its products where it can; tensor() is the words"""
+
+    def __init__(self, A, planes, rescale, a_limbs):
+        _dev_i64(A, "A")
+        assert A.shape[2] == planes.nb and A.shape[3] == planes.K and a_limbs > 0
+        self.A, self.planes, self.rescale, self.a_limbs = A, planes, int(rescale), a_limbs
+        self.shape, self.device = A.shape[:3] + (planes.N,), A.device
+
+    def tensor(self):
+        return einsum_heads_prepared(self.A, self.planes, self.rescale, True, a_limbs=self.a_limbs, dynamic=True)
+
+
 def mla_scores_fused(q_abs, kv, q_pe, pe, rescale1=23, rescale2=21, mul=94, div=695, causal=False,
                      start_pos=0, mask_value=-(64 << 36), a_limbs=0, b_limbs=0, dynamic=False,
                      skip_masked=False, narrow=False):
     """scores = ((score1 + score2) * mul // div) (+ causal mask) with score1 = einsum(q_abs, kv) at
     rescale1 and score2 = einsum(q_pe, pe) at rescale2, in one tensor-core pass (model.py:884-905).
-    narrow (with causal and skip_masked): int32 scores where the limbs prove them to fit.  Returns None when the fused
-    kernel does not take the shape (caller falls back)."""
-    for t, n in ((q_abs, "q_abs"), (kv, "kv"), (q_pe, "q_pe"), (pe, "pe")):
+    narrow (with causal and skip_masked): int32 scores where the limbs prove them to fit.  q_abs may be a HeadsProduct.
+    Returns None when the fused kernel does not take the shape (caller falls back)."""
+    heads = q_abs if isinstance(q_abs, HeadsProduct) else None
+    for t, n in (() if heads else ((q_abs, "q_abs"),)) + ((kv, "kv"), (q_pe, "q_pe"), (pe, "pe")):
         _dev_i64(t, n)
     Bn, S, H, C1 = q_abs.shape
     T, C2 = kv.shape[1], q_pe.shape[3]
@@ -539,11 +556,15 @@ def mla_scores_fused(q_abs, kv, q_pe, pe, rescale1=23, rescale2=21, mul=94, div=
     narrow = narrow and skip_masked and causal and _scores_fit32(a_limbs, b_limbs, C1, C2, rescale1, rescale2, mul, div)
     for dtype, f in ((torch.int32, flags | SCORES_32), (torch.int64, flags)) if narrow else ((torch.int64, flags),):
         out = torch.empty((Bn, S, H, T), dtype=dtype, device=q_abs.device)
+        rest = (kv.data_ptr(), q_pe.data_ptr(), pe.data_ptr(), out.data_ptr(), Bn, S, H, T, C1, C2, int(rescale1), int(rescale2),
+                int(mul), int(div), 1 if causal else 0, int(start_pos), int(mask_value), a_limbs, b_limbs, f)
         with _on(q_abs.device):
-            rc = lib.zkds_mla_scores(q_abs.data_ptr(), kv.data_ptr(), q_pe.data_ptr(), pe.data_ptr(), out.data_ptr(),
-                                     Bn, S, H, T, C1, C2, int(rescale1), int(rescale2), int(mul), int(div),
-                                     1 if causal else 0, int(start_pos), int(mask_value), a_limbs, b_limbs, f, _stream())
-        if rc != 6:          # ZKDS_ERR_UNSUPPORTED
+            if heads is not None:
+                rc = lib.zkds_mla_scores_heads(heads.A.data_ptr(), heads.planes.handle, heads.rescale, heads.a_limbs, *rest, _stream())
+            if heads is None or rc == 6:          # ZKDS_ERR_UNSUPPORTED
+                q = q_abs.tensor() if heads is not None else q_abs
+                rc = lib.zkds_mla_scores(q.data_ptr(), *rest, _stream())
+        if rc != 6:
             _check(rc, "mla_scores_fused")
             return out
     return None
@@ -676,11 +697,13 @@ def softmax_q19_causal(R, C, start_pos=0):
 
 
 def softmax_pv_fused(scores, kv, rescale=23, causal_skip=False, start_pos=0, a_limbs=0, b_limbs=0,
-                     dynamic=False):
+                     dynamic=False, heads=None):
     """einsum_bsht_btc_bshc(softmax_q19(scores), kv, rescale) in one call: scores [B, S, H, T], kv
     [B, T, C] -> [B, S, H, C] (model.py:911-926).  The probabilities go from the softmax kernel straight
     into the limb planes of the contraction and are never stored as int64; `scores` is not modified.
-    causal_skip: only columns t <= start_pos + s of a row are read; scores may then be int32.  Returns None when the
+    causal_skip: only columns t <= start_pos + s of a row are read; scores may then be int32.
+    heads = (planes, rescale, limbs): einsum_heads_prepared(result, planes, rescale, False, limbs, True) instead of the result,
+    [B, S * H / heads, heads, planes.N], with limb planes in between.  Returns None when the
     kernel does not take the shape (use softmax_q19 and the einsum then)."""
     narrow = causal_skip and scores.dtype == torch.int32
     if not (narrow and scores.is_cuda and scores.is_contiguous()):
@@ -690,12 +713,16 @@ def softmax_pv_fused(scores, kv, rescale=23, causal_skip=False, start_pos=0, a_l
     Cd = kv.shape[2]
     assert Bn == kv.shape[0] and T == kv.shape[1]
     lut = _lut_on(EXP2_FRAC_LUT_Q19, scores.device, "softmax_init_q19")
-    out = torch.empty((Bn, S, H, Cd), dtype=torch.int64, device=scores.device)
+    shape = (Bn, S * H // heads[0].nb, heads[0].nb, heads[0].N) if heads else (Bn, S, H, Cd)
+    out = torch.empty(shape, dtype=torch.int64, device=scores.device)
     flags = ALGO_LIMB | (LIMBS_DYNAMIC if dynamic else 0) | (SCORES_32 if narrow else 0)
+    rest = (out.data_ptr(), lut.data_ptr(), int(rescale), Bn, S, H, T, Cd, 1 if causal_skip else 0, int(start_pos), a_limbs, b_limbs, flags)
     with _on(scores.device):
-        rc = lib.zkds_softmax_pv(scores.data_ptr(), kv.data_ptr(), out.data_ptr(), lut.data_ptr(), int(rescale),
-                                 Bn, S, H, T, Cd, 1 if causal_skip else 0, int(start_pos), a_limbs, b_limbs,
-                                 flags, _stream())
+        if heads:
+            assert S * H % heads[0].nb == 0 and heads[0].K == Cd
+            rc = lib.zkds_softmax_pv_heads(scores.data_ptr(), kv.data_ptr(), heads[0].handle, int(heads[1]), int(heads[2]), *rest, _stream())
+        else:
+            rc = lib.zkds_softmax_pv(scores.data_ptr(), kv.data_ptr(), *rest, _stream())
     if rc == 6:
         return None
     _check(rc, "softmax_pv_fused")

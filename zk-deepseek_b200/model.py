@@ -445,8 +445,8 @@ class MLA(nn.Module):
         k_pe, _ = self.wkv_a2(x)
         k_pe = apply_rotary_emb(k_pe.unsqueeze(2), freqs_cis)
         kv_normed, rms = self.kv_norm(kv)
-        ctx = self._core(q_nope, q_pe, kv_normed, k_pe.squeeze(2), bsz, seqlen, start_pos, mask, d)
-        return self._finish(ctx, lim)
+        ctx, projected = self._core(q_nope, q_pe, kv_normed, k_pe.squeeze(2), bsz, seqlen, start_pos, mask, d, through=True)
+        return self._finish(ctx, lim, projected)
 
     def _forward_seq_parallel(self, x, start_pos, freqs_cis, mask):
         """x [1, S / world_size, dim]: this rank's consecutive tokens of one sequence; freqs_cis and mask
@@ -468,8 +468,8 @@ class MLA(nn.Module):
         q_nope = self.wq_b1(q_all).view(1, S, self.n_local_heads, self.qk_nope_head_dim)
         q_pe = self.wq_b2(q_all).view(1, S, self.n_local_heads, self.qk_rope_head_dim)
         q_pe = apply_rotary_emb(q_pe, freqs_cis)
-        ctx = self._core(q_nope, q_pe, full[:, qr:qr + C][None], full[:, qr + C:][None], 1, S, start_pos, mask, None)
-        out = self._project_heads(ctx, ACT_LIMBS)                                       # [1, S, local heads * v]
+        ctx, projected = self._core(q_nope, q_pe, full[:, qr:qr + C][None], full[:, qr + C:][None], 1, S, start_pos, mask, None, through=True)
+        out = self._project_heads(ctx, ACT_LIMBS, projected)                            # [1, S, local heads * v]
         # head-split -> token-split: rank j receives its token block from every rank's heads
         cols = out.shape[-1]
         recv = torch.empty((world_size, s_loc, cols), dtype=torch.int64, device=x.device)
@@ -478,13 +478,27 @@ class MLA(nn.Module):
         rows = recv.permute(1, 0, 2).reshape(1, s_loc, world_size * cols)               # heads in rank order
         return self.wo(rows)
 
-    def _core(self, q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d):
-        """caches, scores, softmax, P . KV for the local heads: returns ctx [b, s, h, c]"""
+    def _core(self, q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d, through=False):
+        """caches, scores, softmax, P . KV for the local heads: returns ctx [b, s, h, c]; through: (ctx, False), or what
+        _project_heads makes of it and True, where the products on both sides of the latent space pass limb planes on"""
+        if not through:
+            return self._attend(q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d, None)
+        heads = None
+        # prompts (up to 64 rows the products of a head read words themselves), with all limbs promised
+        if (bsz * seqlen > 64 and mask is not None and not snark and K.ALGO != K.ALGO_EXACT and 0 < ACT_LIMBS <= 4 and min(self.score_limbs) > 0
+                and K.limb_kernel_takes(self.qk_nope_head_dim, ACT_LIMBS, 5) and K.limb_kernel_takes(self.kv_lora_rank, ACT_LIMBS, 5)):
+            heads = (self._per_head_planes(self.wkv_b_2, True), self.wkv_b_2.shift(), ACT_LIMBS)
+        ctx = self._attend(q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d, heads)
+        return ctx if isinstance(ctx, tuple) else (ctx, False)
+
+    def _attend(self, q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d, heads):
         end_pos = start_pos + seqlen
         lim = ACT_LIMBS
         # q_nope . W_uk per head  (einsum_bshd_hdc_bshc, weight [H, D, C]: K is the middle axis)
         shift1 = self.wkv_b_1.shift()
-        if lim > 0 and K.limb_kernel_takes(self.qk_nope_head_dim, lim, 5):
+        if heads is not None:
+            q_abs = K.HeadsProduct(q_nope.contiguous(), self._per_head_planes(self.wkv_b_1, False), shift1, lim)
+        elif lim > 0 and K.limb_kernel_takes(self.qk_nope_head_dim, lim, 5):
             q_abs = K.einsum_heads_prepared(q_nope.contiguous(), self._per_head_planes(self.wkv_b_1, False),
                                             shift1, True, a_limbs=lim, dynamic=True)
         else:
@@ -532,6 +546,10 @@ class MLA(nn.Module):
                                         self.softmax_scale2, causal=causal, a_limbs=al, b_limbs=bl, dynamic=dyn,
                                         skip_masked=skip, narrow=skip)
             if scores is not None and skip:
+                if heads is not None:
+                    out = K.softmax_pv_fused(scores, kv_in, 23, causal_skip=True, start_pos=0, a_limbs=3, b_limbs=bl, heads=heads)
+                    if out is not None:
+                        return out, True
                 ctx = K.softmax_pv_fused(scores, kv_in, 23, causal_skip=True, start_pos=0, a_limbs=3, b_limbs=bl)
                 if ctx is not None:
                     del scores
@@ -546,6 +564,10 @@ class MLA(nn.Module):
             elif scores is not None and pad:
                 # every row weighs the columns 0 .. end_pos - 1: the rows of all positions as those of one
                 rows = scores.view(bsz, 1, seqlen * scores.shape[2], end_pos + pad)
+                if heads is not None:
+                    out = K.softmax_pv_fused(rows, kv_in, 23, causal_skip=True, start_pos=end_pos - 1, a_limbs=3, b_limbs=bl, heads=heads)
+                    if out is not None:
+                        return out, True
                 ctx = K.softmax_pv_fused(rows, kv_in, 23, causal_skip=True, start_pos=end_pos - 1, a_limbs=3, b_limbs=bl)
                 if ctx is not None:
                     del scores, rows
@@ -556,6 +578,7 @@ class MLA(nn.Module):
                                             self.softmax_scale2, causal=causal, a_limbs=al, b_limbs=bl,
                                             dynamic=dyn)
         if scores is None:      # shape outside the fused kernel: two contractions, tail in the second
+            q_abs = q_abs.tensor() if heads is not None else q_abs
             score1 = K.attention_scores_fused(q_abs, kv_all, 23, a_limbs=al, b_limbs=bl, dynamic=dyn)
             scores = K.attention_scores_fused(q_pe.contiguous(), pe_all, 21, addin=score1,
                                               mul=self.softmax_scale1, div=self.softmax_scale2, causal=causal,
@@ -567,6 +590,10 @@ class MLA(nn.Module):
             saveTensor(f"{d}/scores_softmax_x.bin", scores)
         elif K.ALGO != K.ALGO_EXACT:
             # softmax and P . KV in one call: the probabilities only ever exist as int8 limb planes
+            if heads is not None:
+                out = K.softmax_pv_fused(scores, kv_all, 23, a_limbs=3, b_limbs=bl, heads=heads)
+                if out is not None:
+                    return out, True
             ctx = K.softmax_pv_fused(scores, kv_all, 23, a_limbs=3, b_limbs=bl)
             if ctx is not None:
                 del scores
@@ -581,15 +608,17 @@ class MLA(nn.Module):
         del probs
         return ctx
 
-    def _finish(self, ctx, lim):
-        """ctx [b, s, h, c] -> per-head W_uv, concatenate heads, output projection"""
-        out = self._project_heads(ctx, lim)
+    def _finish(self, ctx, lim, projected=False):
+        """ctx [b, s, h, c] -> per-head W_uv (unless it went through that), concatenate heads, output projection"""
+        out = self._project_heads(ctx, lim, projected)
         if world_size > 1:
             out = _all_gather_last(out)      # heads of every rank, then a column-split wo
         return self.wo(out)
 
-    def _project_heads(self, ctx, lim):
+    def _project_heads(self, ctx, lim, projected=False):
         """ctx [b, s, h, c] -> per-head W_uv -> [b, s, h * v]"""
+        if projected:
+            return ctx.flatten(2)
         shift2 = self.wkv_b_2.shift()
         if lim > 0 and K.limb_kernel_takes(self.kv_lora_rank, lim, 5):
             out = K.einsum_heads_prepared(ctx, self._per_head_planes(self.wkv_b_2, True), shift2, False,
