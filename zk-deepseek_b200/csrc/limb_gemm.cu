@@ -3212,9 +3212,9 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     int pNT = 0, pstages = 0;
     size_t psmem = 0;
     int ew = persistent_epilogue_warps(false);
-    // up to 8 K blocks (K <= 1024); measured: from 12 blocks on the one-tile kernel with its wider tile
-    // (a full 256-column B stack for two-limb weights) wins although it overlaps nothing
-    // (wq_b, K = 1536: 0.70 against 0.85 ms; w2 of the shared expert, K = 2048: 0.68 against 0.93 ms)
+    // up to 8 K blocks (K <= 1024) in narrow tiles whose accumulators have two buffers; a single wide one needs more products behind a
+    // tile (K = 512, 128 heads of 4096 tokens: 218 us narrow, 242 wide; of 777 tokens, four limbs, 110 and 129).  Not where limbs are
+    // written at one K block, which is bound by their stores: whole eights of 112 columns 680 us, of 48 785.
     int64_t max_kb = 8;
     if (switches().persistent_max_kb >= 0) max_kb = switches().persistent_max_kb;
     // few rows: the weights take the MMA's 128 rows (limb_rows_kernel).  Up to 64 rows at any depth, or promised groups of up
@@ -3227,7 +3227,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     const bool by_rows = few > 0 && few <= 64 && !p.skip_k && !p.skip_tiles && !p.addin && !p.ep_div && !p.causal_H &&
                          D * few_rows <= 512 && La * few_rows <= 256 && (kb < 2 ? kb : 2) * rows_stage <= smem_max && mt <= 65535 &&
                          rows_tiles * p.batches * (p.tile_group ? mt : 1) <= 0x7fffffffll / 8;
-    if (!by_rows && !p.R && !p.skip_k && (Kp + kBlockK - 1) / kBlockK <= max_kb && !switches().no_persistent &&
+    const bool wide_planes = p.to_planes.data && kb == 1 && D <= 6 && sum_fits64(La, Lb, p.K, p.addend) && p.batches * mt * nt * 2 > sm_count();
+    if (!by_rows && !p.R && !p.skip_k && !wide_planes && (Kp + kBlockK - 1) / kBlockK <= max_kb && !switches().no_persistent &&
         !(p.tile_group && switches().no_persistent_grouped)) {
         for (int cand : {64, 48, 32, 16}) {
             if (Lb * cand > 256 || 2 * D * cand > 512) continue;
@@ -3435,7 +3436,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     lp.group_shift = p.group_shift; lp.n_split = p.n_split;
     lp.leave_padding = p.tile_group ? p.leave_padding : 0;
     // A lane's own row in global memory is 32 pieces of 16 bytes a store instruction; rows that pass through shared memory cost the
-    // warps two waits for each other a tile.  One K block (128 heads of 4096 tokens, K = 128): 785 us directly, 1175 staged, 718 with
+    // warps two waits for each other a tile.  One K block (128 heads of 4096 tokens, K = 128): 680 us directly, 1175 staged, 718 with
     // words; deeper ones: P . KV of 4096 tokens 4177, 3712, 3631, of 777 tokens (four limbs) 669, 616, 547.  The pass over those words
     // that is saved takes 718, 712 and 195 us.
     lp.out = p.to_planes;

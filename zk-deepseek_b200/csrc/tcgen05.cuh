@@ -214,19 +214,6 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_
         : "memory");
 }
 
-// accumulate flag known at compile time: no predicate set-up in the instruction stream
-__device__ __forceinline__ void umma_i8_acc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
-{
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.eq.u32 p, 1, 1;\n"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n"
-        "}\n"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc)
-        : "memory");
-}
-
 __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
