@@ -1129,3 +1129,19 @@ def test_context_that_stays_limbs_between_its_products(kmod, dev, B, S, H, C, V,
     with pytest.raises(kmod.ZkdsError) as e:
         kmod.device_status(sync=True)
     assert e.value.status == kmod.ERR_RANGE
+
+
+@pytest.mark.parametrize("M", [65, 97, 129, 161, 255])
+@pytest.mark.parametrize("K,bits,limbs", [(100, 20, 3), (300, 20, 3), (300, 37, 5), (300, 45, 6)])
+def test_lanes_behind_the_last_row(kmod, orc, dev, M, K, bits, limbs):
+    """tiles whose last warp has rows in some lanes only, or in the first, several column pieces a warp, sums of 64 and 128 bits,
+    with and without remainders, one K block and more"""
+    rng, N = np.random.default_rng(M + K + limbs), 4010
+    X, W = rand_i64(rng, (1, M, K), bits), rand_i64(rng, (N, K), 13).astype(np.int32)
+    planes = kmod.WeightPlanes(g(W, dev))
+    want = orc.gemm(X, W, 1, 1, 9, orc.R_LEGACY)
+    same(kmod.linear_prepared(g(X, dev), planes, 9, a_limbs=limbs, dynamic=True), want[0], "C")
+    got = kmod.linear_prepared(g(X, dev), planes, 9, a_limbs=limbs, want_remainder=True, dynamic=True)
+    same(got[0], want[0], "C")
+    same(got[1], want[1], "R")
+    kmod.device_status(sync=True)

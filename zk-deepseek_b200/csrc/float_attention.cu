@@ -245,7 +245,7 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid
         uint32_t sp = 0;
         bool ok = true;
         for (int j = first_tile; j <= last_tile; ++j) {
-            ok = mbar_wait(smem_u32(&s.s_full[g]), sp, abort_flag);
+            ok = mbar_wait_warp(smem_u32(&s.s_full[g]), sp, abort_flag);
             sp ^= 1u;
             tc_fence_after();
             float v[2][32];
@@ -311,7 +311,7 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid
             pair_sync();
             l += s.row_max[g][half ^ 1][row];
         }
-        if (ok && first_tile <= last_tile && mbar_wait(smem_u32(&s.o_full[g]), 0, abort_flag)) {
+        if (ok && first_tile <= last_tile && mbar_wait_warp(smem_u32(&s.o_full[g]), 0, abort_flag)) {
             tc_fence_after();
             const float r = 1.0f / l;
             bf16* o = p.out + (long long)t * p.o_tok + head * p.o_head;
@@ -332,6 +332,7 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid
                     }
                     store8(o + c, w);
                 }
+                __syncwarp();
             }
         }
     }
@@ -525,7 +526,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid_c
         const bool row_ok = rr < p.rows;
         const int c_hi = start + rr / p.heads - j0, c_lo = p.window > 0 ? c_hi - p.window + 1 : 0;
         const long long tile = ((long long)b * p.row_tiles + blockIdx.y) * p.chunks + blockIdx.x;
-        if (mbar_wait(smem_u32(&s.s_full), 0, abort_flag)) {
+        if (mbar_wait_warp(smem_u32(&s.s_full), 0, abort_flag)) {
             tc_fence_after();
             float v[2][32];
             tmem_ld32(tq, v[0]);
@@ -561,7 +562,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid_c
                 p.ml[tile * 256 + row] = m;
                 p.ml[tile * 256 + 128 + row] = l;
             }
-            if (mbar_wait(smem_u32(&s.o_full), 0, abort_flag)) {
+            if (mbar_wait_warp(smem_u32(&s.o_full), 0, abort_flag)) {
                 tc_fence_after();
                 float* out = p.part + tile * p.c * 128 + row;
                 for (int c = 0; c < p.c; c += 32) {
@@ -572,6 +573,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ1, const __grid_c
                         for (int i = 0; i < 32; ++i)
                             if (c + i < p.c) out[(long long)(c + i) * 128] = v[0][i];
                     }
+                    __syncwarp();
                 }
             }
         }

@@ -256,11 +256,12 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             int mt, nt;
             const int tile = t / p.ksplit;
             tile_coords(p, tile, mt, nt);
-            if (!mbar_wait(smem_u32(&s.acc_full[buf]), acc_phase, abort_flag)) break;
+            if (!mbar_wait_warp(smem_u32(&s.acc_full[buf]), acc_phase, abort_flag)) break;
             tc_fence_after();
             const int m0 = mt * 256 + (int)rank * kTM + quarter * 32, n0 = nt * p.NT;
             const int pos = (p.e.kind == ZKFP_EPI_ROTATE && m0 + lane < p.M) ? epi_position(p.e, m0 + lane) : 0;
             float* part = p.partial + (((long long)t * 2 + rank) * p.NT) * kTM + quarter * 32 + lane;
+            __syncwarp();
             for (int c = c_begin; c < c_end; c += 32) {
                 float v[32];
                 tmem_ld32(tq + (uint32_t)(buf * 256 + c), v);

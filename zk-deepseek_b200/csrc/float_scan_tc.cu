@@ -365,7 +365,10 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             arrive(bar);
         };
-        auto wait = [&](uint64_t* bar, int phase) { return mbar_wait_polling(smem_u32(bar), (uint32_t)(phase & 1), abort_flag); };
+        // the same answer in every lane, which have met again
+        auto wait = [&](uint64_t* bar, int phase) {
+            return __all_sync(0xffffffffu, mbar_wait_polling(smem_u32(bar), (uint32_t)(phase & 1), abort_flag)) != 0;
+        };
         auto value_tile = [&](int c) { return base + (uint32_t)stage_of(c) * stage_bytes + bytes_q + 2 * kSegB; };
         // values scaled by what is left of them at the chunk's end
         float l_row = 0.f, l_end = 0.f, l_row_next, l_end_next;          // a stage may be refilled once its values are scaled
@@ -430,6 +433,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                         float v[16];
                         tmem_ld16f(ts + (uint32_t)(q * 16), v);
                         if (q) factors(1);
+                        __syncwarp();
                         tmem_ld_wait();
 #pragma unroll
                         for (int i = 0; i < 8; ++i) w[q * 8 + i] = pack_bf16(v[2 * i] * g[2 * i], v[2 * i + 1] * g[2 * i + 1]);

@@ -689,8 +689,8 @@ __device__ __forceinline__ void epilogue_tile(const LimbParams& p, const Epilogu
         i128w sum[8];
         int64_t s64[8];
         gather_chunk<FITS64>(e, nc, p.addend, s64, sum);
-        if (!e.row_ok) continue;
-        finish_chunk<FITS64>(p, e, nc, s64, sum, tail, arow, srow);
+        if (e.row_ok) finish_chunk<FITS64>(p, e, nc, s64, sum, tail, arow, srow);
+        __syncwarp();
     }
 }
 
@@ -750,10 +750,12 @@ __device__ __forceinline__ void epilogue_tile_pipelined(const LimbParams& p, con
         const bool more1 = nc + CW < e.nc_end;
         if (more1) fetch_cols<DD, CW>(e, nc + CW, a1);
         finish_cols<DD, CW>(p, e, nc, a0, tail, arow, srow, tot);
+        __syncwarp();
         if (more1) {
             tmem_ld_wait();
             if (nc + 2 * CW < e.nc_end) fetch_cols<DD, CW>(e, nc + 2 * CW, a0);
             finish_cols<DD, CW>(p, e, nc + CW, a1, tail, arow, srow, tot);
+            __syncwarp();
         }
     }
 }
@@ -784,9 +786,9 @@ __device__ __forceinline__ void add_partials_tile(const LimbParams& p, const Epi
         i128w sum[8];
         int64_t s64[8];
         gather_chunk<FITS64>(e, nc, 0, s64, sum);
-        if (!e.row_ok) continue;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
+            if (!e.row_ok) break;
             unsigned long long* w = tot + (int64_t)(nc + c) * kTileM;
             if (FITS64) {
                 if (s64[c]) atomicAdd(w, (unsigned long long)s64[c]);
@@ -797,6 +799,7 @@ __device__ __forceinline__ void add_partials_tile(const LimbParams& p, const Epi
                 if (hi) atomicAdd(w + (int64_t)e.NT * kTileM, hi);
             }
         }
+        __syncwarp();
     }
 }
 
@@ -1010,9 +1013,10 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
         const bool prof = p.wait_cycles != nullptr && warp == 2 && lane == 0;
         long long ph0 = prof ? clock64() : 0, ph1 = 0, ph2 = 0, ph3 = 0;
-        const bool ok = mbar_wait(bar_accum, 0, abort_flag);
+        const bool ok = mbar_wait_warp(bar_accum, 0, abort_flag);
         tc_fence_after();
         if (prof) ph1 = clock64();
+        __syncwarp();
         const int64_t m = m0 + q * 32 + lane;
         int64_t* crow = p.C + z * p.c_sz + m * p.c_sm;
         int64_t* rrow = p.R ? p.R + z * p.c_sz + m * p.c_sm : nullptr;
@@ -1048,6 +1052,7 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
             if (prof) ph2 = clock64();
             __threadfence();
+            __syncwarp();
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
             if (warp == 2 && lane == 0) {
                 // a CTA that gave up a wait does not count: the tile then stays unfinished and the
@@ -1055,6 +1060,7 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 s_last = 0;
                 if (ok) s_last = atomicAdd(p.tile_counter + tile_id, 1u) == (unsigned)(p.ksplit - 1) ? 1 : 0;
             }
+            __syncwarp();
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
             finish = false;
             if (prof) ph3 = clock64();
@@ -1369,7 +1375,7 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_zeroed);
             if (DIRECT) ok = cut_rows();
-            if (ok) ok = mbar_wait(bar_accum, 0, abort_flag);
+            if (ok) ok = mbar_wait_warp(bar_accum, 0, abort_flag);
             tc_fence_after();
         }
         EpilogueCtx ec;
@@ -1391,16 +1397,16 @@ limb_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                 for (int i = 0; i < 8; ++i) sum[i] = make_i128(s64[i]);
             }
-            if (!ok) continue;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                if (r0 + i >= rows) continue;
+                if (!ok || r0 + i >= rows) continue;
                 if (p.ksplit > 1) {
                     red[(r0 + i) * kTileM + col] = sum[i].lo;
                     if (!p.fits64) red[(rows + r0 + i) * kTileM + col] = (uint64_t)sum[i].hi;
                 } else if (n < p.N && m0 + r0 + i < p.M)
                     rows_store(p, sum[i], shift, z, m0 + r0 + i, n);
             }
+            __syncwarp();
         }
     }
     tc_fence_before();
@@ -1611,6 +1617,7 @@ __device__ __forceinline__ void epilogue_part(const LimbParams& p, uint32_t tq, 
 #pragma unroll
         for (int c = 0; c < CH; c += 2)
             *reinterpret_cast<longlong2*>(srow_ptr + c) = make_longlong2(cv[c], cv[c + 1]);
+        __syncwarp();
     }
     if (two) {
         // second set of diagonals: its own addend and shift, then the two quotients add up
@@ -1632,6 +1639,7 @@ __device__ __forceinline__ void epilogue_part(const LimbParams& p, uint32_t tq, 
 #pragma unroll
             for (int c = 0; c < CH; c += 2)
                 *reinterpret_cast<longlong2*>(srow_ptr + c) = make_longlong2(v2[c], v2[c + 1]);
+            __syncwarp();
         }
     }
     __syncwarp();
@@ -2075,8 +2083,9 @@ limb_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
             }
             const int b = (int)(t % p.nbuf);
             if (prof) t0 = clock64();
-            if (!mbar_wait(bar_tfull + 8 * b, (uint32_t)((t / p.nbuf) & 1), abort_flag, 48u * p.backoff)) break;
+            if (!mbar_wait_warp(bar_tfull + 8 * b, (uint32_t)((t / p.nbuf) & 1), abort_flag, 48u * p.backoff)) break;
             if (prof) w_acc += clock64() - t0;
+            __syncwarp();
             tc_fence_after();
             const uint32_t tq = lane_base + (uint32_t)(b * buf_cols);
             const uint32_t rel = split ? bar_tempty : 0u;
@@ -2092,6 +2101,7 @@ limb_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
                     if (lane == 0) *abort_flag = 1;
                     break;
                 }
+                __syncwarp();
                 ++t;
                 continue;
             }
@@ -2442,7 +2452,7 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                     }
                 continue;
             }
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * buf, turn, abort_flag, 48u * p.backoff))) break;
+            if (!mbar_wait_warp(bar_tfull + 8 * buf, turn, abort_flag, 48u * p.backoff)) break;
             tc_fence_after();
             const uint32_t tq = lanes + (uint32_t)(buf * buf_cols);
             const int64_t m = tc.m0 + q * 32 + lane, at = tc.z * p.c_sz + m * p.c_sm + tc.n0;
@@ -2477,6 +2487,7 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 else if (W == 16) tile_columns_64<16>(p, t, tq, D, col, loaded);
                 else if (W == 8) tile_columns_64<8>(p, t, tq, D, col, loaded);
                 else tile_columns_64<4>(p, t, tq, D, col, loaded);
+                __syncwarp();                          // lanes behind the last row store nothing
                 col += W;
             }
             if constexpr (STAGED) {

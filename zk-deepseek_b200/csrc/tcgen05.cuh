@@ -142,6 +142,9 @@ __device__ __forceinline__ uint32_t elect_one()
 // a value that is the same in every lane, where the compiler can see that
 __device__ __forceinline__ uint32_t uniform(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
 
+// One answer for the whole warp, whose lanes have met again when it is there: also what has to stand in front of tensor-memory loads
+// and stores, which (like their waits, allocation and `bar.sync`) are for warps whose lanes are together.  Behind a branch that only
+// some lanes take, a __syncwarp() does that.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned backoff_ns = 0)
 {
     for (uint32_t it = 0; it < kSpinLimit; ++it) {
@@ -189,6 +192,7 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols)
 {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem),
                  "r"(cols)
                  : "memory");
@@ -197,6 +201,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols)
 
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols)
 {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols)
                  : "memory");
 }
@@ -352,6 +357,7 @@ __device__ __forceinline__ void cluster_sync_all()
 
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t cols)
 {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -359,6 +365,7 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t cols
 
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols)
 {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 
