@@ -24,7 +24,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
 # library -> (translation units, headers)
 LIBRARIES = {
     "libint64gemm.so": (["capi.cu", "fixedpoint.cu", "gemm_exact.cu", "limb_gemm.cu", "converters.cu"],
-                        ["common.cuh", "kernels.h", "tcgen05.cuh", "zkds_int64.h"]),
+                        ["common.cuh", "kernels.h", "range_answer.h", "tcgen05.cuh", "zkds_int64.h"]),
     "libfloatops.so": (["float_capi.cu", "float_ops.cu", "float_gemm.cu", "float_gemm_f32.cu", "float_gemm_tc.cu", "float_attention.cu",
                         "float_grouped.cu", "float_recurrent.cu", "float_scan_tc.cu"],
                        ["common.cuh", "float_common.cuh", "tcgen05.cuh", "zkds_float.h"]),

@@ -24,7 +24,6 @@
 #include <stdlib.h>
 
 #include <atomic>
-#include <mutex>
 
 #include <string.h>
 
@@ -32,6 +31,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "range_answer.h"
 #include "tcgen05.cuh"
 
 namespace zkds {
@@ -2563,7 +2563,7 @@ bool make_plane_map(CUtensorMap* map, void* base, int64_t rows_total, int64_t Kp
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr size_t RangeAnswerBytes = 8 * 4 * sizeof(uint64_t);     // behind the two words: eight measurements' answers
+constexpr size_t RangeAnswerBytes = kRangeSets * 4 * sizeof(uint64_t);     // behind the two words: the measurements' answers
 
 struct DeviceFlags {
     int* host = nullptr;      // mapped, host view
@@ -2745,59 +2745,14 @@ range_kernel(const RangeOf a, const RangeOf b, uint64_t* partial, unsigned* arri
 
 }  // namespace
 
-// The words that one measurement works in and is answered in: one of eight sets of a device, the caller's until it has its answer.
-struct RangeAnswer {
-    static constexpr int kSets = 8;
-    uint64_t* partial = nullptr;
-    unsigned* arrived = nullptr;
-    volatile uint64_t *host = nullptr, *dev = nullptr;
-    uint64_t ticket = 0;
-
-    bool claim()
-    {
-        if (cudaGetDevice(&device_) != cudaSuccess || device_ < 0 || device_ >= 64) return false;
-        Pool& p = pool(device_);
-        std::lock_guard<std::mutex> lk(p.mu);
-        while (set_ < kSets && (p.taken >> set_ & 1)) ++set_;
-        if (set_ == kSets) return false;
-        const size_t each = 256 + (size_t)sm_count() * 8 * 2 * sizeof(uint64_t);
-        size_t fresh = 0;
-        uint8_t* ws = (uint8_t*)workspace_fresh(each * kSets, 7, &fresh);
-        DeviceFlags* fl = flags_for_device();
-        if (!ws || !fl) return false;
-        // the kernel leaves its counter at zero
-        if (fresh && (cudaMemset(ws, 0, each * kSets) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)) return false;
-        p.taken |= 1u << set_;
-        held_ = true;
-        arrived = (unsigned*)(ws + each * set_);
-        partial = (uint64_t*)(ws + each * set_ + 256);
-        host = (volatile uint64_t*)(fl->host + 16) + 4 * set_;
-        dev = (volatile uint64_t*)(fl->dev + 16) + 4 * set_;
-        ticket = ++p.tickets;
-        return true;
-    }
-    ~RangeAnswer()
-    {
-        if (!held_) return;
-        Pool& p = pool(device_);
-        std::lock_guard<std::mutex> lk(p.mu);
-        p.taken &= ~(1u << set_);
-    }
-
-  private:
-    struct Pool {
-        std::mutex mu;
-        unsigned taken = 0;
-        uint64_t tickets = 0;
-    };
-    static Pool& pool(int device)
-    {
-        static Pool pools[64];
-        return pools[device];
-    }
-    int device_ = 0, set_ = 0;
-    bool held_ = false;
-};
+bool range_words(uint64_t** host, uint64_t** dev)
+{
+    DeviceFlags* fl = flags_for_device();
+    if (!fl) return false;
+    *host = (uint64_t*)(fl->host + 16);
+    *dev = (uint64_t*)(fl->dev + 16);
+    return true;
+}
 
 // out[0], out[1] <- ranges of A and B as launch_absmax measures them, of those that are wanted (host words: this waits for the
 // kernel); ZKDS_ERR_UNSUPPORTED for a B that is not contiguous along K, and for rows with gaps between them that fill less than
