@@ -1145,3 +1145,29 @@ def test_lanes_behind_the_last_row(kmod, orc, dev, M, K, bits, limbs):
     same(got[0], want[0], "C")
     same(got[1], want[1], "R")
     kmod.device_status(sync=True)
+
+
+def test_planes_of_tiles_wider_than_a_warp_of_words(kmod, dev):
+    """forced tiles of 160 columns (one-limb keys), where a row is more than a word for every lane: no planes, or the right ones"""
+    import os
+    import subprocess
+    import sys
+    code = """
+import sys, importlib, torch
+sys.path.insert(0, {root!r})
+K = importlib.import_module("zk-deepseek_b200.kernel")
+torch.manual_seed(0)
+dev, B, S, H, T, C, V = torch.device("cuda"), 1, 350, 16, 352, 512, 32
+scores = torch.randint(-9 << 19, 9 << 19, (B, S, H, T), device=dev)
+kv = torch.randint(-100, 100, (B, T, C), device=dev)
+planes = K.WeightPlanes(torch.randint(-(1 << 13), 1 << 13, (H, V, C), device=dev, dtype=torch.int32))
+K.softmax_init_q19()
+for how in (dict(), dict(causal_skip=True, start_pos=2)):
+    ctx = K.softmax_pv_fused(scores, kv, 3, a_limbs=3, b_limbs=1, **how)
+    got = K.softmax_pv_fused(scores, kv, 3, a_limbs=3, b_limbs=1, heads=(planes, 9, 3), **how)
+    assert int(ctx.abs().max()) > 1 << 17
+    assert got is None or torch.equal(got, K.einsum_heads_prepared(ctx, planes, 9, False, a_limbs=3, dynamic=True))
+K.device_status(sync=True)
+""".format(root=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, ZKDS_TILE_NT="160"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]

@@ -2491,7 +2491,8 @@ limb_tiles_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 col += W;
             }
             if constexpr (STAGED) {
-                // eight of the rows a warp, whole rows of the tile a store: NT bytes of every limb side by side
+                // eight of the rows a warp, whole rows of the tile a store: NT bytes of every limb side by side (the launcher takes no
+                // tile of more than 128 columns, a word a lane)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_rows);
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_rows, 0u, abort_flag))) break;
@@ -3230,7 +3231,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     const int64_t nt_eff = (p.N + NT - 1) / NT;
     const size_t plane_rows = p.to_planes.data ? (size_t)kTileM * p.to_planes.L * (NT + 4) : 0;       // see limb_tiles_kernel
     if (p.to_planes.data && (by_rows || p.R || p.tile_group || p.skip_tiles || p.addin || p.ep_div || p.causal_H || switches().no_persistent ||
-                             p.M <= 64 || p.M > 0x7fffffffll || (p.N & 15) || NT < 32 || smem_max < plane_rows ||
+                             p.M <= 64 || p.M > 0x7fffffffll || (p.N & 15) || NT < 32 || NT > 128 || smem_max < plane_rows ||
                              (smem_max - plane_rows) / ((size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK) < 2 || p.to_planes.L > 4 ||
                              p.batches * mt * nt_eff * 2 <= sm_count() || (sum_fits64(La, Lb, p.K, p.addend) ? D > 6 : D > 8)))
         return ZKDS_ERR_UNSUPPORTED;
