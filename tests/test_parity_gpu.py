@@ -1171,3 +1171,34 @@ K.device_status(sync=True)
 """.format(root=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, ZKDS_TILE_NT="160"), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_heads_products_of_refused_calls_are_not_taken(kmod, dev):
+    """scores that the fused kernel refuses (latents that are no multiple of 128) and a second product that it refuses (four limbs on
+    four of 32768 columns) launch nothing; the words are then taken once"""
+    def launched(call):
+        kmod.kernel_timing(2)
+        try:
+            return call(), len(kmod.kernel_timing_records())
+        finally:
+            kmod.kernel_timing(0)
+    rng = np.random.default_rng(2)
+    draw = lambda bits, *shape: g(rand_i64(rng, shape, bits), dev)
+    planes = kmod.WeightPlanes(draw(13, 16, 144, 32).int())
+    heads = kmod.HeadsProduct(draw(20, 1, 130, 16, 32), planes, 17, 3)
+    args = (heads, draw(20, 1, 132, 144), draw(20, 1, 130, 16, 16), draw(20, 1, 132, 16))
+    lib = kmod.lib
+    out = torch.empty((1, 130, 16, 132), dtype=torch.int64, device=dev)
+    rc = launched(lambda: lib.zkds_mla_scores_heads(
+        heads.A.data_ptr(), planes.handle, 17, 3, *(x.data_ptr() for x in args[1:]), out.data_ptr(), 1, 130, 16, 132, 144, 16, 23, 21,
+        94, 695, 1, 0, -(64 << 36), 3, 3, kmod._a_flags(3, True), kmod._stream()))
+    assert rc == (6, 0)
+    for narrow in (False, True):
+        got, n = launched(lambda: kmod.mla_scores_fused(*args, causal=True, skip_masked=True, narrow=narrow, a_limbs=3, b_limbs=3, dynamic=True))
+        assert got is None and n == 1
+    scores, kv = draw(20, 1, 65, 2, 64), draw(20, 1, 64, 32768)
+    wide = kmod.WeightPlanes(draw(30, 2, 16, 32768).int())
+    kmod.softmax_init_q19()
+    for how in (dict(), dict(causal_skip=True)):
+        assert launched(lambda: kmod.softmax_pv_fused(scores, kv, 19, a_limbs=3, b_limbs=3, heads=(wide, 9, 4), **how)) == (None, 0)
+    kmod.device_status(sync=True)

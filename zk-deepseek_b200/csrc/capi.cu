@@ -468,6 +468,10 @@ static int mla_scores(const int64_t* q_abs, const HeadsProduct* heads, const int
     f.skip_tiles = (flags & ZKDS_CAUSAL_SKIP) ? 1 : 0;
     f.out_bits = narrow ? 32 : 64;
     if (heads) {
+        // what the scores refuse is refused before the heads' product is taken
+        f.check_only = 1;
+        if (launch_scores_fused(f, a_limbs, b_limbs, st) != ZKDS_OK) { t_status = ZKDS_ERR_UNSUPPORTED; return t_status; }
+        f.check_only = 0;
         const int64_t pitch = C1 + ((C2 + 15) & ~(int64_t)15), step = B * S * H * pitch;
         f.a1_most = planes_most();
         if (!f.a1_most) return finish(ZKDS_ERR_WORKSPACE, "zkds_mla_scores");
@@ -633,6 +637,11 @@ static int softmax_pv(const HeadsProduct* heads, const int64_t* scores, const in
     }
     // (a row may hold several positions' heads: the weights know how many heads there are)
     const int64_t Hw = heads->weights->pl.nb, rows = B * S * H / Hw, step = rows * Hw * C;
+    Contraction q = heads_problem(*heads, rows, Hw);
+    q.C = out;
+    q.check_only = 1;              // what the second product refuses is refused before the first
+    if (launch_contraction_limb(q, heads->limbs, 0, &heads->weights->pl, st) != ZKDS_OK) { t_status = ZKDS_ERR_UNSUPPORTED; return t_status; }
+    q.check_only = 0;
     unsigned long long* most = planes_most();
     if (!most) return finish(ZKDS_ERR_WORKSPACE, "zkds_softmax_pv");
     int8_t* ctx = (int8_t*)workspace((size_t)heads->limbs * step + 1024, 2);
@@ -640,8 +649,6 @@ static int softmax_pv(const HeadsProduct* heads, const int64_t* scores, const in
     p.to_planes = LimbOut{ctx, heads->limbs, step, C, Hw, 1, rows, S * H / Hw, most};
     int rc = launch_contraction_limb(p, a_limbs, b_limbs, nullptr, st);
     if (rc == ZKDS_OK) {
-        Contraction q = heads_problem(*heads, rows, Hw);
-        q.C = out;
         q.a_planes = ctx; q.a_most = most;
         rc = launch_contraction_limb(q, heads->limbs, 0, &heads->weights->pl, st);
     }

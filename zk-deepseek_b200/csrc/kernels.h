@@ -161,6 +161,7 @@ struct Contraction {
     // memory as int64 (limb kernel only, batches == 1)
     const int64_t* glu_r2;
     const int64_t* glu_lut;
+    int check_only;           // nothing is launched: whether the call would be refused (ZKDS_ERR_UNSUPPORTED)
 };
 
 // CUDA-core path: exact for every input, any shape (gemm_exact.cu)
@@ -200,6 +201,7 @@ struct FusedScores {
     // A1 is there as limb planes: columns [0, K1) of rows of K1 + round16(K2) bytes, [La][batches][M]; A2 is split beside them
     int8_t* a1_planes;
     unsigned long long* a1_most;
+    int check_only;   // as in Contraction
 };
 // new cache rows as limb planes in both layouts the attention contractions read (see zkds_cache_planes_append)
 int launch_cache_planes_append(const int64_t* kv_new, const int64_t* pe_new, int8_t* score_planes,

@@ -3235,6 +3235,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
                              (smem_max - plane_rows) / ((size_t)La * kTileM * kBlockK + (size_t)Lb * NT * kBlockK) < 2 || p.to_planes.L > 4 ||
                              p.batches * mt * nt_eff * 2 <= sm_count() || (sum_fits64(La, Lb, p.K, p.addend) ? D > 6 : D > 8)))
         return ZKDS_ERR_UNSUPPORTED;
+    if (p.batches > 0 && mt * nt_eff > 0x7fffffffll / p.batches) return ZKDS_ERR_UNSUPPORTED;
+    if (p.check_only) return ZKDS_OK;
 
     DeviceFlags* fl = flags_for_device();
     if (!fl) return ZKDS_ERR_WORKSPACE;
@@ -3457,14 +3459,12 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     if (panel < 1) panel = 1;
     if (panel > mt) panel = mt;
     lp.m_tiles = mt; lp.n_tiles = nt_eff; lp.panel_m = panel;
-    if (mt * nt_eff > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
     dim3 grid = p.tile_group ? dim3((unsigned)mt, (unsigned)nt_eff, 1)
                              : dim3((unsigned)(mt * nt_eff * lp.ksplit), 1, (unsigned)p.batches);
     cudaEvent_t* ev = timing_events();
     if (ev) ZKDS_CUDA(cudaEventRecord(ev[0], st));
     if (tiles) {
         const int64_t total_tiles = p.batches * mt * nt_eff;
-        if (total_tiles > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
         auto kernel = !p.to_planes.data ? limb_tiles_kernel<false, false> : staged ? limb_tiles_kernel<true, true> : limb_tiles_kernel<true, false>;
         rc = allow_big_smem(kernel, !p.to_planes.data ? g_attr_tiles : staged ? g_attr_tile_staged : g_attr_tile_planes);
         if (rc != ZKDS_OK) return rc;
@@ -3473,7 +3473,6 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     } else if (persistent) {
         if (psmem < 120 * 1024) psmem = 120 * 1024;
         int64_t total_tiles = p.batches * mt * nt_eff;
-        if (total_tiles > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
         int ctas = sm_count();
         if (total_tiles < ctas) ctas = (int)total_tiles;
         rc = launch_persistent(ew, ctas, psmem, st, tmA, tmB, lp);
@@ -3567,6 +3566,7 @@ int launch_scores_fused(const FusedScores& f, int La, int Lb, cudaStream_t st)
     if (a_rows * La > 0x7fffff00ll || b_rows * Lb > 0x7fffff00ll) return ZKDS_ERR_UNSUPPORTED;
     const int64_t mt = (f.M + kTileM - 1) / kTileM, nt = (f.N + NT - 1) / NT;
     if (f.batches * mt * nt > 0x7fffffffll) return ZKDS_ERR_UNSUPPORTED;
+    if (f.check_only) return ZKDS_OK;
 
     DeviceFlags* fl = flags_for_device();
     if (!fl) return ZKDS_ERR_WORKSPACE;

@@ -554,19 +554,22 @@ def mla_scores_fused(q_abs, kv, q_pe, pe, rescale1=23, rescale2=21, mul=94, div=
     assert kv.shape == (Bn, T, C1) and q_pe.shape == (Bn, S, H, C2) and pe.shape == (Bn, T, C2)
     flags = _a_flags(a_limbs, dynamic) | (CAUSAL_SKIP if (skip_masked and causal) else 0)
     narrow = narrow and skip_masked and causal and _scores_fit32(a_limbs, b_limbs, C1, C2, rescale1, rescale2, mul, div)
-    for dtype, f in ((torch.int32, flags | SCORES_32), (torch.int64, flags)) if narrow else ((torch.int64, flags),):
+    words = ((torch.int32, flags | SCORES_32), (torch.int64, flags)) if narrow else ((torch.int64, flags),)
+    for through, dtype, f in [(True,) + w for w in words if heads] + [(False,) + w for w in words]:
         out = torch.empty((Bn, S, H, T), dtype=dtype, device=q_abs.device)
         rest = (kv.data_ptr(), q_pe.data_ptr(), pe.data_ptr(), out.data_ptr(), Bn, S, H, T, C1, C2, int(rescale1), int(rescale2),
                 int(mul), int(div), 1 if causal else 0, int(start_pos), int(mask_value), a_limbs, b_limbs, f)
         with _on(q_abs.device):
-            if heads is not None:
+            if through:
                 rc = lib.zkds_mla_scores_heads(heads.A.data_ptr(), heads.planes.handle, heads.rescale, heads.a_limbs, *rest, _stream())
-            if heads is None or rc == 6:          # ZKDS_ERR_UNSUPPORTED
-                q = q_abs.tensor() if heads is not None else q_abs
-                rc = lib.zkds_mla_scores(q.data_ptr(), *rest, _stream())
-        if rc != 6:
+            else:
+                if isinstance(q_abs, HeadsProduct):
+                    q_abs = q_abs.tensor()
+                rc = lib.zkds_mla_scores(q_abs.data_ptr(), *rest, _stream())
+        if rc != 6:          # ZKDS_ERR_UNSUPPORTED
             _check(rc, "mla_scores_fused")
             return out
+        del out
     return None
 
 
