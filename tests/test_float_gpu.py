@@ -784,3 +784,24 @@ def test_float32_attention_of_prompts(K, S, start, H, G, D, R, V, window, gated)
     sees = np.array([start + s >= bad and (not window or start + s - bad < window) for s in range(S)])
     assert np.isnan(got[sees]).all() and np.abs(got[~sees] - want[~sees]).max(initial=0) < 2e-5
     K.device_status(sync=True)
+
+
+@pytest.mark.parametrize("M,N,Kd", [(17, 136, 4096), (170, 2056, 328), (321, 4104, 136), (64, 20000, 264)])
+def test_float32_layers_of_rows_that_are_not_finite(K, M, N, Kd):
+    """infinities in every row, in every second weight or only somewhere, and rows of NaN: the outputs that see them are what
+    multiply-adds give, in clusters that share K and alone, with and without an epilogue"""
+    for every in (1, 2, 37):
+        A, W = rnd((M, Kd), "float32", 3), rnd((N, Kd), "float32", 4)
+        A[::every, 5], W[3::every, Kd - 1], A[(every - 1) % M, 9] = float("inf"), float("-inf"), float("nan")
+        out = torch.full((M, N), 7.0, device="cuda")
+        K.linear(A, W, out)
+        want = A.double() @ W.double().T
+        assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+        fine = torch.isfinite(want)
+        assert torch.equal(out[torch.isinf(want)].double(), want[torch.isinf(want)])
+        bound = torch.nan_to_num(A, 0, 0, 0).double().abs() @ torch.nan_to_num(W, 0, 0, 0).double().abs().T
+        assert ((out - want)[fine].abs() <= ((Kd + 8) * 2.0 ** -24 * bound)[fine]).all()
+        aux, gated = rnd((M, N), "float32", 2), torch.empty((M, N), device="cuda")
+        K.linear(A, W, gated, K.GATE, aux=aux)
+        gate = torch.sigmoid(want) * aux
+        assert torch.equal(torch.isnan(gated), torch.isnan(gate)) and (gated - gate)[~torch.isnan(gate)].abs().max() < 1e-4
