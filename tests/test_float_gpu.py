@@ -805,3 +805,18 @@ def test_float32_layers_of_rows_that_are_not_finite(K, M, N, Kd):
         K.linear(A, W, gated, K.GATE, aux=aux)
         gate = torch.sigmoid(want) * aux
         assert torch.equal(torch.isnan(gated), torch.isnan(gate)) and (gated - gate)[~torch.isnan(gate)].abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("M,N,Kd", [(17, 136, 4096), (170, 2056, 328), (64, 1000, 520)])
+@pytest.mark.parametrize("small", [2.0 ** -90, 1e-33, 1e-36, 1e-37, 3e-40])
+def test_float32_layers_of_small_operands(K, M, N, Kd, small):
+    """rows or weights whose last bits lie below bfloat16's smallest number, against operands that bring the result back up, results
+    that are subnormal themselves, sums beyond the range of scaled ones: the limit of test_float32_layers_from_thirds, and a last
+    subnormal bit"""
+    A, W = rnd((M, Kd), "float32", 3), rnd((N, Kd), "float32", 4, Kd ** -0.5)
+    back = min(1 / small, 1e30)
+    for a, w in ((A * small, W * back), (A * back, W * small), (A * 1e-20, W * (small * 1e20)), (A * small, W), (A * 1e20, W * 1e10)):
+        out = torch.full((M, N), 7.0, device="cuda")
+        K.linear(a, w, out)
+        want, bound = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+        assert ((out - want).abs() <= (8 + Kd / 64) * 2.0 ** -24 * bound + 2.0 ** -149).all()

@@ -1,8 +1,10 @@
 // float32 linear layers of more than 16 rows on the tensor cores: out = epilogue(A W^T) from exact bfloat16 thirds.
 //
-// A float is the sum of three bfloat16 numbers exactly: the nearest one, the nearest to what that leaves, and the rest.  Of the nine
-// products of thirds the six largest are taken (what is dropped is below 2^-25 of a product, where a float's own rounding is
-// 2^-24).  On the CUDA cores these layers are bound by FMAs at 64 lanes an SM and clock; here by the pieces of both operands that
+// A float times 2^24 is the sum of three bfloat16 numbers exactly, subnormal ones too: the nearest one, the nearest to what that leaves,
+// and the rest.  (Without the factor, which the sums lose again at the end, bfloat16's smallest numbers cut the last third of what is
+// below 2^-110: error 9e-6 at 2^-118, 2e-3 at 2^-126, where now it is 9e-8 as at 1.)  Operands from 2^104 and sums from 2^80 on leave the range and are taken by multiply-adds, see again_by_fma.  Of the nine
+// products of thirds the six largest are taken: what is dropped is up to 2^-24 of a product, as much as a float's own rounding, of
+// either sign, and 2^-27 on average.  On the CUDA cores these layers are bound by FMAs at 64 lanes an SM and clock; here by the pieces of both operands that
 // have to be in flight (loads of floats, cut into thirds by the threads, 3 x 64 bytes a row and stage) and by 6 MMAs of
 // 128 x NT x 16 for 16 k, a third of what those FMAs take.
 //
@@ -36,6 +38,7 @@ constexpr int kSplitNT = 160;                      // most rows of A in a tile: 
 constexpr int kSplitChunk = 2;                     // stages after which the products of the first thirds are collected
 constexpr int kSplitStages = 4;
 constexpr int kSplitPitch = kSplitN + 4;           // floats between the tokens of the finished sums
+constexpr float kSplitScale = 16777216.f;          // 2^24: the last bit of any float is then a normal number
 constexpr uint32_t kSplitW = kSplitN * kSplitK * 2;     // bytes of one third of the weights in a stage
 
 __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr)
@@ -44,13 +47,16 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr)
 }
 
 // the bfloat16 nearest to each of eight numbers, and what that leaves (exactly: of a float, 16 bits; of those, 8)
-__device__ __forceinline__ void nearest_halves(const float (&x)[8], uint32_t (&half)[4], float (&left)[8])
+__device__ __forceinline__ void nearest_halves(const uint64_t (&x)[4], uint32_t (&half)[4], uint64_t (&left)[4])
 {
+    const uint64_t minus = twice(-1.f);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(half[i]) : "f"(x[2 * i + 1]), "f"(x[2 * i]));
-        left[2 * i] = x[2 * i] - __uint_as_float(half[i] << 16);
-        left[2 * i + 1] = x[2 * i + 1] - __uint_as_float(half[i] & 0xFFFF0000u);
+        asm("{\n\t.reg .f32 a, b;\n\tmov.b64 {a, b}, %1;\n\tcvt.rn.bf16x2.f32 %0, b, a;\n\t}" : "=r"(half[i]) : "l"(x[i]));
+        uint64_t h;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(h) : "r"(half[i] << 16), "r"(half[i] & 0xFFFF0000u));
+        left[i] = x[i];
+        fma2(left[i], h, minus);
     }
 }
 
@@ -305,9 +311,12 @@ linear_split_kernel(const float* __restrict__ A, long long lda, const float* __r
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (!third[u]) continue;
-                const float x[8] = {v[u][0].x, v[u][0].y, v[u][0].z, v[u][0].w, v[u][1].x, v[u][1].y, v[u][1].z, v[u][1].w};
+                uint64_t x[4], m[4], l[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    asm("mov.b64 %0, {%1, %2};\n\tmul.rn.f32x2 %0, %0, %3;" : "=&l"(x[i])
+                        : "f"(i & 1 ? v[u][i >> 1].z : v[u][i >> 1].x), "f"(i & 1 ? v[u][i >> 1].w : v[u][i >> 1].y), "l"(twice(kSplitScale)));
                 uint32_t t[3][4];
-                float m[8], l[8];
                 nearest_halves(x, t[0], m);
                 nearest_halves(m, t[1], l);
                 nearest_halves(l, t[2], m);
@@ -388,6 +397,8 @@ linear_split_kernel(const float* __restrict__ A, long long lda, const float* __r
             again = 1;
             continue;
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] *= 1.f / (kSplitScale * kSplitScale);
         epilogue8(e, e.kind == ZKFP_EPI_ROTATE ? epi_position(e, m) : 0, m, n, v);
     }
     if (ksplit > 1) asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
