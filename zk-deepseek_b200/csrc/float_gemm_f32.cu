@@ -9,10 +9,14 @@
 // 128 x NT x 16 for 16 k, a third of what those FMAs take.
 //
 // Precision: the tensor memory's sums are cut, not rounded, which takes 1.45e-8 of a sum of positive numbers for every 16 k.  So
-// the products of the first thirds are collected after two stages (64 k) and added up in 32 bits, rounded; the other products are
-// 2^-8 of them and less, of either sign, and stay.  Error against 64 bits on normal operands, this kernel and the FMAs: K 520
-// 8.6e-8 and 1.7e-7, K 2048 1.3e-7 and 4.1e-7, K 8192 1.4e-7 and 5.8e-7; on positive ones 8e-8 to 1.7e-7 and 6e-8 to 1.2e-6.
-// (One sum for all products: 1.8e-6 where the FMAs have 1.2e-6.  Collected after every stage: 6e-8 on positive ones, 5 % slower.)
+// the products of the first thirds are collected after one or two stages (32 or 64 k) and added up in 32 bits, rounded; the other
+// products are 2^-8 of them and less, of either sign, and stay.  Relative error against 64 bits (2-norm), this kernel and the FMAs, 17 to
+// 300 rows, 128 to 16384 columns: normal operands, K 128 to 1024 6e-8 to 1.1e-7 and 1.5e-7 to 4.1e-7, K 2048 9.8e-8 to 1.3e-7 and 2.9e-7 to
+// 4.1e-7, K 8192 1.2e-7 to 2.5e-7 and 5.7e-7 to 8.1e-7.  Positive operands are where FMAs in clusters that share a K below 2048 are good
+// (6.5e-8 to 8e-8): a share of up to 512 there is collected after every stage, 5.6e-8 to 8e-8, where two stages have 8.7e-8 to 9.6e-8 and
+// everywhere would cost 5 % (and more additions: K 8192 1.4e-7 -> 1.6e-7).  From K 2048 on positive operands have 8.7e-8 to 1.9e-7, FMAs
+// 9.9e-8 to 3.5e-7.  Above the FMAs: 64 rows, 8192 x 1536 9.0e-8 (8.0e-8) and 33 rows, 16384 x 3072 1.2e-7 (1.0e-7).
+// (One sum for all products: 1.8e-6 where the FMAs have 1.2e-6.)
 //
 // Weights take the MMA's 128 rows, up to 160 rows of A its columns: three sets of sums in 480 of 512 columns of tensor memory.
 // Clusters of up to eight CTAs share K and add their sums through each other's shared memory, in rank order.
@@ -35,7 +39,6 @@ constexpr int kSplitK = 32;                        // k of a stage: rows of 64 b
 constexpr int kSplitWarps = 12;                    // warps that cut operands into thirds and finish the sums
 constexpr int kSplitThreads = 32 * (kSplitWarps + 5);   // one more issues the MMAs, four collect their sums
 constexpr int kSplitNT = 160;                      // most rows of A in a tile: three sets of sums in tensor memory
-constexpr int kSplitChunk = 2;                     // stages after which the products of the first thirds are collected
 constexpr int kSplitStages = 4;
 constexpr int kSplitPitch = kSplitN + 4;           // floats between the tokens of the finished sums
 constexpr float kSplitScale = 16777216.f;          // 2^24: the last bit of any float is then a normal number
@@ -183,6 +186,7 @@ linear_split_kernel(const float* __restrict__ A, long long lda, const float* __r
     const int kblocks = (K + kSplitK - 1) / kSplitK, per = (kblocks + ksplit - 1) / ksplit;
     const int kb0 = share * per, kb1 = min(kblocks, kb0 + per);
     const uint32_t a_third = (uint32_t)NT * kSplitK * 2, stage_bytes = 3 * (kSplitW + a_third), smem0 = smem_u32(base);
+    const int chunk_stages = K < 2048 && per <= 16 ? 1 : 2;      // stages after which the products of the first thirds are collected
     volatile int* abort_flag = &s_abort;
 
     if (tid < kSplitNT * (kSplitN / 8) / 32) s_again[tid] = 0;
@@ -233,7 +237,7 @@ linear_split_kernel(const float* __restrict__ A, long long lda, const float* __r
                     umma_bf16(rest, w[1] + at, a[0] + at, idesc, 1u, one);
                     umma_bf16(rest, w[0] + at, a[1] + at, idesc, 1u, one);
                 }
-                const int in_chunk = (kb - kb0) % kSplitChunk;
+                const int in_chunk = (kb - kb0) % chunk_stages;
                 if (in_chunk == 0 && kb > kb0) {          // the chunk in front has been collected under these
                     if (!(ok = mbar_wait_warp(smem_u32(&s_taken), chunk & 1u, abort_flag))) break;
                     tc_fence_after();
@@ -243,7 +247,7 @@ linear_split_kernel(const float* __restrict__ A, long long lda, const float* __r
                 for (int k = 0; k < kSplitK / 16; ++k)
                     umma_bf16(tm, w[0] + (uint64_t)(k * 2), a[0] + (uint64_t)(k * 2), idesc, in_chunk || k ? 1u : 0u, one);
                 umma_commit(smem_u32(&s_empty[s]), one);
-                if (in_chunk == kSplitChunk - 1 || kb == kb1 - 1) { umma_commit(smem_u32(&s_sum), one); ++sums_made; }
+                if (in_chunk == chunk_stages - 1 || kb == kb1 - 1) { umma_commit(smem_u32(&s_sum), one); ++sums_made; }
                 if (++s == stages) { s = 0; phase ^= 1u; }
             }
             if (!ok) {                                     // no MMA in flight when tensor memory goes back
@@ -255,7 +259,7 @@ linear_split_kernel(const float* __restrict__ A, long long lda, const float* __r
     } else if (warp > kSplitWarps) {
         // the sums of a chunk, 32 rows of tensor memory a warp
         const uint32_t tq = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-        const int chunks = kb1 > kb0 ? (kb1 - kb0 + kSplitChunk - 1) / kSplitChunk : 0;
+        const int chunks = kb1 > kb0 ? (kb1 - kb0 + chunk_stages - 1) / chunk_stages : 0;
         bool ok = true;
         for (int c = 0; c < chunks && ok; ++c) {
             ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_sum), (uint32_t)c & 1u, abort_flag));
