@@ -230,13 +230,52 @@ def test_masked_half_left_out_by_the_rule(M, mo, kmod, dev, monkeypatch, S, al, 
 
     def core(limbs, skip):
         attn.score_limbs, attn.causal_skip = limbs, skip
-        got = attn._core(nope, q_pe, kv, pe, 1, S, 0, t(mo.causal_mask(S), dev), None)
+        got, projected = attn._core(nope, q_pe, kv, pe, 1, S, 0, t(mo.causal_mask(S), dev), None)
         kmod.device_status(sync=True)
+        assert not projected                       # up to 64 rows: words
         return got
     got = core((al, bl), None)
     assert skipped == [True] and served == [True]
     assert torch.equal(got, core((al, bl), False)) and torch.equal(got, core((0, 0), None))
     assert skipped == [True, False, False]
+
+
+@pytest.mark.parametrize("S", [97, 130])
+@pytest.mark.parametrize("al,bl", [(3, 3), (4, 3), (3, 4)])
+def test_masked_half_left_out_between_limb_planes(M, mo, kmod, dev, monkeypatch, S, al, bl):
+    """the same on the route of longer prompts: weights that bring the queries to the ends of their limbs behind the heads' product, which
+    like the context stays limb planes; against the full scores on that route and against words with measured limbs"""
+    a = small_args(M, kv_lora_rank=128, n_heads=64, max_seq_len=160)
+    rng = np.random.default_rng(S + 8 * al + bl)
+    attn, p = M.MLA(0, a).to(dev), mla_weights(rng, a)
+    top = lambda limbs: 127 * (256 ** limbs - 1) // 255
+    near = lambda limbs, *shape: top(limbs) - rng.integers(0, 1000, shape)
+    C, R, H, D = a.kv_lora_rank, a.qk_rope_head_dim, a.n_heads, a.qk_nope_head_dim
+    signs_c, signs_r = rng.choice([-1, 1], C), rng.choice([-1, 1], R)
+    later = np.where(np.arange(S) % 2, 1, -1)[None, :, None]
+    w1 = np.zeros((H, D, C), np.int32)
+    w1[:, 0] = signs_c << 30                                      # q_abs = the first of a head's queries, with these signs
+    p.update(wkv_b_1=w1.reshape(H * D, C), wkv_b_1_scale=30)
+    load_mla(attn, p, dev)
+    nope = np.zeros((1, S, H, D), np.int64)
+    nope[..., 0] = near(al, 1, S, H)
+    nope, q_pe = t(nope, dev), t((near(al, 1, S, H, R) >> 2) * signs_r, dev)
+    kv, pe = t(near(bl, 1, S, C) * signs_c * later, dev), t(near(bl, 1, S, R) * signs_r * later, dev)
+    skipped, scores = [], kmod.mla_scores_fused
+    monkeypatch.setattr(kmod, "mla_scores_fused", lambda *args, skip_masked=False, **kw: (
+        skipped.append(skip_masked), scores(*args, skip_masked=skip_masked, **kw))[1])
+
+    def core(limbs, skip):
+        attn.score_limbs, attn.causal_skip = limbs, skip
+        got, projected = attn._core(nope, q_pe, kv, pe, 1, S, 0, t(mo.causal_mask(S), dev), None)
+        out = attn._project_heads(got, M.ACT_LIMBS, projected)
+        kmod.device_status(sync=True)
+        return out, projected
+    got = core((al, bl), None)
+    assert skipped == [True] and got[1]
+    full, words = core((al, bl), False), core((0, 0), None)
+    assert skipped == [True, False, False] and full[1] and not words[1]
+    assert torch.equal(got[0], full[0]) and torch.equal(got[0], words[0])
 
 
 def test_mla_decode_reads_resident_cache_planes(M, mo, kmod, dev):

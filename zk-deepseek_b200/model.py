@@ -445,7 +445,7 @@ class MLA(nn.Module):
         k_pe, _ = self.wkv_a2(x)
         k_pe = apply_rotary_emb(k_pe.unsqueeze(2), freqs_cis)
         kv_normed, rms = self.kv_norm(kv)
-        ctx, projected = self._core(q_nope, q_pe, kv_normed, k_pe.squeeze(2), bsz, seqlen, start_pos, mask, d, through=True)
+        ctx, projected = self._core(q_nope, q_pe, kv_normed, k_pe.squeeze(2), bsz, seqlen, start_pos, mask, d)
         return self._finish(ctx, lim, projected)
 
     def _forward_seq_parallel(self, x, start_pos, freqs_cis, mask):
@@ -468,7 +468,7 @@ class MLA(nn.Module):
         q_nope = self.wq_b1(q_all).view(1, S, self.n_local_heads, self.qk_nope_head_dim)
         q_pe = self.wq_b2(q_all).view(1, S, self.n_local_heads, self.qk_rope_head_dim)
         q_pe = apply_rotary_emb(q_pe, freqs_cis)
-        ctx, projected = self._core(q_nope, q_pe, full[:, qr:qr + C][None], full[:, qr + C:][None], 1, S, start_pos, mask, None, through=True)
+        ctx, projected = self._core(q_nope, q_pe, full[:, qr:qr + C][None], full[:, qr + C:][None], 1, S, start_pos, mask, None)
         out = self._project_heads(ctx, ACT_LIMBS, projected)                            # [1, S, local heads * v]
         # head-split -> token-split: rank j receives its token block from every rank's heads
         cols = out.shape[-1]
@@ -478,11 +478,9 @@ class MLA(nn.Module):
         rows = recv.permute(1, 0, 2).reshape(1, s_loc, world_size * cols)               # heads in rank order
         return self.wo(rows)
 
-    def _core(self, q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d, through=False):
-        """caches, scores, softmax, P . KV for the local heads: returns ctx [b, s, h, c]; through: (ctx, False), or what
-        _project_heads makes of it and True, where the products on both sides of the latent space pass limb planes on"""
-        if not through:
-            return self._attend(q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d, None)
+    def _core(self, q_nope, q_pe, kv_normed, k_pe, bsz, seqlen, start_pos, mask, d):
+        """caches, scores, softmax, P . KV for the local heads: returns (ctx [b, s, h, c], False), or what _project_heads makes
+        of ctx and True, where the products on both sides of the latent space pass limb planes on"""
         heads = None
         # prompts (up to 64 rows the products of a head read words themselves), with all limbs promised
         if (bsz * seqlen > 64 and mask is not None and not snark and K.ALGO != K.ALGO_EXACT and 0 < ACT_LIMBS <= 4 and min(self.score_limbs) > 0
