@@ -1202,3 +1202,22 @@ def test_heads_products_of_refused_calls_are_not_taken(kmod, dev):
     for how in (dict(), dict(causal_skip=True)):
         assert launched(lambda: kmod.softmax_pv_fused(scores, kv, 19, a_limbs=3, b_limbs=3, heads=(wide, 9, 4), **how)) == (None, 0)
     kmod.device_status(sync=True)
+
+
+@pytest.mark.parametrize("N,K,bits,limbs,rows", [(8192, 8192, 6, 3, (1, 16)), (16384, 2048, 13, 3, (16, 17, 32)), (2304, 18432, 21, 4, (16, 17)),
+                                                 (10240, 8192, 30, 4, (1, 16)), (6144, 7168, 30, 3, (17, 32))])
+def test_few_rows_at_both_sides_of_the_rule(kmod, dev, N, K, bits, limbs, rows):
+    """layers whose rows are cut before the product, as their halves and quarters, which the product cuts itself: the same words"""
+    gen = torch.Generator(device=dev).manual_seed(N)
+    draw = lambda b, shape, dtype: torch.randint(-(1 << b), 1 << b, shape, device=dev, dtype=dtype, generator=gen)
+    W = draw(bits, (N, K), torch.int32)
+    whole = kmod.WeightPlanes(W)
+    for M in rows:
+        X = draw(8 * limbs - 2, (1, M, K), torch.int64)
+        got = kmod.linear_prepared(X, whole, 9, a_limbs=limbs, dynamic=True)
+        for parts in (2, 4):
+            n = N // parts
+            for i in range(parts):
+                want = kmod.linear_prepared(X, kmod.WeightPlanes(W[i * n:(i + 1) * n].contiguous()), 9, a_limbs=limbs, dynamic=True)
+                assert torch.equal(got[..., i * n:(i + 1) * n], want)
+    kmod.device_status(sync=True)

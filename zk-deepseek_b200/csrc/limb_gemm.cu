@@ -1189,10 +1189,10 @@ __device__ __forceinline__ bool put_digits(const int64_t (&v)[8], int L, uint32_
 
 // p.NT = R rows of activations (tmA's box); tmW's box holds 128 weight rows.  grid (n_tiles * ksplit, row tiles, batches); the
 // row tiles of a grouped call are 128 rows apart, others R
-// DIRECT (up to 32 rows): the epilogue warps, which have nothing to do until the sums are complete, read the activations and cut
-// them into limbs on their way into the stages, so that a call is one launch: no pass that writes planes, no range to measure
-// and to clear before.  Every column tile reads and cuts the rows anew, which at 32 rows is half of what the weights move and at 64
-// would be as much.  One sequence through two blocks and the head: 114 -> 72 launches, 1401 -> 1272 us; 64 sequences, whose routed
+// DIRECT (up to 32 rows, where rows_cut_by_product says so): the epilogue warps, which have nothing to do until the sums are complete,
+// read the activations and cut them into limbs on their way into the stages, so that a call is one launch: no pass that writes planes,
+// no range to measure and to clear before.  Every column tile reads and cuts the rows anew, which at 32 rows is as much as weights of two
+// limbs move.  One sequence through two blocks and the head: 114 -> 72 launches, 1401 -> 1272 us; 64 sequences, whose routed
 // experts take it: 3174 -> 3126.
 template <bool DIRECT>
 __global__ void __launch_bounds__(kRowsThreads, 2)
@@ -3130,6 +3130,29 @@ static int rows_clusters(int size, size_t smem)
     return n;
 }
 
+// Whether limb_rows_kernel cuts the rows itself.  That saves two launches, 7 us, and costs some tenths of a microsecond for every K block
+// that an SM works through: the next block's words are requested one block ahead, which a busy L2 answers later than the weights of a
+// stage take, and from 17 rows on they are as many bytes as these.  So the line lies at so much work, by how long a block of these weights takes
+// (us, cut by the product / planes; 3 limbs of activations):
+//   up to 16 rows  two limbs of weights: at any size (36864 x 7168 by 1 and 16 rows 104 / 111, 109 / 113)
+//                  one limb: up to 48 MB (6144 x 7168 27 / 29, 30 / 31; 12288 x 7168 42 / 37, 50 / 41)
+//                  three and four: up to 240 MB, 280 of three by three, 480 for one row (8192 x 7168 of four 62 / 68, 69 / 70; 7168 x 16384 103 / 109,
+//                  118 / 112; 36864 x 7168 190 / 186, 228 / 190; 12288 x 7168 of three 66 / 74, 70 / 76); five and more: at any size (12288 x 7168
+//                  101 / 115, 98 / 104)
+//   17 to 32 rows  up to eight K blocks an SM and, with fewer than four limbs, 64 in all (2048 x 7168 24 / 29, 30 / 31; 4096 x 7168 36 / 34,
+//                  41 / 35; 36864 x 7168 125 / 113, 130 / 115; 1024 x 18432 37 / 31); four limbs up to 140 MB (4096 x 7168 45 / 49, 50 / 51;
+//                  6144 x 7168 64 / 66, 72 / 68), five and more up to 300 (8192 x 7168 79 / 86, 85 / 88; 12288 x 7168 108 / 108, 124 / 108)
+//   experts        (up to 32 rows promised, of which few hold data: 64 x 4096 x 7168 by 1, 8, 17, 32 rows each 611 / 670, 618 / 670,
+//                  662 / 674, 775 / 678) but for four limbs at a K below 4096 (64 x 7168 x 2048 763 / 762, 849 / 762), where the same eight K blocks hold
+static bool rows_cut_by_product(int La, int Lb, int few, bool experts, int64_t rows_tiles, int64_t kblocks, int64_t weight_bytes)
+{
+    const int64_t mb = weight_bytes / 1000000;
+    const bool shallow = rows_tiles * kblocks <= 8 * (int64_t)sm_count();
+    if (experts) return Lb < 4 || kblocks >= 32 || shallow;
+    if (few <= 16) return Lb == 2 || Lb >= 5 || mb <= (Lb == 1 ? 48 : few == 1 ? 480 : La + Lb <= 6 ? 280 : 240);
+    return (shallow && (Lb >= 4 || kblocks <= 64)) || (Lb >= 4 && mb <= (Lb == 4 ? 140 : 300));
+}
+
 int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* pre_b, cudaStream_t st)
 {
     if (pre_b) Lb = pre_b->L;
@@ -3241,7 +3264,8 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     DeviceFlags* fl = flags_for_device();
     if (!fl) return ZKDS_ERR_WORKSPACE;
     const bool direct = by_rows && few <= kDirectRows && La <= 7 && p.a_div == 1 && !p.softmax_lut && !p.glu_lut && p.a_n_parts == 0 &&
-                        !p.a_planes;
+                        !p.a_planes && rows_cut_by_product(La, Lb, few, p.tile_group, rows_tiles * p.batches * (p.tile_group ? mt : 1), kb,
+                                                           (p.tile_group ? 1 : nbB) * p.N * p.K * Lb);
     int8_t* pa = p.a_planes ? const_cast<int8_t*>(p.a_planes) : direct ? nullptr : (int8_t*)workspace((size_t)La * a_rows * Kp + 1024, 0);
     if (!pa && !direct) return ZKDS_ERR_WORKSPACE;
     unsigned long long* d_absmax = nullptr;
