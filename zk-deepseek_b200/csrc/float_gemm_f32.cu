@@ -2,11 +2,11 @@
 //
 // A float times 2^24 is the sum of three bfloat16 numbers exactly, subnormal ones too: the nearest one, the nearest to what that leaves,
 // and the rest.  (Without the factor, which the sums lose again at the end, bfloat16's smallest numbers cut the last third of what is
-// below 2^-110: error 9e-6 at 2^-118, 2e-3 at 2^-126, where now it is 9e-8 as at 1.)  Operands from 2^104 and sums from 2^80 on leave the range and are taken by multiply-adds, see again_by_fma.  Of the nine
-// products of thirds the six largest are taken: what is dropped is up to 2^-24 of a product, as much as a float's own rounding, of
-// either sign, and 2^-27 on average.  On the CUDA cores these layers are bound by FMAs at 64 lanes an SM and clock; here by the pieces of both operands that
-// have to be in flight (loads of floats, cut into thirds by the threads, 3 x 64 bytes a row and stage) and by 6 MMAs of
-// 128 x NT x 16 for 16 k, a third of what those FMAs take.
+// below 2^-110: error 9e-6 at 2^-118, 2e-3 at 2^-126, where now it is 9e-8 as at 1.)  Operands from 2^104 and sums from 2^80 on leave the
+// range and are taken by multiply-adds, see again_by_fma.  Of the nine products of thirds the six largest are taken: what is dropped is
+// up to 2^-24 of a product, as much as a float's own rounding, of either sign, and 2^-27 on average.  On the CUDA cores these layers are
+// bound by FMAs at 64 lanes an SM and clock; here by the pieces of both operands that have to be in flight (loads of floats, cut into
+// thirds by the threads, 3 x 64 bytes a row and stage) and by 6 MMAs of 128 x NT x 16 for 16 k, a third of what those FMAs take.
 //
 // Precision: the tensor memory's sums are cut, not rounded, which takes 1.45e-8 of a sum of positive numbers for every 16 k.  So
 // the products of the first thirds are collected after one or two stages (32 or 64 k) and added up in 32 bits, rounded; the other
@@ -21,7 +21,7 @@
 // Weights take the MMA's 128 rows, up to 160 rows of A its columns: three sets of sums in 480 of 512 columns of tensor memory.
 // Clusters of up to eight CTAs share K and add their sums through each other's shared memory, in rank order.
 // 300 rows, 2048 x 2048: 80 -> 32 us; 16384 x 2048: 477 -> 158 us; 17 rows, 1344 x 2048: 19 -> 13 us; a prompt of 300 tokens at
-// width 2048 2.69 -> 1.30 ms.
+// width 2048 2.69 -> 1.30 ms, 1.10 with attention_f32_kernel.
 #include <float.h>
 #include <math.h>
 
@@ -474,7 +474,8 @@ SplitPlan split_plan(const zkfp_linear_args& a)
 // 25 and 27; from K 128 on 9.0 and 8.7, 41 and 33); a handful of CTAs for more rows than that kernel's tiles need to fill the chip
 // (640 x 328: 300 rows 14.1 and 16.2 us with 20 CTAs, 700 rows 18.9 and 16.9 with 50); up to 32 rows, which it has a tile for,
 // where more than half and fewer than three quarters of the SMs would hold a tile (17 rows, 10304 x 2048: 51 to 56 and 60 us;
-// 2048 x 2048 23 and 17, 16384 x 2048 78 and 66); and what it refuses.
+// 2048 x 2048 23 and 17, 16384 x 2048 78 and 66); and what it refuses.  With 34 to 48 tiles up to 32 rows are slower here (4384 x 2048
+// 33.3 and 35.4 us, 6144 x 2048 33.3 and 37.2, 4384 x 8192 112 and 121) and stay for their error, a third of the FMAs'.
 bool linear_split_takes(const zkfp_linear_args& a)
 {
     if (a.K < 128 || (a.M + 63) / 64 > 65535) return false;

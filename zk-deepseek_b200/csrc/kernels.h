@@ -80,10 +80,6 @@ int launch_peer_barrier(unsigned long long* const* flag_bases, int n_parts, int 
                         unsigned* status, cudaStream_t st);
 
 // ---- contractions ---------------------------------------------------------------
-// One batched contraction  C[z][m][n] = (addend + sum_k A(z,m,k) * B(z,n,k)) >> shift
-// with the sum held in 128 bits.  A is int64 with unit k-stride; B is int32 or int64
-// with arbitrary n- and k-strides (so the MLA einsums map onto it without copies).
-// a_div / b_div are C truncating divisors applied to each element before the product.
 // Where a contraction leaves its results as limb planes for the next one instead of as words: row m of batch z at
 // data[l * step + ((m / div) * rq + (m % div) * rr + z * rz) * pitch], one byte a column and limb l < L <= 4; most <- the largest
 // magnitude (as a split measures it; zeroed by the launch).  A result that L limbs do not hold raises the limb flag.
@@ -94,6 +90,10 @@ struct LimbOut {
     unsigned long long* most;
 };
 
+// One batched contraction  C[z][m][n] = (addend + sum_k A(z,m,k) * B(z,n,k)) >> shift
+// with the sum held in 128 bits.  A is int64 with unit k-stride; B is int32 or int64
+// with arbitrary n- and k-strides (so the MLA einsums map onto it without copies).
+// a_div / b_div are C truncating divisors applied to each element before the product.
 struct Contraction {
     const int64_t* A;
     const void* B;

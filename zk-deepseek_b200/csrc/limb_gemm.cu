@@ -2649,11 +2649,11 @@ int launch_split_t(const T* X, int8_t* planes, int L, int64_t nb, int64_t rows, 
     return check_launch();
 }
 
-// Both operands' ranges in one launch: 2048 consecutive elements of a row a step of a block, its loads all in flight, one
-// atomic a block.  Bound by the bytes read.  32 x 7168 by 576 x 7168 int64, the whole product with its ranges measured:
-// 78.3 -> 60.8 us.  An operand without gaps is one long row, since a step of a short row would leave most of its threads without
+// Both operands' ranges in one launch: 2048 consecutive elements of a row a step of a block, its loads all in flight.  Bound by the
+// bytes read.  32 x 7168 by 576 x 7168 int64, the whole product with its ranges measured, against a launch an operand: 78.3 -> 60.8 us.
+// An operand without gaps is one long row, since a step of a short row would leave most of its threads without
 // work: 262144 x 8, row by row 1004 us for the product, as one row 278 (absmax_kernel 290).  absmax_kernel (a 64-bit division and
-// one load an element, an atomic a warp: 10.8 us each for 32 and 576 rows of 7168) is left for short rows with gaps, for sources
+// one load an element: 10.8 us each for 32 and 576 rows of 7168) is left for short rows with gaps, for sources
 // that are not contiguous along K and for the other entry points that measure.
 struct RangeOf {
     const void* X;
@@ -3204,7 +3204,7 @@ int launch_contraction_limb(const Contraction& p, int La, int Lb, const Planes* 
     int ew = persistent_epilogue_warps(false);
     // up to 8 K blocks (K <= 1024) in narrow tiles whose accumulators have two buffers; a single wide one needs more products behind a
     // tile (K = 512, 128 heads of 4096 tokens: 218 us narrow, 242 wide; of 777 tokens, four limbs, 110 and 129).  Not where limbs are
-    // written at one K block, which is bound by their stores: whole eights of 112 columns 680 us, of 48 785.
+    // written at one K block, which is bound by their stores: whole eights of 112 columns 680 us (690 within the layer), of 48 785.
     int64_t max_kb = 8;
     if (switches().persistent_max_kb >= 0) max_kb = switches().persistent_max_kb;
     // few rows: the weights take the MMA's 128 rows (limb_rows_kernel).  Up to 64 rows at any depth, or promised groups of up
