@@ -1194,8 +1194,12 @@ def test_heads_products_of_refused_calls_are_not_taken(kmod, dev):
         94, 695, 1, 0, -(64 << 36), 3, 3, kmod._a_flags(3, True), kmod._stream()))
     assert rc == (6, 0)
     for narrow in (False, True):
-        got, n = launched(lambda: kmod.mla_scores_fused(*args, causal=True, skip_masked=True, narrow=narrow, a_limbs=3, b_limbs=3, dynamic=True))
+        fresh = kmod.HeadsProduct(heads.A, planes, 17, 3)
+        got, n = launched(lambda: kmod.mla_scores_fused(fresh, *args[1:], causal=True, skip_masked=True, narrow=narrow, a_limbs=3, b_limbs=3,
+                                                        dynamic=True))
         assert got is None and n == 1
+        words, n = launched(fresh.tensor)                  # what the caller goes on with
+        assert n == 0 and torch.equal(words, heads.tensor())
     scores, kv = draw(20, 1, 65, 2, 64), draw(20, 1, 64, 32768)
     wide = kmod.WeightPlanes(draw(30, 2, 16, 32768).int())
     kmod.softmax_init_q19()

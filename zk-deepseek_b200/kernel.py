@@ -527,16 +527,18 @@ def _scores_fit32(a_limbs, b_limbs, C1, C2, rescale1, rescale2, mul, div):
 
 class HeadsProduct:
     """einsum_heads_prepared(A, planes, rescale, True, a_limbs, True) that has not been taken: mla_scores_fused leaves it as limb planes
-    between its products where it can; tensor() is the words"""
+    between its products where it can; tensor() is the words, taken once (one object stands for one product: A stays as it is)"""
 
     def __init__(self, A, planes, rescale, a_limbs):
         _dev_i64(A, "A")
         assert A.shape[2] == planes.nb and A.shape[3] == planes.K and a_limbs > 0
         self.A, self.planes, self.rescale, self.a_limbs = A, planes, int(rescale), a_limbs
-        self.shape, self.device = A.shape[:3] + (planes.N,), A.device
+        self.shape, self.device, self._words = A.shape[:3] + (planes.N,), A.device, None
 
     def tensor(self):
-        return einsum_heads_prepared(self.A, self.planes, self.rescale, True, a_limbs=self.a_limbs, dynamic=True)
+        if self._words is None:
+            self._words = einsum_heads_prepared(self.A, self.planes, self.rescale, True, a_limbs=self.a_limbs, dynamic=True)
+        return self._words
 
 
 def mla_scores_fused(q_abs, kv, q_pe, pe, rescale1=23, rescale2=21, mul=94, div=695, causal=False,
