@@ -721,8 +721,8 @@ def test_trace_and_generate_programs(float_libpath, tmp_path, case, dtype):
                                     (321, 2056, 4104), (33, 20000, 264)])
 def test_float32_layers_from_thirds(K, M, N, Kd):
     """the tensor-core products of bfloat16 thirds: edges of the tiles of 160 rows and 128 columns, ragged blocks of K, shares.
-    The limit is that of 32-bit sums in chunks of 64 and then one by one: (64 / 16 + Kd / 64 + 4) roundings of 2^-24 of the sum of
-    absolute products, a few times what they add up to by chance"""
+    The limit is that of 32-bit sums in chunks of 64 (or 32, of at most 512 k a share) and then one by one: (64 / 16 + Kd / 64 + 4)
+    roundings of 2^-24 of the sum of absolute products, a few times what they add up to by chance"""
     for scale in (1.0, 2.0 ** -60, 2.0 ** 60):
         A, W = rnd((M, Kd), "float32", 3) * scale, rnd((N, Kd), "float32", 4, Kd ** -0.5)
         out = torch.full((M, N), 7.0, device="cuda")

@@ -73,8 +73,8 @@ __device__ __forceinline__ float4 peer_sums(uint32_t own, unsigned rank)
 }
 
 // Outputs whose sum is not finite, once more: thirds of an infinity are no number.  `again` marks them, eight columns a bit, 16 bits a
-// row, of `rows` rows from m0 on.  What has a NaN in its row or its weights is none; the rest is taken by multiply-adds, 512 threads
-// with eight columns of five rows each, 32 k at a time through shared memory.
+// row, of `rows` rows from m0 on.  What has a NaN in its row or its weights is none; the rest, finite neighbours in the same eight
+// among it, is taken by multiply-adds, 512 threads with eight columns of five rows each, 32 k at a time through shared memory.
 // 300 rows, 16384 x 2048, against a thread an output that walked all of K by itself: rows of NaN 24.9 -> 0.31 ms, one of them 0.85 -> 0.30,
 // an infinity in every row 25.0 -> 1.33 (finite 0.17; linear_f32_kernel 0.48 on any of them); 2048 x 8192: 12.9 -> 0.26, 2.0 -> 0.25, 12.9 ->
 // 1.71 (0.09; 0.29).
